@@ -26,7 +26,7 @@ on the same scene and configuration, a bounded sample of the frame per step,
 counting the rays its scene traces.
 
 At N=1 the same line carries `sections`: the ray-intersection kernel (2^24
-rays x 1,048,576-triangle soup, binary and 4-wide layouts, bit-exact against
+rays x 1,048,576-triangle soup, scene types bvh and qbvh, bit-exact against
 the reference), the plain one-scene renderer on the headline frame, the
 adjoint path replay's backward/forward time, and the 64-scene batch against
 the plain renderers.
@@ -51,19 +51,12 @@ sys.path.insert(0, ROOT)
 NUM_TRIS = 1 << 20
 NUM_RAYS = 1 << 24
 NODE_BYTES = 32      # compact binary node (6 f32 + 2 u32), per slab test
-NODE4_BYTES = 128    # 4-wide node, per node fetch (four slab tests)
+WIDE_BOX_BYTES = 12  # an eighth of what a visit of an 8-wide node reads (96 B), per box test
 TRI_BYTES = 48       # TriAccel record, per triangle test
 RAY_IO_BYTES = 32 + 16
 # The headline metric, one string for both arms (the reference's renderer and
 # this core's batched wavefront path trace the same frame).
 FRAME_METRIC = "Mrays/s @1080p path tracing (pt.mis)"
-QNODE_BYTES = 24     # quantised binary node (48 B: grid, 16-bit planes, children), per slab test
-
-
-def node_bytes(layout: str, any_hit: bool) -> int:
-    """Node bytes per slab test of a render walk under the batch layout."""
-    quantised = layout == "bvh_q16" or (layout == "bvh_qshadow" and any_hit)
-    return QNODE_BYTES if quantised else NODE_BYTES
 
 # Headline frame: the full path tracer on the terrain + icospheres scene.
 FRAME_W, FRAME_H = 1920, 1080
@@ -181,13 +174,12 @@ def profile_value(name, key):
     return None
 
 
-def load_traffic(layout, num_rays):
+def load_traffic(num_rays):
     """DRAM bytes (read + write) of one full-size traversal launch of the
     intersection API, from the committed ncu summary of the kernel: its line
     `dram_bytes_per_ray: X` (measured on a smaller capture, scaled by the
     rays of this launch), or None."""
-    kernel_layout = {"bvh": "bvh2", "qbvh": "bvh4"}[layout]
-    v = profile_value(f"trace_closest_{kernel_layout}_intersect", "dram_bytes_per_ray")
+    v = profile_value("trace_closest_bvh2_intersect", "dram_bytes_per_ray")
     return None if v is None else int(v * num_rays)
 
 
@@ -326,12 +318,11 @@ def _batch_launches(cfg, stats, bounces):
     return stats["waves"] * (5 + 4 * bounces) + 1
 
 
-def frame_roofline(prof_count, prof_time, layout="bvh"):
+def frame_roofline(prof_count, prof_time):
     """Roofline of the dominant kernel of the frame, the closest-hit
     traversal of the path queues (and, beside it, the shadow traversal):
-    algorithmic bytes per ray (32 B ray + 16 B hit + 32 B per binary-node
-    slab test, 24 B for a quantised node, + 48 B per TriAccel test, the
-    tests counted on the same samples by the counting kernel) over the
+    algorithmic bytes per ray (32 B ray + 16 B hit + 96 B per 8-wide node
+    visit, 12 B per box test, + 48 B per TriAccel test, the tests counted on the same samples by the counting kernel) over the
     launches' summed device time."""
     peak, peak_kind = measured_peaks()
     out = {}
@@ -342,7 +333,7 @@ def frame_roofline(prof_count, prof_time, layout="bvh"):
             continue
         nb = c["node_tests"] / rays
         tb = c["tri_tests"] / rays
-        bpr = RAY_IO_BYTES + node_bytes(layout, kind == "shadow") * nb + TRI_BYTES * tb
+        bpr = RAY_IO_BYTES + WIDE_BOX_BYTES * nb + TRI_BYTES * tb
         achieved = bpr * rays / (t["trace_ms"] / 1e3) / 1e9
         out[kind] = {"achieved": round(achieved, 1), "frac": round(achieved / peak, 4),
                      "bytes_per_ray": round(bpr, 2), "node_tests_per_ray": round(nb, 3),
@@ -355,9 +346,9 @@ def frame_roofline(prof_count, prof_time, layout="bvh"):
             "achieved": main["achieved"], "peak": peak, "unit": "GB/s", "frac": main["frac"],
             "traffic": None if traffic_per_ray is None else int(traffic_per_ray * main["rays"] / main["launches"]),
             "peak_source": peak_kind,
-            "why_not_hbm": "the tree and triangles (~250 MB) mostly hit in L2; each ray's walk is a chain of "
-                           "dependent node fetches with a third of the lanes active, so the kernel is bound by "
-                           "fetch latency and divergence, not DRAM bandwidth",
+            "why_not_hbm": "the tree and triangles (~220 MB) mostly hit in L2; each ray's walk is a chain of "
+                           "dependent node visits of ~250 instructions, so the kernel is bound by the ALU pipe, "
+                           "divergence and fetch latency, not DRAM bandwidth",
             "kernels": out}
 
 
@@ -462,7 +453,7 @@ def run_ours(args):
                "inputs": "the render parameters of the step (the scene stays resident in HBM)"}
 
     frame_layout = batch.config["layout"]
-    roofline = frame_roofline(prof_count, prof_time, frame_layout)
+    roofline = frame_roofline(prof_count, prof_time)
     launches = _batch_launches(batch.config, stats, FRAME_MAX_PV - 1) * args.steps
     batch.close()
 
@@ -548,9 +539,9 @@ def _terrain_parity(r, layout="bvh"):
 def intersect_section(args, dev, layout, cpu_baseline, want_ref_hits):
     """The ray-intersection kernel alone: 2^24 rays (origins U[-2,2]^3,
     directions uniform on the sphere) against 1,048,576 random triangles
-    (centres U[-1,1]^3, edges N(0, 0.01^2)), closest hit. Layout "bvh" is the
-    binary SAH tree that reproduces the reference BVHScene; "qbvh" its 4-wide
-    collapse. One launch per step over the batch (512 MB of rays, larger
+    (centres U[-1,1]^3, edges N(0, 0.01^2)), closest hit, scene type "bvh" or
+    "qbvh" (the same walk and hits). Bytes per ray: the reference walk's slab and
+    TriAccel tests. One launch per step over the batch (512 MB of rays, larger
     than L2)."""
     import torch
     from lightmetrica_b200 import native
@@ -582,10 +573,7 @@ def intersect_section(args, dev, layout, cpu_baseline, want_ref_hits):
                                            ctypes.c_void_p(counters.data_ptr()), sptr))
     scene.status(stream.cuda_stream)
     node_tests, tri_tests = int(counters[0]), int(counters[1])
-    if layout == "bvh":
-        bytes_per_ray = RAY_IO_BYTES + NODE_BYTES * node_tests / n + TRI_BYTES * tri_tests / n
-    else:
-        bytes_per_ray = RAY_IO_BYTES + NODE4_BYTES * (node_tests / 4) / n + TRI_BYTES * tri_tests / n
+    bytes_per_ray = RAY_IO_BYTES + NODE_BYTES * node_tests / n + TRI_BYTES * tri_tests / n
     hit_frac = float((hits["tri_id"] >= 0).float().mean())
 
     steps, warm = max(3, args.steps), max(3, args.warmup)
@@ -604,19 +592,16 @@ def intersect_section(args, dev, layout, cpu_baseline, want_ref_hits):
     peak, peak_kind = measured_peaks()
     achieved = bytes_per_ray * n / (avg_ms / 1e3) / 1e9
     out = {"workload": f"ray-intersection: 2^{n.bit_length() - 1} rays x 1,048,576-triangle soup, closest hit",
-           "layout": {"bvh": "binary SAH BVH (reference bvh, bit-exact)",
-                      "qbvh": "4-wide collapse of the reference tree, 128 B nodes (bit-exact)"}[layout],
+           "layout": f"{layout}: 8-wide compressed collapse of the reference tree, 128 B nodes (bit-exact)",
            "Mrays_per_s": round(n / (avg_ms / 1e3) / 1e6, 1),
            "kernel_ms": {"avg": round(avg_ms, 4), "min": round(min(launch_ms), 4), "max": round(max(launch_ms), 4)},
            "steps": steps, "hit_fraction": round(hit_frac, 4),
            "roofline": {"bound": "latency", "denominator": "hbm", "achieved": round(achieved, 1), "peak": peak,
-                        "unit": "GB/s", "frac": round(achieved / peak, 4), "traffic": load_traffic(layout, n),
+                        "unit": "GB/s", "frac": round(achieved / peak, 4), "traffic": load_traffic(n),
                         "peak_source": peak_kind, "bytes_per_ray": round(bytes_per_ray, 2),
                         "node_tests_per_ray": round(node_tests / n, 3), "tri_tests_per_ray": round(tri_tests / n, 4)},
            "bvh_nodes": info["num_nodes"], "bvh_depth": info["max_depth"],
            "build_seconds": round(info["build_seconds"], 3)}
-    if layout == "qbvh":
-        out["node_fetches_per_ray"] = round(node_tests / 4 / n, 3)
     if not args.no_e2e and layout == "bvh":
         out["e2e"] = run_e2e(args, scene, rays, hits, dev)
     ids = hits["tri_id"].cpu().numpy()

@@ -46,17 +46,18 @@ enum {
 
 /* ------------------------------------------------------------- scene ---- */
 
-/* Acceleration layouts. BVH2 reproduces the reference `bvh` scene
- * (src/liblightmetrica/scene.bvh.cpp) exactly: same tree, same traversal
- * order, same float arithmetic, hence bit-identical closest hits. */
+/* Scene types. Both BVH layouts answer the intersection entry points with the
+ * reference `bvh` scene's closest hits (src/liblightmetrica/scene.bvh.cpp), bit
+ * for bit, and walk the same 8-wide compressed collapse of its tree; renders
+ * walk the same kind of collapse of the render tree. The two names are the
+ * reference's scene components (`bvh`, `qbvh`); the last two are accepted as
+ * batch layouts. */
 enum {
-    LMGPU_LAYOUT_BVH2 = 0,   /* binary, children-in-parent 64 B nodes */
-    LMGPU_LAYOUT_BVH4 = 1,   /* 4-wide collapse of the same tree, 128 B nodes */
+    LMGPU_LAYOUT_BVH2 = 0,
+    LMGPU_LAYOUT_BVH4 = 1,
     LMGPU_LAYOUT_NAIVE = 2,  /* brute force over all triangles (tiny scenes) */
-    LMGPU_LAYOUT_BVH2Q = 3,  /* batch renders only: the binary render tree with 48 B nodes whose child
-                                boxes are 16-bit planes on a per-node grid (boxes only grow) */
-    LMGPU_LAYOUT_BVH2_QSHADOW = 4   /* batch renders only: float binary nodes for bounce rays,
-                                       quantised ones (LMGPU_LAYOUT_BVH2Q) for shadow rays */
+    LMGPU_LAYOUT_BVH2Q = 3,         /* batch configurations only: as LMGPU_LAYOUT_BVH2 */
+    LMGPU_LAYOUT_BVH2_QSHADOW = 4   /* batch configurations only: as LMGPU_LAYOUT_BVH2 */
 };
 
 /* BSDFs (reference diffuse.cpp, mirror.cpp, plugin.diffusemirror). */
@@ -124,8 +125,9 @@ typedef struct {
     int32_t film_height;
     int32_t layout;             /* LMGPU_LAYOUT_* */
     int32_t build_threads;      /* host threads for the BVH build, 0 = all */
-    int32_t max_stack_entries;  /* traversal stack bound per ray, 0 = automatic (2 * tree depth + 4,
-                                   enough for every walk); a smaller bound makes the walks that
+    int32_t max_stack_entries;  /* traversal stack bound per ray, 0 = automatic (enough for every
+                                   walk: the wide tree's depth, and 2 * tree depth + 4 in the
+                                   reference's own walk); a smaller bound makes the walks that
                                    need more fail with LMGPU_ERR_STACK_OVERFLOW (the status word
                                    the kernels raise). The multi-scene batch always uses the
                                    largest compiled bound. */
@@ -138,8 +140,9 @@ typedef struct {
     int64_t num_leaves;
     int32_t max_depth;
     int32_t layout;
-    int64_t device_bytes;       /* bytes in HBM of the traversal data: every tree in both layouts,
-                                   the quantised render nodes and the triangle records */
+    int64_t device_bytes;       /* bytes in HBM of the traversal data: the reference's tree (binary
+                                   and 8-wide), the render tree (8-wide), the triangle records and
+                                   leaf boxes */
     double build_seconds;       /* host BVH build time */
     float bounds_min[3];        /* Scene::GetAABBTriangles */
     float bounds_max[3];
@@ -302,7 +305,12 @@ typedef struct {
 
 /* Forward pass: renders `params` with `diff` into a DEVICE image (W*H*3,
  * accumulated with atomics, already rescaled by W*H/num_samples; the caller
- * zeroes it). Same estimator as lmgpu_render. */
+ * zeroes it). Same estimator as lmgpu_render. Both passes run budgets of 2^16
+ * samples or more as waves of up to 2^23 paths over a workspace that is
+ * allocated in stream order from a pool of the device (at most
+ * 220 + 16 * (max_path_vertices - 1) bytes per path; kept for the next call until
+ * lmgpu_render_release); smaller budgets, and streams being captured, run
+ * one thread per sample without it. */
 int lmgpu_adjoint_forward(LmgpuScene* scene, const LmgpuRenderParams* params,
                           const LmgpuDiffParams* diff, float* image_device,
                           void* stream, LmgpuRenderStats* stats);
@@ -339,7 +347,8 @@ enum {
 };
 
 typedef struct LmgpuBatchConfig {
-    int32_t layout;               /* LMGPU_LAYOUT_BVH2, _BVH4, _BVH2Q or _BVH2_QSHADOW for every scene */
+    int32_t layout;               /* LMGPU_LAYOUT_BVH2, _BVH4, _BVH2Q or _BVH2_QSHADOW: every one walks the
+                                     scenes' 8-wide render trees */
     int32_t wave_paths;           /* paths in flight: the capacity of the ray and shadow queues
                                      (per pool), in [1024, 2^27] */
     int32_t shade_blocks_per_sm;  /* grid of the shading kernel (blocks of 128 threads per SM) */
@@ -388,7 +397,7 @@ int lmgpu_batch_render(LmgpuBatch* batch, const LmgpuRenderParams* params, float
  * batch renders with direct launches in fixed waves (no graph; its
  * configuration is otherwise kept), records CUDA events on `stream` around
  * every traversal launch and, with count_tests, counts each traversal's
- * binary-node slab tests (four per 4-wide node) and TriAccel tests with a
+ * box tests (eight per node visit) and TriAccel tests with a
  * counting copy of the traversal kernel, whose times are then not the
  * render's. Films as lmgpu_batch_render_device; synchronises. */
 typedef struct {
@@ -396,7 +405,7 @@ typedef struct {
     int64_t launches[2];        /* traversal launches of each kind */
     double trace_ms[2];         /* summed device time of those launches */
     double render_ms;           /* device time of the whole render */
-    uint64_t node_tests[2];     /* count_tests only: slab tests per kind */
+    uint64_t node_tests[2];     /* count_tests only: box tests per kind */
     uint64_t tri_tests[2];      /* count_tests only: TriAccel tests per kind */
 } LmgpuTraceProfile;
 int lmgpu_batch_profile(LmgpuBatch* batch, const LmgpuRenderParams* params, void* const* films_device,
@@ -405,8 +414,7 @@ int lmgpu_batch_profile(LmgpuBatch* batch, const LmgpuRenderParams* params, void
 /* Autotuner: renders the batch with each scene's sample count scaled by
  * `sample_fraction` (0 < f <= 1; raised for a candidate until the trial
  * holds four of its waves, eight in overlap mode, or the whole render) under candidate
- * configurations (mode, BVH layout, paths in flight, shading grid, overlap
- * bounce), coordinate by coordinate, keeps the one with the least device
+ * configurations (mode, paths in flight, shading grid, overlap bounce), coordinate by coordinate, keeps the one with the least device
  * time per sample (a candidate must beat the incumbent, which starts as the
  * batch's configuration, by more than 0.5 %), stores it as the batch's
  * configuration and returns it
@@ -480,10 +488,10 @@ int lmgpu_abi_version(void);
  * timeouts raised inside kernels come back here as LMGPU_ERR_* codes. */
 int lmgpu_scene_status(LmgpuScene* scene, void* stream);
 
-/* Measurement variant of lmgpu_intersect: additionally adds the number of
- * binary-node slab tests and TriAccel tests of the batch to two DEVICE
- * unsigned long long counters (the reference's per-ray work, counted the way
- * scene.bvh.cpp:405-473 performs it). */
+/* Measurement variant of lmgpu_intersect: the same hits by the reference's own
+ * walk (one thread per ray), adding the number of its binary-node slab tests and
+ * TriAccel tests to two DEVICE unsigned long long counters (the reference's
+ * per-ray work, counted the way scene.bvh.cpp:405-473 performs it). */
 int lmgpu_intersect_counted(LmgpuScene* scene, const LmgpuRaysSoA* rays, int64_t n,
                             LmgpuHitsSoA* hits, unsigned long long* counters_device,
                             void* stream);

@@ -3,7 +3,7 @@ reference, whose RenderProcessScheduler renders one scene at a time,
 sched.mt.cpp:93-266).
 
     batch = SceneBatch([scene_a, scene_b, ...])       # built Scene objects
-    batch.autotune(renderers, num_samples)            # optional: layout, wave size, shading grid
+    batch.autotune(renderers, num_samples)            # optional: mode, wave size, shading grid
     films = batch.render(renderers, num_samples)      # one (H, W, 3) film per scene
 
 Each scene keeps its own camera, film, renderer parameters (technique shared
@@ -25,9 +25,8 @@ import numpy as np
 from . import native as N
 from .render import Renderer
 
-# "bvh": binary float nodes, "qbvh": 4-wide, "bvh_q16": binary nodes with
-# 16-bit quantised child boxes, "bvh_qshadow": float nodes for bounce rays
-# and quantised ones for shadow rays (the last two: batch renders only).
+# Accepted layout names; renders walk the scenes' 8-wide compressed render trees
+# under every one of them.
 LAYOUTS = {"bvh": N.LAYOUT_BVH2, "qbvh": N.LAYOUT_BVH4, "bvh_q16": N.LAYOUT_BVH2Q,
            "bvh_qshadow": N.LAYOUT_BVH2_QSHADOW}
 MODES = {"waves": N.BATCH_WAVES, "stream": N.BATCH_STREAM, "overlap": N.BATCH_OVERLAP}
@@ -138,7 +137,7 @@ class SceneBatch:
                 sample_offsets=None) -> dict:
         """One measurement render (lmgpu_batch_profile): direct launches in
         fixed waves with CUDA events around every traversal launch; with
-        `count_tests`, the slab and TriAccel tests of every ray (counting
+        `count_tests`, the box and TriAccel tests of every ray (counting
         kernels: their times are not the render's)."""
         import torch
         fp64 = films[0].dtype == torch.float64
@@ -157,7 +156,7 @@ class SceneBatch:
         return out
 
     def autotune(self, renderers, num_samples, sample_fraction: float = 0.125, stream=None) -> dict:
-        """Chooses mode, layout, wave size, shading grid and overlap bounce by timing scaled-down
+        """Chooses mode, wave size, shading grid and overlap bounce by timing scaled-down
         renders of this batch (each candidate on at least four of its waves, or
         the whole render; compared by time per sample); the choice becomes the
         batch's configuration. trial_ms is the winner's time at sample_fraction."""

@@ -31,7 +31,7 @@ BUILD_DIR = os.path.join(HERE, "_build")
 
 CU_SOURCES = ["api.cu", "pathtrace.cu", "adjoint.cu", "noalloc.cu", "batch.cu", "eval.cu"]
 CPP_SOURCES = ["builder.cpp"]
-HEADERS = ["layout.h", "builder.h", "internal.h", "scene.cuh", "trace.cuh", "trace4.cuh",
+HEADERS = ["layout.h", "builder.h", "internal.h", "scene.cuh", "trace.cuh", "trace8.cuh",
            "shading.cuh", "rng.cuh", "pathtrace.cuh", "trace_kernels.cuh", "pt_kernels.cuh"]
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]

@@ -1,23 +1,34 @@
 // Differentiable rendering: a forward / adjoint pair over the path tracer
 // with per-triangle diffuse albedo and per-light emission as parameters.
 //
-// Both passes run the same per-sample path (the reference's pt / pt.direct /
-// pt.mis loops, pathtrace*.cpp) one thread per sample. The adjoint pass does
-// not store path vertices from the forward pass: it replays every path from
-// its counter-based random numbers (recomputation instead of checkpointing)
-// and, for each radiance contribution c splatted at pixel p, adds
+// Both passes run the reference's pt / pt.direct / pt.mis paths (pathtrace*.cpp)
+// as waves of the renderers' own kernels (pt_kernels.cuh) under a context that
+// replaces albedo and emission. The adjoint pass does not store path vertices from
+// the forward pass: it replays every path from its counter-based random
+// numbers and, for each radiance contribution c splatted at pixel p, adds
 // dL/dI_p * c / R_t to the gradient of the albedo R of every diffuse vertex t
 // on the contribution's prefix (c is linear in each of them) and
-// dL/dI_p * c / Le to the emission of its light. A path's contributions come
-// in order of non-decreasing prefix length ("depth"), so the replay keeps,
-// for the first RECORDED_VERTS vertices, the sum of the weights
-// w = dL/dI_p * c whose prefix ends there and turns them into suffix sums
-// once the path is done: one set of atomics per vertex instead of one per
-// (contribution, vertex). Emission gradients are summed per thread and per
-// block before they reach global memory, since every path adds to the same
-// few lights. Russian-roulette probabilities and MIS weights are held at
-// their sampled values, which keeps the estimator unbiased for the diffuse
-// BSDFs (their sampling densities do not depend on R).
+// dL/dI_p * c / Le to the emission of its light. While a wave runs, each
+// path keeps per vertex the triangle and the sum of the weights
+// w = dL/dI_p * c whose prefix ends there; once the wave is done the weights are
+// turned into suffix sums: one set of atomics per vertex instead of one per
+// (contribution, vertex). Emission gradients go to double-precision partial sums
+// (EMISSION_COPIES of them, since every path adds to the same few lights).
+// Russian-roulette probabilities and MIS weights are held at their sampled
+// values, which keeps the estimator unbiased for the diffuse BSDFs (their
+// sampling densities do not depend on R).
+//
+// Waves against one thread per sample (k_diff; measured on the refined Cornell box,
+// 512 x 512, 32 samples per pixel, up to 8 vertices, forward + backward):
+// one thread per sample over the binary tree 35.2 ms, over the 8-wide tree (more
+// registers, one ray's leaves hold up its warp) 61.5 ms, waves 16.0 ms.
+// One thread per sample stays for batches below WAVE_MIN_SAMPLES samples, whose
+// launches would cost more than the walk, and for streams being captured (a
+// wave's workspace is allocated in stream order).
+//
+// The tail of a path of more vertices than a wave records (RECORDED_VERTS;
+// UNBOUNDED_VERTS where the depth has no bound) is run by one thread from the path's
+// queued ray (k_diff_tail). In k_diff and in that kernel:
 //
 // Paths deeper than RECORDED_VERTS vertices: the weights of all
 // contributions deeper than that are summed into one total W_tail while the
@@ -35,14 +46,20 @@
 // max_path_vertices = -1) does not end either.
 #include <cuda_runtime.h>
 #include <algorithm>
+#include <cstdint>
 #include <cstring>
 
 #include "../../include/lmgpu.h"
 #include "internal.h"
 #include "pathtrace.cuh"
+#include "pt_kernels.cuh"
 #include "rng.cuh"
 #include "trace.cuh"
-#include "trace4.cuh"
+#include "trace8.cuh"
+#include "trace_kernels.cuh"
+#include <memory>
+#include <mutex>
+#include <unordered_map>
 
 namespace lmgpu {
 namespace {
@@ -60,39 +77,35 @@ struct DiffConsts {
     const float* emission;   // 3 per area light or null
 };
 
-template <int LAYOUT, bool ANY, int STACK>
+template <bool NAIVE, bool ANY, int STACK>
 __device__ __forceinline__ int32_t cast_ray(const DeviceScene& s, V3 o, V3 d, float tmin, float tmax, Hit& h,
-                                            int2* stack, int32_t* status)
+                                            uint2* stack, int32_t* status)
 {
     RayIn in;
     in.o[0] = o.x; in.o[1] = o.y; in.o[2] = o.z;
     in.d[0] = d.x; in.d[1] = d.y; in.d[2] = d.z;
     in.tmin = tmin; in.tmax = tmax;
     TraversalRay r;
-    setup_ray<LAYOUT != LMGPU_LAYOUT_NAIVE>(r, in);   // a render ray (the naive scan keeps the exact setup)
+    setup_ray<!NAIVE>(r, in);   // a render ray (the naive scan keeps the exact setup)
     h.tri = -1;
     if (s.num_tris == 0) return -1;
-    bool ok;
-    const int cap = s.stack_cap < STACK ? s.stack_cap : STACK;
-    // The renderers' walks and triangle test: the wavefront kernels' own.
-    if (LAYOUT == LMGPU_LAYOUT_BVH2 && ANY && LMGPU_TRACE_ANYHIT_WALK)   // visibility: the any-hit walk
-        ok = trace_bvh2_any<true>(s.bvh2, s.tris, s.root_ref, s.root_box, r, h, reinterpret_cast<int*>(stack), cap, nullptr);
-    else if (LAYOUT == LMGPU_LAYOUT_BVH2) ok = trace_bvh2<ANY, true>(s.bvh2, s.tris, s.root_ref, s.root_box, r, h, stack, cap, nullptr);
-    else if (LAYOUT == LMGPU_LAYOUT_BVH4) ok = trace_bvh4<ANY, true>(s.bvh4, s.tris, s.root_ref4, s.root_box, r, h, stack, cap, nullptr);
-    else { trace_naive<ANY>(s.tris_by_id, s.num_tris, r, h, nullptr); ok = true; }
+    bool ok = true;
+    // The renderers' walk and triangle test: the wavefront kernels' own.
+    if (NAIVE) trace_naive<ANY>(s.tris_by_id, s.num_tris, r, h, nullptr);
+    else ok = trace8<ANY>(s.bvh8, s.tris8, s.check_boxes ? s.boxes8 : nullptr, r, h, stack, s.stack8_cap < STACK ? s.stack8_cap : STACK);
     if (!ok) { atomicOr(status, STATUS_STACK_OVERFLOW); h.tri = -1; }
     return h.tri;
 }
 
-template <int LAYOUT, int STACK>
-__device__ __forceinline__ bool visible(const DeviceScene& s, V3 a, V3 b, int2* stack, int32_t* status)
+template <bool NAIVE, int STACK>
+__device__ __forceinline__ bool visible(const DeviceScene& s, V3 a, V3 b, uint2* stack, int32_t* status)
 {
     const V3 d = b - a;
     const float len = sqrtf(length2(d));
     const V3 dn = d / len;
     const float maxt = len * (1.0f - EPS_F);
     Hit h;
-    if (cast_ray<LAYOUT, true, STACK>(s, a, dn, EPS_F, maxt, h, stack, status) >= 0) return false;
+    if (cast_ray<NAIVE, true, STACK>(s, a, dn, EPS_F, maxt, h, stack, status) >= 0) return false;
     float t;
     if (s.has_env && env_sphere_intersect(s, a, dn, EPS_F, maxt, t)) return false;
     return true;
@@ -230,9 +243,9 @@ __device__ __noinline__ void save_point(PathPoint* dst, const PathPoint& src) { 
 // second replay of a deep path's tail; otherwise, in the adjoint, the state
 // on arrival at depth RECORDED_VERTS is saved in *ck and *deep set. Both
 // instantiations compute the same path from the same state.
-template <int TECH, int LAYOUT, int STACK, bool BACKWARD, bool TAIL>
+template <int TECH, bool NAIVE, int STACK, bool BACKWARD, bool TAIL>
 __device__ __forceinline__ void bounce_loop(const DeviceScene& s, const DiffConsts& c, uint64_t key, int path_pixel,
-                                            PathPoint& pp, PathPoint* ck, bool* deep, Replay& rp, int2* stack,
+                                            PathPoint& pp, PathPoint* ck, bool* deep, Replay& rp, uint2* stack,
                                             float* image, const float* dL, float* d_albedo, EmissionSum& es,
                                             float* s_de, float* d_emission, int32_t* status)
 {
@@ -240,7 +253,7 @@ __device__ __forceinline__ void bounce_loop(const DeviceScene& s, const DiffCons
         if (c.max_pv != -1 && pp.k >= c.max_pv) break;
         if (BACKWARD && !TAIL && pp.nv == RECORDED_VERTS) { save_point(ck, pp); *deep = true; }
         Hit h;
-        const int tri = cast_ray<LAYOUT, false, STACK>(s, pp.ro, pp.rd, pp.tmin, FLT_MAX, h, stack, status);
+        const int tri = cast_ray<NAIVE, false, STACK>(s, pp.ro, pp.rd, pp.tmin, FLT_MAX, h, stack, status);
         Geom g;
         const V3 wi = -pp.rd;
         V3 Le = v3(0, 0, 0);
@@ -306,7 +319,7 @@ __device__ __forceinline__ void bounce_loop(const DeviceScene& s, const DiffCons
                 const V3 fs = eval_bsdf(m, g, wi, ppL, pb);
                 const float G = geometry_term(g.p, g.sn, false, lp.p, lp.n, false);
                 const V3 Lel = emitted(lp.Le, lp.n, -ppL);
-                if (G != 0.0f && !is_zero(fs) && !is_zero(Lel) && visible<LAYOUT, STACK>(s, g.p, lp.p, stack, status)) {
+                if (G != 0.0f && !is_zero(fs) && !is_zero(Lel) && visible<NAIVE, STACK>(s, g.p, lp.p, stack, status)) {
                     float w = 1.0f;
                     if (TECH == LMGPU_RENDER_PT_MIS) { const float pdl = lp.pdf_area / G; w = pdl / (pdl + pb); }
                     contribute<BACKWARD>(c, s, rp, TAIL, pp.nv, li, path_pixel, pp.thr * fs * Lel * (w * G / lp.pdf_area),
@@ -337,7 +350,7 @@ __device__ __forceinline__ void bounce_loop(const DeviceScene& s, const DiffCons
     }
 }
 
-template <int TECH, int LAYOUT, int STACK, bool BACKWARD>
+template <int TECH, bool NAIVE, int STACK, bool BACKWARD>
 // 8 resident blocks per SM (64 registers, some spills): on the refined
 // Cornell box, forward / backward 22.2 / 33.1 ms against 24.9 / 36.2 ms at the
 // unconstrained 94-96 registers (5 blocks); 6, 10 and 12 blocks were slower
@@ -346,7 +359,7 @@ template <int TECH, int LAYOUT, int STACK, bool BACKWARD>
 __global__ void __launch_bounds__(128, 8) k_diff(const DeviceScene s, const DiffConsts c, float* image, const float* dL,
                                               float* d_albedo, float* d_emission, int32_t* status)
 {
-    int2 stack[STACK];
+    uint2 stack[STACK];
     Replay rp;
     __shared__ float s_de[3 * SHARED_LIGHTS];
     EmissionSum es;
@@ -395,7 +408,7 @@ __global__ void __launch_bounds__(128, 8) k_diff(const DeviceScene s, const Diff
                 if (camera_project(s.cam, cp, ppL, lrx, lry, We) && We > 0.0f) {
                     const float G = geometry_term(cp, v3(0, 0, 1), true, lp.p, lp.n, false);
                     const V3 Le = emitted(lp.Le, lp.n, -ppL);
-                    if (G != 0.0f && !is_zero(Le) && visible<LAYOUT, STACK>(s, cp, lp.p, stack, status)) {
+                    if (G != 0.0f && !is_zero(Le) && visible<NAIVE, STACK>(s, cp, lp.p, stack, status)) {
                         float w = 1.0f;
                         if (TECH == LMGPU_RENDER_PT_MIS) { const float pdl = lp.pdf_area / G; w = pdl / (pdl + We); }
                         contribute<BACKWARD>(c, s, rp, false, 0, li, film_pixel(s.cam, lrx, lry),
@@ -412,14 +425,14 @@ __global__ void __launch_bounds__(128, 8) k_diff(const DeviceScene s, const Diff
         PathPoint ck;
         bool deep = false;
         if (alive)
-            bounce_loop<TECH, LAYOUT, STACK, BACKWARD, false>(s, c, key, path_pixel, pp, &ck, &deep, rp, stack, image, dL,
+            bounce_loop<TECH, NAIVE, STACK, BACKWARD, false>(s, c, key, path_pixel, pp, &ck, &deep, rp, stack, image, dL,
                                                               d_albedo, es, s_de, d_emission, status);
         if (BACKWARD) {
             flush_albedo(c, s, rp, min(pp.nv, RECORDED_VERTS), d_albedo);
             // The tail of a path deeper than RECORDED_VERTS: replayed from the
             // checkpoint taken on arrival at that depth.
             if (deep)
-                bounce_loop<TECH, LAYOUT, STACK, BACKWARD, true>(s, c, key, path_pixel, ck, nullptr, nullptr, rp, stack,
+                bounce_loop<TECH, NAIVE, STACK, BACKWARD, true>(s, c, key, path_pixel, ck, nullptr, nullptr, rp, stack,
                                                                  image, dL, d_albedo, es, s_de, d_emission, status);
         }
     }
@@ -432,13 +445,379 @@ __global__ void __launch_bounds__(128, 8) k_diff(const DeviceScene s, const Diff
     }
 }
 
-template <int TECH, int LAYOUT, int STACK>
+// ------------------------------------------------------------- waves ----
+
+// Samples from which a pass runs as waves.
+constexpr int64_t WAVE_MIN_SAMPLES = int64_t(1) << 16;
+constexpr int64_t WAVE_PATHS = int64_t(1) << 23;   // paths in flight (a workspace of 350 bytes a path at 8 vertices)
+constexpr int UNBOUNDED_VERTS = 20;                // vertices a wave follows a path of unbounded depth
+constexpr int EMISSION_COPIES = 512;
+
+// The renderers' context with parameters in place of the scene's albedo and
+// emission. The adjoint's shadow rays carry the weight dL/dI_p * c in place of c, and
+// their light.
+template <bool BACKWARD>
+struct DiffScene : RenderContext {
+    static constexpr bool TABLE = false, STREAM = false;
+    DeviceScene s;
+    RenderConsts rc;
+    float scale;
+    const float* albedo;
+    const float* emission_of;
+    float* image;            // forward
+    const float* dL;         // adjoint, from here on
+    float4* record;          // [vertex][path]: weight, triangle
+    int64_t stride;
+    int32_t* vertices;       // surface vertices of each path
+    int32_t hit_no;          // shadow pass: the vertex its rays leave from
+    double* d_emission;      // [copy][light][3]
+    int32_t copies;
+
+    __device__ __forceinline__ const DeviceScene& scene(int) const { return s; }
+    __device__ __forceinline__ const RenderConsts& consts(int) const { return rc; }
+    __device__ __forceinline__ int64_t wave_count(int64_t n) const { return n; }
+    __device__ __forceinline__ int64_t sample_of(int, int64_t i) const { return rc.sample_base + i; }
+    __device__ __forceinline__ int begin_path(const PathState&, int64_t j, int64_t& i, int64_t& sample) const
+    {
+        i = j;
+        sample = rc.sample_base + j;
+        return 0;
+    }
+    __device__ __forceinline__ int path_depth(const PathState&, int64_t, int k) const { return k; }
+
+    __device__ __forceinline__ V3 Le_of(const DeviceScene&, int li) const
+    {
+        if (li >= s.num_area_lights) return load3(s.env_Le);
+        return emission_of ? load3(emission_of + 3 * li) : load3(s.area_lights[li].Le);
+    }
+    __device__ __forceinline__ Material material(const DeviceScene&, int prim, int32_t tri) const
+    {
+        Material m = material_of(s, prim);
+        if (albedo && m.type == LMGPU_BSDF_DIFFUSE) m.R = load3(albedo + 3 * (int64_t)tri);
+        return m;
+    }
+    __device__ __forceinline__ V3 area_Le(const DeviceScene&, int li) const { return Le_of(s, li); }
+    __device__ __forceinline__ void light_sample(const DeviceScene&, LightPoint& lp) const { lp.Le = Le_of(s, lp.light); }
+    __device__ __forceinline__ V3 weight(int pixel, V3 c) const
+    {
+        return v3(dL[3 * pixel] * c.x, dL[3 * pixel + 1] * c.y, dL[3 * pixel + 2] * c.z) * scale;
+    }
+    __device__ __forceinline__ V3 path_weight(const PathState& st, int64_t i, V3 c) const
+    {
+        const float2 r = st.raster[i];
+        return weight(film_pixel(s.cam, r.x, r.y), c);
+    }
+    __device__ __forceinline__ void add_record(int vertex, int64_t i, V3 w) const
+    {
+        float4& q = record[vertex * stride + i];
+        const float4 v = q;
+        q = make_float4(v.x + w.x, v.y + w.y, v.z + w.z, v.w);
+    }
+    __device__ __forceinline__ void add_emission(int li, V3 w) const
+    {
+        if (li >= s.num_area_lights) return;
+        const V3 Le = Le_of(s, li);
+        const int copy = (int)((blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) & (unsigned)(copies - 1));
+        double* dst = d_emission + 3 * ((int64_t)copy * s.num_area_lights + li);
+        if (Le.x != 0.0f) atomicAdd(dst, (double)(w.x / Le.x));
+        if (Le.y != 0.0f) atomicAdd(dst + 1, (double)(w.y / Le.y));
+        if (Le.z != 0.0f) atomicAdd(dst + 2, (double)(w.z / Le.z));
+    }
+    __device__ __forceinline__ void start(int64_t i) const { if (BACKWARD) vertices[i] = 0; }
+    __device__ __forceinline__ void vertex(const PathState&, int64_t i, int k, int32_t tri) const
+    {
+        if (!BACKWARD) return;
+        record[(int64_t)(k - 1) * stride + i] = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(tri));
+        vertices[i] = k;
+    }
+    __device__ __forceinline__ void emission(const PathState& st, int64_t i, int k, int li, V3 c) const
+    {
+        if (!BACKWARD) { RenderContext::emission(st, i, k, li, c); return; }
+        const V3 w = path_weight(st, i, c);
+        if (is_zero(w)) return;
+        if (k >= 2) add_record(k - 2, i, w);       // its prefix ends at the vertex before the hit
+        add_emission(li, w);
+    }
+    __device__ __forceinline__ V3 nee(const PathState& st, int64_t i, V3 c) const { return BACKWARD ? path_weight(st, i, c) : c; }
+    __device__ __forceinline__ V3 camera_nee(int pixel, V3 c) const { return BACKWARD ? weight(pixel, c) : c; }
+    __device__ __forceinline__ int shadow_tag(int, int light) const { return BACKWARD ? light : 0; }
+    __device__ __forceinline__ void lit(float4* L, int32_t dest, V3 c, int tag) const
+    {
+        if (!BACKWARD) { RenderContext::lit(L, dest, c, tag); return; }
+        add_record(hit_no - 1, dest, c);
+        add_emission(tag, c);
+    }
+    __device__ __forceinline__ void lit_pixel(int tag, int pixel, V3 c) const
+    {
+        if (BACKWARD) add_emission(tag, c);
+        else film_add(image, pixel, c * scale);
+    }
+};
+
+// Before a bounce: clear its output queue and the shadow queue.
+__global__ void k_diff_prep(uint32_t* counters, int qout)
+{
+    counters[qout] = 0;
+    counters[2] = 0;
+}
+
+// Forward, end of a wave: each path's radiance to its pixel.
+__global__ void __launch_bounds__(128) k_diff_splat(const DiffScene<false> ctx, const PathState st, int64_t n)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float2 r = st.raster[i];
+    film_add(ctx.image, film_pixel(ctx.s.cam, r.x, r.y), f3(st.L[i]) * ctx.scale);
+}
+
+// Adjoint, end of a wave: the albedo gradient weight of a vertex is the sum of
+// the weights of every contribution whose prefix contains it: the suffix sum of
+// the recorded weights plus the tail's (left in st.L by k_diff_tail, else 0).
+// Bound by its atomics: three per vertex with a non-zero weight.
+__global__ void __launch_bounds__(128) k_diff_flush(const DiffScene<true> ctx, const DiffConsts c, const PathState st, int64_t n,
+                                                    float* d_albedo)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    V3 S = f3(st.L[i]);
+    for (int v = ctx.vertices[i] - 1; v >= 0; v--) {
+        const float4 q = ctx.record[v * ctx.stride + i];
+        S = S + f3(q);
+        add_albedo_grad(c, ctx.s, __float_as_int(q.w), S, d_albedo);
+    }
+}
+
+__global__ void k_diff_emission(const double* part, int copies, int n, float* d_emission)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    double sum = 0.0;
+    for (int k = 0; k < copies; k++) sum += part[(int64_t)k * n + i];
+    if (sum != 0.0) atomicAdd(d_emission + i, (float)sum);
+}
+
+// The paths still alive after a wave's last bounce, one thread each from their
+// queued ray. Their vertices count from RECORDED_VERTS on, so that every
+// contribution is "deeper than the record" (see the head of this file); the one
+// found by the first hit belongs to the wave's last vertex.
+template <int TECH, int STACK, bool BACKWARD>
+__global__ void __launch_bounds__(128) k_diff_tail(const DiffScene<BACKWARD> ctx, const DiffConsts c, const PathState st, int q, int k0,
+                                                   float* d_albedo, float* d_emission, int32_t* status)
+{
+    uint2 stack[STACK];
+    Replay rp;
+    __shared__ float s_de[3 * SHARED_LIGHTS];
+    EmissionSum es;
+    es.light = -1;
+    es.g = v3(0, 0, 0);
+    if (BACKWARD) {
+        for (int i = threadIdx.x; i < 3 * SHARED_LIGHTS; i += blockDim.x) s_de[i] = 0.0f;
+        __syncthreads();
+    }
+    const int64_t n = (int64_t)st.counters[q];
+    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x) {
+        const float4 o4 = st.qo[q][j], d4 = st.qd[q][j], t4 = st.qt[q][j];
+        const float4 n4 = TECH == LMGPU_RENDER_PT ? make_float4(0, 0, 1, 0) : st.qn[q][j];
+        const int64_t i = queued_path(d4);
+        const uint64_t key = sample_key(c.seed, (uint64_t)ctx.sample_of(0, i));
+        const float2 rs = st.raster[i];
+        const int pixel = film_pixel(ctx.s.cam, rs.x, rs.y);
+        PathPoint pp, ck;
+        pp.ro = f3(o4); pp.rd = f3(d4); pp.thr = f3(t4);
+        pp.prev_p = pp.ro; pp.prev_n = f3(n4);
+        pp.prev_deg = (__float_as_uint(n4.w) & PREV_DEGENERATED) != 0;
+        pp.prev_spec = (__float_as_uint(n4.w) & PREV_SPECULAR) != 0;
+        pp.prev_pdf = t4.w;
+        pp.tmin = queued_tmin(d4);
+        pp.k = k0;
+        pp.nv = BACKWARD ? RECORDED_VERTS : k0 - 1;
+        bool deep = false;
+        if (BACKWARD) rp.w[RECORDED_VERTS - 1] = rp.w[TAIL_SUM] = rp.w[RUN_SUM] = v3(0, 0, 0);
+        bounce_loop<TECH, false, STACK, BACKWARD, false>(ctx.s, c, key, pixel, pp, &ck, &deep, rp, stack, ctx.image, ctx.dL, d_albedo,
+                                                         es, s_de, d_emission, status);
+        if (BACKWARD) {
+            st.L[i] = f4(rp.w[TAIL_SUM] + rp.w[RECORDED_VERTS - 1], 0.0f);
+            if (deep)
+                bounce_loop<TECH, false, STACK, BACKWARD, true>(ctx.s, c, key, pixel, ck, nullptr, nullptr, rp, stack, ctx.image, ctx.dL,
+                                                                d_albedo, es, s_de, d_emission, status);
+        }
+    }
+    if (BACKWARD) {
+        flush_emission(es, s_de, d_emission);
+        __syncthreads();
+        const int m = 3 * min(ctx.s.num_area_lights, SHARED_LIGHTS);
+        for (int i = threadIdx.x; i < m; i += blockDim.x)
+            if (s_de[i] != 0.0f) atomicAdd(d_emission + i, s_de[i]);
+    }
+}
+
+// Stream-ordered memory of the waves' workspaces, one pool per device: calls
+// on several streams or threads each get their own, and what they return stays
+// in the pool for the next call until lmgpu_render_release.
+struct DiffPool {
+    std::mutex mu;
+    cudaMemPool_t pool = nullptr;
+};
+DiffPool& diff_pool(int device)
+{
+    static std::mutex map_mu;
+    static std::unordered_map<int, std::unique_ptr<DiffPool>> all;
+    std::lock_guard<std::mutex> lock(map_mu);
+    auto& e = all[device];
+    if (!e) e.reset(new DiffPool);
+    return *e;
+}
+cudaError_t diff_pool_of(int device, cudaMemPool_t* out)
+{
+    DiffPool& p = diff_pool(device);
+    std::lock_guard<std::mutex> lock(p.mu);
+    if (!p.pool) {
+        cudaMemPoolProps props;
+        std::memset(&props, 0, sizeof(props));
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        cudaError_t e = cudaMemPoolCreate(&p.pool, &props);
+        if (e != cudaSuccess) { p.pool = nullptr; return e; }
+        uint64_t keep = UINT64_MAX;
+        e = cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        if (e != cudaSuccess) { cudaMemPoolDestroy(p.pool); p.pool = nullptr; return e; }
+    }
+    *out = p.pool;
+    return cudaSuccess;
+}
+
+template <int TECH, int STACK, bool BACKWARD>
+int run_diff_waves(LmgpuScene* sc, const DiffConsts& c, float* image, const float* dL, float* da, float* de, cudaStream_t stream)
+{
+    using Ctx = DiffScene<BACKWARD>;
+    const DeviceScene& s = sc->rdev;
+    if (c.max_pv != -1 && c.max_pv <= 1) return LMGPU_OK;      // no vertex beyond the camera
+    const int limit = c.max_pv == -1 ? UNBOUNDED_VERTS : RECORDED_VERTS;
+    const int bounces = c.max_pv == -1 ? limit : std::min(c.max_pv - 1, limit);
+    const bool tail = c.max_pv == -1 || c.max_pv - 1 > limit;
+    const int lights = s.num_area_lights;
+    int copies = 1;
+    while (2 * copies <= EMISSION_COPIES && 2 * copies * std::max(lights, 1) <= 64 * EMISSION_COPIES) copies *= 2;
+    // Workspace: counters, work slots, emission partial sums, then the path state.
+    const int slots = 2 * bounces + 1;
+    const size_t emission_bytes = BACKWARD ? (size_t)copies * lights * 3 * sizeof(double) : 0;
+    const size_t head = (256 + slots * sizeof(unsigned long long) + emission_bytes + 255) / 256 * 256;
+    const size_t per_path = 16 * 13 + 8 + (BACKWARD ? 4 + 16 * (size_t)bounces : 0);
+    cudaMemPool_t pool = nullptr;
+    LMGPU_CUDA_TRY(diff_pool_of(sc->device, &pool));
+    int64_t P = std::min(c.num_samples, WAVE_PATHS);
+    char* mem = nullptr;
+    for (;;) {
+        const cudaError_t e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&mem), head + (size_t)P * per_path + 256, pool, stream);
+        if (e == cudaSuccess) break;
+        cudaGetLastError();
+        if (e != cudaErrorMemoryAllocation) return cuda_fail(e, "cudaMallocFromPoolAsync");
+        if (P <= WAVE_MIN_SAMPLES) return fail(LMGPU_ERR_OOM, "differentiable render workspace allocation failed");
+        P = (P + 1) / 2;
+    }
+    PathState st{};
+    st.counters = reinterpret_cast<uint32_t*>(mem);
+    unsigned long long* work = reinterpret_cast<unsigned long long*>(mem + 256);
+    char* p = mem + head;
+    auto take = [&](size_t b) { char* r = p; p += b; return r; };
+    Ctx ctx;
+    ctx.record = reinterpret_cast<float4*>(take(BACKWARD ? 16 * (size_t)P * bounces : 0));
+    for (int q = 0; q < 2; q++) {
+        st.qo[q] = reinterpret_cast<float4*>(take(16 * (size_t)P));
+        st.qd[q] = reinterpret_cast<float4*>(take(16 * (size_t)P));
+        st.qt[q] = reinterpret_cast<float4*>(take(16 * (size_t)P));
+        st.qn[q] = reinterpret_cast<float4*>(take(16 * (size_t)P));
+    }
+    st.hit = reinterpret_cast<float4*>(take(16 * (size_t)P));
+    st.L = reinterpret_cast<float4*>(take(16 * (size_t)P));
+    st.sh_o = reinterpret_cast<float4*>(take(16 * (size_t)P));
+    st.sh_d = reinterpret_cast<float4*>(take(16 * (size_t)P));
+    st.sh_c = reinterpret_cast<float4*>(take(16 * (size_t)P));
+    st.raster = reinterpret_cast<float2*>(take(8 * (size_t)P));
+    ctx.vertices = reinterpret_cast<int32_t*>(take(BACKWARD ? 4 * (size_t)P : 0));
+    for (uint32_t& q : st.cap) q = (uint32_t)P;
+#if LMGPU_BOUNDS_CHECK
+    for (uint32_t& q : st.cap) q = (uint32_t)std::min<int64_t>(P, check_limit_from_env("LMGPU_CHECK_QUEUE_LIMIT"));
+#endif
+    st.status = sc->d_status;
+    ctx.s = s;
+    ctx.rc.technique = TECH;
+    ctx.rc.rr_depth = c.rr_depth;
+    ctx.rc.max_pv = c.max_pv;
+    ctx.rc.sampling = c.sampling;
+    ctx.rc.seed = c.seed;
+    ctx.rc.pixels = c.pixels;
+    ctx.rc.inv_pixels = c.inv_pixels;
+    ctx.scale = c.scale;
+    ctx.albedo = c.albedo;
+    ctx.emission_of = c.emission;
+    ctx.image = image;
+    ctx.dL = dL;
+    ctx.stride = P;
+    ctx.hit_no = 0;
+    ctx.d_emission = reinterpret_cast<double*>(mem + 256 + slots * sizeof(unsigned long long));
+    ctx.copies = copies;
+    cudaError_t e = emission_bytes ? cudaMemsetAsync(ctx.d_emission, 0, emission_bytes, stream) : cudaSuccess;
+    auto closest = k_trace_persistent<STACK, false, PathRayIO<false>>;
+    auto any = k_trace_persistent<STACK, true, ShadowIO<Ctx>>;
+    for (int64_t base = 0; base < c.num_samples && e == cudaSuccess; base += P) {
+        const int64_t n = std::min(P, c.num_samples - base);
+        const int64_t full = (n + 127) / 128;
+        const unsigned shade = (unsigned)std::min<int64_t>(full, 148 * 8);
+        const unsigned rays = (unsigned)std::min<int64_t>(full, resident_blocks(closest));
+        const unsigned shadows = (unsigned)std::min<int64_t>(full, resident_blocks(any));
+        ctx.rc.sample_base = c.sample_offset + base;
+        auto shadow = [&](int k) {
+            ctx.hit_no = k;
+            ShadowIO<Ctx> io{ st.counters + 2, st.sh_o, st.sh_d, st.sh_c, st.L, ctx };
+            any<<<shadows, 128, 0, stream>>>(s, io, sc->d_status, work + 2 * k, nullptr);
+        };
+        k_wave_begin<<<1, 128, 0, stream>>>(st.counters, work, slots);
+        k_pt_init<TECH, Ctx><<<(unsigned)full, 128, 0, stream>>>(ctx, st, n, 0);
+        if (TECH != LMGPU_RENDER_PT) shadow(0);
+        for (int k = 1; k <= bounces; k++) {
+            const int qin = (k - 1) & 1;
+            k_diff_prep<<<1, 1, 0, stream>>>(st.counters, 1 - qin);
+            PathRayIO<false> io{ st.counters + qin, st.qo[qin], st.qd[qin], st.hit, nullptr };
+            closest<<<rays, 128, 0, stream>>>(s, io, sc->d_status, work + 2 * k - 1, nullptr);
+            k_pt_shade<TECH, Ctx><<<shade, 128, 0, stream>>>(ctx, st, k, qin, 1 - qin);
+            if (TECH != LMGPU_RENDER_PT) shadow(k);
+        }
+        if (tail) k_diff_tail<TECH, STACK, BACKWARD><<<shade, 128, 0, stream>>>(ctx, c, st, bounces & 1, bounces + 1, da, de, sc->d_status);
+        if constexpr (BACKWARD) k_diff_flush<<<(unsigned)full, 128, 0, stream>>>(ctx, c, st, n, da);
+        else k_diff_splat<<<(unsigned)full, 128, 0, stream>>>(ctx, st, n);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess && emission_bytes) {
+        k_diff_emission<<<(unsigned)((3 * lights + 127) / 128), 128, 0, stream>>>(ctx.d_emission, copies, 3 * lights, de);
+        e = cudaGetLastError();
+    }
+    const cudaError_t f = cudaFreeAsync(mem, stream);
+    if (e != cudaSuccess) return cuda_fail(e, "differentiable render wave");
+    if (f != cudaSuccess) return cuda_fail(f, "cudaFreeAsync");
+    return LMGPU_OK;
+}
+
+// Whether a pass runs as waves (see the head of this file).
+bool diff_as_waves(const LmgpuScene* sc, const DiffConsts& c, cudaStream_t stream)
+{
+    if (sc->dev.layout == LMGPU_LAYOUT_NAIVE || c.num_samples < WAVE_MIN_SAMPLES || sc->rdev.num_tris == 0) return false;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return cap == cudaStreamCaptureStatusNone;
+}
+
+template <int TECH, bool NAIVE, int STACK>
 int launch_diff_l(LmgpuScene* sc, const DiffConsts& c, bool backward, float* image, const float* dL, float* da,
                   float* de, cudaStream_t st)
 {
     const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((c.num_samples + 127) / 128, 148 * 16));
-    if (backward) k_diff<TECH, LAYOUT, STACK, true><<<blocks, 128, 0, st>>>(sc->rdev, c, image, dL, da, de, sc->d_status);
-    else k_diff<TECH, LAYOUT, STACK, false><<<blocks, 128, 0, st>>>(sc->rdev, c, image, dL, da, de, sc->d_status);
+    if (backward) k_diff<TECH, NAIVE, STACK, true><<<blocks, 128, 0, st>>>(sc->rdev, c, image, dL, da, de, sc->d_status);
+    else k_diff<TECH, NAIVE, STACK, false><<<blocks, 128, 0, st>>>(sc->rdev, c, image, dL, da, de, sc->d_status);
     LMGPU_CUDA_TRY(cudaGetLastError());
     return LMGPU_OK;
 }
@@ -447,20 +826,23 @@ template <int TECH, int STACK>
 int launch_diff_s(LmgpuScene* sc, const DiffConsts& c, bool backward, float* image, const float* dL, float* da,
                   float* de, cudaStream_t st)
 {
-    switch (sc->dev.layout) {
-    case LMGPU_LAYOUT_BVH2: return launch_diff_l<TECH, LMGPU_LAYOUT_BVH2, STACK>(sc, c, backward, image, dL, da, de, st);
-    case LMGPU_LAYOUT_BVH4: return launch_diff_l<TECH, LMGPU_LAYOUT_BVH4, STACK>(sc, c, backward, image, dL, da, de, st);
-    default: return launch_diff_l<TECH, LMGPU_LAYOUT_NAIVE, 1>(sc, c, backward, image, dL, da, de, st);
-    }
+    if (sc->dev.layout == LMGPU_LAYOUT_NAIVE) return launch_diff_l<TECH, true, 1>(sc, c, backward, image, dL, da, de, st);
+    return launch_diff_l<TECH, false, STACK>(sc, c, backward, image, dL, da, de, st);
 }
 
 template <int TECH>
 int launch_diff_t(LmgpuScene* sc, const DiffConsts& c, bool backward, float* image, const float* dL, float* da,
                   float* de, cudaStream_t st)
 {
-    const int cap = sc->rdev.stack_cap;
-    if (cap <= 32) return launch_diff_s<TECH, 32>(sc, c, backward, image, dL, da, de, st);
-    if (cap <= 64) return launch_diff_s<TECH, 64>(sc, c, backward, image, dL, da, de, st);
+    const int cap = sc->rdev.stack8_cap;
+    if (cap <= 128 && diff_as_waves(sc, c, st)) {
+        if (cap <= 32)
+            return backward ? run_diff_waves<TECH, 32, true>(sc, c, image, dL, da, de, st)
+                            : run_diff_waves<TECH, 32, false>(sc, c, image, dL, da, de, st);
+        return backward ? run_diff_waves<TECH, 256, true>(sc, c, image, dL, da, de, st)
+                        : run_diff_waves<TECH, 256, false>(sc, c, image, dL, da, de, st);
+    }
+    if (cap <= 16) return launch_diff_s<TECH, 16>(sc, c, backward, image, dL, da, de, st);
     if (cap <= 128) return launch_diff_s<TECH, 128>(sc, c, backward, image, dL, da, de, st);
     return fail(LMGPU_ERR_UNSUPPORTED, "BVH too deep for the differentiable path (stack 128)");
 }
@@ -518,6 +900,15 @@ int launch_diff(LmgpuScene* sc, const LmgpuRenderParams* p, const LmgpuDiffParam
 }
 
 }  // namespace
+
+int release_diff_pool(int device)
+{
+    DiffPool& p = diff_pool(device);
+    std::lock_guard<std::mutex> lock(p.mu);
+    if (p.pool) LMGPU_CUDA_TRY(cudaMemPoolTrimTo(p.pool, 0));
+    return LMGPU_OK;
+}
+
 }  // namespace lmgpu
 
 using namespace lmgpu;

@@ -13,7 +13,6 @@
 #include "builder.h"
 #include "internal.h"
 #include "trace.cuh"
-#include "trace4.cuh"
 #include "trace_kernels.cuh"
 #include <condition_variable>
 #include <functional>
@@ -127,30 +126,31 @@ __global__ void k_check_bvh2(const Bvh2Node* nodes, int64_t num, int64_t limit, 
     if (!ref_in_range(nodes[i].left, limit, tris, ntris) || !ref_in_range(nodes[i].right, limit, tris, ntris))
         atomicOr(status, STATUS_BOUNDS);
 }
-__global__ void k_check_bvh4(const Bvh4Node* nodes, int64_t num, int64_t limit, int32_t root,
-                             const TriRecord* tris, int64_t ntris, int32_t* status)
+__global__ void k_check_bvh8(const Bvh8Node* nodes, int64_t num, int64_t limit, const TriRecord* tris, int64_t ntris,
+                             int32_t* status)
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0 && !ref_in_range(root, limit, tris, ntris)) atomicOr(status, STATUS_BOUNDS);
+    if (i == 0 && limit < 1) atomicOr(status, STATUS_BOUNDS);
     if (i >= num) return;
-    for (int c = 0; c < 4; c++) {
-        const int32_t r = nodes[i].child[c];
-        if (r != BVH4_EMPTY && !ref_in_range(r, limit, tris, ntris)) atomicOr(status, STATUS_BOUNDS);
-    }
+    const uint32_t inner = nodes[i].exps >> 24, valid = nodes[i].valid;
+    if ((inner & ~valid) || (int64_t)nodes[i].child_base + __popc(inner) > limit) atomicOr(status, STATUS_BOUNDS);
+    for (int c = 0; c < 8; c++)
+        if ((valid & ~inner) >> c & 1u)
+            if (nodes[i].start[c] > 0x7fffffffu || !leaf_in_range(~(int32_t)nodes[i].start[c], tris, ntris))
+                atomicOr(status, STATUS_BOUNDS);
 }
 
-// Checks the uploaded trees of `d` (node counts n2 / n4, triangle count
+// Checks the uploaded trees of `d` (node counts n2 / n8, triangle count
 // ntris) into the scene's status word and consumes it.
-int check_trees(LmgpuScene* s, const DeviceScene& d, int64_t n2, int64_t n4, int64_t ntris)
+int check_trees(LmgpuScene* s, const DeviceScene& d, int64_t n2, int64_t n8, int64_t ntris)
 {
     if (ntris <= 0) return LMGPU_OK;
     const int64_t lim = check_limit_from_env("LMGPU_CHECK_NODE_LIMIT");
     if (n2 > 0)
         k_check_bvh2<<<(unsigned)((n2 + 127) / 128), 128>>>(d.bvh2, n2, std::min(n2, lim), d.root_ref, d.tris, ntris,
                                                             s->d_status);
-    if (n4 > 0)
-        k_check_bvh4<<<(unsigned)((n4 + 127) / 128), 128>>>(d.bvh4, n4, std::min(n4, lim), d.root_ref4, d.tris, ntris,
-                                                            s->d_status);
+    if (n8 > 0)
+        k_check_bvh8<<<(unsigned)((n8 + 127) / 128), 128>>>(d.bvh8, n8, std::min(n8, lim), d.tris8, ntris, s->d_status);
     LMGPU_CUDA_TRY(cudaGetLastError());
     return consume_status(s, nullptr);
 }
@@ -276,16 +276,53 @@ int create_impl(const LmgpuSceneDesc* desc, LmgpuScene** out)
     if (!err.empty()) return fail(LMGPU_ERR_INVALID, err);
     const bool render_tree = desc->layout != LMGPU_LAYOUT_NAIVE && desc->render_tree == LMGPU_RENDER_TREE_SAH &&
                              b.num_tris > 0;
-    if (render_tree) {
-        try {
-            build_render_tree(b, desc->build_threads);
-        } catch (const std::bad_alloc&) {
-            return fail(LMGPU_ERR_OOM, "host allocation failed during the render tree build");
-        }
-    }
-
     CameraGpu cam;
     if (!setup_camera(*desc, cam)) return fail(LMGPU_ERR_INVALID, "invalid camera");
+
+    // The trees every traversal walks. The reference's: origins up to
+    // WIDE_ORIGIN_LIMIT times the scene's largest coordinate (the boxes grow with the
+    // bound; rays from farther away take the reference's own walk). The
+    // render tree: rays start in the scene's bounds or at the camera; far from the
+    // origin (coordinates beyond FAR_FROM_ORIGIN times the scene's extent) its candidate
+    // hits are also tested against their float leaf boxes.
+    constexpr double WIDE_ORIGIN_LIMIT = 8.0, FAR_FROM_ORIGIN = 8.0;
+    Bvh8Tree wide, rwide;
+    double scene_max = 0.0, extent = 0.0, wide_limit = 0.0;
+    bool far = false;
+    if (desc->layout != LMGPU_LAYOUT_NAIVE && b.num_tris > 0) {
+        for (int c = 0; c < 3; c++) {
+            scene_max = std::max(scene_max, (double)std::max(std::fabs(b.bounds.mn[c]), std::fabs(b.bounds.mx[c])));
+            extent = std::max(extent, (double)b.bounds.mx[c] - b.bounds.mn[c]);
+        }
+        // (scales at which a plane distance could overflow or go subnormal: none)
+        wide_limit = scene_max > 1e-20 && scene_max < 1e15 ? WIDE_ORIGIN_LIMIT * scene_max : -1.0;
+        far = scene_max > FAR_FROM_ORIGIN * extent;
+        double ray_max = scene_max;
+        if (cam.valid)
+            for (int c = 0; c < 3; c++) ray_max = std::max(ray_max, (double)std::fabs(cam.position[c]));
+        // The reference tree's collapse beside the render tree's build: both read
+        // only what build_scene made.
+        bool short_of_memory = false;
+        std::thread side([&] {
+            try {
+                collapse_bvh8(b, b.bvh2, b.tris, b.bvh2_root, b.root_box, WIDE_ORIGIN_LIMIT * scene_max, true, true,
+                              desc->build_threads, wide);
+            } catch (...) {
+                short_of_memory = true;
+            }
+        });
+        bool main_short = false;
+        try {
+            if (render_tree) {
+                build_render_tree(b, desc->build_threads);
+                collapse_bvh8(b, b.rbvh2, b.rtris, b.rbvh2_root, b.rroot_box, ray_max, false, far, desc->build_threads, rwide);
+            }
+        } catch (...) {
+            main_short = true;
+        }
+        side.join();
+        if (short_of_memory || main_short) return fail(LMGPU_ERR_OOM, "host allocation failed during the tree builds");
+    }
 
     LmgpuScene* s = new (std::nothrow) LmgpuScene;
     if (!s) return fail(LMGPU_ERR_OOM, "host allocation failed");
@@ -295,7 +332,6 @@ int create_impl(const LmgpuSceneDesc* desc, LmgpuScene** out)
     d.layout = desc->layout;
     d.num_tris = b.num_tris;
     d.root_ref = b.bvh2_root;
-    d.root_ref4 = b.bvh4_root;
     d.stack_cap = 2 * b.max_depth + 4;
     if (desc->max_stack_entries > 0 && desc->max_stack_entries < d.stack_cap) d.stack_cap = desc->max_stack_entries;
     std::memcpy(d.root_box, b.root_box, sizeof(d.root_box));
@@ -305,7 +341,12 @@ int create_impl(const LmgpuSceneDesc* desc, LmgpuScene** out)
     auto up = [&](auto& vec, auto** dst) { if (rc == LMGPU_OK) rc = upload(s, vec, dst); };
     up(b.tris, &d.tris);
     up(b.bvh2, &d.bvh2);
-    up(b.bvh4, &d.bvh4);
+    up(wide.nodes, &d.bvh8);
+    up(wide.tris, &d.tris8);
+    up(wide.boxes, &d.boxes8);
+    d.stack8_cap = wide.depth;
+    if (desc->max_stack_entries > 0 && desc->max_stack_entries < d.stack8_cap) d.stack8_cap = desc->max_stack_entries;
+    d.wide_limit = (float)wide_limit;
     std::vector<TriRecord> by_id;
     if (desc->layout == LMGPU_LAYOUT_NAIVE) {
         by_id.resize(b.tris.size());
@@ -414,22 +455,15 @@ int create_impl(const LmgpuSceneDesc* desc, LmgpuScene** out)
     s->rdev = d;
     if (render_tree) {
         DeviceScene& r = s->rdev;
-        up(b.rtris, &r.tris);
-        up(b.rbvh2, &r.bvh2);
-        up(b.rbvh4, &r.bvh4);
-        r.root_ref = b.rbvh2_root;
-        r.root_ref4 = b.rbvh4_root;
-        std::memcpy(r.root_box, b.rroot_box, sizeof(r.root_box));
-        r.stack_cap = 2 * b.rmax_depth + 4;
-        if (desc->max_stack_entries > 0 && desc->max_stack_entries < r.stack_cap) r.stack_cap = desc->max_stack_entries;
+        up(rwide.nodes, &r.bvh8);
+        up(rwide.tris, &r.tris8);
+        up(rwide.boxes, &r.boxes8);
+        r.stack8_cap = rwide.depth;
+        if (desc->max_stack_entries > 0 && desc->max_stack_entries < r.stack8_cap) r.stack8_cap = desc->max_stack_entries;
+        r.bvh2 = nullptr;              // renders have no use for the reference's walk
+        r.tris = nullptr;
     }
-    // The quantised copy of the binary tree renders traverse (batch layout
-    // LMGPU_LAYOUT_BVH2Q); rays start in the scene's bounds or at the camera.
-    if (desc->layout != LMGPU_LAYOUT_NAIVE && b.num_tris > 0) {
-        const std::vector<Bvh2QNode> qn = quantize_bvh2(render_tree ? b.rbvh2 : b.bvh2, b.bounds,
-                                                        cam.valid ? cam.position : nullptr);
-        up(qn, &s->rdev.bvh2q);
-    }
+    s->rdev.check_boxes = far ? 1 : 0;
     if (rc != LMGPU_OK) { lmgpu_scene_destroy(s); return rc; }
 
     // Scratch: status word and the persistent kernels' work counter.
@@ -443,9 +477,9 @@ int create_impl(const LmgpuSceneDesc* desc, LmgpuScene** out)
     LMGPU_CUDA_TRY(cudaMemset(st, 0, scratch));
 #if LMGPU_BOUNDS_CHECK
     if (desc->layout != LMGPU_LAYOUT_NAIVE) {
-        rc = check_trees(s, s->dev, (int64_t)b.bvh2.size(), (int64_t)b.bvh4.size(), (int64_t)b.tris.size());
+        rc = check_trees(s, s->dev, (int64_t)b.bvh2.size(), (int64_t)wide.nodes.size(), (int64_t)b.tris.size());
         if (rc == LMGPU_OK && render_tree)
-            rc = check_trees(s, s->rdev, (int64_t)b.rbvh2.size(), (int64_t)b.rbvh4.size(), (int64_t)b.rtris.size());
+            rc = check_trees(s, s->rdev, 0, (int64_t)rwide.nodes.size(), (int64_t)rwide.tris.size());
         if (rc != LMGPU_OK) { lmgpu_scene_destroy(s); return rc; }
     }
 #endif
@@ -457,17 +491,12 @@ int create_impl(const LmgpuSceneDesc* desc, LmgpuScene** out)
     info.max_depth = b.max_depth;
     info.layout = desc->layout;
     info.build_seconds = b.build_seconds;
-    // Everything uploaded for traversal: both layouts of each tree (a batch
-    // may pick either), the quantised copy of the render view's binary tree,
-    // and the triangle records.
-    int64_t bytes = 0;
-    bytes += (int64_t)b.tris.size() * sizeof(TriRecord);
-    bytes += (int64_t)b.bvh4.size() * sizeof(Bvh4Node) + (int64_t)b.bvh2.size() * sizeof(Bvh2Node);
-    if (render_tree) {
-        bytes += (int64_t)b.rtris.size() * sizeof(TriRecord);
-        bytes += (int64_t)b.rbvh4.size() * sizeof(Bvh4Node) + (int64_t)b.rbvh2.size() * sizeof(Bvh2Node);
-    }
-    if (s->rdev.bvh2q) bytes += (int64_t)(render_tree ? b.rbvh2 : b.bvh2).size() * sizeof(Bvh2QNode);
+    // Everything uploaded for traversal: the reference's tree (binary and
+    // 8-wide) and the render tree (8-wide), with their triangle records.
+    int64_t bytes = (int64_t)b.tris.size() * sizeof(TriRecord) + (int64_t)b.bvh2.size() * sizeof(Bvh2Node);
+    for (const Bvh8Tree* t : { &wide, &rwide })
+        bytes += (int64_t)t->nodes.size() * sizeof(Bvh8Node) + (int64_t)t->tris.size() * sizeof(TriRecord) +
+                 (int64_t)t->boxes.size() * sizeof(LeafBox);
     info.device_bytes = bytes;
     for (int c = 0; c < 3; c++) { info.bounds_min[c] = b.bounds.mn[c]; info.bounds_max[c] = b.bounds.mx[c]; }
     info.render_tree = render_tree ? LMGPU_RENDER_TREE_SAH : LMGPU_RENDER_TREE_REFERENCE;
@@ -516,7 +545,6 @@ __device__ __forceinline__ void store_hit(const LmgpuHitsSoA& hits, int64_t i, c
 
 // I/O policy of the intersection API: SoA or AoS rays in, hit arrays out.
 struct ApiHitIO {
-    static constexpr int MIN_BLOCKS = LMGPU_TRACE_API_MIN_BLOCKS;
     RaySrc rays;
     int64_t n;
     LmgpuHitsSoA hits;
@@ -535,14 +563,47 @@ struct ApiAnyIO {
     __device__ void store(int64_t i, const Hit& h, const TraversalRay&) const { occluded[i] = h.tri >= 0 ? 1 : 0; }
 };
 
-int launch_intersect(LmgpuScene* sc, const RaySrc& rays, int64_t n, const LmgpuHitsSoA& hits,
-                     cudaStream_t stream, unsigned long long* counters)
+int launch_intersect(LmgpuScene* sc, const RaySrc& rays, int64_t n, const LmgpuHitsSoA& hits, cudaStream_t stream)
 {
     if (n == 0) return LMGPU_OK;
-    if (!counters) return launch_trace<false>(sc, ApiHitIO{ rays, n, hits }, n, stream);
-    // The counting instantiation of the same persistent kernel the path
-    // tracer's measurement renders use.
-    return launch_trace<false, ApiHitIO, true>(sc, ApiHitIO{ rays, n, hits }, n, stream, counters);
+    return launch_trace<false>(sc, ApiHitIO{ rays, n, hits }, n, stream);
+}
+
+// The reference's own walk of every ray, one thread each, counting its slab
+// and TriAccel tests (lmgpu_intersect_counted; measurement only).
+template <int STACK>
+__global__ void __launch_bounds__(128) k_intersect_counted(const DeviceScene s, const ApiHitIO io, int32_t* status,
+                                                           unsigned long long* counts)
+{
+    int2 stack[STACK];
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    TraceStats st{ 0, 0 };
+    if (i < io.n) {
+        TraversalRay r;
+        setup_ray(r, io.load(i));
+        Hit h;
+        if (!trace_bvh2<false>(s.bvh2, s.tris, s.root_ref, s.root_box, r, h, stack, s.stack_cap < STACK ? s.stack_cap : STACK, &st)) {
+            atomicOr(status, STATUS_STACK_OVERFLOW);
+            h.tri = -1;
+        }
+        io.store(i, h, r);
+    }
+    add_trace_stats(st, counts);
+}
+
+int launch_counted(LmgpuScene* sc, const RaySrc& rays, int64_t n, const LmgpuHitsSoA& hits, cudaStream_t stream,
+                   unsigned long long* counters)
+{
+    if (n == 0) return LMGPU_OK;
+    const DeviceScene& s = sc->dev;
+    if (s.layout == LMGPU_LAYOUT_NAIVE || s.num_tris == 0) return fail(LMGPU_ERR_UNSUPPORTED, "traversal counters need a BVH layout");
+    const ApiHitIO io{ rays, n, hits };
+    const unsigned blocks = (unsigned)((n + 127) / 128);
+    if (s.stack_cap <= 64) k_intersect_counted<64><<<blocks, 128, 0, stream>>>(s, io, sc->d_status, counters);
+    else if (s.stack_cap <= 256) k_intersect_counted<256><<<blocks, 128, 0, stream>>>(s, io, sc->d_status, counters);
+    else return fail(LMGPU_ERR_UNSUPPORTED, "BVH deeper than the largest compiled traversal stack (256)");
+    LMGPU_CUDA_TRY(cudaGetLastError());
+    return LMGPU_OK;
 }
 
 // Exposed for the measurement path (traversal counters).
@@ -719,7 +780,7 @@ int intersect_host_staged(LmgpuScene* scene, const float* rays_aos, int64_t n, v
         rs.aos = reinterpret_cast<const float4*>(hp.rays[k]);
         float* dh = hp.hits[k];
         LmgpuHitsSoA H{ reinterpret_cast<int32_t*>(dh), dh + chunk, dh + 2 * chunk, dh + 3 * chunk };
-        rc = launch_intersect(scene, rs, m, H, st, nullptr);
+        rc = launch_intersect(scene, rs, m, H, st);
         if (rc != LMGPU_OK) break;
         for (int a = 0; a < 4 && rc == LMGPU_OK; a++) {
             if (!outs[a]) continue;
@@ -798,7 +859,7 @@ int lmgpu_intersect(LmgpuScene* scene, const LmgpuRaysSoA* rays, int64_t n, Lmgp
     if (const int rc = check_scene_device(scene)) return rc;
     if (n > 0 && (!rays->ox || !rays->oy || !rays->oz || !rays->dx || !rays->dy || !rays->dz || !rays->tmin || !rays->tmax))
         return fail(LMGPU_ERR_INVALID, "null ray array");
-    return launch_intersect(scene, soa_src(*rays), n, *hits, static_cast<cudaStream_t>(stream), nullptr);
+    return launch_intersect(scene, soa_src(*rays), n, *hits, static_cast<cudaStream_t>(stream));
 }
 
 int lmgpu_occluded(LmgpuScene* scene, const LmgpuRaysSoA* rays, int64_t n, uint8_t* occluded, void* stream)
@@ -843,7 +904,7 @@ int lmgpu_intersect_host(LmgpuScene* scene, const float* rays_aos, int64_t n, in
         std::memset(&src, 0, sizeof(src));
         src.aos = reinterpret_cast<const float4*>(dr);
         LmgpuHitsSoA H{ reinterpret_cast<int32_t*>(dh), dh + chunk, dh + 2 * chunk, dh + 3 * chunk };
-        rc = launch_intersect(scene, src, m, H, st, nullptr);
+        rc = launch_intersect(scene, src, m, H, st);
         if (rc != LMGPU_OK) break;
         for (int a = 0; a < 4 && rc == LMGPU_OK; a++) {
             if (!outs[a]) continue;
@@ -866,7 +927,7 @@ int lmgpu_intersect_counted(LmgpuScene* scene, const LmgpuRaysSoA* rays, int64_t
 {
     if (!scene || !rays || !hits || !counters_device || n < 0) return fail(LMGPU_ERR_INVALID, "null argument");
     if (const int rc = check_scene_device(scene)) return rc;
-    return launch_intersect(scene, soa_src(*rays), n, *hits, static_cast<cudaStream_t>(stream), counters_device);
+    return launch_counted(scene, soa_src(*rays), n, *hits, static_cast<cudaStream_t>(stream), counters_device);
 }
 
 // Host-only build (no device work): info and, optionally, the leaf triangle
@@ -894,9 +955,7 @@ int lmgpu_scene_build_host(const LmgpuSceneDesc* desc, LmgpuSceneInfo* info, int
     info->max_depth = b.max_depth;
     info->layout = desc->layout;
     info->build_seconds = b.build_seconds;
-    info->device_bytes = (int64_t)b.tris.size() * sizeof(TriRecord) +
-                         (desc->layout == LMGPU_LAYOUT_BVH4 ? (int64_t)b.bvh4.size() * sizeof(Bvh4Node)
-                                                            : (int64_t)b.bvh2.size() * sizeof(Bvh2Node));
+    info->device_bytes = (int64_t)b.tris.size() * sizeof(TriRecord) + (int64_t)b.bvh2.size() * sizeof(Bvh2Node);
     for (int c = 0; c < 3; c++) { info->bounds_min[c] = b.bounds.mn[c]; info->bounds_max[c] = b.bounds.mx[c]; }
     // The render tree, as lmgpu_scene_create builds it.
     if (desc->layout != LMGPU_LAYOUT_NAIVE && desc->render_tree == LMGPU_RENDER_TREE_SAH && b.num_tris > 0) {

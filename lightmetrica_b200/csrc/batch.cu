@@ -56,13 +56,13 @@ constexpr int STREAM_CHECK_EVERY = 8;      // graph launches between checks of t
 constexpr int NSTATS = 4;
 
 struct GraphKey {
-    int tech = -1, fp64 = -1, layout = -1, stack = -1, bounces = -1, bounded = -1, shade_blocks = -1, mode = -1;
+    int tech = -1, fp64 = -1, stack = -1, bounces = -1, bounded = -1, shade_blocks = -1, mode = -1;
     int split = -1;
     int64_t paths = -1;
     int num_scenes = -1;
     bool operator==(const GraphKey& o) const
     {
-        return tech == o.tech && fp64 == o.fp64 && layout == o.layout && stack == o.stack && bounces == o.bounces &&
+        return tech == o.tech && fp64 == o.fp64 && stack == o.stack && bounces == o.bounces &&
                bounded == o.bounded && shade_blocks == o.shade_blocks && paths == o.paths && num_scenes == o.num_scenes &&
                mode == o.mode && split == o.split;
     }
@@ -153,14 +153,6 @@ __global__ void k_batch_setup(WaveCtl* wave, int pools, int64_t total, int64_t s
     for (int i = 0; i < NSTATS; i++) stats[i] = 0;
 }
 
-// Start of a wave: clear the queue counters and this wave's traversal work
-// counters.
-__global__ void k_wave_begin(uint32_t* counters, unsigned long long* work, int slots)
-{
-    for (int i = threadIdx.x; i < slots; i += blockDim.x) work[i] = 0;
-    if (threadIdx.x < 4) counters[threadIdx.x] = 0;
-}
-
 // Before bounce k: tally the rays about to be traced and the shadow rays of
 // the previous pass, then clear the output queue and the shadow queue. The
 // totals are shared by the path pools (atomics: pools run concurrently).
@@ -234,23 +226,16 @@ __global__ void k_stream_plan(StreamCtl* ctl, uint32_t* counters, int q, unsigne
 
 // ------------------------------------------------------- wave builder ----
 
-// Kernel layout of each walk: LMGPU_LAYOUT_BVH2_QSHADOW traces bounce rays
-// through the float binary nodes and shadow rays through the quantised ones.
-constexpr int walk_layout(int layout, bool any_hit)
-{
-    return layout == LMGPU_LAYOUT_BVH2_QSHADOW ? (any_hit ? LMGPU_LAYOUT_BVH2Q : LMGPU_LAYOUT_BVH2) : layout;
-}
-
 // Launches one persistent traversal of `io`. During a measurement render
 // (b->prof) the launch is bracketed by CUDA events and, when counting, runs
 // the counting instantiation of the same kernel.
-template <int LAYOUT, int STACK, bool ANY_HIT, class IO>
+template <int STACK, bool ANY_HIT, class IO>
 void launch_traversal(const LmgpuBatch* b, int blocks, const DeviceScene& proto, const IO& io,
                       unsigned long long* work, cudaStream_t s)
 {
     TraceProfileRun* p = b->prof;
     if (!p) {
-        k_trace_persistent<walk_layout(LAYOUT, ANY_HIT), STACK, ANY_HIT, IO><<<blocks, 128, 0, s>>>(proto, io, b->d_status, work, nullptr);
+        k_trace_persistent<STACK, ANY_HIT, IO><<<blocks, 128, 0, s>>>(proto, io, b->d_status, work, nullptr);
         return;
     }
     cudaEvent_t e[2] = { nullptr, nullptr };
@@ -258,10 +243,10 @@ void launch_traversal(const LmgpuBatch* b, int blocks, const DeviceScene& proto,
         if (p->error == cudaSuccess) p->error = cudaEventCreate(&x);
     if (p->error == cudaSuccess) p->error = cudaEventRecord(e[0], s);
     if (p->count)
-        k_trace_persistent<walk_layout(LAYOUT, ANY_HIT), STACK, ANY_HIT, IO, true><<<blocks, 128, 0, s>>>(
+        k_trace_persistent<STACK, ANY_HIT, IO, true><<<blocks, 128, 0, s>>>(
             proto, io, b->d_status, work, p->d_counts + (ANY_HIT ? 2 : 0));
     else
-        k_trace_persistent<walk_layout(LAYOUT, ANY_HIT), STACK, ANY_HIT, IO><<<blocks, 128, 0, s>>>(proto, io, b->d_status, work, nullptr);
+        k_trace_persistent<STACK, ANY_HIT, IO><<<blocks, 128, 0, s>>>(proto, io, b->d_status, work, nullptr);
     if (p->error == cudaSuccess) p->error = cudaEventRecord(e[1], s);
     for (cudaEvent_t x : e)
         if (x) p->events.push_back(x);
@@ -279,7 +264,7 @@ struct Launch {
 // One wave of path pool l: head = begin, init, camera shadow pass, bounces
 // 1 .. T-1; tail = bounces T .. K, splat, advance. The traversal launches of
 // bounce k use work slots slot_of(k) and slot_of(k) + 1 of the pool.
-template <int TECH, class F, int LAYOUT, int STACK>
+template <int TECH, class F, int STACK>
 struct Wave {
     using Ctx = SceneTable<float>;     // init / shade use no film
     using FilmCtx = SceneTable<F>;
@@ -299,7 +284,7 @@ struct Wave {
     {
         const PathState& st = b->st[l];
         ShadowIO<FilmCtx> io{ st.counters + 2, st.sh_o, st.sh_d, st.sh_c, st.L, film_ctx(b, l) };
-        launch_traversal<LAYOUT, STACK, true>(b, L.shadow_blocks, L.proto, io, work(b, l) + slot, s);
+        launch_traversal<STACK, true>(b, L.shadow_blocks, L.proto, io, work(b, l) + slot, s);
     }
 
     static void bounce(const LmgpuBatch* b, const Launch& L, int l, int k, int slot, cudaStream_t s)
@@ -308,7 +293,7 @@ struct Wave {
         const int qin = (k - 1) & 1;
         k_bounce_prep<<<1, 1, 0, s>>>(st.counters, qin, k, b->d_stats);
         PathRayIO<true> io{ st.counters + qin, st.qo[qin], st.qd[qin], st.hit, b->d_table };
-        launch_traversal<LAYOUT, STACK, false>(b, L.trace_blocks, L.proto, io, work(b, l) + slot, s);
+        launch_traversal<STACK, false>(b, L.trace_blocks, L.proto, io, work(b, l) + slot, s);
         k_pt_shade<TECH, Ctx><<<L.shade_blocks, 128, 0, s>>>(ctx(b, l), st, k, qin, 1 - qin);
         if (TECH != LMGPU_RENDER_PT) shadow(b, L, l, slot + 1, s);
     }
@@ -343,12 +328,12 @@ struct Wave {
 
     static void warm(Launch& L)
     {
-        L.trace_blocks = resident_blocks(k_trace_persistent<walk_layout(LAYOUT, false), STACK, false, PathRayIO<true>>);
-        L.shadow_blocks = resident_blocks(k_trace_persistent<walk_layout(LAYOUT, true), STACK, true, ShadowIO<FilmCtx>>);
+        L.trace_blocks = resident_blocks(k_trace_persistent<STACK, false, PathRayIO<true>>);
+        L.shadow_blocks = resident_blocks(k_trace_persistent<STACK, true, ShadowIO<FilmCtx>>);
     }
 };
 
-template <int TECH, class F, int LAYOUT, int STACK>
+template <int TECH, class F, int STACK>
 struct Stream {
     using Ctx = StreamTable<float>;    // init / shade use no film
     using FilmCtx = StreamTable<F>;
@@ -367,11 +352,11 @@ struct Stream {
         k_stream_plan<<<1, 1, 0, s>>>(b->d_ctl, st.counters, q, b->d_stats, work);
         k_pt_init<TECH, Ctx><<<(unsigned)((L.paths + 127) / 128), 128, 0, s>>>(make<Ctx>(b), st, 0, q);
         PathRayIO<true> io{ st.counters + q, st.qo[q], st.qd[q], st.hit, b->d_table };
-        launch_traversal<LAYOUT, STACK, false>(b, L.trace_blocks, L.proto, io, work, s);
+        launch_traversal<STACK, false>(b, L.trace_blocks, L.proto, io, work, s);
         k_pt_shade<TECH, Ctx><<<L.shade_blocks, 128, 0, s>>>(make<Ctx>(b), st, 0, q, 1 - q);
         if (TECH != LMGPU_RENDER_PT) {
             ShadowIO<FilmCtx> sio{ st.counters + 2, st.sh_o, st.sh_d, st.sh_c, st.L, make<FilmCtx>(b) };
-            launch_traversal<LAYOUT, STACK, true>(b, L.shadow_blocks, L.proto, sio, work + 1, s);
+            launch_traversal<STACK, true>(b, L.shadow_blocks, L.proto, sio, work + 1, s);
         }
         k_pt_retire<FilmCtx><<<L.shade_blocks, 128, 0, s>>>(make<FilmCtx>(b), st);
     }
@@ -384,8 +369,8 @@ struct Stream {
 
     static void warm(Launch& L)
     {
-        L.trace_blocks = resident_blocks(k_trace_persistent<walk_layout(LAYOUT, false), STACK, false, PathRayIO<true>>);
-        L.shadow_blocks = resident_blocks(k_trace_persistent<walk_layout(LAYOUT, true), STACK, true, ShadowIO<FilmCtx>>);
+        L.trace_blocks = resident_blocks(k_trace_persistent<STACK, false, PathRayIO<true>>);
+        L.shadow_blocks = resident_blocks(k_trace_persistent<STACK, true, ShadowIO<FilmCtx>>);
     }
 };
 
@@ -507,7 +492,7 @@ int make_plan(LmgpuBatch* b, const LmgpuRenderParams* params, void* const* films
         pl.total += p.num_samples;
         if (p.max_path_vertices == -1) pl.bounded = false;
         else max_pv = std::max(max_pv, p.max_path_vertices);
-        cap = std::max(cap, sc->rdev.stack_cap);
+        cap = std::max(cap, sc->rdev.stack8_cap);
     }
     if (pl.total >= (int64_t(1) << 62)) return fail(LMGPU_ERR_INVALID, "sample count too large");
     pl.bounces = pl.bounded ? max_pv - 1 : GRAPH_BOUNCES_UNBOUNDED;
@@ -515,8 +500,7 @@ int make_plan(LmgpuBatch* b, const LmgpuRenderParams* params, void* const* films
         pl.bounded = false;
         pl.bounces = GRAPH_BOUNCES_UNBOUNDED;
     }
-    if (cap <= 64) pl.stack = 64;
-    else if (cap <= 128) pl.stack = 128;
+    if (cap <= 32) pl.stack = 32;
     else if (cap <= 256) pl.stack = 256;
     else return fail(LMGPU_ERR_UNSUPPORTED, "BVH deeper than the largest compiled traversal stack (256)");
     return LMGPU_OK;
@@ -532,7 +516,6 @@ int upload_table(LmgpuBatch* b, const LmgpuRenderParams* params, void* const* fi
         const LmgpuRenderParams& p = params[i];
         BatchEntry& e = b->h_table[i];
         e.s = b->scenes[i]->rdev;
-        e.s.layout = b->cfg.layout;
         e.rc.technique = p.technique;
         e.rc.rr_depth = p.rr_depth;
         e.rc.max_pv = p.max_path_vertices;
@@ -555,23 +538,22 @@ int upload_table(LmgpuBatch* b, const LmgpuRenderParams* params, void* const* fi
 
 // Stream mode: `iterations` returns the iterations run (including at most
 // 2 * STREAM_CHECK_EVERY - 1 empty ones after the last path retired).
-template <int TECH, class F, int LAYOUT, int STACK>
+template <int TECH, class F, int STACK>
 int run_stream(LmgpuBatch* b, const Plan& pl, int64_t P, cudaStream_t s, int64_t& iterations)
 {
-    using S = Stream<TECH, F, LAYOUT, STACK>;
+    using S = Stream<TECH, F, STACK>;
     Launch L;
     L.paths = P;
     L.shade_blocks = std::max(1, b->cfg.shade_blocks_per_sm) * b->sms;
     L.proto = b->scenes[0]->rdev;
-    L.proto.layout = LAYOUT;
-    L.proto.stack_cap = STACK;        // every scene of the batch: the largest bound
+    L.proto.stack8_cap = STACK;       // every scene of the batch: the largest bound
     S::warm(L);
     const unsigned setup_blocks = (unsigned)std::min<int64_t>((P + 255) / 256, 148 * 16);
     k_stream_setup<<<setup_blocks, 256, 0, s>>>(b->d_ctl, pl.total, P, b->st[0].free_slots, b->st[0].counters, b->d_stats);
     LMGPU_CUDA_TRY(cudaGetLastError());
     if (b->cfg.use_graph) {
         GraphKey key;
-        key.tech = TECH; key.fp64 = pl.fp64; key.layout = LAYOUT; key.stack = STACK; key.bounces = 0;
+        key.tech = TECH; key.fp64 = pl.fp64; key.stack = STACK; key.bounces = 0;
         key.bounded = 0; key.shade_blocks = L.shade_blocks; key.paths = P; key.num_scenes = (int)b->scenes.size();
         key.mode = LMGPU_BATCH_STREAM;
         if (!b->exec || !(b->key == key)) {
@@ -616,16 +598,15 @@ int run_stream(LmgpuBatch* b, const Plan& pl, int64_t P, cudaStream_t s, int64_t
 // after them; floor(W / 2) periods cover W waves (a wave past the last
 // sample has no paths and costs only its launches). Depth must be
 // bounded: the tail is a fixed sequence of bounces.
-template <int TECH, class F, int LAYOUT, int STACK>
+template <int TECH, class F, int STACK>
 int run_overlap(LmgpuBatch* b, const Plan& pl, int64_t P, cudaStream_t s, int64_t& waves)
 {
-    using W = Wave<TECH, F, LAYOUT, STACK>;
+    using W = Wave<TECH, F, STACK>;
     Launch L;
     L.paths = P;
     L.shade_blocks = std::max(1, b->cfg.shade_blocks_per_sm) * b->sms;
     L.proto = b->scenes[0]->rdev;
-    L.proto.layout = LAYOUT;
-    L.proto.stack_cap = STACK;        // every scene of the batch: the largest bound
+    L.proto.stack8_cap = STACK;       // every scene of the batch: the largest bound
     W::warm(L);
     const int K = pl.bounces;
     const int T = std::min(b->cfg.overlap_bounce > 0 ? b->cfg.overlap_bounce : DEFAULT_OVERLAP_BOUNCE, K + 1);
@@ -661,7 +642,7 @@ int run_overlap(LmgpuBatch* b, const Plan& pl, int64_t P, cudaStream_t s, int64_
     };
     if (b->cfg.use_graph) {
         GraphKey key;
-        key.tech = TECH; key.fp64 = pl.fp64; key.layout = LAYOUT; key.stack = STACK; key.bounces = K;
+        key.tech = TECH; key.fp64 = pl.fp64; key.stack = STACK; key.bounces = K;
         key.bounded = 1; key.shade_blocks = L.shade_blocks; key.paths = P; key.num_scenes = (int)b->scenes.size();
         key.mode = LMGPU_BATCH_OVERLAP; key.split = T;
         if (!b->exec || !b->exec_head || !b->exec_tail || !(b->key == key)) {
@@ -697,18 +678,17 @@ int run_overlap(LmgpuBatch* b, const Plan& pl, int64_t P, cudaStream_t s, int64_
     return LMGPU_OK;
 }
 
-template <int TECH, class F, int LAYOUT, int STACK>
+template <int TECH, class F, int STACK>
 int run_waves(LmgpuBatch* b, const Plan& pl, int64_t P, cudaStream_t s, int64_t& waves)
 {
-    if (b->cfg.mode == LMGPU_BATCH_STREAM) return run_stream<TECH, F, LAYOUT, STACK>(b, pl, P, s, waves);
-    if (b->cfg.mode == LMGPU_BATCH_OVERLAP && pl.bounded) return run_overlap<TECH, F, LAYOUT, STACK>(b, pl, P, s, waves);
-    using W = Wave<TECH, F, LAYOUT, STACK>;
+    if (b->cfg.mode == LMGPU_BATCH_STREAM) return run_stream<TECH, F, STACK>(b, pl, P, s, waves);
+    if (b->cfg.mode == LMGPU_BATCH_OVERLAP && pl.bounded) return run_overlap<TECH, F, STACK>(b, pl, P, s, waves);
+    using W = Wave<TECH, F, STACK>;
     Launch L;
     L.paths = P;
     L.shade_blocks = std::max(1, b->cfg.shade_blocks_per_sm) * b->sms;
     L.proto = b->scenes[0]->rdev;
-    L.proto.layout = LAYOUT;
-    L.proto.stack_cap = STACK;        // every scene of the batch: the largest bound
+    L.proto.stack8_cap = STACK;       // every scene of the batch: the largest bound
     W::warm(L);
     waves = (pl.total + P - 1) / P;
     k_batch_setup<<<1, 1, 0, s>>>(b->d_wave, 1, pl.total, P, b->d_stats);
@@ -716,7 +696,7 @@ int run_waves(LmgpuBatch* b, const Plan& pl, int64_t P, cudaStream_t s, int64_t&
 
     if (b->cfg.use_graph) {
         GraphKey key;
-        key.tech = TECH; key.fp64 = pl.fp64; key.layout = LAYOUT; key.stack = STACK; key.bounces = pl.bounces;
+        key.tech = TECH; key.fp64 = pl.fp64; key.stack = STACK; key.bounces = pl.bounces;
         key.bounded = pl.bounded; key.shade_blocks = L.shade_blocks; key.paths = P; key.num_scenes = (int)b->scenes.size();
         key.mode = LMGPU_BATCH_WAVES;
         if (!b->exec || !(b->key == key)) {
@@ -749,34 +729,20 @@ int run_waves(LmgpuBatch* b, const Plan& pl, int64_t P, cudaStream_t s, int64_t&
     return LMGPU_OK;
 }
 
-template <int TECH, class F, int LAYOUT>
+template <int TECH, class F>
 int dispatch_stack(LmgpuBatch* b, const Plan& pl, int64_t P, cudaStream_t s, int64_t& waves)
 {
-    switch (pl.stack) {
-    case 64: return run_waves<TECH, F, LAYOUT, 64>(b, pl, P, s, waves);
-    case 128: return run_waves<TECH, F, LAYOUT, 128>(b, pl, P, s, waves);
-    default: return run_waves<TECH, F, LAYOUT, 256>(b, pl, P, s, waves);
-    }
-}
-
-template <int TECH, class F>
-int dispatch_layout(LmgpuBatch* b, const Plan& pl, int64_t P, cudaStream_t s, int64_t& waves)
-{
-    switch (b->cfg.layout) {
-    case LMGPU_LAYOUT_BVH4: return dispatch_stack<TECH, F, LMGPU_LAYOUT_BVH4>(b, pl, P, s, waves);
-    case LMGPU_LAYOUT_BVH2Q: return dispatch_stack<TECH, F, LMGPU_LAYOUT_BVH2Q>(b, pl, P, s, waves);
-    case LMGPU_LAYOUT_BVH2_QSHADOW: return dispatch_stack<TECH, F, LMGPU_LAYOUT_BVH2_QSHADOW>(b, pl, P, s, waves);
-    default: return dispatch_stack<TECH, F, LMGPU_LAYOUT_BVH2>(b, pl, P, s, waves);
-    }
+    if (pl.stack == 32) return run_waves<TECH, F, 32>(b, pl, P, s, waves);
+    return run_waves<TECH, F, 256>(b, pl, P, s, waves);
 }
 
 template <class F>
 int dispatch_tech(LmgpuBatch* b, const Plan& pl, int64_t P, cudaStream_t s, int64_t& waves)
 {
     switch (pl.tech) {
-    case LMGPU_RENDER_PT: return dispatch_layout<LMGPU_RENDER_PT, F>(b, pl, P, s, waves);
-    case LMGPU_RENDER_PT_DIRECT: return dispatch_layout<LMGPU_RENDER_PT_DIRECT, F>(b, pl, P, s, waves);
-    default: return dispatch_layout<LMGPU_RENDER_PT_MIS, F>(b, pl, P, s, waves);
+    case LMGPU_RENDER_PT: return dispatch_stack<LMGPU_RENDER_PT, F>(b, pl, P, s, waves);
+    case LMGPU_RENDER_PT_DIRECT: return dispatch_stack<LMGPU_RENDER_PT_DIRECT, F>(b, pl, P, s, waves);
+    default: return dispatch_stack<LMGPU_RENDER_PT_MIS, F>(b, pl, P, s, waves);
     }
 }
 
@@ -1132,7 +1098,7 @@ int lmgpu_batch_autotune(LmgpuBatch* b, const LmgpuRenderParams* params, double 
     best.use_graph = 1;
     double best_t = 1e30;
     rc = trial(best, best_t);
-    // Coordinate descent: mode, layout, then paths in flight, shading grid
+    // Coordinate descent: mode, then paths in flight, shading grid
     // and (overlap mode) the first tail bounce.
     for (int m : { LMGPU_BATCH_WAVES, LMGPU_BATCH_STREAM, LMGPU_BATCH_OVERLAP }) {
         if (rc != LMGPU_OK || m == best.mode) continue;
@@ -1141,16 +1107,8 @@ int lmgpu_batch_autotune(LmgpuBatch* b, const LmgpuRenderParams* params, double 
         double t;
         if ((rc = trial(c, t)) == LMGPU_OK && better(t, best_t)) { best = c; best_t = t; }
     }
-    const int layouts[] = { LMGPU_LAYOUT_BVH2, LMGPU_LAYOUT_BVH4, LMGPU_LAYOUT_BVH2Q, LMGPU_LAYOUT_BVH2_QSHADOW };
     const int waves[] = { 1 << 21, 1 << 22, 1 << 23, 1 << 24, 1 << 25, 1 << 26, 1 << 27 };
     const int grids[] = { 4, 8, 16 };
-    for (int l : layouts) {
-        if (rc != LMGPU_OK || l == best.layout) continue;
-        LmgpuBatchConfig c = best;
-        c.layout = l;
-        double t;
-        if ((rc = trial(c, t)) == LMGPU_OK && better(t, best_t)) { best = c; best_t = t; }
-    }
     int64_t largest = 0;
     for (int w : waves) {
         // Waves beyond the sample count behave like a wave of the sample count.

@@ -17,8 +17,11 @@
 #include <cmath>
 #include <cfloat>
 #include <cstring>
+#include <exception>
 #include <functional>
 #include <limits>
+#include <mutex>
+#include <system_error>
 #include <thread>
 
 namespace lmgpu {
@@ -239,48 +242,6 @@ int32_t flatten_bvh2(const std::vector<BuildNode>& nodes, int32_t ni, std::vecto
     return id;
 }
 
-// 4-wide collapse: each 4-node holds the (up to) four grandchildren of a
-// binary internal node; a binary child that is a leaf occupies its slot pair
-// alone.
-int32_t flatten_bvh4(const std::vector<BuildNode>& nodes, int32_t ni, std::vector<Bvh4Node>& out)
-{
-    const BuildNode& n = nodes[ni];
-    if (n.leaf) return ~n.begin;
-    const int32_t id = static_cast<int32_t>(out.size());
-    out.emplace_back();
-    int32_t slot_node[4] = { -1, -1, -1, -1 };
-    int32_t axis_pair[2] = { -1, -1 };
-    const int32_t kids[2] = { n.left, n.right };
-    for (int p = 0; p < 2; p++) {
-        const BuildNode& c = nodes[kids[p]];
-        if (c.leaf) { slot_node[2 * p] = kids[p]; }
-        else { slot_node[2 * p] = c.left; slot_node[2 * p + 1] = c.right; axis_pair[p] = c.axis; }
-    }
-    {
-        Bvh4Node& o = out[id];
-        for (int k = 0; k < 4; k++) {
-            if (slot_node[k] < 0) {
-                // Empty slot: a box no ray can enter (lo > hi on every axis).
-                o.lox[k] = o.loy[k] = o.loz[k] = FLT_MAX;
-                o.hix[k] = o.hiy[k] = o.hiz[k] = -FLT_MAX;
-                o.child[k] = BVH4_EMPTY;
-                continue;
-            }
-            const HostAabb& b = nodes[slot_node[k]].bound;
-            o.lox[k] = b.mn[0]; o.hix[k] = b.mx[0];
-            o.loy[k] = b.mn[1]; o.hiy[k] = b.mx[1];
-            o.loz[k] = b.mn[2]; o.hiz[k] = b.mx[2];
-        }
-        o.axis_top = n.axis;
-        o.axis_l = axis_pair[0];
-        o.axis_r = axis_pair[1];
-        o.pad = 0;
-    }
-    for (int k = 0; k < 4; k++)
-        if (slot_node[k] >= 0) out[id].child[k] = flatten_bvh4(nodes, slot_node[k], out);
-    return id;
-}
-
 // ------------------------------------------------------------ render tree
 
 // Render tree: binned SAH over all three axes (the reference bins only the
@@ -405,49 +366,435 @@ struct RenderBuilder {
 
 }  // namespace
 
-std::vector<Bvh2QNode> quantize_bvh2(const std::vector<Bvh2Node>& nodes, const HostAabb& bounds,
-                                     const float* extra)
+// ------------------------------------------------------- 8-wide collapse
+
+namespace {
+
+// Cost model of the collapse: a wide node's visit costs 1, a triangle test
+// BVH8_TRI_COST, weighted by surface area. A triangle test runs with few lanes
+// active (about 6 of 32, against 22 in a node visit), which makes it as dear as a
+// visit: 0.3, 0.6 and 1.0 gave 1.82, 1.65 and 1.60 ms for 2^23 random rays through a
+// 1,048,576-triangle soup, 1.51, 1.48 and 1.47 ms for 5.3 M shadow rays of a
+// 3.4 M-triangle terrain. Leaves of more than BVH8_MAX_LEAF triangles are not formed
+// by merging (6: slower on both).
+constexpr float BVH8_TRI_COST = 1.0f;
+constexpr int BVH8_MAX_LEAF = 3;
+
+struct Box {
+    float lo[3], hi[3];
+};
+inline float half_area(const Box& b)
 {
-    double M = 0.0;
-    for (int c = 0; c < 3; c++) {
-        M = std::max(M, (double)std::fabs(bounds.mn[c]));
-        M = std::max(M, (double)std::fabs(bounds.mx[c]));
-        if (extra) M = std::max(M, (double)std::fabs(extra[c]));
+    const float dx = b.hi[0] - b.lo[0], dy = b.hi[1] - b.lo[1], dz = b.hi[2] - b.lo[2];
+    return dx * dy + dy * dz + dz * dx;
+}
+inline void box_join(Box& a, const Box& b)
+{
+    for (int k = 0; k < 3; k++) { a.lo[k] = std::min(a.lo[k], b.lo[k]); a.hi[k] = std::max(a.hi[k], b.hi[k]); }
+}
+inline Box box_empty()
+{
+    return Box{ { FLT_MAX, FLT_MAX, FLT_MAX }, { -FLT_MAX, -FLT_MAX, -FLT_MAX } };
+}
+
+// fn(0) .. fn(n - 1) on up to `threads` threads; the first exception is
+// rethrown once all have ended.
+template <class Fn>
+void parallel_for(int threads, size_t n, Fn fn)
+{
+    threads = static_cast<int>(std::min<size_t>((size_t)threads, n));
+    std::atomic<size_t> next{0};
+    std::exception_ptr failed;
+    std::mutex mu;
+    auto work = [&] {
+        try {
+            for (size_t i; (i = next.fetch_add(1)) < n;) fn(i);
+        } catch (...) {
+            std::lock_guard<std::mutex> lock(mu);
+            if (!failed) failed = std::current_exception();
+            next.store(n);
+        }
+    };
+    std::vector<std::thread> pool;
+    pool.reserve((size_t)std::max(threads, 1));
+    try {
+        for (int t = 1; t < threads; t++) pool.emplace_back(work);
+    } catch (const std::system_error&) {
+        // fewer threads than asked for
     }
-    // 16 ulps of the largest magnitude a ray origin or a plane takes
-    const double min_step = 16.0 * (M > 0.0 ? std::ldexp(1.0, std::ilogb(M) - 23) : std::ldexp(1.0, -126));
-    std::vector<Bvh2QNode> out(nodes.size());
-    for (size_t i = 0; i < nodes.size(); i++) {
-        const Bvh2Node& n = nodes[i];
-        const float* ax[3] = { n.bx, n.by, n.bz };
-        Bvh2QNode& o = out[i];
-        uint32_t exps = (uint32_t)(n.axis & 0xff) << 24;
+    work();
+    for (auto& t : pool) t.join();
+    if (failed) std::rethrow_exception(failed);
+}
+
+// How far outside its triangle's bounding box a point that TriAccel::Intersect
+// reports as hit can lie, for ray origins and triangles whose coordinates are at
+// most B and M. With eps = 2^-24 and Wald's projection: the projected point
+// (hu, hv) is off by e0 = 4 eps (B + 4M); the barycentrics by e0 times the row
+// norms of the inverse edge matrix plus the relative error K of its float
+// determinant (large for slivers); each of the three edge tests then lets the
+// point out by that times the longest edge L, and the plane equation adds its own
+// rounding and tilt.
+double triaccel_slack(const float* A, const float* B_, const float* C, double B, double M)
+{
+    const double eps = std::ldexp(1.0, -24);
+    double b[3], c[3], L = 0.0;
+    for (int k = 0; k < 3; k++) {
+        b[k] = (double)C[k] - A[k];
+        c[k] = (double)B_[k] - A[k];
+        L = std::max(L, std::max(std::fabs(b[k]), std::fabs(c[k])));
+    }
+    const double N[3] = { c[1] * b[2] - c[2] * b[1], c[2] * b[0] - c[0] * b[2], c[0] * b[1] - c[1] * b[0] };
+    const double Nk = std::max(std::fabs(N[0]), std::max(std::fabs(N[1]), std::fabs(N[2])));
+    const double base = 32.0 * eps * (B + 4.0 * M);
+    if (!(Nk > 0.0)) return base + 2.0 * M;
+    const double K = 16.0 * eps * L * L / Nk;
+    const double delta = 4.0 * eps * (B + 4.0 * M) * (4.0 * L / Nk) + 4.0 * K + 16.0 * eps;
+    return std::min(base + 9.0 * delta * L + 4.0 * K * L, 4.0 * M + base);
+}
+
+// The dynamic programme of the collapse (Ylitie et al. 2017, section 4.1) over a binary
+// tree in DFS pre-order: cost[n][i - 1] is the least cost of node n's subtree
+// as at most i children of some wide node, i = 1 .. 7.
+struct Collapse {
+    static constexpr int W = 8;
+    const BuiltScene& s;
+    const std::vector<Bvh2Node>& nodes;
+    const std::vector<TriRecord>& tris;
+    double magnitude = 0.0;
+    bool exact = false;
+    std::vector<int32_t> run;            // triangles of the leaf starting at a record
+    std::vector<Box> record_box;         // per record (inflated when exact)
+    std::vector<Box> box;                // per binary node (inflated when exact)
+    std::vector<int32_t> count;          // triangles below
+    std::vector<float> cost;             // W - 1 per node
+    std::vector<uint8_t> split;          // W + 1 per node: slots of the left child when node takes j (0: takes j - 1)
+    std::vector<uint8_t> leaf;           // the node's subtree becomes one leaf
+
+    struct Item {
+        int32_t ref;
+        Box b;
+    };
+
+    Collapse(const BuiltScene& s_, const std::vector<Bvh2Node>& n, const std::vector<TriRecord>& t)
+        : s(s_), nodes(n), tris(t) {}
+
+    Box tri_box(const TriRecord& t) const
+    {
+        const float* p[3];
+        for (int c = 0; c < 3; c++) p[c] = &s.positions[3 * (size_t)s.tri_vidx[3 * (size_t)t.tri_id + c]];
+        Box b;
+        const float e = exact ? (float)(triaccel_slack(p[0], p[1], p[2], magnitude, scene_max) * 1.001) : 0.0f;
         for (int k = 0; k < 3; k++) {
-            const double lo = std::min(ax[k][0], ax[k][2]), hi = std::max(ax[k][1], ax[k][3]);
-            // 65,520 steps cover the box, its two-step margins and the
-            // origin's rounding; a power of two, so q * step is exact.
-            const double need = std::max(min_step, (hi - lo) / 65520.0);
+            b.lo[k] = std::min(p[0][k], std::min(p[1][k], p[2][k])) - e;
+            b.hi[k] = std::max(p[0][k], std::max(p[1][k], p[2][k])) + e;
+        }
+        return b;
+    }
+    Item item(int32_t ref) const
+    {
+        if (ref >= 0) return Item{ ref, box[(size_t)ref] };
+        Item it{ ref, box_empty() };
+        for (size_t i = (size_t)~ref;; i++) {
+            box_join(it.b, record_box[i]);
+            if (tris[i].k_flags & TRI_LAST_IN_LEAF) break;
+        }
+        return it;
+    }
+    // Costs of a child as at most 1 .. 7 children.
+    void costs_of(const Item& it, float* c) const
+    {
+        if (it.ref < 0) std::fill(c, c + (W - 1), half_area(it.b) * (float)run[(size_t)~it.ref] * BVH8_TRI_COST);
+        else std::memcpy(c, &cost[(size_t)it.ref * (W - 1)], (W - 1) * sizeof(float));
+    }
+    void solve(size_t n)
+    {
+        const Item l = item(nodes[n].left), r = item(nodes[n].right);
+        Box u = l.b;
+        box_join(u, r.b);
+        box[n] = u;
+        count[n] = (l.ref < 0 ? run[(size_t)~l.ref] : count[(size_t)l.ref]) + (r.ref < 0 ? run[(size_t)~r.ref] : count[(size_t)r.ref]);
+        const float area = half_area(u);
+        float cl[W - 1], cr[W - 1], dist[W + 1];
+        costs_of(l, cl);
+        costs_of(r, cr);
+        for (int j = 2; j <= W; j++) {
+            float best = cl[0] + cr[j - 2];
+            int at = 1;
+            for (int k = 2; k < j; k++) {
+                const float c = cl[k - 1] + cr[j - k - 1];
+                if (c < best) { best = c; at = k; }
+            }
+            dist[j] = best;
+            split[n * (W + 1) + (size_t)j] = (uint8_t)at;
+        }
+        const float inner = area + dist[W];
+        const float as_leaf = count[n] <= BVH8_MAX_LEAF ? area * (float)count[n] * BVH8_TRI_COST : FLT_MAX;
+        leaf[n] = as_leaf <= inner;
+        float* c = &cost[n * (W - 1)];
+        c[0] = std::min(as_leaf, inner);
+        for (int j = 2; j < W; j++) {
+            if (dist[j] < c[j - 2]) c[j - 1] = dist[j];
+            else { c[j - 1] = c[j - 2]; split[n * (W + 1) + (size_t)j] = 0; }
+        }
+    }
+    // Children of a wide node that give binary subtree `it` j slots.
+    void gather(const Item& it, int j, Item* out, int& n) const
+    {
+        if (it.ref < 0) { out[n++] = it; return; }
+        const uint8_t* sp = &split[(size_t)it.ref * (W + 1)];
+        j = std::min(j, W - 1);
+        while (j > 1 && sp[j] == 0) j--;
+        if (j == 1) { out[n++] = it; return; }
+        gather(item(nodes[(size_t)it.ref].left), sp[j], out, n);
+        gather(item(nodes[(size_t)it.ref].right), j - sp[j], out, n);
+    }
+    bool is_leaf(const Item& it) const { return it.ref < 0 || leaf[(size_t)it.ref]; }
+    void emit_tris(int32_t ref, std::vector<TriRecord>& out) const
+    {
+        if (ref >= 0) { emit_tris(nodes[(size_t)ref].left, out); emit_tris(nodes[(size_t)ref].right, out); return; }
+        for (size_t i = (size_t)~ref;; i++) {
+            out.push_back(tris[i]);
+            out.back().k_flags &= ~TRI_LAST_IN_LEAF;
+            if (tris[i].k_flags & TRI_LAST_IN_LEAF) return;
+        }
+    }
+    double scene_max = 0.0;
+
+    // Writes the wide node of binary subtree `ref` to `node`, its leaves to `out_tris`, and
+    // returns its internal children in slot order. Indices are relative to
+    // the lists' present sizes.
+    struct Made {
+        int32_t ref[W];
+        int n = 0;
+    };
+    Made make(const Item* in, int n, Bvh8Node& node, std::vector<TriRecord>& out_tris, uint32_t child_base) const
+    {
+        Box u = box_empty();
+        for (int i = 0; i < n; i++) box_join(u, in[i].b);
+        // Greedy assignment of children to octant slots: the best remaining
+        // (child, slot) pair by projection of the child's centre on the slot's diagonal.
+        int slot_of[W], child_in[W];
+        for (int i = 0; i < W; i++) { slot_of[i] = -1; child_in[i] = -1; }
+        float toward[W][W];
+        for (int i = 0; i < n; i++) {
+            float cen[3];
+            for (int k = 0; k < 3; k++) cen[k] = (in[i].b.lo[k] + in[i].b.hi[k]) - (u.lo[k] + u.hi[k]);
+            for (int sl = 0; sl < W; sl++)
+                toward[i][sl] = (sl & 1 ? cen[0] : -cen[0]) + (sl & 2 ? cen[1] : -cen[1]) + (sl & 4 ? cen[2] : -cen[2]);
+        }
+        for (int r = 0; r < n; r++) {
+            float best = -FLT_MAX;
+            int bi = -1, bs = -1;
+            for (int i = 0; i < n; i++) {
+                if (slot_of[i] >= 0) continue;
+                for (int sl = 0; sl < W; sl++) {
+                    if (child_in[sl] >= 0) continue;
+                    if (bi < 0 || toward[i][sl] > best) { best = toward[i][sl]; bi = i; bs = sl; }
+                }
+            }
+            slot_of[bi] = bs;
+            child_in[bs] = bi;
+        }
+        std::memset(&node, 0, sizeof(node));
+        // Grid: steps are powers of two, at least 16 ulps of the largest
+        // magnitude, so that a visit's rounding stays inside the planes' margin.
+        const double top = std::max(magnitude, scene_max);
+        const double ulp = top > 0.0 ? std::ldexp(1.0, std::ilogb(top) - 23) : std::ldexp(1.0, -126);
+        uint8_t q[6][W];
+        uint32_t exps = 0;
+        for (int k = 0; k < 3; k++) {
+            const double extra = 4.0 * ulp;
+            const double need = std::max(16.0 * ulp, ((double)u.hi[k] - u.lo[k] + 2.0 * extra) / 253.0);
             int E = std::ilogb(need);
             if (std::ldexp(1.0, E) < need) E++;
             E = std::min(std::max(E, -126), 127);
-            const double step = std::ldexp(1.0, E);
-            const double od = lo - 2.0 * step;
+            const double step = std::ldexp(1.0, E), inv_step = std::ldexp(1.0, -E);
+            const double m = extra + step / 64.0;
+            const double od = (double)u.lo[k] - m - step / 64.0;
             float of = (float)od;
             if ((double)of > od) of = std::nextafter(of, -std::numeric_limits<float>::infinity());
-            o.origin[k] = of;
-            for (int c = 0; c < 2; c++) {
-                const double clo = ax[k][2 * c], chi = ax[k][2 * c + 1];
-                const double qlo = std::max(0.0, std::floor((clo - (double)of) / step) - 2.0);
-                const double qhi = std::min(65535.0, std::ceil((chi - (double)of) / step) + 2.0);
-                o.q[2 * k + c] = (uint32_t)qlo | ((uint32_t)qhi << 16);
+            node.origin[k] = of;
+            for (int sl = 0; sl < W; sl++) {
+                q[k][sl] = 255;          // an unused slot: lo > hi
+                q[3 + k][sl] = 0;
+                if (child_in[sl] < 0) continue;
+                const Box& b = in[child_in[sl]].b;
+                // (both quotients are in [0, 255]: truncation is the floor)
+                q[k][sl] = (uint8_t)std::min(255.0, std::max(0.0, ((double)b.lo[k] - m - of) * inv_step));
+                const double hi = std::min(255.0, std::max(0.0, ((double)b.hi[k] + m - of) * inv_step));
+                q[3 + k][sl] = (uint8_t)((double)(int)hi < hi ? (int)hi + 1 : (int)hi);
             }
             exps |= (uint32_t)(E + 127) << (8 * k);
         }
-        o.exps = exps;
-        o.left = n.left;
-        o.right = n.right;
+        Made made;
+        uint32_t inner = 0;
+        for (int sl = 0; sl < W; sl++) {
+            if (child_in[sl] < 0) continue;
+            const Item& it = in[child_in[sl]];
+            node.valid |= 1u << sl;
+            if (!is_leaf(it)) {
+                inner |= 1u << sl;
+                made.ref[made.n++] = it.ref;
+            } else {
+                node.start[sl] = (uint32_t)out_tris.size();
+                emit_tris(it.ref, out_tris);
+                out_tris.back().k_flags |= TRI_LAST_IN_LEAF;
+            }
+        }
+        node.exps = exps | inner << 24;
+        node.child_base = child_base;
+        std::memcpy(node.lox, q[0], W); std::memcpy(node.loy, q[1], W); std::memcpy(node.loz, q[2], W);
+        std::memcpy(node.hix, q[3], W); std::memcpy(node.hiy, q[4], W); std::memcpy(node.hiz, q[5], W);
+        return made;
     }
-    return out;
+    Made make_from(int32_t ref, Bvh8Node& node, std::vector<TriRecord>& out_tris, uint32_t child_base) const
+    {
+        Item in[W];
+        int n = 0;
+        const int k = split[(size_t)ref * (W + 1) + W];
+        gather(item(nodes[(size_t)ref].left), k, in, n);
+        gather(item(nodes[(size_t)ref].right), W - k, in, n);
+        return make(in, n, node, out_tris, child_base);
+    }
+    // Depth-first emission below the wide node already made at out.nodes[0].
+    struct Todo {
+        size_t at;
+        int32_t ref;
+        int depth;
+    };
+    void emit(std::vector<Todo> stack, Bvh8Tree& out) const
+    {
+        while (!stack.empty()) {
+            const Todo t = stack.back();
+            stack.pop_back();
+            out.depth = std::max(out.depth, t.depth);
+            Bvh8Node node;
+            const size_t base = out.nodes.size();
+            const Made m = make_from(t.ref, node, out.tris, (uint32_t)base);
+            out.nodes[t.at] = node;
+            out.nodes.resize(base + (size_t)m.n);
+            for (int i = m.n - 1; i >= 0; i--) stack.push_back(Todo{ base + (size_t)i, m.ref[i], t.depth + 1 });
+        }
+    }
+};
+
+}  // namespace
+
+void collapse_bvh8(const BuiltScene& s, const std::vector<Bvh2Node>& nodes, const std::vector<TriRecord>& tris,
+                   int32_t root, const float* root_box, double magnitude, bool exact, bool boxes, int threads,
+                   Bvh8Tree& out)
+{
+    out = Bvh8Tree{};
+    if (tris.empty()) return;
+    if (threads <= 0) threads = static_cast<int>(std::max(1u, std::thread::hardware_concurrency()));
+    Collapse C(s, nodes, tris);
+    C.exact = exact;
+    C.magnitude = magnitude;
+    for (int k = 0; k < 3; k++)
+        C.scene_max = std::max(C.scene_max, std::max((double)std::fabs(s.bounds.mn[k]), (double)std::fabs(s.bounds.mx[k])));
+    if (tris.size() < 8192) threads = 1;
+    C.record_box.resize(tris.size());
+    const size_t chunk = 16384;
+    parallel_for(threads, (tris.size() + chunk - 1) / chunk, [&](size_t t) {
+        for (size_t i = t * chunk; i < std::min(tris.size(), (t + 1) * chunk); i++) C.record_box[i] = C.tri_box(tris[i]);
+    });
+    C.run.assign(tris.size(), 0);
+    for (size_t i = 0, first = 0; i < tris.size(); i++)
+        if (tris[i].k_flags & TRI_LAST_IN_LEAF) { C.run[first] = (int32_t)(i + 1 - first); first = i + 1; }
+    if (root < 0) {                                   // one leaf
+        out.nodes.resize(1);
+        const Collapse::Item it = C.item(root);
+        C.make(&it, 1, out.nodes[0], out.tris, 1);
+        out.depth = 1;
+    } else {
+        const size_t n = nodes.size();
+        C.box.resize(n);
+        C.count.resize(n);
+        C.cost.resize(n * (Collapse::W - 1));
+        C.split.assign(n * (Collapse::W + 1), 0);
+        C.leaf.resize(n);
+        // Pre-order: a subtree is the index range [ref, end). Subtrees of at most
+        // n / 64 nodes are solved in parallel, the nodes above them afterwards.
+        struct Range { size_t at, end; };
+        std::vector<Range> tasks;
+        std::vector<size_t> above;
+        std::vector<Range> open{ Range{ (size_t)root, n } };
+        while (!open.empty()) {
+            const Range r = open.back();
+            open.pop_back();
+            if (r.end - r.at <= std::max<size_t>(n / 64, 1024)) { tasks.push_back(r); continue; }
+            above.push_back(r.at);
+            const int32_t l = nodes[r.at].left, rt = nodes[r.at].right;
+            if (l >= 0) open.push_back(Range{ (size_t)l, rt >= 0 ? (size_t)rt : r.end });
+            if (rt >= 0) open.push_back(Range{ (size_t)rt, r.end });
+        }
+        parallel_for(threads, tasks.size(), [&](size_t t) {
+            for (size_t i = tasks[t].end; i-- > tasks[t].at;) C.solve(i);
+        });
+        std::sort(above.begin(), above.end());
+        for (size_t i = above.size(); i-- > 0;) C.solve(above[i]);
+        // The top of the wide tree breadth first until there are enough subtrees
+        // to share among the threads; each subtree's nodes and triangles then
+        // follow in one block.
+        std::vector<Collapse::Todo> front{ Collapse::Todo{ 0, root, 1 } };
+        out.nodes.resize(1);
+        const size_t want = threads > 1 ? 4 * (size_t)threads : 0;
+        for (size_t head = 0; head < front.size() && front.size() - head < want;) {
+            const Collapse::Todo t = front[head++];
+            Bvh8Node node;
+            const size_t base = out.nodes.size();
+            const Collapse::Made m = C.make_from(t.ref, node, out.tris, (uint32_t)base);
+            out.nodes[t.at] = node;
+            out.nodes.resize(base + (size_t)m.n);
+            out.depth = std::max(out.depth, t.depth);
+            for (int i = 0; i < m.n; i++) front.push_back(Collapse::Todo{ base + (size_t)i, m.ref[i], t.depth + 1 });
+            if (head == front.size() || front.size() - head >= want) {
+                front.erase(front.begin(), front.begin() + (ptrdiff_t)head);
+                break;
+            }
+        }
+        std::vector<Bvh8Tree> part(front.size());
+        parallel_for(threads, front.size(), [&](size_t t) {
+            part[t].nodes.resize(1);
+            C.emit({ Collapse::Todo{ 0, front[t].ref, front[t].depth } }, part[t]);
+        });
+        for (size_t t = 0; t < part.size(); t++) {
+            // Local node 0 is the front node itself; node i > 0 lands at base + i - 1.
+            const uint32_t node_base = (uint32_t)out.nodes.size() - 1, tri_base = (uint32_t)out.tris.size();
+            for (Bvh8Node& x : part[t].nodes) {
+                x.child_base += node_base;
+                for (int sl = 0; sl < Collapse::W; sl++)
+                    if ((x.valid & ~(x.exps >> 24)) >> sl & 1u) x.start[sl] += tri_base;
+            }
+            out.nodes[front[t].at] = part[t].nodes[0];
+            out.nodes.insert(out.nodes.end(), part[t].nodes.begin() + 1, part[t].nodes.end());
+            out.tris.insert(out.tris.end(), part[t].tris.begin(), part[t].tris.end());
+            out.depth = std::max(out.depth, part[t].depth);
+            part[t] = Bvh8Tree{};
+        }
+    }
+    if (!boxes) return;
+    std::vector<LeafBox> by_id(tris.size());
+    auto put = [&](int32_t ref, const float* x, const float* y, const float* z) {
+        LeafBox b{ { x[0], y[0], z[0] }, { x[1], y[1], z[1] }, { 0.0f, 0.0f } };
+        for (size_t i = (size_t)~ref;; i++) {
+            by_id[tris[i].tri_id] = b;
+            if (tris[i].k_flags & TRI_LAST_IN_LEAF) break;
+        }
+    };
+    if (root < 0) {
+        const float x[2] = { root_box[0], root_box[3] }, y[2] = { root_box[1], root_box[4] }, z[2] = { root_box[2], root_box[5] };
+        put(root, x, y, z);
+    }
+    for (const Bvh2Node& n : nodes) {
+        if (n.left < 0) put(n.left, n.bx, n.by, n.bz);
+        if (n.right < 0) put(n.right, n.bx + 2, n.by + 2, n.bz + 2);
+    }
+    out.boxes.resize(tris.size());
+    parallel_for(threads, (tris.size() + chunk - 1) / chunk, [&](size_t t) {
+        for (size_t i = t * chunk; i < std::min(tris.size(), (t + 1) * chunk); i++) out.boxes[i] = by_id[out.tris[i].tri_id];
+    });
 }
 
 void build_render_tree(BuiltScene& s, int threads)
@@ -489,8 +836,6 @@ void build_render_tree(BuiltScene& s, int threads)
     s.rbvh2.clear();
     s.rbvh2.reserve((size_t)std::max<int64_t>(1, ntris));
     s.rbvh2_root = flatten_bvh2(B.pool, root, s.rbvh2);
-    s.rbvh4.clear();
-    s.rbvh4_root = flatten_bvh4(B.pool, root, s.rbvh4);
     const HostAabb& rb = B.pool[root].bound;
     for (int c = 0; c < 3; c++) { s.rroot_box[c] = rb.mn[c]; s.rroot_box[3 + c] = rb.mx[c]; }
     s.rnum_nodes = (int64_t)B.pool.size();
@@ -629,8 +974,6 @@ std::string build_scene(const std::vector<PrimitiveInput>& prims, int threads, b
             if (n.leaf) s.tris[(size_t)(n.end - 1)].k_flags |= TRI_LAST_IN_LEAF;
         s.bvh2.reserve((size_t)std::max<int64_t>(1, ntris));
         s.bvh2_root = flatten_bvh2(s.nodes, s.root, s.bvh2);
-        s.bvh4.reserve((size_t)std::max<int64_t>(1, ntris / 2));
-        s.bvh4_root = flatten_bvh4(s.nodes, s.root, s.bvh4);
         const HostAabb& rb = s.nodes[s.root].bound;
         for (int c = 0; c < 3; c++) { s.root_box[c] = rb.mn[c]; s.root_box[3 + c] = rb.mx[c]; }
         s.max_stack = s.max_depth + 2;

@@ -45,8 +45,6 @@ struct BuiltScene {
     std::vector<Bvh2Node> bvh2;
     int32_t bvh2_root = 0;            // root reference
     float root_box[6] = {0, 0, 0, 0, 0, 0};
-    std::vector<Bvh4Node> bvh4;
-    int32_t bvh4_root = 0;
     int32_t max_stack = 0;            // traversal stack bound for this tree
     double build_seconds = 0.0;
 
@@ -57,8 +55,6 @@ struct BuiltScene {
     std::vector<Bvh2Node> rbvh2;
     int32_t rbvh2_root = 0;
     float rroot_box[6] = {0, 0, 0, 0, 0, 0};
-    std::vector<Bvh4Node> rbvh4;
-    int32_t rbvh4_root = 0;
     int64_t rnum_nodes = 0;
     int64_t rnum_leaves = 0;
     int32_t rmax_depth = 0;
@@ -75,13 +71,25 @@ struct PrimitiveInput {
     const float* transform;   // 16 floats column-major or nullptr
 };
 
-// The quantised copy of a binary tree (same node order and references) for
-// rays that start within `bounds` (or at `extra`, a camera position): the
-// grid step of an axis is a power of two no finer than 16 float ulps of the
-// largest coordinate magnitude, so the decode's rounding stays below the
-// two-step margin around every box.
-std::vector<Bvh2QNode> quantize_bvh2(const std::vector<Bvh2Node>& nodes, const HostAabb& bounds,
-                                     const float* extra);
+// An 8-wide compressed tree, its triangle records in leaf order and, when asked
+// for, the binary leaf's box of every record.
+struct Bvh8Tree {
+    std::vector<Bvh8Node> nodes;      // the root is node 0
+    std::vector<TriRecord> tris;
+    std::vector<LeafBox> boxes;
+    int32_t depth = 0;                // nodes on the longest path from the root
+};
+
+// Collapses the binary tree `nodes` / `tris` (the reference's or the render
+// tree) of a built scene into `out`.
+//   magnitude  largest coordinate magnitude a ray origin takes
+//   exact      the tree serves the reference-exact walk: every box is inflated by
+//              the distance outside its triangle at which TriAccel::Intersect
+//              can still report a hit for rays from within `magnitude`
+//   boxes      also write each record's binary leaf box
+void collapse_bvh8(const BuiltScene& s, const std::vector<Bvh2Node>& nodes, const std::vector<TriRecord>& tris,
+                   int32_t root, const float* root_box, double magnitude, bool exact, bool boxes, int threads,
+                   Bvh8Tree& out);
 
 // Builds everything; returns an empty string on success, else an error.
 std::string build_scene(const std::vector<PrimitiveInput>& prims, int threads, bool want_bvh,

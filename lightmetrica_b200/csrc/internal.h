@@ -69,6 +69,9 @@ int64_t workspace_paths_for_bytes(size_t bytes);
 int render_device_preallocated(LmgpuScene* sc, const LmgpuRenderParams& p, void* film, cudaStream_t stream,
                                void* ws_mem, size_t ws_bytes, uint32_t* host_counts);
 
+// Gives the differentiable passes' pooled workspace memory back (adjoint.cu).
+int release_diff_pool(int device);
+
 // Reads and clears the device status word; maps it to an LMGPU status.
 int consume_status(LmgpuScene* s, cudaStream_t stream);
 // The LMGPU status (and message) of a non-zero device status word.

@@ -1,16 +1,21 @@
 // Device data layout of a built scene, shared by the host builder (g++) and
 // the CUDA kernels (nvcc). Plain structs only.
 //
-// HBM layout of the binary accelerator (LMGPU_LAYOUT_BVH2):
-//   Bvh2Node[num_internal]  64 B each, DFS pre-order, both children's boxes
-//                           stored in the parent so one node fetch (4 x 16 B)
-//                           serves both slab tests of a traversal step.
-//   TriRecord[num_tris]     48 B each, the reference TriAccel constants
-//                           (triaccel.h:31-47) permuted into leaf order
-//                           (bvhTriIndices of scene.bvh.cpp:193); leaves are
-//                           contiguous runs ended by TRI_LAST_IN_LEAF.
-// A child reference >= 0 is an internal node index; < 0 is a leaf whose
-// first TriRecord is ~ref.
+// HBM layout of an accelerator:
+//   Bvh8Node[]   128 B each, the 8-wide compressed collapse of a binary tree
+//                that every traversal walks.
+//   TriRecord[]  48 B each, the reference TriAccel constants
+//                (triaccel.h:31-47) in the wide tree's leaf order; leaves
+//                are contiguous runs ended by TRI_LAST_IN_LEAF.
+//   LeafBox[]    32 B each, the binary leaf's box of every triangle (the
+//                reference's tree; the render tree far from the origin).
+// and, for the reference's own depth-first walk (rays the wide walk hands back,
+// work counts, full hit records):
+//   Bvh2Node[]   64 B each, DFS pre-order, both children's boxes stored in
+//                the parent; a child reference >= 0 is an internal node index, < 0
+//                a leaf whose first TriRecord is ~ref.
+//   TriRecord[]  the same records in the reference's leaf order
+//                (bvhTriIndices of scene.bvh.cpp:193).
 #pragma once
 #include <stdint.h>
 
@@ -30,37 +35,37 @@ struct alignas(16) Bvh2Node {
 };
 static_assert(sizeof(Bvh2Node) == 64, "Bvh2Node is 64 B");
 
-// 4-wide collapse of the binary tree. Children are the grandchildren of a
-// binary node in the reference's DFS order for a ray with all direction
-// components positive; the three split axes let the kernel recover the
-// reference order for any ray: child slot s = (h << 1) | l where h is the
-// top split's side and l the second split's side.
-struct alignas(16) Bvh4Node {
-    float lox[4], hix[4];
-    float loy[4], hiy[4];
-    float loz[4], hiz[4];
-    int32_t child[4];      // child references (0x7fffffff = empty slot)
-    int32_t axis_top;      // split axis between slot pairs {0,1} and {2,3}
-    int32_t axis_l;        // split axis inside {0,1} (-1: slot pair is one child)
-    int32_t axis_r;        // split axis inside {2,3}
-    int32_t pad;
-};
-static_assert(sizeof(Bvh4Node) == 128, "Bvh4Node is 128 B");
-constexpr int32_t BVH4_EMPTY = 0x7fffffff;
-
-// Quantised binary node (LMGPU_LAYOUT_BVH2Q, render trees only): the same
-// tree as Bvh2Node with each child box on a per-node grid. Axis k's planes
-// sit at origin[k] + q * 2^(e_k - 127) for 16-bit q, where e_k is byte k of
-// `exps`. quantize_bvh2 (builder.cpp) chooses grid and q so that every
-// quantised box contains its child's float box with a margin of two grid
-// steps. 48 B: three 16-byte loads per visit instead of four.
-struct alignas(16) Bvh2QNode {
+// 8-wide compressed node (after Ylitie, Karras, Laine, "Efficient Incoherent
+// Ray Traversal on GPUs Through Compressed Wide BVHs", HPG 2017): up to eight
+// children, each child's box on a per-node grid of 8-bit planes. Axis k's planes sit
+// at origin[k] + q * 2^(e_k - 127), e_k byte k of `exps`; collapse_bvh8
+// (builder.cpp) rounds them outward with a margin, so a box only grows.
+// Slot s holds a child whose centre lies towards the corner of the node given
+// by s's bits (bit k set: the high side of axis k), so that the slots taken in
+// the order s ^ (signs of the ray's direction) run roughly near to far.
+// Internal children are consecutive nodes from `child_base` in slot order; a
+// leaf child is the run of TriRecords from start[s], ended by TRI_LAST_IN_LEAF.
+// A visit reads the first 96 bytes as three 32-byte loads; start[] is read
+// when a leaf is tested.
+struct alignas(128) Bvh8Node {
     float origin[3];
-    uint32_t exps;         // e_x | e_y << 8 | e_z << 16 | split axis << 24
-    uint32_t q[6];         // axis k: q[2k] left child, q[2k + 1] right child, each lo | hi << 16
-    int32_t left, right;   // child references as in Bvh2Node
+    uint32_t exps;         // e_x | e_y << 8 | e_z << 16 | mask of internal children << 24
+    uint32_t child_base;
+    uint32_t valid;        // mask of the slots in use
+    uint32_t pad0[2];
+    uint32_t lox[2], loy[2], loz[2], hix[2];   // byte s of each pair: slot s
+    uint32_t hiy[2], hiz[2], pad1[4];
+    uint32_t start[8];
 };
-static_assert(sizeof(Bvh2QNode) == 48, "Bvh2QNode is 48 B");
+static_assert(sizeof(Bvh8Node) == 128, "Bvh8Node is 128 B");
+
+// Box of a triangle's leaf in the binary tree (lo.xyz hi.x | hi.yz - -), by
+// position in the wide tree's triangle array.
+struct alignas(16) LeafBox {
+    float lo[3], hi[3];
+    float pad[2];
+};
+static_assert(sizeof(LeafBox) == 32, "LeafBox is 32 B");
 
 struct alignas(16) TriRecord {
     uint32_t k_flags;      // TriAccel::k | TRI_LAST_IN_LEAF

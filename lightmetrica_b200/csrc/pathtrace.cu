@@ -21,7 +21,6 @@
 #include "rng.cuh"
 #include "shading.cuh"
 #include "trace.cuh"
-#include "trace4.cuh"
 #include "trace_kernels.cuh"
 
 namespace lmgpu {
@@ -29,21 +28,19 @@ namespace {
 
 // ------------------------------------------------------ full hit record ----
 
-template <int LAYOUT, bool ANY_HIT, int STACK>
+template <bool NAIVE, int STACK>
 __device__ __forceinline__ bool trace_scene(const DeviceScene& s, TraversalRay& r, Hit& h, int2* stack)
 {
     if (s.num_tris == 0) { h.tri = -1; return true; }   // empty scene: no node arrays exist
-    if (LAYOUT == LMGPU_LAYOUT_BVH2)
-        return trace_bvh2<ANY_HIT>(s.bvh2, s.tris, s.root_ref, s.root_box, r, h, stack, s.stack_cap < STACK ? s.stack_cap : STACK, nullptr);
-    if (LAYOUT == LMGPU_LAYOUT_BVH4)
-        return trace_bvh4<ANY_HIT>(s.bvh4, s.tris, s.root_ref4, s.root_box, r, h, stack, s.stack_cap < STACK ? s.stack_cap : STACK, nullptr);
-    trace_naive<ANY_HIT>(s.tris_by_id, s.num_tris, r, h, nullptr);
+    if (!NAIVE)
+        return trace_bvh2<false>(s.bvh2, s.tris, s.root_ref, s.root_box, r, h, stack, s.stack_cap < STACK ? s.stack_cap : STACK, nullptr);
+    trace_naive<false>(s.tris_by_id, s.num_tris, r, h, nullptr);
     return true;
 }
 
 // Scene::Intersect (scene.cpp:67-72): triangles, then the environment's
 // emitter shape on a miss. kind: 0 miss, 1 triangle, 2 environment.
-template <int LAYOUT, int STACK>
+template <bool NAIVE, int STACK>
 __global__ void __launch_bounds__(128) k_intersect_full(const DeviceScene s, const float* __restrict__ rays, int64_t n,
                                                         int32_t* tri_id, float* t_out, float* geom, int32_t* kind,
                                                         int32_t* status)
@@ -58,7 +55,7 @@ __global__ void __launch_bounds__(128) k_intersect_full(const DeviceScene s, con
     TraversalRay r;
     setup_ray(r, in);
     Hit h;
-    if (!trace_scene<LAYOUT, false, STACK>(s, r, h, stack)) { atomicOr(status, STATUS_STACK_OVERFLOW); h.tri = -1; }
+    if (!trace_scene<NAIVE, STACK>(s, r, h, stack)) { atomicOr(status, STATUS_STACK_OVERFLOW); h.tri = -1; }
     Geom g;
     int k = 0;
     float t = 0.0f;
@@ -89,11 +86,10 @@ void launch_full(const LmgpuScene* sc, const float* rays, int64_t n, int32_t* id
     const int threads = 128;
     const int64_t blocks = (n + threads - 1) / threads;
     const DeviceScene& s = sc->dev;
-    switch (s.layout) {
-    case LMGPU_LAYOUT_BVH2: k_intersect_full<LMGPU_LAYOUT_BVH2, STACK><<<blocks, threads>>>(s, rays, n, id, t, g, kind, sc->d_status); break;
-    case LMGPU_LAYOUT_BVH4: k_intersect_full<LMGPU_LAYOUT_BVH4, STACK><<<blocks, threads>>>(s, rays, n, id, t, g, kind, sc->d_status); break;
-    default: k_intersect_full<LMGPU_LAYOUT_NAIVE, 1><<<blocks, threads>>>(s, rays, n, id, t, g, kind, sc->d_status); break;
-    }
+    if (s.layout == LMGPU_LAYOUT_NAIVE)
+        k_intersect_full<true, 1><<<blocks, threads>>>(s, rays, n, id, t, g, kind, sc->d_status);
+    else
+        k_intersect_full<false, STACK><<<blocks, threads>>>(s, rays, n, id, t, g, kind, sc->d_status);
 }
 
 // ------------------------------------------------------------ driver ------
@@ -158,7 +154,7 @@ template <class F>
 int shadow_pass(LmgpuScene* sc, const PathState& st, const OneScene<F>& ctx, int64_t max_rays, cudaStream_t stream)
 {
     ShadowIO<OneScene<F>> io{ st.counters + 2, st.sh_o, st.sh_d, st.sh_c, st.L, ctx };
-    return launch_trace<true, ShadowIO<OneScene<F>>>(sc, io, max_rays, stream, nullptr, true);
+    return launch_trace<true, ShadowIO<OneScene<F>>>(sc, io, max_rays, stream);
 }
 
 int read_counts(Workspace& ws, cudaStream_t stream)
@@ -222,7 +218,7 @@ int render_waves(LmgpuScene* sc, const LmgpuRenderParams& p, F* film, cudaStream
             stats.rays_traced += n;
             stats.max_bounces_run = std::max(stats.max_bounces_run, k);
             PathRayIO<false> io{ st.counters + qin, st.qo[qin], st.qd[qin], st.hit, nullptr };
-            rc = launch_trace<false, PathRayIO<false>>(sc, io, n, stream, nullptr, true);
+            rc = launch_trace<false, PathRayIO<false>>(sc, io, n, stream);
             if (rc != LMGPU_OK) break;
             LMGPU_CUDA_TRY(cudaMemsetAsync(st.counters + (1 - qin), 0, 4, stream));
             LMGPU_CUDA_TRY(cudaMemsetAsync(st.counters + 2, 0, 4, stream));
@@ -548,8 +544,9 @@ int lmgpu_render_release(void)
     hb.out = nullptr;
     hb.pinned = nullptr;
     hb.film_bytes = hb.out_bytes = 0;
+    const int rc = release_diff_pool(dev);
     if (first != cudaSuccess) return cuda_fail(first, what);
-    return LMGPU_OK;
+    return rc;
 }
 
 }  // extern "C"

@@ -67,6 +67,9 @@ struct PathState {
     int32_t* status;
 };
 
+__device__ __forceinline__ V3 f3(float4 q) { return v3(q.x, q.y, q.z); }
+__device__ __forceinline__ float4 f4(V3 v, float w) { return make_float4(v.x, v.y, v.z, w); }
+
 struct RenderConsts {
     int32_t technique;
     int32_t rr_depth;
@@ -78,14 +81,54 @@ struct RenderConsts {
     double inv_pixels;     // 1 / pixels
 };
 
+template <class F>
+__device__ __forceinline__ void film_add(F* film, int pixel, V3 c)
+{
+    if (pixel < 0 || (c.x == 0.0f && c.y == 0.0f && c.z == 0.0f)) return;
+    atomicAdd(film + 3 * pixel, (F)c.x);
+    atomicAdd(film + 3 * pixel + 1, (F)c.y);
+    atomicAdd(film + 3 * pixel + 2, (F)c.z);
+}
+
 // ------------------------------------------------------------ contexts ----
 
+// What a context may change of the light transport and of where contributions
+// go; the renderers keep the scene's own values and sum each path's radiance.
+// (The differentiable passes' context overrides all of these, adjoint.cu.)
+struct RenderContext {
+    __device__ __forceinline__ Material material(const DeviceScene& s, int prim, int32_t) const { return material_of(s, prim); }
+    __device__ __forceinline__ V3 area_Le(const DeviceScene& s, int li) const { return load3(s.area_lights[li].Le); }
+    __device__ __forceinline__ void light_sample(const DeviceScene&, LightPoint&) const {}
+    // A new path, and a surface vertex (hit number k) of path i.
+    __device__ __forceinline__ void start(int64_t) const {}
+    __device__ __forceinline__ void vertex(const PathState&, int64_t, int, int32_t) const {}
+    // Emission c of light li found by hit number k of path i.
+    __device__ __forceinline__ void emission(const PathState& st, int64_t i, int, int, V3 c) const
+    {
+        const V3 L = f3(st.L[i]) + c;
+        st.L[i] = f4(L, 0.0f);
+    }
+    // The contribution a shadow ray carries for path i or (camera vertex) for a
+    // pixel, and the tag stored with it.
+    __device__ __forceinline__ V3 nee(const PathState&, int64_t, V3 c) const { return c; }
+    __device__ __forceinline__ V3 camera_nee(int, V3 c) const { return c; }
+    __device__ __forceinline__ int shadow_tag(int sid, int) const { return sid; }
+    // A visible shadow ray's contribution to path dest (>= 0).
+    __device__ __forceinline__ void lit(float4* L, int32_t dest, V3 c, int) const
+    {
+        const float4 l = L[dest];
+        L[dest] = make_float4(l.x + c.x, l.y + c.y, l.z + c.z, 0.0f);
+    }
+};
+
 template <class F>
-struct OneScene {
+struct OneScene : RenderContext {
     static constexpr bool TABLE = false;
     DeviceScene s;
     RenderConsts rc;
     F* film;
+    OneScene() = default;
+    __host__ __device__ OneScene(const DeviceScene& scene, const RenderConsts& consts, F* out) : s(scene), rc(consts), film(out) {}
     __device__ __forceinline__ const DeviceScene& scene(int) const { return s; }
     __device__ __forceinline__ const RenderConsts& consts(int) const { return rc; }
     __device__ __forceinline__ int64_t wave_count(int64_t n) const { return n; }
@@ -98,6 +141,7 @@ struct OneScene {
     __device__ __forceinline__ int path_scene(const PathState&, int64_t) const { return 0; }
     __device__ __forceinline__ int64_t sample_of(int, int64_t i) const { return rc.sample_base + i; }
     __device__ __forceinline__ F* film_of(int) const { return film; }
+    __device__ __forceinline__ void lit_pixel(int, int pixel, V3 c) const { film_add(film, pixel, c); }
     // New path number j of this launch: its slot i and scene-local sample.
     __device__ __forceinline__ int begin_path(const PathState&, int64_t j, int64_t& i, int64_t& sample) const
     {
@@ -127,12 +171,13 @@ struct WaveCtl {
 };
 
 template <class F>
-struct SceneTable {
+struct SceneTable : RenderContext {
     static constexpr bool TABLE = true;
     const BatchEntry* table;
     const int64_t* begins;   // num_scenes + 1 ascending sample boundaries
     int32_t num_scenes;
     const WaveCtl* wave;
+    SceneTable(const BatchEntry* t, const int64_t* b, int32_t n, const WaveCtl* w) : table(t), begins(b), num_scenes(n), wave(w) {}
     __device__ __forceinline__ const DeviceScene& scene(int sid) const { return table[sid].s; }
     __device__ __forceinline__ const RenderConsts& consts(int sid) const { return table[sid].rc; }
     __device__ __forceinline__ int64_t wave_count(int64_t) const { return wave->count; }
@@ -154,6 +199,7 @@ struct SceneTable {
         return table[sid].rc.sample_base + (wave->base + i - table[sid].begin);
     }
     __device__ __forceinline__ F* film_of(int sid) const { return static_cast<F*>(table[sid].film); }
+    __device__ __forceinline__ void lit_pixel(int sid, int pixel, V3 c) const { film_add(film_of(sid), pixel, c); }
     __device__ __forceinline__ int begin_path(const PathState& st, int64_t j, int64_t& i, int64_t& sample) const
     {
         i = j;
@@ -179,7 +225,7 @@ struct StreamCtl {
 };
 
 template <class F>
-struct StreamTable {
+struct StreamTable : RenderContext {
     static constexpr bool TABLE = true;
     static constexpr bool STREAM = true;
     const BatchEntry* table;
@@ -188,6 +234,8 @@ struct StreamTable {
     const StreamCtl* ctl;
     const int64_t* sample;            // PathState::sample
     unsigned long long* max_depth;    // statistics: deepest bounce reached
+    StreamTable(const BatchEntry* t, const int64_t* b, int32_t n, const StreamCtl* c, const int64_t* s, unsigned long long* d)
+        : table(t), begins(b), num_scenes(n), ctl(c), sample(s), max_depth(d) {}
     __device__ __forceinline__ const DeviceScene& scene(int sid) const { return table[sid].s; }
     __device__ __forceinline__ const RenderConsts& consts(int sid) const { return table[sid].rc; }
     __device__ __forceinline__ int64_t wave_count(int64_t) const { return ctl->n_new; }
@@ -197,6 +245,7 @@ struct StreamTable {
         return table[sid].rc.sample_base + (sample[i] - table[sid].begin);
     }
     __device__ __forceinline__ F* film_of(int sid) const { return static_cast<F*>(table[sid].film); }
+    __device__ __forceinline__ void lit_pixel(int sid, int pixel, V3 c) const { film_add(film_of(sid), pixel, c); }
     __device__ __forceinline__ int begin_path(const PathState& st, int64_t j, int64_t& i, int64_t& local) const
     {
         i = st.free_slots[ctl->free_base + j];
@@ -251,9 +300,6 @@ __device__ __forceinline__ uint32_t queue_append(const PathState& st, int q, boo
     return slot;
 }
 
-__device__ __forceinline__ V3 f3(float4 q) { return v3(q.x, q.y, q.z); }
-__device__ __forceinline__ float4 f4(V3 v, float w) { return make_float4(v.x, v.y, v.z, w); }
-
 // A queued ray's minT is Eps, except pt's camera rays (minT 0,
 // pathtrace.cpp:187, 245); the flag shares the word of the path slot
 // (slots < 2^31).
@@ -275,15 +321,6 @@ __device__ __forceinline__ float queued_tmin(float4 d)
 }
 __device__ __forceinline__ int queued_scene(float4 o) { return __float_as_int(o.w); }
 
-template <class F>
-__device__ __forceinline__ void film_add(F* film, int pixel, V3 c)
-{
-    if (pixel < 0 || (c.x == 0.0f && c.y == 0.0f && c.z == 0.0f)) return;
-    atomicAdd(film + 3 * pixel, (F)c.x);
-    atomicAdd(film + 3 * pixel + 1, (F)c.y);
-    atomicAdd(film + 3 * pixel + 2, (F)c.z);
-}
-
 // RenderUtils::Visible (renderutils.cpp:58-70) as a queued shadow ray:
 // minT = Eps, maxT = |target - p| (1 - Eps).
 __device__ __forceinline__ void write_shadow(const PathState& st, uint32_t slot, V3 p, V3 target, V3 c, int32_t dest,
@@ -299,12 +336,15 @@ __device__ __forceinline__ void write_shadow(const PathState& st, uint32_t slot,
 // Camera vertex of pt.direct / pt.mis (numPathVertices == 1): a light sample
 // seen through the pinhole, splatted at its own raster position
 // (pathtrace.direct.cpp:206-250, pathtrace.mis.cpp:188-247).
-template <int TECH>
-__device__ __forceinline__ bool camera_nee(const DeviceScene& s, uint64_t key, V3& target, V3& c, int32_t& dest)
+template <int TECH, class Ctx>
+__device__ __forceinline__ bool camera_nee(const Ctx& ctx, const DeviceScene& s, uint64_t key, V3& target, V3& c, int32_t& dest,
+                                           int& light)
 {
     LightPoint lp;
     if (!sample_light(s, rng_uniform(key, dim_vertex(1) + DIM_LIGHT), rng_uniform(key, dim_vertex(1) + DIM_LIGHT + 1), lp))
         return false;
+    ctx.light_sample(s, lp);
+    light = lp.light;
     const V3 cp = load3(s.cam.position);
     const V3 ppL = normalize(lp.p - cp);
     float rx, ry, We;
@@ -319,8 +359,11 @@ __device__ __forceinline__ bool camera_nee(const DeviceScene& s, uint64_t key, V
     }
     c = Le * (w * We * G / lp.pdf_area);
     target = lp.p;
-    dest = ~film_pixel(s.cam, rx, ry);
-    return !is_zero(c) && dest != ~(-1);
+    const int pixel = film_pixel(s.cam, rx, ry);
+    dest = ~pixel;
+    if (is_zero(c) || pixel < 0) return false;
+    c = ctx.camera_nee(pixel, c);
+    return !is_zero(c);
 }
 
 // ------------------------------------------------------------- kernels ----
@@ -351,6 +394,7 @@ __global__ void __launch_bounds__(128) k_pt_init(const Ctx ctx, const PathState 
     const V3 cp = load3(s.cam.position);
     st.raster[i] = make_float2(rx, ry);
     st.L[i] = make_float4(0, 0, 0, 0);
+    ctx.start(i);
     V3 thr = v3(1, 1, 1);
     // No vertex beyond the camera: the path contributes nothing (the
     // one-scene driver skips such waves before launching).
@@ -358,9 +402,10 @@ __global__ void __launch_bounds__(128) k_pt_init(const Ctx ctx, const PathState 
     if (TECH != LMGPU_RENDER_PT && alive) {
         V3 target, c;
         int32_t dest;
-        const bool shadow = camera_nee<TECH>(s, key, target, c, dest);
+        int light = 0;
+        const bool shadow = camera_nee<TECH>(ctx, s, key, target, c, dest, light);
         const uint32_t sslot = queue_append(st, 2, shadow);
-        if (shadow && slot_ok(sslot)) write_shadow(st, sslot, cp, target, c, dest, sid);
+        if (shadow && slot_ok(sslot)) write_shadow(st, sslot, cp, target, c, dest, ctx.shadow_tag(sid, light));
         if (rc.rr_depth != -1 && 1 >= rc.rr_depth) {
             const float p = fminf(0.5f, luminance(thr));
             if (rng_uniform(key, dim_vertex(1) + DIM_RR) > p) alive = false;
@@ -378,35 +423,10 @@ __global__ void __launch_bounds__(128) k_pt_init(const Ctx ctx, const PathState 
 
 // Closest-hit traversal of the queued rays (writes hit records). With a
 // scene table each ray is traced in its own path's scene.
-// Both path-tracer queues refill traversal lanes once 20 are idle and pause
-// a descent once fewer than 16 lanes still descend. Measured with the render
-// walks (1080p terrain frame / 64-scene batch): 166.7 / 793.9 ms against
-// 171.0 / 804.6 ms at (24, 24); pausing below 20 lanes or refilling 16 at a
-// time was slower, pausing below 28 slower still.
-#ifndef LMGPU_PT_REFILL_MIN
-#define LMGPU_PT_REFILL_MIN 20
-#endif
-#ifndef LMGPU_PT_EXIT_BELOW
-#define LMGPU_PT_EXIT_BELOW 16
-#endif
-constexpr int PATH_QUEUE_REFILL_MIN = LMGPU_PT_REFILL_MIN;
-constexpr int PATH_QUEUE_EXIT_BELOW = LMGPU_PT_EXIT_BELOW;
-// The shadow queue's speculative any-hit walk refills at 12 idle lanes
-// (shadow traversal of the 1080p frame 45.3 -> 44.2 ms; 8 and 28 were
-// slower, and pausing below 8, 12 or 24 lanes instead of 16 did not help).
-#ifndef LMGPU_PT_SHADOW_REFILL_MIN
-#define LMGPU_PT_SHADOW_REFILL_MIN 12
-#endif
-#ifndef LMGPU_PT_SHADOW_EXIT_BELOW
-#define LMGPU_PT_SHADOW_EXIT_BELOW LMGPU_PT_EXIT_BELOW
-#endif
-
 template <bool TABLE>
 struct PathRayIO {
     static constexpr bool PER_RAY_SCENE = TABLE;
     static constexpr bool RENDER = true;
-    static constexpr int REFILL_MIN = PATH_QUEUE_REFILL_MIN;
-    static constexpr int EXIT_BELOW = PATH_QUEUE_EXIT_BELOW;
     const uint32_t* count_ptr;
     const float4* qo;
     const float4* qd;
@@ -436,8 +456,6 @@ template <class Ctx>
 struct ShadowIO {
     static constexpr bool PER_RAY_SCENE = Ctx::TABLE;
     static constexpr bool RENDER = true;
-    static constexpr int REFILL_MIN = LMGPU_PT_SHADOW_REFILL_MIN;
-    static constexpr int EXIT_BELOW = LMGPU_PT_SHADOW_EXIT_BELOW;
     const uint32_t* count_ptr;
     const float4* sh_o;
     const float4* sh_d;
@@ -466,12 +484,8 @@ struct ShadowIO {
         if (s.has_env && env_sphere_intersect(s, o, d, r.tmin, sh_o[j].w, te)) return;
         const V3 c = f3(c4);
         const int32_t dest = __float_as_int(sh_d[j].w);
-        if (dest >= 0) {
-            const float4 l = L[dest];
-            L[dest] = make_float4(l.x + c.x, l.y + c.y, l.z + c.z, 0.0f);
-        } else {
-            film_add(ctx.film_of(sid), ~dest, c);
-        }
+        if (dest >= 0) ctx.lit(L, dest, c, sid);
+        else ctx.lit_pixel(sid, ~dest, c);
     }
 };
 
@@ -506,6 +520,7 @@ __global__ void __launch_bounds__(128, LMGPU_PT_SHADE_MIN_BLOCKS) k_pt_shade(con
         Geom g;
         BsdfSample bs;
         V3 sh_target = v3(0, 0, 0), sh_c = v3(0, 0, 0);
+        int sh_tag = 0;
         if (valid) {
             const DeviceScene& s = ctx.scene(sid);
             const RenderConsts& rc = ctx.consts(sid);
@@ -518,6 +533,7 @@ __global__ void __launch_bounds__(128, LMGPU_PT_SHADE_MIN_BLOCKS) k_pt_shade(con
             const int32_t tri = __float_as_int(h4.x);
             V3 Le = v3(0, 0, 0);
             float light_pdf_area = 0.0f;   // EvaluatePositionPDF of the light that was hit
+            int hit_light = s.num_area_lights;
             bool hit_surface = false;
             Material m;
             m.type = LMGPU_BSDF_BLACK;
@@ -534,11 +550,12 @@ __global__ void __launch_bounds__(128, LMGPU_PT_SHADE_MIN_BLOCKS) k_pt_shade(con
                 const int prim = s.tri_prim[tri];
                 const int li = s.prim_light[prim];
                 if (li >= 0) {
-                    const AreaLightGpu al = s.area_lights[li];
-                    Le = emitted(load3(al.Le), g.sn, wi);
-                    light_pdf_area = al.inv_area;
+                    Le = emitted(ctx.area_Le(s, li), g.sn, wi);
+                    light_pdf_area = s.area_lights[li].inv_area;
+                    hit_light = li;
                 }
-                m = material_of(s, prim);
+                m = ctx.material(s, prim, tri);
+                ctx.vertex(st, i, k, tri);
                 hit_surface = true;
             }
             // ---- emission reached by BSDF sampling (the path's radiance is
@@ -558,10 +575,7 @@ __global__ void __launch_bounds__(128, LMGPU_PT_SHADE_MIN_BLOCKS) k_pt_shade(con
                         add = false;
                     }
                 }
-                if (add) {
-                    const V3 L = f3(st.L[i]) + c;
-                    st.L[i] = f4(L, 0.0f);
-                }
+                if (add) ctx.emission(st, i, k, hit_light, c);
             }
             const int v = k + 1;   // numPathVertices once this hit is accepted
             alive = hit_surface;
@@ -570,6 +584,7 @@ __global__ void __launch_bounds__(128, LMGPU_PT_SHADE_MIN_BLOCKS) k_pt_shade(con
                 // ---- next-event estimation at vertex v
                 LightPoint lp;
                 if (sample_light(s, rng_uniform(key, dim_vertex(v) + DIM_LIGHT), rng_uniform(key, dim_vertex(v) + DIM_LIGHT + 1), lp)) {
+                    ctx.light_sample(s, lp);
                     const V3 ppL = normalize(lp.p - g.p);
                     float pdf_bsdf;
                     const V3 fs = eval_bsdf(m, g, wi, ppL, pdf_bsdf);
@@ -582,7 +597,9 @@ __global__ void __launch_bounds__(128, LMGPU_PT_SHADE_MIN_BLOCKS) k_pt_shade(con
                             w = pdf_dl / (pdf_dl + pdf_bsdf);
                         }
                         sh_c = thr * fs * Lel * (w * G / lp.pdf_area);
+                        if (!is_zero(sh_c)) sh_c = ctx.nee(st, i, sh_c);
                         sh_target = lp.p;
+                        sh_tag = ctx.shadow_tag(sid, lp.light);
                         shadow = !is_zero(sh_c);
                     }
                 }
@@ -609,7 +626,7 @@ __global__ void __launch_bounds__(128, LMGPU_PT_SHADE_MIN_BLOCKS) k_pt_shade(con
             }
         }
         const uint32_t sslot = queue_append(st, 2, shadow);
-        if (shadow && slot_ok(sslot)) write_shadow(st, sslot, g.p, sh_target, sh_c, i, sid);
+        if (shadow && slot_ok(sslot)) write_shadow(st, sslot, g.p, sh_target, sh_c, i, sh_tag);
         const uint32_t slot = queue_append(st, qout, alive);
         if (alive && slot_ok(slot)) {
             queue_ray<TECH>(st, qout, slot, g.p, bs.wo, i, sid, false, thr, bs.pdf, g.sn, bs.specular ? PREV_SPECULAR : 0u);
@@ -640,6 +657,14 @@ __global__ void __launch_bounds__(128) k_pt_retire(const Ctx ctx, const PathStat
         film_add(ctx.film_of(sid), film_pixel(ctx.scene(sid).cam, r.x, r.y), f3(st.L[i]));
         st.free_slots[base + j] = i;
     }
+}
+
+// Start of a wave: clear the queue counters and this wave's traversal work
+// counters (static: each translation unit launches its own).
+static __global__ void k_wave_begin(uint32_t* counters, unsigned long long* work, int slots)
+{
+    for (int i = threadIdx.x; i < slots; i += blockDim.x) work[i] = 0;
+    if (threadIdx.x < 4) counters[threadIdx.x] = 0;
 }
 
 // Film splat of each path's radiance at its raster position.

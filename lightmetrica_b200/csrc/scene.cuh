@@ -50,14 +50,18 @@ struct CameraGpu {
 struct DeviceScene {
     // ---- accelerator
     int32_t layout;
-    int32_t root_ref;      // BVH2 root reference
-    int32_t root_ref4;     // BVH4 root reference
+    int32_t stack8_cap;    // stack bound of the 8-wide walk
+    const Bvh8Node* bvh8;         // root: node 0
+    const TriRecord* tris8;       // its leaf order
+    const LeafBox* boxes8;        // binary leaf box per tris8 record (the reference's tree; renders with check_boxes)
+    int32_t check_boxes;          // renders: test boxes8 on every candidate hit (scene far from the origin)
+    float wide_limit;             // the reference's tree: origins up to this magnitude take the 8-wide walk
+    // The reference's own walk (the reference's tree only).
+    int32_t root_ref;
     int32_t stack_cap;
-    float root_box[6];     // lo.xyz, hi.xyz
+    float root_box[6];            // lo.xyz, hi.xyz
     const Bvh2Node* bvh2;
-    const Bvh4Node* bvh4;
-    const Bvh2QNode* bvh2q;       // render view: the quantised copy of bvh2 (LMGPU_LAYOUT_BVH2Q)
-    const TriRecord* tris;        // leaf order
+    const TriRecord* tris;        // the reference's leaf order
     const TriRecord* tris_by_id;  // TriAccel order (naive layout)
     int64_t num_tris;
 

@@ -1,0 +1,273 @@
+// Traversal of the 8-wide compressed tree (Bvh8Node): the box test of a
+// node's eight children, the exact walk's certificate, and a one-thread walk.
+//
+// A visit is about 250 instructions a warp, half of them on the ALU pipe (48 byte
+// permutes turn plane bytes into floats, 32 three-input min/max): with 22 of 32
+// lanes active the walk issues on 75 % of cycles. It replaces the binary
+// tree's visits (64-byte nodes as four 16-byte loads, L1 at 83 % of its
+// wavefront peak on the bounce rays of a 3.4 M-triangle terrain): 38 visits of a
+// bounce ray became 14.6, each of three 32-byte loads. Measured, binary -> 8-wide
+// (one B200, render arithmetic): 2^23 random rays through a 1,048,576-triangle soup
+// 2.97 -> 1.60 ms (exact, with the certificate below: 3.17 -> 2.32 ms);
+// on the terrain 8.3 M camera rays 1.52 -> 1.44 ms, 5.3 M bounce rays
+// 1.98 -> 1.51 ms, 5.3 M shadow rays 2.30 -> 1.47 ms. Float planes (224-byte nodes)
+// took 2.5 / 2.2 ms on the soup / bounce rays, a 4-wide node of 8-bit planes
+// 2.0 / 1.54 ms.
+#pragma once
+#include <type_traits>
+#include "trace.cuh"
+
+namespace lmgpu {
+
+// 32 bytes of read-only data by one load (sm_100).
+struct Words8 { uint32_t w[8]; };
+__device__ __forceinline__ Words8 load32(const void* p)
+{
+    Words8 v;
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(v.w[0]), "=r"(v.w[1]), "=r"(v.w[2]), "=r"(v.w[3]), "=r"(v.w[4]), "=r"(v.w[5]), "=r"(v.w[6]), "=r"(v.w[7])
+        : "l"(p));
+    return v;
+}
+
+// x * s + b and y * s + b, each rounded once (packed, sm_100).
+__device__ __forceinline__ void fma_pair(float x, float y, float s, float b, float& a, float& c)
+{
+    asm("{\n\t.reg .b64 p, q, r;\n\t"
+        "mov.b64 p, {%2, %3};\n\t"
+        "mov.b64 q, {%4, %4};\n\t"
+        "mov.b64 r, {%5, %5};\n\t"
+        "fma.rn.f32x2 p, p, q, r;\n\t"
+        "mov.b64 {%0, %1}, p;\n\t}"
+        : "=f"(a), "=f"(c) : "f"(x), "f"(y), "f"(s), "f"(b));
+}
+
+// Byte B of `word` as the float 2^15 + byte: one byte permute puts it into the
+// second mantissa byte under the exponent of 2^15. The 2^15 * step / d this adds is
+// taken off the axis' bias, which rounds that at 2^-9 of a grid step, inside the
+// margin of step / 64 that collapse_bvh8 leaves.
+template <int B>
+__device__ __forceinline__ float plane_byte(uint32_t word)
+{
+    return __uint_as_float(__byte_perm(word, 0x47000000u, 0x7404 | (B << 4)));
+}
+
+// One lane's walk: the group of deferred children it is in (bits 0-7 of mask: hit
+// internal children still to visit, nearest first at bit 0; bits 8-15: which slots
+// are internal) and the leaves found (bit s of leaves: slot s of leaf_node).
+struct Walk8 {
+    uint32_t base, mask;
+    uint32_t leaf_node, leaves;
+    int sp;
+};
+
+__device__ __forceinline__ void walk8_begin(Walk8& w, uint32_t oct)
+{
+    // The root as slot 0 of a group of one: child index popc(0) = 0.
+    w.base = 0;
+    w.mask = (1u << oct) | (1u << 8);
+    w.leaves = 0;
+    w.sp = 0;
+}
+
+// Visit order is slot ^ oct: exchanges the bits of an 8-bit slot mask so.
+__device__ __forceinline__ uint32_t order_mask(uint32_t m, uint32_t oct)
+{
+    if (oct & 1u) m = ((m & 0x55u) << 1) | ((m >> 1) & 0x55u);
+    if (oct & 2u) m = ((m & 0x33u) << 2) | ((m >> 2) & 0x33u);
+    if (oct & 4u) m = ((m & 0x0fu) << 4) | ((m >> 4) & 0x0fu);
+    return m;
+}
+
+// Takes the nearest child of the current group (which has one) and returns its node.
+__device__ __forceinline__ uint32_t walk8_next(Walk8& w, uint32_t oct)
+{
+    const uint32_t slot = (uint32_t)(__ffs(w.mask) - 1) ^ oct;
+    w.mask &= w.mask - 1;
+    return w.base + __popc((w.mask >> 8) & ((1u << slot) - 1u));
+}
+
+// Tests the eight child boxes of `node` against the ray's [tmin, tmax]: sets the
+// group of hit internal children and the hit leaves (`w.leaves` must be empty).
+// A ray made by setup_ray<true>; oct = the signs of its direction.
+__device__ __forceinline__ void walk8_visit(Walk8& w, const Bvh8Node* __restrict__ nodes, uint32_t node,
+                                            const TraversalRay& r, uint32_t oct)
+{
+    const char* p = reinterpret_cast<const char*>(nodes + node);
+    const Words8 h = load32(p), a = load32(p + 32), b = load32(p + 64);
+    const float sx = __uint_as_float((h.w[3] << 23) & 0x7f800000u) * r.inv_min[0];
+    const float sy = __uint_as_float((h.w[3] << 15) & 0x7f800000u) * r.inv_min[1];
+    const float sz = __uint_as_float((h.w[3] << 7) & 0x7f800000u) * r.inv_min[2];
+    const float bx = fmaf(-32768.0f, sx, fmaf(__uint_as_float(h.w[0]), r.inv_min[0], r.inv_max[0]));
+    const float by = fmaf(-32768.0f, sy, fmaf(__uint_as_float(h.w[1]), r.inv_min[1], r.inv_max[1]));
+    const float bz = fmaf(-32768.0f, sz, fmaf(__uint_as_float(h.w[2]), r.inv_min[2], r.inv_max[2]));
+    const bool nx = oct & 1u, ny = oct & 2u, nz = oct & 4u;
+    uint32_t miss = 0;
+#pragma unroll
+    for (int q = 1; q >= 0; q--) {
+        const uint32_t lx = a.w[q], ly = a.w[2 + q], lz = a.w[4 + q], ux = a.w[6 + q], uy = b.w[q], uz = b.w[2 + q];
+        const uint32_t near_x = nx ? ux : lx, far_x = nx ? lx : ux;
+        const uint32_t near_y = ny ? uy : ly, far_y = ny ? ly : uy;
+        const uint32_t near_z = nz ? uz : lz, far_z = nz ? lz : uz;
+        auto child = [&](auto B) {
+            constexpr int I = decltype(B)::value;
+            float x0, x1, y0, y1, z0, z1;
+            fma_pair(plane_byte<I>(near_x), plane_byte<I>(far_x), sx, bx, x0, x1);
+            fma_pair(plane_byte<I>(near_y), plane_byte<I>(far_y), sy, by, y0, y1);
+            fma_pair(plane_byte<I>(near_z), plane_byte<I>(far_z), sz, bz, z0, z1);
+            const float tn = fmaxf(fmaxf(x0, y0), fmaxf(z0, r.tmin));
+            const float tf = fminf(fminf(x1, y1), fminf(z1, r.tmax));
+            miss = __funnelshift_l(__float_as_uint(tf - tn), miss, 1);   // shifts in the sign: 1 = entry after exit
+        };
+        child(std::integral_constant<int, 3>{});
+        child(std::integral_constant<int, 2>{});
+        child(std::integral_constant<int, 1>{});
+        child(std::integral_constant<int, 0>{});
+    }
+    const uint32_t hit = ~miss & h.w[5], inner = h.w[3] >> 24;
+    w.base = h.w[4];
+    w.mask = order_mask(hit & inner, oct) | (inner << 8);
+    w.leaf_node = node;
+    w.leaves = hit & ~inner;
+}
+
+// First record of the next hit leaf.
+__device__ __forceinline__ const float4* walk8_leaf(const Bvh8Node* __restrict__ nodes, const TriRecord* __restrict__ tris,
+                                                    uint32_t node, uint32_t& leaves)
+{
+    const uint32_t slot = (uint32_t)(__ffs(leaves) - 1);
+    leaves &= leaves - 1;
+    return reinterpret_cast<const float4*>(tris + __ldg(&nodes[node].start[slot]));
+}
+
+// ------------------------------------------------------- candidate hits ----
+
+// The slab test of the record's binary leaf box, in the arithmetic of render
+// rays (multiply-adds): whether a walk through float boxes would have come to
+// this triangle. Renders far from the origin make it (DeviceScene::check_boxes):
+// there the triangle test's rounding reports hits outside the triangle, and the
+// 8-bit boxes let more of them through than float boxes do.
+__device__ __forceinline__ bool leaf_box_render(const LeafBox* __restrict__ boxes, int64_t at, const TraversalRay& r)
+{
+    const float4 a = __ldg(reinterpret_cast<const float4*>(boxes + at));
+    const float4 b = __ldg(reinterpret_cast<const float4*>(boxes + at) + 1);
+    float x0, x1, y0, y1, z0, z1;
+    fma_pair(a.x, a.w, r.inv_min[0], r.inv_max[0], x0, x1);
+    fma_pair(a.y, b.x, r.inv_min[1], r.inv_max[1], y0, y1);
+    fma_pair(a.z, b.y, r.inv_min[2], r.inv_max[2], z0, z1);
+    const float tn = fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fminf(z0, z1));
+    const float tf = fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fmaxf(z0, z1));
+    return tn <= tf && tf > r.tmin && tn < r.tmax;
+}
+
+// Exact walk. The reference's answer for a ray is a fold over the triangles whose
+// leaf box passes its slab test with t_enter < maxT (the ancestors' boxes then
+// pass too: the test is monotone under containment) and whose TriAccel test
+// passes. Call S the candidates at the ray's own maxT. If A in S has the least t
+// and every other member has t > max(t_A, t_enter_A), the reference finds A
+// whatever the order: its leaf is entered before any maxT that another hit can
+// have set, and nothing is accepted after it. The wide walk therefore culls at
+// max(t_A, t_enter_A), tests each candidate's leaf box with the reference's
+// arithmetic, and hands the ray back (HIT_TIED) when two candidates lie within that
+// window of one another; such rays, and rays for which the inflated boxes prove
+// nothing (exact_wide_ok), take the reference's own walk.
+constexpr int32_t HIT_TIED = -2;
+
+__device__ __forceinline__ bool leaf_box_exact(const LeafBox* __restrict__ boxes, int64_t at, const TraversalRay& r,
+                                               float& te)
+{
+    const float4 a = __ldg(reinterpret_cast<const float4*>(boxes + at));
+    const float4 b = __ldg(reinterpret_cast<const float4*>(boxes + at) + 1);
+    TraversalRay e;
+    RayIn in;
+#pragma unroll
+    for (int c = 0; c < 3; c++) { in.o[c] = r.o[c]; in.d[c] = r.d[c]; }
+    in.tmin = r.tmin;
+    in.tmax = r.tmax;
+    setup_ray(e, in);
+    return slab_intrinsic(e, a.x, a.w, a.y, b.x, a.z, b.y, te);
+}
+
+// A candidate hit (t, u, v) of record `at` within the current window; tmax0 is
+// the ray's own maxT.
+__device__ __forceinline__ void exact_candidate(const LeafBox* __restrict__ boxes, int64_t at, int32_t tri, float t,
+                                                float u, float v, float tmax0, TraversalRay& r, Hit& h)
+{
+    float te;
+    if (!leaf_box_exact(boxes, at, r, te) || !(te < tmax0) || h.tri == HIT_TIED) return;
+    const float window = fmaxf(t, te);
+    if (h.tri >= 0 && (t >= h.t || h.t <= window)) { h.tri = HIT_TIED; return; }
+    h.tri = tri; h.t = t; h.u = u; h.v = v;
+    r.tmax = window;
+}
+
+// Whether the inflated boxes cover this ray: a finite origin within the
+// magnitude they were built for, and every direction component zero or with a
+// finite inverse.
+__device__ __forceinline__ bool exact_wide_ok(const RayIn& in, float limit)
+{
+    bool ok = true;
+    const float inf = __int_as_float(0x7f800000);
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        ok = ok && fabsf(in.o[c]) <= limit;
+        ok = ok && (in.d[c] == 0.0f || fabsf(__frcp_rn(in.d[c])) < inf) && fabsf(in.d[c]) < inf;
+    }
+    return ok;
+}
+
+// --------------------------------------------------------- one thread ----
+
+// Closest (or any) render hit by one thread; `stack` holds `cap` groups.
+// Between triangles hit at the same distance the higher id wins, whatever the
+// order of the tests. Returns false on stack overflow.
+template <bool ANY_HIT>
+__device__ __forceinline__ bool trace8(const Bvh8Node* __restrict__ nodes, const TriRecord* __restrict__ tris,
+                                       const LeafBox* __restrict__ boxes, TraversalRay& r, Hit& h, uint2* stack, int cap)
+{
+    const uint32_t oct = r.neg & 7u;
+    Walk8 w;
+    walk8_begin(w, oct);
+    h.tri = -1;
+    for (;;) {
+        // Descend to the next leaves: the lanes of a warp meet again before they
+        // test triangles.
+        while (w.leaves == 0) {
+            if ((w.mask & 0xffu) == 0) {
+                if (w.sp == 0) break;
+                const uint2 e = stack[--w.sp];
+                w.base = e.x;
+                w.mask = e.y;
+            }
+            const uint32_t node = walk8_next(w, oct);
+            if (w.mask & 0xffu) {
+                if (w.sp >= cap) return false;
+                stack[w.sp++] = make_uint2(w.base, w.mask);
+            }
+            walk8_visit(w, nodes, node, r, oct);
+        }
+        if (w.leaves == 0) return true;
+        const float4* p = walk8_leaf(nodes, tris, w.leaf_node, w.leaves);
+        for (;;) {
+            const float4 q0 = __ldg(p), q1 = __ldg(p + 1), q2 = __ldg(p + 2);
+            float u, v, t;
+            if (triaccel_intersect_fast(q0, q1, q2, r, r.tmax, u, v, t) &&
+                (!boxes || leaf_box_render(boxes, (p - reinterpret_cast<const float4*>(tris)) / 3, r))) {
+                const int32_t id = static_cast<int32_t>(__float_as_uint(q2.z));
+                if (t < r.tmax || id > h.tri) {
+                    r.tmax = t;
+                    h.tri = id; h.t = t; h.u = u; h.v = v;
+                    if (ANY_HIT) return true;
+                }
+            }
+            if (__float_as_uint(q0.x) & TRI_LAST_IN_LEAF) {
+                if (w.leaves == 0) break;
+                p = walk8_leaf(nodes, tris, w.leaf_node, w.leaves);
+            } else {
+                p += 3;
+            }
+        }
+    }
+}
+
+}  // namespace lmgpu

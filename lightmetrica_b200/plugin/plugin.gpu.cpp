@@ -37,7 +37,7 @@
 // renderer goes to an internal "mt" scheduler configured with the same node.
 //
 // Configuration of the scene: <layout>bvh</layout> (default; bit-exact) or
-// qbvh (4-wide collapse of the same tree, also bit-exact).
+// qbvh (the same hits).
 #include <lightmetrica/scene.h>
 #include <lightmetrica/primitive.h>
 #include <lightmetrica/primitives.h>

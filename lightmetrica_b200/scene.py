@@ -188,8 +188,8 @@ _LAYOUTS = {"bvh": N.LAYOUT_BVH2, "qbvh": N.LAYOUT_BVH4, "naive": N.LAYOUT_NAIVE
 
 class Scene:
     """GPU implementation of the reference Scene component. `impl` names the
-    accelerator: "bvh" (binary, bit-identical to the reference BVHScene),
-    "qbvh" (4-wide collapse of the same tree, also bit-identical) or "naive"."""
+    accelerator: "bvh" or "qbvh" (bit-identical to the reference BVHScene,
+    through the same 8-wide collapse of its tree) or "naive"."""
 
     def __init__(self, impl: str = "bvh"):
         if impl not in _LAYOUTS:

@@ -1,0 +1,74 @@
+"""The differentiable passes as waves against the one-thread passes: a budget
+large enough for waves equals the weighted sum of its parts, each small enough
+for one thread per sample (same samples, same random numbers; the sums are
+accumulated in another order)."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from lightmetrica_b200 import create_renderer, create_scene, native as N, scenes
+from lightmetrica_b200.diff import light_emission, triangle_albedo
+
+pytestmark = pytest.mark.gpu
+
+WAVE_MIN = 1 << 16      # samples from which a pass runs as waves
+PART = 1 << 15
+
+
+def _closed_box():
+    """Mirrors and diffuse faces all around: no path leaves."""
+    prims = scenes.cornell_box(32, 32, variant="mixed")
+    prims.environment_light = None
+    prims.add(scenes.Primitive(mesh=scenes._mesh([scenes._quad((0, 0, 1.0), (1, 0, 1.0), (1, 1, 1.0), (0, 1, 1.0), (0, 0, -1))]),
+                               bsdf=scenes.PerfectMirrorBSDF((0.9, 0.9, 0.9))))
+    prims.camera.eye = (0.5, 0.5, 0.9)
+    return prims
+
+
+def _pass(scene, params, diff, torch, albedo, emission, dL, backward):
+    st = N.RenderStats()
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    if not backward:
+        img = torch.zeros(dL.numel(), device="cuda")
+        N.check(N.lib().lmgpu_adjoint_forward(scene.handle, ctypes.byref(params), ctypes.byref(diff), img.data_ptr(), stream,
+                                              ctypes.byref(st)))
+        scene.status(stream.value)
+        return (img.double().cpu().numpy(),)
+    da, de = torch.zeros_like(albedo), torch.zeros_like(emission)
+    N.check(N.lib().lmgpu_adjoint_backward(scene.handle, ctypes.byref(params), ctypes.byref(diff), dL.data_ptr(), da.data_ptr(),
+                                           de.data_ptr(), stream, ctypes.byref(st)))
+    scene.status(stream.value)
+    return da.double().cpu().numpy(), de.double().cpu().numpy()
+
+
+@pytest.mark.parametrize("technique,box,max_pv,rr,n", [
+    ("pt.mis", "mixed", 9, 3, WAVE_MIN), ("pt.direct", "classic", 2, 1, WAVE_MIN + 1), ("pt", "mixed", 9, -1, WAVE_MIN + 77),
+    ("pt.mis", "closed", 45, -1, WAVE_MIN),          # beyond the vertices a wave records: tails
+    ("pt", "closed", -1, 8, WAVE_MIN),               # unbounded depth: tails
+    ("pt.direct", "closed", 33, -1, WAVE_MIN + 5)])  # exactly the recorded vertices
+def test_waves_equal_the_sum_of_one_thread_passes(cuda, technique, box, max_pv, rr, n):
+    import torch
+    prims = _closed_box() if box == "closed" else scenes.cornell_box(32, 32, variant=box)
+    scene = create_scene("bvh")
+    scene.load(prims)
+    scene.configure({})
+    scene.build()
+    r = create_renderer(technique)
+    r.configure({"rr_depth": rr, "max_path_vertices": max_pv, "sampler": {"rng_seed": 5}})
+    albedo = torch.from_numpy(triangle_albedo(prims) * np.float32(0.9)).cuda()
+    emission = torch.from_numpy(light_emission(prims)).cuda()
+    dL = 1.0 + 0.5 * torch.rand((32, 32, 3), generator=torch.Generator(device="cuda").manual_seed(1), device="cuda")
+    diff = N.DiffParams(albedo.data_ptr(), emission.data_ptr())
+    for backward in (False, True):
+        whole = _pass(scene, r.params(n), diff, torch, albedo, emission, dL, backward)
+        parts = [np.zeros_like(x) for x in whole]
+        for off in range(0, n, PART):
+            m = min(PART, n - off)
+            for acc, x in zip(parts, _pass(scene, r.params(m, sample_offset=off), diff, torch, albedo, emission, dL, backward)):
+                acc += x * (m / n)                   # a pass scales by W*H / its own samples
+        for got, want in zip(whole, parts):
+            # Single-precision sums of up to n terms in two orders: rounding of sqrt(n) ulps of the largest partial sums.
+            assert np.linalg.norm(got - want) <= 4 * np.sqrt(n) * 6e-8 * np.linalg.norm(want) + 1e-12
+            assert np.linalg.norm(want) > 0 or max_pv == 2   # (one bounce: light seen directly, no albedo on any prefix)
+    scene.close()
