@@ -524,6 +524,8 @@ int upload_table(LmgpuBatch* b, const LmgpuRenderParams* params, void* const* fi
         e.rc.sample_base = p.sample_offset;
         e.rc.pixels = (int64_t)e.s.cam.width * e.s.cam.height;
         e.rc.inv_pixels = 1.0 / double(e.rc.pixels);
+        e.rc.order = sample_order(p.num_samples, e.s.cam.width, e.s.cam.height, p.sampling == LMGPU_SAMPLING_STRATIFIED);
+        e.rc.path_base = 0;
         e.begin = begin;
         e.film = films[i];
         b->h_begins[i] = begin;

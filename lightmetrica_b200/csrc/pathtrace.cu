@@ -193,10 +193,12 @@ int render_waves(LmgpuScene* sc, const LmgpuRenderParams& p, F* film, cudaStream
     c.seed = p.seed;
     c.pixels = pixels;
     c.inv_pixels = 1.0 / double(pixels);
+    c.sample_base = p.sample_offset;
+    c.order = sample_order(p.num_samples, s.cam.width, s.cam.height, p.sampling == LMGPU_SAMPLING_STRATIFIED);
     const int shade_blocks = 148 * 8;
     for (int64_t base = 0; base < p.num_samples && rc == LMGPU_OK; base += P) {
         const int64_t cnt = std::min<int64_t>(P, p.num_samples - base);
-        c.sample_base = p.sample_offset + base;
+        c.path_base = base;
         const OneScene<F> ctx{ s, c, film };
         stats.waves++;
         stats.paths += cnt;
@@ -286,11 +288,10 @@ DeviceWorkspace& device_workspace(int device)
     return *e;
 }
 
-template <class F>
-__global__ void k_rescale(const F* film, float* out, int64_t n, double scale)
+__global__ void k_rescale(const double* film, float* out, int64_t n, double scale)
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = (float)((double)film[i] * scale);
+    if (i < n) out[i] = (float)(film[i] * scale);
 }
 
 // lmgpu_render's film buffers, one set per device, kept between calls: the
@@ -497,17 +498,19 @@ int lmgpu_render(LmgpuScene* scene, const LmgpuRenderParams* params, float* film
     if (rc != LMGPU_OK) return rc;
     if (!film_host) return fail(LMGPU_ERR_INVALID, "null film");
     const int64_t n = 3 * (int64_t)scene->dev.cam.width * scene->dev.cam.height;
-    const size_t esize = params->film_fp64 ? sizeof(double) : sizeof(float);
+    // The sums are made in double whatever the caller's film type: a float film's rounding
+    // grows with the samples of a pixel (4e-3 of a constant pixel at 40,000).
+    LmgpuRenderParams p = *params;
+    p.film_fp64 = 1;
     HostFilmBuffers& hb = host_film_buffers(scene->device);
     std::lock_guard<std::mutex> lock(hb.mu);
-    if ((rc = ensure_host_film(hb, n * esize, n * sizeof(float))) != LMGPU_OK) return rc;
-    LMGPU_CUDA_TRY(cudaMemsetAsync(hb.film, 0, n * esize, nullptr));
-    if ((rc = lmgpu_render_device(scene, params, hb.film, nullptr, stats)) != LMGPU_OK) return rc;
+    if ((rc = ensure_host_film(hb, n * sizeof(double), n * sizeof(float))) != LMGPU_OK) return rc;
+    LMGPU_CUDA_TRY(cudaMemsetAsync(hb.film, 0, n * sizeof(double), nullptr));
+    if ((rc = lmgpu_render_device(scene, &p, hb.film, nullptr, stats)) != LMGPU_OK) return rc;
     // Rescale(W * H / num_samples) (sched.mt.cpp:250-256, hdrfilm.cpp:334-341).
     const double scale = double(scene->dev.cam.width) * scene->dev.cam.height / double(params->num_samples);
     const unsigned blocks = (unsigned)((n + 255) / 256);
-    if (params->film_fp64) k_rescale<double><<<blocks, 256>>>(static_cast<const double*>(hb.film), hb.out, n, scale);
-    else k_rescale<float><<<blocks, 256>>>(static_cast<const float*>(hb.film), hb.out, n, scale);
+    k_rescale<<<blocks, 256>>>(static_cast<const double*>(hb.film), hb.out, n, scale);
     LMGPU_CUDA_TRY(cudaGetLastError());
     LMGPU_CUDA_TRY(cudaMemcpyAsync(hb.pinned, hb.out, n * sizeof(float), cudaMemcpyDeviceToHost, nullptr));
     LMGPU_CUDA_TRY(cudaStreamSynchronize(nullptr));

@@ -75,6 +75,63 @@ __device__ __forceinline__ void stratified_raster(int64_t sample, int64_t pixels
     ry = (float(y) + u1) / float(height);
 }
 
+// The order in which a render's paths take its samples. Sample j of a
+// stratified render belongs to pixel j mod (W*H), so the samples come in planes of W*H.
+// Paths take whole planes pixel by pixel, the pixels in blocks of 8 x 4, so that a warp's
+// camera rays, first hits and first shadow rays lie together. Any order renders
+// the same paths (a path depends on its sample index alone). A trailing part of a
+// plane, and uniform sampling (samples lie anywhere), keep the index order.
+// Measured against the index order: six-scene batch 26.6 -> 25.1 ms, terrain
+// 641 x 359 x 8 1.95 -> 1.91 ms, 1080p terrain frame 15.14 -> 15.10 ms. Plane by plane
+// within a block took 5 % longer on the batch and 2 % on the frame. (The differentiable
+// passes keep the index order: a warp on one pixel adds its gradients to one triangle,
+// 16.2 -> 16.3 ms.)
+struct SampleOrder {
+    int64_t ordered;       // samples in whole planes (0: index order)
+    int64_t planes, pixels;
+    double inv_planes;
+    uint32_t width, height;
+};
+
+inline SampleOrder sample_order(int64_t num_samples, int width, int height, bool stratified)
+{
+    SampleOrder o;
+    o.pixels = (int64_t)width * height;
+    o.planes = stratified && o.pixels > 0 ? num_samples / o.pixels : 0;
+    o.ordered = o.planes * o.pixels;
+    o.inv_planes = o.planes > 0 ? 1.0 / double(o.planes) : 0.0;
+    o.width = (uint32_t)width;
+    o.height = (uint32_t)height;
+    return o;
+}
+
+// Sample index (from the render's first) of path number l: a permutation of
+// [0, num_samples). l < 2^53, so the double-precision quotient is off by at most one.
+__host__ __device__ __forceinline__ int64_t ordered_sample(const SampleOrder& o, int64_t l)
+{
+    if (l >= o.ordered) return l;
+    int64_t q = (int64_t)(double(l) * o.inv_planes);
+    int64_t plane = l - q * o.planes;
+    if (plane < 0) { plane += o.planes; q--; }
+    else if (plane >= o.planes) { plane -= o.planes; q++; }
+    uint32_t p = (uint32_t)q;
+    const uint32_t w = o.width, band = p / (4u * w);
+    if (4u * band + 4u <= o.height) {          // four whole rows: blocks, then the columns left over
+        uint32_t r = p - band * 4u * w, x, y;
+        const uint32_t w8 = w & ~7u;
+        if (r < 4u * w8) {
+            x = (r >> 5 << 3) | (r & 7u);
+            y = (r >> 3) & 3u;
+        } else {
+            r -= 4u * w8;
+            y = r / (w - w8);
+            x = w8 + (r - y * (w - w8));
+        }
+        p = (4u * band + y) * w + x;
+    }
+    return plane * o.pixels + p;
+}
+
 // SampleAndEstimateDirection (perspectivecamera.cpp:216-240): raster in
 // [0,1]^2 -> world direction; pdf = importance (projected solid angle);
 // the estimated weight We/pdf is 1.

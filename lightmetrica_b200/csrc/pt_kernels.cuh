@@ -76,9 +76,11 @@ struct RenderConsts {
     int32_t max_pv;
     int32_t sampling;
     uint64_t seed;
-    int64_t sample_base;   // OneScene: sample index of the wave's path 0; SceneTable: the scene's sample offset
+    int64_t sample_base;   // the scene's sample offset (differentiable passes: sample index of the wave's path 0)
     int64_t pixels;
     double inv_pixels;     // 1 / pixels
+    SampleOrder order;     // path numbers to sample indices (renders)
+    int64_t path_base;     // OneScene: path number of the wave's path 0
 };
 
 template <class F>
@@ -88,6 +90,35 @@ __device__ __forceinline__ void film_add(F* film, int pixel, V3 c)
     atomicAdd(film + 3 * pixel, (F)c.x);
     atomicAdd(film + 3 * pixel + 1, (F)c.y);
     atomicAdd(film + 3 * pixel + 2, (F)c.z);
+}
+
+// The film adds of a warp (all its lanes call it) whose neighbouring lanes mostly
+// share a pixel (see SampleOrder): each run of lanes with the same pixel is summed by
+// shuffles and added once. Splat of a 1080p x 8 wave: 169 -> 125 us; and a float film
+// takes up to 32 times fewer roundings.
+template <class F>
+__device__ __forceinline__ void film_add_runs(F* film, int pixel, V3 c)
+{
+    constexpr unsigned FULL = 0xffffffffu;
+    const unsigned lane = threadIdx.x & 31u;
+    const unsigned long long key = pixel < 0 ? 0ull : reinterpret_cast<unsigned long long>(film + 3 * (int64_t)pixel);
+    const unsigned long long before = __shfl_up_sync(FULL, key, 1);
+    const bool head = lane == 0 || before != key;
+    const unsigned heads = __ballot_sync(FULL, head);
+    if (heads == FULL) { film_add(film, pixel, c); return; }
+    const int run = __popc(heads & ((2u << lane) - 1u));
+    F x = (F)c.x, y = (F)c.y, z = (F)c.z;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int other = __shfl_down_sync(FULL, run, o);
+        const F a = __shfl_down_sync(FULL, x, o), b = __shfl_down_sync(FULL, y, o), d = __shfl_down_sync(FULL, z, o);
+        if (other == run && lane + o < 32) { x += a; y += b; z += d; }
+    }
+    if (!head || key == 0 || (x == (F)0 && y == (F)0 && z == (F)0)) return;
+    F* p = reinterpret_cast<F*>(key);
+    atomicAdd(p, x);
+    atomicAdd(p + 1, y);
+    atomicAdd(p + 2, z);
 }
 
 // ------------------------------------------------------------ contexts ----
@@ -135,11 +166,14 @@ struct OneScene : RenderContext {
     // Scene index and scene-local sample index of wave path i.
     __device__ __forceinline__ int locate(int64_t i, int64_t& sample) const
     {
-        sample = rc.sample_base + i;
+        sample = sample_of(0, i);
         return 0;
     }
     __device__ __forceinline__ int path_scene(const PathState&, int64_t) const { return 0; }
-    __device__ __forceinline__ int64_t sample_of(int, int64_t i) const { return rc.sample_base + i; }
+    __device__ __forceinline__ int64_t sample_of(int, int64_t i) const
+    {
+        return rc.sample_base + ordered_sample(rc.order, rc.path_base + i);
+    }
     __device__ __forceinline__ F* film_of(int) const { return film; }
     __device__ __forceinline__ void lit_pixel(int, int pixel, V3 c) const { film_add(film, pixel, c); }
     // New path number j of this launch: its slot i and scene-local sample.
@@ -190,13 +224,13 @@ struct SceneTable : RenderContext {
             if (begins[mid] <= g) lo = mid;
             else hi = mid;
         }
-        sample = table[lo].rc.sample_base + (g - begins[lo]);
+        sample = table[lo].rc.sample_base + ordered_sample(table[lo].rc.order, g - begins[lo]);
         return lo;
     }
     __device__ __forceinline__ int path_scene(const PathState& st, int64_t i) const { return st.scene[i]; }
     __device__ __forceinline__ int64_t sample_of(int sid, int64_t i) const
     {
-        return table[sid].rc.sample_base + (wave->base + i - table[sid].begin);
+        return table[sid].rc.sample_base + ordered_sample(table[sid].rc.order, wave->base + i - table[sid].begin);
     }
     __device__ __forceinline__ F* film_of(int sid) const { return static_cast<F*>(table[sid].film); }
     __device__ __forceinline__ void lit_pixel(int sid, int pixel, V3 c) const { film_add(film_of(sid), pixel, c); }
@@ -242,7 +276,7 @@ struct StreamTable : RenderContext {
     __device__ __forceinline__ int path_scene(const PathState& st, int64_t i) const { return st.scene[i]; }
     __device__ __forceinline__ int64_t sample_of(int sid, int64_t i) const
     {
-        return table[sid].rc.sample_base + (sample[i] - table[sid].begin);
+        return table[sid].rc.sample_base + ordered_sample(table[sid].rc.order, sample[i] - table[sid].begin);
     }
     __device__ __forceinline__ F* film_of(int sid) const { return static_cast<F*>(table[sid].film); }
     __device__ __forceinline__ void lit_pixel(int sid, int pixel, V3 c) const { film_add(film_of(sid), pixel, c); }
@@ -256,7 +290,7 @@ struct StreamTable : RenderContext {
             if (begins[mid] <= g) lo = mid;
             else hi = mid;
         }
-        local = table[lo].rc.sample_base + (g - begins[lo]);
+        local = table[lo].rc.sample_base + ordered_sample(table[lo].rc.order, g - begins[lo]);
         st.scene[i] = lo;
         st.sample[i] = g;
         st.depth[i] = 1;
@@ -672,10 +706,10 @@ template <class Ctx>
 __global__ void __launch_bounds__(128) k_pt_splat(const Ctx ctx, const PathState st, int64_t count)
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= ctx.wave_count(count)) return;
-    const int sid = ctx.path_scene(st, i);
-    const float2 r = st.raster[i];
-    film_add(ctx.film_of(sid), film_pixel(ctx.scene(sid).cam, r.x, r.y), f3(st.L[i]));
+    const bool valid = i < ctx.wave_count(count);
+    const int sid = valid ? ctx.path_scene(st, i) : 0;
+    const float2 r = valid ? st.raster[i] : make_float2(-1.0f, 0.0f);
+    film_add_runs(ctx.film_of(sid), film_pixel(ctx.scene(sid).cam, r.x, r.y), valid ? f3(st.L[i]) : v3(0, 0, 0));
 }
 
 }  // namespace lmgpu

@@ -132,7 +132,9 @@ class RenderProcessScheduler:
         import time
         import torch
         W, H = cam.film.width, cam.film.height
-        dev_film = torch.zeros(W * H * 3, dtype=torch.float64 if self.film_fp64 else torch.float32, device="cuda")
+        # Many small passes into one film: a double film, so that a pass's rounding
+        # does not grow with the passes before it.
+        dev_film = torch.zeros(W * H * 3, dtype=torch.float64, device="cuda")
         stream = torch.cuda.current_stream().cuda_stream
         timed = self.termination_mode == "time"
         chunk = self.num_samples if timed else max(W * H, self.num_samples // 64)
@@ -152,7 +154,7 @@ class RenderProcessScheduler:
                 if done >= self.num_samples:
                     break
                 n = min(chunk, self.num_samples - done)
-            p = renderer.params(n, sample_offset=done, film_fp64=self.film_fp64, wave_paths=self.wave_paths)
+            p = renderer.params(n, sample_offset=done, film_fp64=True, wave_paths=self.wave_paths)
             st = N.RenderStats()
             N.check(N.lib().lmgpu_render_device(scene.handle, ctypes.byref(p), ctypes.c_void_p(dev_film.data_ptr()),
                                                 ctypes.c_void_p(stream), ctypes.byref(st)))

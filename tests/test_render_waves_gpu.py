@@ -1,0 +1,59 @@
+"""The waves of the renderers where they can go wrong: the order in which paths take
+samples (ragged films, parts of a sample plane), bounces traced together with the
+shadow rays before them (deep and many waves), few rays spread over the GPU, and
+ties between coincident triangles."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from lightmetrica_b200 import create_renderer, create_scene, native as N, scenes
+from lightmetrica_b200.batch import SceneBatch
+from lightmetrica_b200.scene import soup_primitives
+from lightmetrica_b200.workloads import random_rays, random_soup, rays_soa
+
+pytestmark = pytest.mark.gpu
+
+
+def _built(prims):
+    s = create_scene("bvh")
+    s.load(prims)
+    s.configure({})
+    s.build()
+    return s
+
+
+def _render(scene, renderer, n, torch, offset=0, wave_paths=0, fp64=True):
+    cam = scene.main_camera()
+    film = torch.zeros(cam.film.width * cam.film.height * 3, dtype=torch.float64 if fp64 else torch.float32, device="cuda")
+    p = renderer.params(n, sample_offset=offset, film_fp64=fp64, wave_paths=wave_paths)
+    st = N.RenderStats()
+    N.check(N.lib().lmgpu_render_device(scene.handle, ctypes.byref(p), ctypes.c_void_p(film.data_ptr()),
+                                        ctypes.c_void_p(torch.cuda.current_stream().cuda_stream), ctypes.byref(st)))
+    return film.cpu().numpy(), st
+
+
+def _renderer(tech, max_pv, rr, sampling="stratified"):
+    r = create_renderer(tech)
+    r.configure({"rr_depth": rr, "max_path_vertices": max_pv, "sampler": {"rng_seed": 3, "sampling": sampling}})
+    return r
+
+
+# A path's radiance is the same in every order; a double film sums it with relative errors of 2^-53 an addition.
+SUMS = dict(rtol=1e-11, atol=1e-13)
+
+
+@pytest.mark.parametrize("w,h,n,split", [(1, 1, 5, 2), (3, 2, 6, 1), (7, 5, 100, 33), (8, 4, 64, 32), (9, 7, 63 * 3 + 11, 70),
+                                         (33, 13, 429 * 8, 429 * 3), (64, 36, 2304 * 33, 2304 * 32 + 1)])
+@pytest.mark.parametrize("tech", ["pt", "pt.mis"])
+def test_any_split_renders_the_same_samples(cuda, tech, w, h, n, split):
+    import torch
+    s = _built(scenes.cornell_box(w, h, variant="mixed"))
+    r = _renderer(tech, 6, 3)
+    whole, _ = _render(s, r, n, torch)
+    parts = _render(s, r, split, torch)[0] + _render(s, r, n - split, torch, offset=split)[0]
+    assert whole.any()
+    np.testing.assert_allclose(whole, parts, **SUMS)
+    single, _ = _render(s, r, n, torch, fp64=False)
+    np.testing.assert_allclose(single, whole, rtol=n * 6e-8, atol=1e-6)   # n additions of 2^-24 relative error each
+    s.close()
