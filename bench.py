@@ -310,12 +310,14 @@ def _sum_over_ranks(value, dev, world):
 
 def _batch_launches(cfg, stats, bounces):
     """Kernels one batch render launches (captured or direct): per wave
-    k_wave_begin, init, the camera-vertex shadow pass, `bounces` x (bounce
-    prep, closest hit, shade, shadow), splat, k_wave_end, plus one setup
-    kernel; stream mode: six kernels per iteration."""
+    k_wave_begin, init, `bounces` x (trace, shade), splat, k_wave_end, a shadow
+    pass of its own for the camera vertex and the first three vertices after it,
+    one for the last vertex of deeper waves (the traces of the bounces between take
+    theirs along), plus one setup kernel; stream mode: six kernels per iteration."""
     if cfg["mode"] == "stream":
         return 6 * stats["waves"] + 1
-    return stats["waves"] * (5 + 4 * bounces) + 1
+    shadows = min(bounces + 1, 4) + (1 if bounces >= 4 else 0)
+    return stats["waves"] * (4 + 2 * bounces + shadows) + 1
 
 
 def frame_roofline(prof_count, prof_time):
@@ -665,8 +667,7 @@ def _timed_device_renders(L, scene, renderer, num_samples, film, stream, reps, n
 
 
 def render_section(args, dev):
-    """The plain one-scene wavefront renderer (lmgpu_render_device: the host
-    reads each bounce's queue sizes back to size the next launch) on the
+    """The plain one-scene wavefront renderer (lmgpu_render_device) on the
     headline frame, and end to end through the scheduler (host film)."""
     import torch
     from lightmetrica_b200 import create_renderer, create_scene, create_scheduler, native, scenes

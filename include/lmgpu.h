@@ -257,7 +257,7 @@ int lmgpu_render(LmgpuScene* scene, const LmgpuRenderParams* params,
 /* Device variant: accumulates un-rescaled contributions into a DEVICE film
  * (float, or double when film_fp64) on `stream`; the caller rescales by
  * W*H/num_samples. The call returns once the render's device work is done
- * (it reads each bounce's queue sizes back to size the next launch). Waves
+ * (a wave of more than 8 bounces asks every 4 whether a path is left). Waves
  * hold `wave_paths` paths (0 = 2^27, fewer if device memory is short) in a
  * workspace of about 216 bytes per path that is shared by all scenes of the
  * device and kept until exit; calls on one device take turns. */
@@ -286,8 +286,8 @@ int lmgpu_render_release(void);
  * array's device address, so make it before any stream capture. All calls
  * share the one array, and the counters in it are cleared at the start of
  * each wave, but calls that overlap on the GPU race: run them one after
- * another. Like lmgpu_render_device, the call reads each bounce's queue
- * sizes back to the host, so it synchronises `stream` after every bounce. */
+ * another. Like lmgpu_render_device, the call synchronises `stream` within
+ * deep waves and at its end. */
 int lmgpu_render_device_noalloc(LmgpuScene* scene, const LmgpuRenderParams* params,
                                 void* film_device, void* stream);
 

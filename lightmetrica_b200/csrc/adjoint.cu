@@ -554,13 +554,6 @@ struct DiffScene : RenderContext {
     }
 };
 
-// Before a bounce: clear its output queue and the shadow queue.
-__global__ void k_diff_prep(uint32_t* counters, int qout)
-{
-    counters[qout] = 0;
-    counters[2] = 0;
-}
-
 // Forward, end of a wave: each path's radiance to its pixel.
 __global__ void __launch_bounds__(128) k_diff_splat(const DiffScene<false> ctx, const PathState st, int64_t n)
 {
@@ -614,7 +607,7 @@ __global__ void __launch_bounds__(128) k_diff_tail(const DiffScene<BACKWARD> ctx
         for (int i = threadIdx.x; i < 3 * SHARED_LIGHTS; i += blockDim.x) s_de[i] = 0.0f;
         __syncthreads();
     }
-    const int64_t n = (int64_t)st.counters[q];
+    const int64_t n = (int64_t)st.counters[ring_rays(k0)];
     for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x) {
         const float4 o4 = st.qo[q][j], d4 = st.qd[q][j], t4 = st.qt[q][j];
         const float4 n4 = TECH == LMGPU_RENDER_PT ? make_float4(0, 0, 1, 0) : st.qn[q][j];
@@ -699,10 +692,9 @@ int run_diff_waves(LmgpuScene* sc, const DiffConsts& c, float* image, const floa
     const int lights = s.num_area_lights;
     int copies = 1;
     while (2 * copies <= EMISSION_COPIES && 2 * copies * std::max(lights, 1) <= 64 * EMISSION_COPIES) copies *= 2;
-    // Workspace: counters, work slots, emission partial sums, then the path state.
-    const int slots = 2 * bounces + 1;
+    // Workspace: counters, emission partial sums, then the path state.
     const size_t emission_bytes = BACKWARD ? (size_t)copies * lights * 3 * sizeof(double) : 0;
-    const size_t head = (256 + slots * sizeof(unsigned long long) + emission_bytes + 255) / 256 * 256;
+    const size_t head = (256 + emission_bytes + 255) / 256 * 256;
     const size_t per_path = 16 * 13 + 8 + (BACKWARD ? 4 + 16 * (size_t)bounces : 0);
     cudaMemPool_t pool = nullptr;
     LMGPU_CUDA_TRY(diff_pool_of(sc->device, &pool));
@@ -718,7 +710,6 @@ int run_diff_waves(LmgpuScene* sc, const DiffConsts& c, float* image, const floa
     }
     PathState st{};
     st.counters = reinterpret_cast<uint32_t*>(mem);
-    unsigned long long* work = reinterpret_cast<unsigned long long*>(mem + 256);
     char* p = mem + head;
     auto take = [&](size_t b) { char* r = p; p += b; return r; };
     Ctx ctx;
@@ -756,33 +747,37 @@ int run_diff_waves(LmgpuScene* sc, const DiffConsts& c, float* image, const floa
     ctx.dL = dL;
     ctx.stride = P;
     ctx.hit_no = 0;
-    ctx.d_emission = reinterpret_cast<double*>(mem + 256 + slots * sizeof(unsigned long long));
+    ctx.d_emission = reinterpret_cast<double*>(mem + 256);
     ctx.copies = copies;
     cudaError_t e = emission_bytes ? cudaMemsetAsync(ctx.d_emission, 0, emission_bytes, stream) : cudaSuccess;
-    auto closest = k_trace_persistent<STACK, false, PathRayIO<false>>;
-    auto any = k_trace_persistent<STACK, true, ShadowIO<Ctx>>;
+    auto closest = k_trace_persistent<STACK, TRACE_CLOSEST, PathRayIO<false>>;
+    auto both = k_trace_persistent<STACK, TRACE_MIXED, BounceIO<Ctx>>;
+    auto any = k_trace_persistent<STACK, TRACE_ANY, ShadowIO<Ctx>>;
+    auto work = [&](int word) { return work_counter(st.counters, word); };
     for (int64_t base = 0; base < c.num_samples && e == cudaSuccess; base += P) {
         const int64_t n = std::min(P, c.num_samples - base);
         const int64_t full = (n + 127) / 128;
         const unsigned shade = (unsigned)std::min<int64_t>(full, 148 * 8);
-        const unsigned rays = (unsigned)std::min<int64_t>(full, resident_blocks(closest));
-        const unsigned shadows = (unsigned)std::min<int64_t>(full, resident_blocks(any));
+        auto grid = [&](auto kernel, int64_t blocks) { return (unsigned)std::min<int64_t>(blocks, resident_blocks(kernel)); };
         ctx.rc.sample_base = c.sample_offset + base;
-        auto shadow = [&](int k) {
-            ctx.hit_no = k;
-            ShadowIO<Ctx> io{ st.counters + 2, st.sh_o, st.sh_d, st.sh_c, st.L, ctx };
-            any<<<shadows, 128, 0, stream>>>(s, io, sc->d_status, work + 2 * k, nullptr);
-        };
-        k_wave_begin<<<1, 128, 0, stream>>>(st.counters, work, slots);
-        k_pt_init<TECH, Ctx><<<(unsigned)full, 128, 0, stream>>>(ctx, st, n, 0);
-        if (TECH != LMGPU_RENDER_PT) shadow(0);
+        k_wave_begin<<<1, 128, 0, stream>>>(st.counters);
+        k_pt_init<TECH, Ctx><<<(unsigned)full, 128, 0, stream>>>(ctx, st, n, 0, ring_rays(1), ring_shadow(0));
         for (int k = 1; k <= bounces; k++) {
             const int qin = (k - 1) & 1;
-            k_diff_prep<<<1, 1, 0, stream>>>(st.counters, 1 - qin);
-            PathRayIO<false> io{ st.counters + qin, st.qo[qin], st.qd[qin], st.hit, nullptr };
-            closest<<<rays, 128, 0, stream>>>(s, io, sc->d_status, work + 2 * k - 1, nullptr);
-            k_pt_shade<TECH, Ctx><<<shade, 128, 0, stream>>>(ctx, st, k, qin, 1 - qin);
-            if (TECH != LMGPU_RENDER_PT) shadow(k);
+            const auto io = ray_queue<false>(st, qin, ring_rays(k), nullptr);
+            ctx.hit_no = k - 1;
+            if (TECH == LMGPU_RENDER_PT) {
+                closest<<<grid(closest, full), 128, 0, stream>>>(s, io, sc->d_status, work(ring_work(k)), nullptr);
+            } else {
+                const BounceIO<Ctx> bio{ io, shadow_queue(st, ring_shadow(k - 1), ctx) };
+                both<<<grid(both, 2 * full), 128, 0, stream>>>(s, bio, sc->d_status, work(ring_work(k)), nullptr);
+            }
+            k_pt_shade<TECH, Ctx><<<shade, 128, 0, stream>>>(ctx, st, k, qin, nullptr);
+        }
+        if (TECH != LMGPU_RENDER_PT) {
+            ctx.hit_no = bounces;
+            any<<<grid(any, full), 128, 0, stream>>>(s, shadow_queue(st, ring_shadow(bounces), ctx), sc->d_status,
+                                                     work(ring_shadow_work(bounces)), nullptr);
         }
         if (tail) k_diff_tail<TECH, STACK, BACKWARD><<<shade, 128, 0, stream>>>(ctx, c, st, bounces & 1, bounces + 1, da, de, sc->d_status);
         if constexpr (BACKWARD) k_diff_flush<<<(unsigned)full, 128, 0, stream>>>(ctx, c, st, n, da);

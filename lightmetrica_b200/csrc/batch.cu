@@ -39,7 +39,7 @@ using namespace lmgpu;
 
 namespace {
 
-constexpr int WORK_SLOTS = 160;            // traversal launches per wave: 2 per bounce + 1
+constexpr int WORK_SLOTS = 4;              // stream mode: closest-hit and shadow launches of an iteration pair
 constexpr int POOLS = 2;                   // path pools (overlap mode uses both)
 constexpr int DEFAULT_OVERLAP_BOUNCE = 3;
 constexpr int GRAPH_BOUNCES_UNBOUNDED = 24;
@@ -92,7 +92,7 @@ struct LmgpuBatch {
     StreamCtl* d_ctl = nullptr;
     int64_t* h_done = nullptr;              // pinned: StreamCtl::done and ::iterations
     unsigned long long* d_stats = nullptr;
-    unsigned long long* d_work = nullptr;   // WORK_SLOTS per path pool
+    unsigned long long* d_work = nullptr;   // stream mode (WORK_SLOTS)
     int32_t* d_status = nullptr;
     BatchEntry* h_table = nullptr;          // pinned staging
     int64_t* h_begins = nullptr;
@@ -153,25 +153,11 @@ __global__ void k_batch_setup(WaveCtl* wave, int pools, int64_t total, int64_t s
     for (int i = 0; i < NSTATS; i++) stats[i] = 0;
 }
 
-// Before bounce k: tally the rays about to be traced and the shadow rays of
-// the previous pass, then clear the output queue and the shadow queue. The
-// totals are shared by the path pools (atomics: pools run concurrently).
-__global__ void k_bounce_prep(uint32_t* counters, int qin, int k, unsigned long long* stats)
-{
-    const uint32_t n = counters[qin];
-    atomicAdd(stats + 0, (unsigned long long)n);
-    atomicAdd(stats + 1, (unsigned long long)counters[2]);
-    if (n > 0) atomicMax(stats + 2, (unsigned long long)k);
-    counters[1 - qin] = 0;
-    counters[2] = 0;
-}
-
 // End of a wave (after the splat): last shadow tally, advance the pool to
 // its next wave.
-__global__ void k_wave_end(WaveCtl* wave, uint32_t* counters, unsigned long long* stats)
+__global__ void k_wave_end(WaveCtl* wave, const uint32_t* last_shadow, unsigned long long* stats)
 {
-    atomicAdd(stats + 1, (unsigned long long)counters[2]);
-    counters[2] = 0;
+    atomicAdd(stats + 1, (unsigned long long)*last_shadow);
     const int64_t base = wave->base + wave->stride;
     wave->base = base;
     const int64_t left = wave->total - base;
@@ -229,13 +215,13 @@ __global__ void k_stream_plan(StreamCtl* ctl, uint32_t* counters, int q, unsigne
 // Launches one persistent traversal of `io`. During a measurement render
 // (b->prof) the launch is bracketed by CUDA events and, when counting, runs
 // the counting instantiation of the same kernel.
-template <int STACK, bool ANY_HIT, class IO>
+template <int STACK, int MODE, class IO>
 void launch_traversal(const LmgpuBatch* b, int blocks, const DeviceScene& proto, const IO& io,
                       unsigned long long* work, cudaStream_t s)
 {
     TraceProfileRun* p = b->prof;
     if (!p) {
-        k_trace_persistent<STACK, ANY_HIT, IO><<<blocks, 128, 0, s>>>(proto, io, b->d_status, work, nullptr);
+        k_trace_persistent<STACK, MODE, IO><<<blocks, 128, 0, s>>>(proto, io, b->d_status, work, nullptr);
         return;
     }
     cudaEvent_t e[2] = { nullptr, nullptr };
@@ -243,14 +229,14 @@ void launch_traversal(const LmgpuBatch* b, int blocks, const DeviceScene& proto,
         if (p->error == cudaSuccess) p->error = cudaEventCreate(&x);
     if (p->error == cudaSuccess) p->error = cudaEventRecord(e[0], s);
     if (p->count)
-        k_trace_persistent<STACK, ANY_HIT, IO, true><<<blocks, 128, 0, s>>>(
-            proto, io, b->d_status, work, p->d_counts + (ANY_HIT ? 2 : 0));
+        k_trace_persistent<STACK, MODE, IO, true><<<blocks, 128, 0, s>>>(
+            proto, io, b->d_status, work, p->d_counts + (MODE == TRACE_ANY ? 2 : 0));
     else
-        k_trace_persistent<STACK, ANY_HIT, IO><<<blocks, 128, 0, s>>>(proto, io, b->d_status, work, nullptr);
+        k_trace_persistent<STACK, MODE, IO><<<blocks, 128, 0, s>>>(proto, io, b->d_status, work, nullptr);
     if (p->error == cudaSuccess) p->error = cudaEventRecord(e[1], s);
     for (cudaEvent_t x : e)
         if (x) p->events.push_back(x);
-    if (e[0] && e[1]) p->kinds.push_back(ANY_HIT ? 1 : 0);
+    if (e[0] && e[1]) p->kinds.push_back(MODE == TRACE_ANY ? 1 : 0);
 }
 
 struct Launch {
@@ -258,16 +244,20 @@ struct Launch {
     int shade_blocks;
     int trace_blocks;          // closest-hit grid
     int shadow_blocks;         // any-hit grid
+    int bounce_blocks;         // grid of both in one launch (waves)
     DeviceScene proto;         // template scene for the traversal kernel (layout only)
 };
 
-// One wave of path pool l: head = begin, init, camera shadow pass, bounces
-// 1 .. T-1; tail = bounces T .. K, splat, advance. The traversal launches of
-// bounce k use work slots slot_of(k) and slot_of(k) + 1 of the pool.
-template <int TECH, class F, int STACK>
+// One wave of path pool l: head = begin, init, bounces 1 .. T-1; tail = bounces
+// T .. K, the last shadow pass, splat, advance. From bounce TABLE_MERGE on a bounce
+// traces its rays together with the previous vertices' shadow rays; a measurement
+// render (b->prof) always traces the two apart. SOLO: one scene, whose accelerator the
+// traversals take from their parameters instead of from each ray's scene.
+template <int TECH, class F, int STACK, bool SOLO>
 struct Wave {
     using Ctx = SceneTable<float>;     // init / shade use no film
-    using FilmCtx = SceneTable<F>;
+    using FilmCtx = std::conditional_t<SOLO, SoloTable<F>, SceneTable<F>>;
+    static bool merged(const LmgpuBatch* b, int k) { return TECH != LMGPU_RENDER_PT && !b->prof && k >= TABLE_MERGE; }
 
     static Ctx ctx(const LmgpuBatch* b, int l)
     {
@@ -277,59 +267,65 @@ struct Wave {
     {
         return FilmCtx{ b->d_table, b->d_begins, (int32_t)b->scenes.size(), b->d_wave + l };
     }
-    static unsigned long long* work(const LmgpuBatch* b, int l) { return b->d_work + (size_t)l * WORK_SLOTS; }
-    static int slot_of(int k) { return (TECH != LMGPU_RENDER_PT ? 1 : 0) + 2 * (k - 1); }
 
-    static void shadow(const LmgpuBatch* b, const Launch& L, int l, int slot, cudaStream_t s)
+    static void shadow(const LmgpuBatch* b, const Launch& L, int l, int k, cudaStream_t s)
     {
         const PathState& st = b->st[l];
-        ShadowIO<FilmCtx> io{ st.counters + 2, st.sh_o, st.sh_d, st.sh_c, st.L, film_ctx(b, l) };
-        launch_traversal<STACK, true>(b, L.shadow_blocks, L.proto, io, work(b, l) + slot, s);
+        launch_traversal<STACK, TRACE_ANY>(b, L.shadow_blocks, L.proto, shadow_queue(st, ring_shadow(k), film_ctx(b, l)),
+                                           work_counter(st.counters, ring_shadow_work(k)), s);
     }
 
-    static void bounce(const LmgpuBatch* b, const Launch& L, int l, int k, int slot, cudaStream_t s)
+    static void bounce(const LmgpuBatch* b, const Launch& L, int l, int k, cudaStream_t s)
     {
         const PathState& st = b->st[l];
         const int qin = (k - 1) & 1;
-        k_bounce_prep<<<1, 1, 0, s>>>(st.counters, qin, k, b->d_stats);
-        PathRayIO<true> io{ st.counters + qin, st.qo[qin], st.qd[qin], st.hit, b->d_table };
-        launch_traversal<STACK, false>(b, L.trace_blocks, L.proto, io, work(b, l) + slot, s);
-        k_pt_shade<TECH, Ctx><<<L.shade_blocks, 128, 0, s>>>(ctx(b, l), st, k, qin, 1 - qin);
-        if (TECH != LMGPU_RENDER_PT) shadow(b, L, l, slot + 1, s);
+        unsigned long long* work = work_counter(st.counters, ring_work(k));
+        const auto rays = ray_queue<!SOLO>(st, qin, ring_rays(k), b->d_table);
+        if (!merged(b, k)) {
+            launch_traversal<STACK, TRACE_CLOSEST>(b, L.trace_blocks, L.proto, rays, work, s);
+        } else {
+            const BounceIO<FilmCtx> io{ rays, shadow_queue(st, ring_shadow(k - 1), film_ctx(b, l)) };
+            k_trace_persistent<STACK, TRACE_MIXED, BounceIO<FilmCtx>><<<L.bounce_blocks, 128, 0, s>>>(L.proto, io, b->d_status, work, nullptr);
+        }
+        k_pt_shade<TECH, Ctx><<<L.shade_blocks, 128, 0, s>>>(ctx(b, l), st, k, qin, b->d_stats);
+        if (TECH != LMGPU_RENDER_PT && !merged(b, k + 1)) shadow(b, L, l, k, s);
     }
 
     static void head(const LmgpuBatch* b, const Launch& L, int l, int T, cudaStream_t s)
     {
         const PathState& st = b->st[l];
-        k_wave_begin<<<1, 128, 0, s>>>(st.counters, work(b, l), WORK_SLOTS);
-        k_pt_init<TECH, Ctx><<<(unsigned)((L.paths + 127) / 128), 128, 0, s>>>(ctx(b, l), st, 0, 0);
-        if (TECH != LMGPU_RENDER_PT) shadow(b, L, l, 0, s);
-        for (int k = 1; k < T; k++) bounce(b, L, l, k, slot_of(k), s);
+        k_wave_begin<<<1, 128, 0, s>>>(st.counters);
+        k_pt_init<TECH, Ctx><<<(unsigned)((L.paths + 127) / 128), 128, 0, s>>>(ctx(b, l), st, 0, 0, ring_rays(1), ring_shadow(0));
+        if (TECH != LMGPU_RENDER_PT && !merged(b, 1)) shadow(b, L, l, 0, s);
+        for (int k = 1; k < T; k++) bounce(b, L, l, k, s);
     }
 
     static void tail(const LmgpuBatch* b, const Launch& L, int l, int T, int K, cudaStream_t s)
     {
-        for (int k = T; k <= K; k++) bounce(b, L, l, k, slot_of(k), s);
-        tail_end(b, L, l, s);
+        for (int k = T; k <= K; k++) bounce(b, L, l, k, s);
+        tail_end(b, L, l, K, s);
     }
 
-    // Pool 0: init + bounces 1..K (+ splat and wave advance when `finish`).
+    // Pool 0: init + bounces 1..K (+ last shadow pass, splat and wave advance when `finish`).
     static void body(const LmgpuBatch* b, const Launch& L, int K, bool finish, cudaStream_t s)
     {
         head(b, L, 0, K + 1, s);
-        if (finish) tail_end(b, L, 0, s);
+        if (finish) tail_end(b, L, 0, K, s);
     }
 
-    static void tail_end(const LmgpuBatch* b, const Launch& L, int l, cudaStream_t s)
+    // After the last bounce K.
+    static void tail_end(const LmgpuBatch* b, const Launch& L, int l, int K, cudaStream_t s)
     {
+        if (merged(b, K + 1)) shadow(b, L, l, K, s);
         k_pt_splat<FilmCtx><<<(unsigned)((L.paths + 127) / 128), 128, 0, s>>>(film_ctx(b, l), b->st[l], 0);
-        k_wave_end<<<1, 1, 0, s>>>(b->d_wave + l, b->st[l].counters, b->d_stats);
+        k_wave_end<<<1, 1, 0, s>>>(b->d_wave + l, b->st[l].counters + ring_shadow(K), b->d_stats);
     }
 
     static void warm(Launch& L)
     {
-        L.trace_blocks = resident_blocks(k_trace_persistent<STACK, false, PathRayIO<true>>);
-        L.shadow_blocks = resident_blocks(k_trace_persistent<STACK, true, ShadowIO<FilmCtx>>);
+        L.trace_blocks = resident_blocks(k_trace_persistent<STACK, TRACE_CLOSEST, PathRayIO<!SOLO>>);
+        L.shadow_blocks = resident_blocks(k_trace_persistent<STACK, TRACE_ANY, ShadowIO<FilmCtx>>);
+        L.bounce_blocks = resident_blocks(k_trace_persistent<STACK, TRACE_MIXED, BounceIO<FilmCtx>>);
     }
 };
 
@@ -350,14 +346,12 @@ struct Stream {
         const PathState& st = b->st[0];
         unsigned long long* work = b->d_work + 2 * q;
         k_stream_plan<<<1, 1, 0, s>>>(b->d_ctl, st.counters, q, b->d_stats, work);
-        k_pt_init<TECH, Ctx><<<(unsigned)((L.paths + 127) / 128), 128, 0, s>>>(make<Ctx>(b), st, 0, q);
-        PathRayIO<true> io{ st.counters + q, st.qo[q], st.qd[q], st.hit, b->d_table };
-        launch_traversal<STACK, false>(b, L.trace_blocks, L.proto, io, work, s);
-        k_pt_shade<TECH, Ctx><<<L.shade_blocks, 128, 0, s>>>(make<Ctx>(b), st, 0, q, 1 - q);
-        if (TECH != LMGPU_RENDER_PT) {
-            ShadowIO<FilmCtx> sio{ st.counters + 2, st.sh_o, st.sh_d, st.sh_c, st.L, make<FilmCtx>(b) };
-            launch_traversal<STACK, true>(b, L.shadow_blocks, L.proto, sio, work + 1, s);
-        }
+        k_pt_init<TECH, Ctx><<<(unsigned)((L.paths + 127) / 128), 128, 0, s>>>(make<Ctx>(b), st, 0, q, COUNTER_RAYS[q], COUNTER_SHADOW);
+        launch_traversal<STACK, TRACE_CLOSEST>(b, L.trace_blocks, L.proto, ray_queue<true>(st, q, COUNTER_RAYS[q], b->d_table), work, s);
+        k_pt_shade<TECH, Ctx><<<L.shade_blocks, 128, 0, s>>>(make<Ctx>(b), st, 0, q, nullptr);
+        if (TECH != LMGPU_RENDER_PT)
+            launch_traversal<STACK, TRACE_ANY>(b, L.shadow_blocks, L.proto, shadow_queue(st, COUNTER_SHADOW, make<FilmCtx>(b)),
+                                               work + 1, s);
         k_pt_retire<FilmCtx><<<L.shade_blocks, 128, 0, s>>>(make<FilmCtx>(b), st);
     }
 
@@ -369,8 +363,8 @@ struct Stream {
 
     static void warm(Launch& L)
     {
-        L.trace_blocks = resident_blocks(k_trace_persistent<STACK, false, PathRayIO<true>>);
-        L.shadow_blocks = resident_blocks(k_trace_persistent<STACK, true, ShadowIO<FilmCtx>>);
+        L.trace_blocks = resident_blocks(k_trace_persistent<STACK, TRACE_CLOSEST, PathRayIO<true>>);
+        L.shadow_blocks = resident_blocks(k_trace_persistent<STACK, TRACE_ANY, ShadowIO<FilmCtx>>);
     }
 };
 
@@ -600,10 +594,10 @@ int run_stream(LmgpuBatch* b, const Plan& pl, int64_t P, cudaStream_t s, int64_t
 // after them; floor(W / 2) periods cover W waves (a wave past the last
 // sample has no paths and costs only its launches). Depth must be
 // bounded: the tail is a fixed sequence of bounces.
-template <int TECH, class F, int STACK>
+template <int TECH, class F, int STACK, bool SOLO>
 int run_overlap(LmgpuBatch* b, const Plan& pl, int64_t P, cudaStream_t s, int64_t& waves)
 {
-    using W = Wave<TECH, F, STACK>;
+    using W = Wave<TECH, F, STACK, SOLO>;
     Launch L;
     L.paths = P;
     L.shade_blocks = std::max(1, b->cfg.shade_blocks_per_sm) * b->sms;
@@ -680,12 +674,12 @@ int run_overlap(LmgpuBatch* b, const Plan& pl, int64_t P, cudaStream_t s, int64_
     return LMGPU_OK;
 }
 
-template <int TECH, class F, int STACK>
+template <int TECH, class F, int STACK, bool SOLO>
 int run_waves(LmgpuBatch* b, const Plan& pl, int64_t P, cudaStream_t s, int64_t& waves)
 {
     if (b->cfg.mode == LMGPU_BATCH_STREAM) return run_stream<TECH, F, STACK>(b, pl, P, s, waves);
-    if (b->cfg.mode == LMGPU_BATCH_OVERLAP && pl.bounded) return run_overlap<TECH, F, STACK>(b, pl, P, s, waves);
-    using W = Wave<TECH, F, STACK>;
+    if (b->cfg.mode == LMGPU_BATCH_OVERLAP && pl.bounded) return run_overlap<TECH, F, STACK, SOLO>(b, pl, P, s, waves);
+    using W = Wave<TECH, F, STACK, SOLO>;
     Launch L;
     L.paths = P;
     L.shade_blocks = std::max(1, b->cfg.shade_blocks_per_sm) * b->sms;
@@ -715,17 +709,16 @@ int run_waves(LmgpuBatch* b, const Plan& pl, int64_t P, cudaStream_t s, int64_t&
         LMGPU_CUDA_TRY(cudaGetLastError());
         if (pl.bounded) continue;
         // Unbounded depth: finish the wave's remaining bounces directly.
-        const int slot = (TECH != LMGPU_RENDER_PT ? 1 : 0);   // counters reused: clear before each launch
-        for (int k = pl.bounces + 1;; k++) {
-            const int qin = (k - 1) & 1;
-            LMGPU_CUDA_TRY(cudaMemcpyAsync(b->h_counts, b->st[0].counters, 16, cudaMemcpyDeviceToHost, s));
+        int k = pl.bounces + 1;
+        for (;; k++) {
+            LMGPU_CUDA_TRY(cudaMemcpyAsync(b->h_counts, b->st[0].counters + ring_rays(0), RING * sizeof(uint32_t),
+                                           cudaMemcpyDeviceToHost, s));
             LMGPU_CUDA_TRY(cudaStreamSynchronize(s));
-            if (b->h_counts[qin] == 0) break;
-            LMGPU_CUDA_TRY(cudaMemsetAsync(b->d_work + slot, 0, 2 * sizeof(unsigned long long), s));
-            W::bounce(b, L, 0, k, slot, s);
+            if (b->h_counts[k & (RING - 1)] == 0) break;
+            W::bounce(b, L, 0, k, s);
             LMGPU_CUDA_TRY(cudaGetLastError());
         }
-        W::tail_end(b, L, 0, s);
+        W::tail_end(b, L, 0, k - 1, s);
         LMGPU_CUDA_TRY(cudaGetLastError());
     }
     return LMGPU_OK;
@@ -734,8 +727,10 @@ int run_waves(LmgpuBatch* b, const Plan& pl, int64_t P, cudaStream_t s, int64_t&
 template <int TECH, class F>
 int dispatch_stack(LmgpuBatch* b, const Plan& pl, int64_t P, cudaStream_t s, int64_t& waves)
 {
-    if (pl.stack == 32) return run_waves<TECH, F, 32>(b, pl, P, s, waves);
-    return run_waves<TECH, F, 256>(b, pl, P, s, waves);
+    const bool solo = b->scenes.size() == 1 && b->scenes[0]->rdev.num_tris > 0;
+    if (pl.stack == 32)
+        return solo ? run_waves<TECH, F, 32, true>(b, pl, P, s, waves) : run_waves<TECH, F, 32, false>(b, pl, P, s, waves);
+    return solo ? run_waves<TECH, F, 256, true>(b, pl, P, s, waves) : run_waves<TECH, F, 256, false>(b, pl, P, s, waves);
 }
 
 template <class F>
@@ -848,7 +843,7 @@ int lmgpu_batch_create(LmgpuScene* const* scenes, int32_t num_scenes, LmgpuBatch
     dm(reinterpret_cast<void**>(&b->d_ctl), sizeof(StreamCtl));
     hm(reinterpret_cast<void**>(&b->h_done), 2 * sizeof(int64_t));
     dm(reinterpret_cast<void**>(&b->d_stats), NSTATS * sizeof(unsigned long long));
-    dm(reinterpret_cast<void**>(&b->d_work), POOLS * WORK_SLOTS * sizeof(unsigned long long));
+    dm(reinterpret_cast<void**>(&b->d_work), WORK_SLOTS * sizeof(unsigned long long));
     dm(reinterpret_cast<void**>(&b->d_status), sizeof(int32_t));
     hm(reinterpret_cast<void**>(&b->h_table), n * sizeof(BatchEntry));
     hm(reinterpret_cast<void**>(&b->h_begins), (n + 1) * sizeof(int64_t));

@@ -6,8 +6,8 @@
 // memory manager forbids device allocations, or a process already at its
 // memory budget. This entry point runs the same waves over a fixed workspace
 // that lives in this file's static device array instead, so a call allocates
-// nothing. Like lmgpu_render_device, it reads each bounce's queue sizes back
-// to the host, so it synchronises its stream after every bounce.
+// nothing. Like lmgpu_render_device, it synchronises its stream when a deep wave asks
+// whether any path is left, and at the end of the call.
 #include <cuda_runtime.h>
 #include <mutex>
 

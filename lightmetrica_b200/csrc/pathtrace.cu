@@ -4,8 +4,7 @@
 // Path state lives in HBM as structure-of-arrays (float4 records, 16-byte
 // coalesced accesses); surviving paths and shadow rays are appended to
 // compacted queues with one warp-aggregated atomic per warp (ballot/popc).
-// The driver reads the queue counts back after each pass to size the next
-// launch; the multi-scene batch (batch.cu) keeps them on the device instead.
+// Queue lengths stay on the device; the driver asks for them only to end deep waves.
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cstring>
@@ -138,7 +137,7 @@ void carve_state(PathState& st, char* p, size_t P)
 
 int ensure_workspace(Workspace& ws, int64_t paths)
 {
-    if (!ws.host_counts) LMGPU_CUDA_TRY(cudaMallocHost(&ws.host_counts, 16));
+    if (!ws.host_counts) LMGPU_CUDA_TRY(cudaMallocHost(&ws.host_counts, WS_HEADER_BYTES));
     if (ws.capacity >= paths && ws.mem) return LMGPU_OK;
     if (ws.mem) { cudaFree(ws.mem); ws.mem = nullptr; ws.capacity = 0; }
     const size_t P = (size_t)paths;
@@ -150,24 +149,39 @@ int ensure_workspace(Workspace& ws, int64_t paths)
     return LMGPU_OK;
 }
 
-template <class F>
-int shadow_pass(LmgpuScene* sc, const PathState& st, const OneScene<F>& ctx, int64_t max_rays, cudaStream_t stream)
+// Launches one traversal of a wave's rays (their number is on the device).
+template <int STACK, int MODE, class IO>
+int trace_wave(LmgpuScene* sc, const IO& io, unsigned long long* work, int64_t max_rays, cudaStream_t stream)
 {
-    ShadowIO<OneScene<F>> io{ st.counters + 2, st.sh_o, st.sh_d, st.sh_c, st.L, ctx };
-    return launch_trace<true, ShadowIO<OneScene<F>>>(sc, io, max_rays, stream);
-}
-
-int read_counts(Workspace& ws, cudaStream_t stream)
-{
-    LMGPU_CUDA_TRY(cudaMemcpyAsync(ws.host_counts, ws.st.counters, 16, cudaMemcpyDeviceToHost, stream));
-    LMGPU_CUDA_TRY(cudaStreamSynchronize(stream));
+    const DeviceScene& s = sc->rdev;
+    if (s.layout == LMGPU_LAYOUT_NAIVE || s.num_tris == 0) {
+        const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((max_rays + 127) / 128, 148 * 64));
+        if constexpr (MODE == TRACE_MIXED) {
+            k_trace_naive<false><<<blocks, 128, 0, stream>>>(s, io.closest);
+            k_trace_naive<true><<<blocks, 128, 0, stream>>>(s, io.shadow);
+        } else {
+            k_trace_naive<MODE == TRACE_ANY, IO><<<blocks, 128, 0, stream>>>(s, io);
+        }
+    } else {
+        auto k = k_trace_persistent<STACK, MODE, IO>;
+        const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(resident_blocks(k), (max_rays + 127) / 128));
+        k<<<blocks, 128, 0, stream>>>(s, io, sc->d_status, work, nullptr);
+    }
+    LMGPU_CUDA_TRY(cudaGetLastError());
     return LMGPU_OK;
 }
 
-template <int TECH, class F>
+// Bounces launched before the host first asks whether any path is left, and from
+// then on between questions: a launch over an empty queue takes about 2 us on the
+// device, a question (copy, wait, next launch) about 12.
+constexpr int FIRST_CHECK = 8, CHECK_EVERY = 4;
+
+// `counts`: host memory of 4 words, or of the whole header (`with_stats`).
+template <int TECH, int STACK, class F>
 int render_waves(LmgpuScene* sc, const LmgpuRenderParams& p, F* film, cudaStream_t stream, LmgpuRenderStats& stats,
-                 Workspace& ws)
+                 Workspace& ws, bool with_stats)
 {
+    using Ctx = OneScene<F>;
     const DeviceScene& s = sc->rdev;
     const int64_t pixels = (int64_t)s.cam.width * s.cam.height;
     int64_t P = p.wave_paths > 0 ? p.wave_paths : DEFAULT_WAVE_PATHS;
@@ -195,62 +209,79 @@ int render_waves(LmgpuScene* sc, const LmgpuRenderParams& p, F* film, cudaStream
     c.inv_pixels = 1.0 / double(pixels);
     c.sample_base = p.sample_offset;
     c.order = sample_order(p.num_samples, s.cam.width, s.cam.height, p.sampling == LMGPU_SAMPLING_STRATIFIED);
+    unsigned long long* totals = work_counter(st.counters, COUNTER_STATS);
+    auto work = [&](int word) { return work_counter(st.counters, word); };
     const int shade_blocks = 148 * 8;
+    LMGPU_CUDA_TRY(cudaMemsetAsync(totals, 0, 3 * sizeof(unsigned long long), stream));
     for (int64_t base = 0; base < p.num_samples && rc == LMGPU_OK; base += P) {
         const int64_t cnt = std::min<int64_t>(P, p.num_samples - base);
         c.path_base = base;
-        const OneScene<F> ctx{ s, c, film };
+        const Ctx ctx{ s, c, film };
         stats.waves++;
         stats.paths += cnt;
         if (c.max_pv != -1 && c.max_pv <= 1) continue;   // no path vertex beyond the camera
-        LMGPU_CUDA_TRY(cudaMemsetAsync(st.counters, 0, 16, stream));
-        k_pt_init<TECH, OneScene<F>><<<(unsigned)((cnt + 127) / 128), 128, 0, stream>>>(ctx, st, cnt, 0);
+        LMGPU_CUDA_TRY(cudaMemsetAsync(st.counters, 0, COUNTER_WORDS * sizeof(uint32_t), stream));
+        k_pt_init<TECH, Ctx><<<(unsigned)((cnt + 127) / 128), 128, 0, stream>>>(ctx, st, cnt, 0, ring_rays(1), ring_shadow(0));
         LMGPU_CUDA_TRY(cudaGetLastError());
-        if (TECH != LMGPU_RENDER_PT) {
-            if ((rc = read_counts(ws, stream)) != LMGPU_OK) break;
-            stats.shadow_rays += ws.host_counts[2];
-            if (ws.host_counts[2]) rc = shadow_pass(sc, st, ctx, ws.host_counts[2], stream);
-        }
-        int qin = 0;
-        for (int k = 1; rc == LMGPU_OK; k++) {
-            if (c.max_pv != -1 && k >= c.max_pv) break;
-            if ((rc = read_counts(ws, stream)) != LMGPU_OK) break;
-            const uint32_t n = ws.host_counts[qin];
-            if (n == 0) break;
-            stats.rays_traced += n;
-            stats.max_bounces_run = std::max(stats.max_bounces_run, k);
-            PathRayIO<false> io{ st.counters + qin, st.qo[qin], st.qd[qin], st.hit, nullptr };
-            rc = launch_trace<false, PathRayIO<false>>(sc, io, n, stream);
-            if (rc != LMGPU_OK) break;
-            LMGPU_CUDA_TRY(cudaMemsetAsync(st.counters + (1 - qin), 0, 4, stream));
-            LMGPU_CUDA_TRY(cudaMemsetAsync(st.counters + 2, 0, 4, stream));
-            const unsigned blocks = (unsigned)std::min<int64_t>((n + 127) / 128, shade_blocks);
-            k_pt_shade<TECH, OneScene<F>><<<blocks, 128, 0, stream>>>(ctx, st, k, qin, 1 - qin);
-            LMGPU_CUDA_TRY(cudaGetLastError());
-            if (TECH != LMGPU_RENDER_PT) {
-                if ((rc = read_counts(ws, stream)) != LMGPU_OK) break;
-                stats.shadow_rays += ws.host_counts[2];
-                if (ws.host_counts[2]) rc = shadow_pass(sc, st, ctx, ws.host_counts[2], stream);
+        const unsigned blocks = (unsigned)std::min<int64_t>((cnt + 127) / 128, shade_blocks);
+        int k = 1;
+        for (; c.max_pv == -1 || k < c.max_pv; k++) {
+            if (k > FIRST_CHECK && (k - FIRST_CHECK - 1) % CHECK_EVERY == 0) {
+                LMGPU_CUDA_TRY(cudaMemcpyAsync(ws.host_counts, st.counters + ring_rays(0), RING * sizeof(uint32_t),
+                                               cudaMemcpyDeviceToHost, stream));
+                LMGPU_CUDA_TRY(cudaStreamSynchronize(stream));
+                if (ws.host_counts[k & (RING - 1)] == 0) break;
             }
-            qin = 1 - qin;
-        }
-        if (rc == LMGPU_OK) {
-            k_pt_splat<OneScene<F>><<<(unsigned)((cnt + 127) / 128), 128, 0, stream>>>(ctx, st, cnt);
+            const int q = (k - 1) & 1;
+            const auto rays = ray_queue<false>(st, q, ring_rays(k), nullptr);
+            if (TECH == LMGPU_RENDER_PT) {
+                rc = trace_wave<STACK, TRACE_CLOSEST>(sc, rays, work(ring_work(k)), cnt, stream);
+            } else {
+                const BounceIO<Ctx> io{ rays, shadow_queue(st, ring_shadow(k - 1), ctx) };
+                rc = trace_wave<STACK, TRACE_MIXED>(sc, io, work(ring_work(k)), 2 * cnt, stream);
+            }
+            if (rc != LMGPU_OK) break;
+            k_pt_shade<TECH, Ctx><<<blocks, 128, 0, stream>>>(ctx, st, k, q, totals);
             LMGPU_CUDA_TRY(cudaGetLastError());
+        }
+        if (rc == LMGPU_OK && TECH != LMGPU_RENDER_PT)     // the last vertices' shadow rays
+            rc = trace_wave<STACK, TRACE_ANY>(sc, shadow_queue(st, ring_shadow(k - 1), ctx), work(ring_shadow_work(k - 1)), cnt, stream);
+        if (rc == LMGPU_OK) {
+            k_pt_splat<Ctx><<<(unsigned)((cnt + 127) / 128), 128, 0, stream>>>(ctx, st, cnt);
+            LMGPU_CUDA_TRY(cudaGetLastError());
+            if (with_stats) {
+                LMGPU_CUDA_TRY(cudaMemcpyAsync(ws.host_counts, st.counters, WS_HEADER_BYTES, cudaMemcpyDeviceToHost, stream));
+                LMGPU_CUDA_TRY(cudaStreamSynchronize(stream));
+                stats.shadow_rays += ws.host_counts[ring_shadow(k - 1)];
+            }
         }
     }
-    stats.rays_traced += stats.shadow_rays;
+    if (rc == LMGPU_OK && with_stats && stats.waves > 0 && !(c.max_pv != -1 && c.max_pv <= 1)) {
+        const unsigned long long* t = work_counter(ws.host_counts, COUNTER_STATS);
+        stats.shadow_rays += (int64_t)t[1];
+        stats.rays_traced = (int64_t)t[0] + stats.shadow_rays;
+        stats.max_bounces_run = (int)t[2];
+    }
     return rc;
+}
+
+template <int TECH, class F>
+int render_waves_stack(LmgpuScene* sc, const LmgpuRenderParams& p, F* film, cudaStream_t stream, LmgpuRenderStats& stats,
+                       Workspace& ws, bool with_stats)
+{
+    if (sc->rdev.stack8_cap <= 32) return render_waves<TECH, 32>(sc, p, film, stream, stats, ws, with_stats);
+    if (sc->rdev.stack8_cap <= 256) return render_waves<TECH, 256>(sc, p, film, stream, stats, ws, with_stats);
+    return fail(LMGPU_ERR_UNSUPPORTED, "BVH deeper than the largest compiled traversal stack (256)");
 }
 
 template <class F>
 int render_dispatch(LmgpuScene* sc, const LmgpuRenderParams& p, F* film, cudaStream_t stream, LmgpuRenderStats& stats,
-                    Workspace& ws)
+                    Workspace& ws, bool with_stats)
 {
     switch (p.technique) {
-    case LMGPU_RENDER_PT: return render_waves<LMGPU_RENDER_PT, F>(sc, p, film, stream, stats, ws);
-    case LMGPU_RENDER_PT_DIRECT: return render_waves<LMGPU_RENDER_PT_DIRECT, F>(sc, p, film, stream, stats, ws);
-    case LMGPU_RENDER_PT_MIS: return render_waves<LMGPU_RENDER_PT_MIS, F>(sc, p, film, stream, stats, ws);
+    case LMGPU_RENDER_PT: return render_waves_stack<LMGPU_RENDER_PT>(sc, p, film, stream, stats, ws, with_stats);
+    case LMGPU_RENDER_PT_DIRECT: return render_waves_stack<LMGPU_RENDER_PT_DIRECT>(sc, p, film, stream, stats, ws, with_stats);
+    case LMGPU_RENDER_PT_MIS: return render_waves_stack<LMGPU_RENDER_PT_MIS>(sc, p, film, stream, stats, ws, with_stats);
     default: return fail(LMGPU_ERR_INVALID, "unknown technique");
     }
 }
@@ -395,20 +426,8 @@ int render_device_preallocated(LmgpuScene* sc, const LmgpuRenderParams& p, void*
     carve_workspace(ws, ws_mem, cap, host_counts);
     LmgpuRenderStats stats;
     std::memset(&stats, 0, sizeof(stats));
-    switch (q.technique) {
-    case LMGPU_RENDER_PT:
-        rc = q.film_fp64 ? render_waves<LMGPU_RENDER_PT, double>(sc, q, static_cast<double*>(film), stream, stats, ws)
-                         : render_waves<LMGPU_RENDER_PT, float>(sc, q, static_cast<float*>(film), stream, stats, ws);
-        break;
-    case LMGPU_RENDER_PT_DIRECT:
-        rc = q.film_fp64 ? render_waves<LMGPU_RENDER_PT_DIRECT, double>(sc, q, static_cast<double*>(film), stream, stats, ws)
-                         : render_waves<LMGPU_RENDER_PT_DIRECT, float>(sc, q, static_cast<float*>(film), stream, stats, ws);
-        break;
-    default:
-        rc = q.film_fp64 ? render_waves<LMGPU_RENDER_PT_MIS, double>(sc, q, static_cast<double*>(film), stream, stats, ws)
-                         : render_waves<LMGPU_RENDER_PT_MIS, float>(sc, q, static_cast<float*>(film), stream, stats, ws);
-        break;
-    }
+    rc = q.film_fp64 ? render_dispatch(sc, q, static_cast<double*>(film), stream, stats, ws, false)
+                     : render_dispatch(sc, q, static_cast<float*>(film), stream, stats, ws, false);
     if (rc == LMGPU_OK) rc = consume_status(sc, stream);
     return rc;
 }
@@ -475,8 +494,8 @@ int lmgpu_render_device(LmgpuScene* scene, const LmgpuRenderParams* params, void
     LMGPU_CUDA_TRY(cudaEventCreate(&e0));
     LMGPU_CUDA_TRY(cudaEventCreate(&e1));
     LMGPU_CUDA_TRY(cudaEventRecord(e0, s));
-    if (params->film_fp64) rc = render_dispatch(scene, *params, static_cast<double*>(film_device), s, st, dw.ws);
-    else rc = render_dispatch(scene, *params, static_cast<float*>(film_device), s, st, dw.ws);
+    if (params->film_fp64) rc = render_dispatch(scene, *params, static_cast<double*>(film_device), s, st, dw.ws, true);
+    else rc = render_dispatch(scene, *params, static_cast<float*>(film_device), s, st, dw.ws, true);
     if (rc == LMGPU_OK) {
         cudaError_t e = cudaEventRecord(e1, s);
         if (e == cudaSuccess) e = cudaEventSynchronize(e1);

@@ -40,6 +40,26 @@ namespace lmgpu {
 constexpr uint32_t PREV_DEGENERATED = 1u;   // previous vertex is the pinhole
 constexpr uint32_t PREV_SPECULAR = 2u;      // last BSDF sample was specular
 
+// The 256-byte header of a path state: queue lengths and traversal work counters.
+// A wave keeps a ring of four per kind, by bounce number: bounce k's shading fills the
+// rays of bounce k + 1 and the shadow rays of bounce k, and clears the counters that
+// bounce k + 1 will fill, so that bounces follow one another without a launch
+// between them to clear counters and without the host.
+constexpr int COUNTER_RAYS[2] = { 0, 1 };     // stream mode: ray queues by parity, shadow rays, retired paths
+constexpr int COUNTER_SHADOW = 2, COUNTER_RETIRE = 3;
+constexpr int RING = 4;
+__host__ __device__ constexpr int ring_rays(int k) { return 8 + (k & (RING - 1)); }
+__host__ __device__ constexpr int ring_shadow(int k) { return 12 + (k & (RING - 1)); }
+// (64-bit counters, by word) the launch that traces bounce k's rays, and shadow rays traced by themselves
+__host__ __device__ constexpr int ring_work(int k) { return 16 + 2 * (k & (RING - 1)); }
+__host__ __device__ constexpr int ring_shadow_work(int k) { return 24 + 2 * (k & (RING - 1)); }
+constexpr int COUNTER_WORDS = 32;
+constexpr int COUNTER_STATS = 32;             // one scene: 3 64-bit totals as LmgpuBatch::d_stats
+__host__ __device__ __forceinline__ unsigned long long* work_counter(uint32_t* counters, int word)
+{
+    return reinterpret_cast<unsigned long long*>(counters + word);
+}
+
 // Device pointers of one wave's path state (capacity paths). The two ray
 // queues hold each live path's ray and its state between bounces in queue
 // order (see queue_ray), so the traversal and the shading read them, and
@@ -55,7 +75,7 @@ struct PathState {
     float4* sh_o;      // shadow ray origin, maxT
     float4* sh_d;      // direction, target (int bits: path index, or ~pixel)
     float4* sh_c;      // contribution, scene index (int bits)
-    uint32_t* counters;   // [0], [1] ray queues; [2] shadow queue
+    uint32_t* counters;   // see COUNTER_*
     int32_t* scene;    // per path scene index (SceneTable, StreamTable)
     int64_t* sample;   // per path batch-global sample index (StreamTable)
     int32_t* depth;    // per path index k of its next bounce (StreamTable)
@@ -245,6 +265,13 @@ struct SceneTable : RenderContext {
     static constexpr bool STREAM = false;
 };
 
+// The table of a batch of one scene: traversals need no scene per ray.
+template <class F>
+struct SoloTable : SceneTable<F> {
+    static constexpr bool TABLE = false;
+    using SceneTable<F>::SceneTable;
+};
+
 // Plan of one regenerating iteration, written by a one-thread kernel.
 struct StreamCtl {
     int64_t next;          // next batch-global sample to start
@@ -301,7 +328,7 @@ struct StreamTable : RenderContext {
 
 // ------------------------------------------------------------- helpers ----
 
-// Warp-aggregated append to queue q (counters[q]): returns this lane's slot
+// Warp-aggregated append to queue q (its length at counters[word]): returns this lane's slot
 // (the whole warp must reach the call). In the bounds-checked build a slot
 // at or beyond the queue's capacity is not handed out: the lane gets
 // NO_SLOT (slot_ok is false), the status word records
@@ -311,9 +338,9 @@ struct StreamTable : RenderContext {
 constexpr uint32_t NO_SLOT = 0xffffffffu;
 __device__ __forceinline__ bool slot_ok(uint32_t slot) { return !LMGPU_BOUNDS_CHECK || slot != NO_SLOT; }
 
-__device__ __forceinline__ uint32_t queue_append(const PathState& st, int q, bool want)
+__device__ __forceinline__ uint32_t queue_append(const PathState& st, int word, int q, bool want)
 {
-    uint32_t* counter = &st.counters[q];
+    uint32_t* counter = &st.counters[word];
     const unsigned active = __activemask();
     const unsigned mask = __ballot_sync(active, want);
     if (!want) return NO_SLOT;
@@ -405,9 +432,10 @@ __device__ __forceinline__ bool camera_nee(const Ctx& ctx, const DeviceScene& s,
 // Wave initialisation: raster sample and camera ray; for pt.direct / pt.mis
 // the whole camera vertex (light sample, Russian roulette). `count` is the
 // wave's path count for OneScene (the tables read it from the device); new
-// rays join ray queue q.
+// rays join ray queue q (length at counters[rays]), shadow rays the shadow queue
+// (length at counters[shadows]).
 template <int TECH, class Ctx>
-__global__ void __launch_bounds__(128) k_pt_init(const Ctx ctx, const PathState st, int64_t count, int q)
+__global__ void __launch_bounds__(128) k_pt_init(const Ctx ctx, const PathState st, int64_t count, int q, int rays, int shadows)
 {
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= ctx.wave_count(count)) return;
@@ -438,7 +466,7 @@ __global__ void __launch_bounds__(128) k_pt_init(const Ctx ctx, const PathState 
         int32_t dest;
         int light = 0;
         const bool shadow = camera_nee<TECH>(ctx, s, key, target, c, dest, light);
-        const uint32_t sslot = queue_append(st, 2, shadow);
+        const uint32_t sslot = queue_append(st, shadows, 2, shadow);
         if (shadow && slot_ok(sslot)) write_shadow(st, sslot, cp, target, c, dest, ctx.shadow_tag(sid, light));
         if (rc.rr_depth != -1 && 1 >= rc.rr_depth) {
             const float p = fminf(0.5f, luminance(thr));
@@ -446,11 +474,11 @@ __global__ void __launch_bounds__(128) k_pt_init(const Ctx ctx, const PathState 
             else thr = thr / p;
         }
     }
-    const uint32_t slot = queue_append(st, q, alive);
+    const uint32_t slot = queue_append(st, rays, q, alive);
     if (alive && slot_ok(slot))
         queue_ray<TECH>(st, q, slot, cp, dir, i, sid, TECH == LMGPU_RENDER_PT, thr, pdf_cam, v3(0, 0, 1), PREV_DEGENERATED);
     if (Ctx::STREAM) {                           // a path that ends at the camera retires at once
-        const uint32_t r = queue_append(st, 3, !alive);
+        const uint32_t r = queue_append(st, COUNTER_RETIRE, 3, !alive);
         if (!alive && slot_ok(r)) st.retire[r] = (int32_t)i;
     }
 }
@@ -523,6 +551,35 @@ struct ShadowIO {
     }
 };
 
+// The two queues of one launch (TRACE_MIXED): bounce k's rays and the shadow rays of
+// the vertices before them. One launch has one tail of long rays instead of two.
+// Measured, two launches -> one (us): terrain 641 x 359 x 8, bounces 1 to 5:
+// 354 -> 294, 435 -> 405, 146 -> 94, 129 -> 67, 125 -> 46; 1080p x 8 through the batch's
+// scene table, bounces 2, 3, 4: 4391 -> 4801, 1641 -> 1766, 1060 -> 1109, from 5 on
+// 1509 -> 820 in all. A full queue of each kind runs better by itself there, so scene
+// tables merge from bounce TABLE_MERGE on (when most paths have ended), other waves
+// always.
+constexpr int TABLE_MERGE = 5;
+template <class Ctx>
+struct BounceIO {
+    static constexpr bool PER_RAY_SCENE = Ctx::TABLE;
+    static constexpr bool RENDER = true;
+    PathRayIO<Ctx::TABLE> closest;
+    ShadowIO<Ctx> shadow;
+    __device__ int64_t count() const { return closest.count() + shadow.count(); }
+};
+
+template <bool TABLE>
+__host__ __device__ inline PathRayIO<TABLE> ray_queue(const PathState& st, int q, int word, const BatchEntry* table)
+{
+    return PathRayIO<TABLE>{ st.counters + word, st.qo[q], st.qd[q], st.hit, table };
+}
+template <class Ctx>
+__host__ __device__ inline ShadowIO<Ctx> shadow_queue(const PathState& st, int word, const Ctx& ctx)
+{
+    return ShadowIO<Ctx>{ st.counters + word, st.sh_o, st.sh_d, st.sh_c, st.L, ctx };
+}
+
 // Shading of the hits of iteration k: emission at the hit (vertex k + 1),
 // then for pt.direct / pt.mis next-event estimation at it, Russian roulette
 // and BSDF sampling; pt samples the BSDF first and applies Russian roulette
@@ -535,9 +592,24 @@ struct ShadowIO {
 #endif
 template <int TECH, class Ctx>
 __global__ void __launch_bounds__(128, LMGPU_PT_SHADE_MIN_BLOCKS) k_pt_shade(const Ctx ctx, const PathState st, int kw,
-                                                                            int qin, int qout)
+                                                                            int qin, unsigned long long* stats)
 {
-    const int64_t count = (int64_t)st.counters[qin];
+    const int qout = 1 - qin;
+    const int rays_in = Ctx::STREAM ? qin : ring_rays(kw), rays_out = Ctx::STREAM ? qout : ring_rays(kw + 1);
+    const int shadows = Ctx::STREAM ? COUNTER_SHADOW : ring_shadow(kw);
+    const int64_t count = (int64_t)st.counters[rays_in];
+    if (!Ctx::STREAM && blockIdx.x == 0 && threadIdx.x == 0) {
+        // What bounce k + 1 will fill or count with was last used by bounce k - 2.
+        if (stats) {
+            atomicAdd(stats + 0, (unsigned long long)count);
+            atomicAdd(stats + 1, (unsigned long long)st.counters[ring_shadow(kw - 1)]);
+            if (count > 0) atomicMax(stats + 2, (unsigned long long)kw);
+        }
+        st.counters[ring_rays(kw + 2)] = 0;
+        st.counters[ring_shadow(kw + 1)] = 0;
+        *work_counter(st.counters, ring_work(kw + 1)) = 0;
+        *work_counter(st.counters, ring_shadow_work(kw + 1)) = 0;
+    }
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     // Whole warps iterate together so that the queue appends stay warp-wide.
     const int64_t rounds = (count + stride - 1) / stride;
@@ -659,16 +731,16 @@ __global__ void __launch_bounds__(128, LMGPU_PT_SHADE_MIN_BLOCKS) k_pt_shade(con
                 if (alive && TECH == LMGPU_RENDER_PT && rc.max_pv != -1 && k + 1 >= rc.max_pv) alive = false;
             }
         }
-        const uint32_t sslot = queue_append(st, 2, shadow);
+        const uint32_t sslot = queue_append(st, shadows, 2, shadow);
         if (shadow && slot_ok(sslot)) write_shadow(st, sslot, g.p, sh_target, sh_c, i, sh_tag);
-        const uint32_t slot = queue_append(st, qout, alive);
+        const uint32_t slot = queue_append(st, rays_out, qout, alive);
         if (alive && slot_ok(slot)) {
             queue_ray<TECH>(st, qout, slot, g.p, bs.wo, i, sid, false, thr, bs.pdf, g.sn, bs.specular ? PREV_SPECULAR : 0u);
             if (Ctx::STREAM) st.depth[i] = k + 1;
         }
         if constexpr (Ctx::STREAM) {
             const bool done = valid && !alive;
-            const uint32_t r = queue_append(st, 3, done);
+            const uint32_t r = queue_append(st, COUNTER_RETIRE, 3, done);
             if (done && slot_ok(r)) st.retire[r] = i;
             const unsigned m = __reduce_max_sync(__activemask(), valid ? (unsigned)k : 0u);
             if ((threadIdx.x & 31u) == (unsigned)(__ffs(__activemask()) - 1)) atomicMax(ctx.max_depth, (unsigned long long)m);
@@ -682,7 +754,7 @@ __global__ void __launch_bounds__(128, LMGPU_PT_SHADE_MIN_BLOCKS) k_pt_shade(con
 template <class Ctx>
 __global__ void __launch_bounds__(128) k_pt_retire(const Ctx ctx, const PathState st)
 {
-    const int64_t n = (int64_t)st.counters[3];
+    const int64_t n = (int64_t)st.counters[COUNTER_RETIRE];
     const int64_t base = ctx.ctl->free_count;
     for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x) {
         const int32_t i = st.retire[j];
@@ -693,12 +765,10 @@ __global__ void __launch_bounds__(128) k_pt_retire(const Ctx ctx, const PathStat
     }
 }
 
-// Start of a wave: clear the queue counters and this wave's traversal work
-// counters (static: each translation unit launches its own).
-static __global__ void k_wave_begin(uint32_t* counters, unsigned long long* work, int slots)
+// Start of a wave: clear its counters (static: each translation unit launches its own).
+static __global__ void k_wave_begin(uint32_t* counters)
 {
-    for (int i = threadIdx.x; i < slots; i += blockDim.x) work[i] = 0;
-    if (threadIdx.x < 4) counters[threadIdx.x] = 0;
+    if (threadIdx.x < COUNTER_WORDS) counters[threadIdx.x] = 0;
 }
 
 // Film splat of each path's radiance at its raster position.

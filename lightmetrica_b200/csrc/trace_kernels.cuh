@@ -49,6 +49,10 @@ struct render_rays : std::false_type {};
 template <class IO>
 struct render_rays<IO, std::void_t<decltype(IO::RENDER)>> : std::bool_constant<IO::RENDER> {};
 
+// Which question a traversal launch asks of its rays. TRACE_MIXED answers two queues
+// in one launch: io.closest's rays first, then io.shadow's (any hit).
+constexpr int TRACE_CLOSEST = 0, TRACE_ANY = 1, TRACE_MIXED = 2;
+
 // Adds each lane's counts to counts[0] (box tests: eight per node visit) and
 // counts[1] (TriAccel tests); the whole warp calls it.
 __device__ __forceinline__ void add_trace_stats(const TraceStats& st, unsigned long long* counts)
@@ -98,7 +102,7 @@ __device__ __forceinline__ void reference_walk(const DeviceScene& s, int32_t* st
 // For a multi-scene I/O policy each lane switches to its new ray's scene at
 // refill; an empty scene is a miss. The COUNT instantiation (measurement
 // runs only) also adds the rays' box and TriAccel tests to counts[0..1].
-template <int STACK, bool ANY_HIT, class IO, bool COUNT = false>
+template <int STACK, int MODE, class IO, bool COUNT = false>
 __global__ void __launch_bounds__(128, LMGPU_TRACE_MIN_BLOCKS)
 k_trace_persistent(const __grid_constant__ DeviceScene s, const __grid_constant__ IO io, int32_t* status,
                    unsigned long long* next_ray, unsigned long long* counts)
@@ -112,6 +116,8 @@ k_trace_persistent(const __grid_constant__ DeviceScene s, const __grid_constant_
     __shared__ int64_t back_sh[RENDER ? 1 : 4][RENDER ? 1 : BACK_LIST];   // rays handed back (exact)
     int back = 0;                              // entries in the warp's list
     bool hand_back = false;                    // this lane's ray joins it
+    int64_t n_closest = 0;
+    if constexpr (MODE == TRACE_MIXED) n_closest = io.closest.count();
     const int64_t n = io.count();
     const unsigned lane = threadIdx.x & 31u;
     const int cap = s.stack8_cap < STACK ? s.stack8_cap : STACK;
@@ -130,6 +136,22 @@ k_trace_persistent(const __grid_constant__ DeviceScene s, const __grid_constant_
     int64_t idx = -1;
     bool live = false;
     bool exhausted = n <= 0;
+    bool any = MODE == TRACE_ANY;              // this lane's ray stops at its first hit
+    auto load = [&](int64_t j) -> RayIn {
+        if constexpr (MODE == TRACE_MIXED) return any ? io.shadow.load(j - n_closest) : io.closest.load(j);
+        else return io.load(j);
+    };
+    auto store = [&](int64_t j) {
+        if constexpr (MODE == TRACE_MIXED) {
+            if (any) io.shadow.store(j - n_closest, h, r);
+            else io.closest.store(j, h, r);
+        } else io.store(j, h, r);
+    };
+    auto ray_scene = [&](int64_t j) -> const DeviceScene& {
+        if constexpr (MODE == TRACE_MIXED) return any ? io.shadow.ray_scene(j - n_closest) : io.closest.ray_scene(j);
+        else if constexpr (TABLE) return io.ray_scene(j);
+        else return s;
+    };
     for (;;) {
         const unsigned need = __ballot_sync(FULL, !live);
         if constexpr (!RENDER) {
@@ -143,8 +165,8 @@ k_trace_persistent(const __grid_constant__ DeviceScene s, const __grid_constant_
                 __syncwarp();
                 for (int i = (int)lane; i < back; i += 32) {
                     idx = back_sh[threadIdx.x >> 5][i];
-                    reference_walk<ANY_HIT, STACK>(s, status, io.load(idx), r, h);
-                    io.store(idx, h, r);
+                    reference_walk<MODE == TRACE_ANY, STACK>(s, status, load(idx), r, h);
+                    store(idx);
                 }
                 __syncwarp();
                 back = 0;
@@ -159,13 +181,14 @@ k_trace_persistent(const __grid_constant__ DeviceScene s, const __grid_constant_
             if (!live) {
                 idx = (int64_t)base + __popc(need & ((1u << lane) - 1u));
                 if (idx < n) {
-                    const RayIn in = io.load(idx);
+                    if constexpr (MODE == TRACE_MIXED) any = idx >= n_closest;
+                    const RayIn in = load(idx);
                     setup_ray<true>(r, in);
                     oct = r.neg & 7u;
                     h.tri = -1;
                     live = true;
                     if constexpr (TABLE) {
-                        const DeviceScene& rs = io.ray_scene(idx);
+                        const DeviceScene& rs = ray_scene(idx);
                         nodes = rs.bvh8;
                         tris = rs.tris8;
                         live = rs.num_tris > 0;
@@ -177,7 +200,7 @@ k_trace_persistent(const __grid_constant__ DeviceScene s, const __grid_constant_
                         }
                     }
                     if (live) walk8_begin(w, oct);
-                    else if (!hand_back) io.store(idx, h, r);
+                    else if (!hand_back) store(idx);
                 }
             }
         } else if (exhausted && need == FULL && !__any_sync(FULL, hand_back)) {
@@ -230,21 +253,23 @@ k_trace_persistent(const __grid_constant__ DeviceScene s, const __grid_constant_
                 if constexpr (RENDER) {
                     if (triaccel_intersect_fast(q0, q1, q2, r, r.tmax, u, v, t)) {
                         bool take = t < r.tmax || id > h.tri;
-                        if (TABLE ? io.ray_scene(idx).check_boxes : s.check_boxes) {
+                        bool check = s.check_boxes;
+                        if constexpr (TABLE) check = ray_scene(idx).check_boxes;
+                        if (check) {
                             const LeafBox* boxes = s.boxes8;
-                            if constexpr (TABLE) boxes = io.ray_scene(idx).boxes8;
+                            if constexpr (TABLE) boxes = ray_scene(idx).boxes8;
                             take = take && leaf_box_render(boxes, (p - reinterpret_cast<const float4*>(tris)) / 3, r);
                         }
                         if (take) {
                             r.tmax = t;
                             h.tri = id; h.t = t; h.u = u; h.v = v;
-                            if (ANY_HIT) { done = true; break; }
+                            if (any) { done = true; break; }
                         }
                     }
                 } else {
                     if (triaccel_intersect(q0, q1, q2, r, r.tmax, u, v, t)) {
                         const int64_t at = (p - reinterpret_cast<const float4*>(tris)) / 3;
-                        if (ANY_HIT) {
+                        if (any) {
                             float te;
                             if (leaf_box_exact(s.boxes8, at, r, te) && te < r.tmax) {
                                 h.tri = id;
@@ -252,7 +277,7 @@ k_trace_persistent(const __grid_constant__ DeviceScene s, const __grid_constant_
                                 break;
                             }
                         } else {
-                            exact_candidate(s.boxes8, at, id, t, u, v, io.load(idx).tmax, r, h);
+                            exact_candidate(s.boxes8, at, id, t, u, v, load(idx).tmax, r, h);
                         }
                     }
                 }
@@ -264,7 +289,7 @@ k_trace_persistent(const __grid_constant__ DeviceScene s, const __grid_constant_
                 }
             }
             pend = 0;
-            if constexpr (!RENDER && !ANY_HIT) {
+            if constexpr (!RENDER && MODE == TRACE_CLOSEST) {
                 if (h.tri == HIT_TIED) {
                     hand_back = true;
                     done = true;
@@ -279,7 +304,7 @@ k_trace_persistent(const __grid_constant__ DeviceScene s, const __grid_constant_
         }
         if (pend == 0 && w.leaves == 0 && (w.mask & 0xffu) == 0 && w.sp == 0) {
             live = false;
-            if (!hand_back) io.store(idx, h, r);
+            if (!hand_back) store(idx);
         }
     }
     if (COUNT) add_trace_stats(stats, counts);
@@ -324,7 +349,7 @@ int launch_trace_stack(LmgpuScene* sc, const DeviceScene& s, const IO& io, int64
     // kernels queued on different streams never share one.
     unsigned long long* work = sc->d_work + (sc->work_slot++ % LmgpuScene::WORK_SLOTS);
     LMGPU_CUDA_TRY(cudaMemsetAsync(work, 0, sizeof(unsigned long long), stream));
-    auto k = k_trace_persistent<STACK, ANY_HIT, IO>;
+    auto k = k_trace_persistent<STACK, ANY_HIT ? TRACE_ANY : TRACE_CLOSEST, IO>;
     int64_t blocks = resident_blocks(k);
     if (max_rays > 0) blocks = std::max<int64_t>(1, std::min<int64_t>(blocks, (max_rays + 127) / 128));
     k<<<blocks, 128, 0, stream>>>(s, io, sc->d_status, work, nullptr);
@@ -332,18 +357,17 @@ int launch_trace_stack(LmgpuScene* sc, const DeviceScene& s, const IO& io, int64
     return LMGPU_OK;
 }
 
-// Render policies trace the scene's render view (its render tree), the
-// others the reference's tree. The stack bound is the wide walk's, for exact
-// rays also that of the reference's walk they may be handed to.
+// The intersection API's launch (the reference's tree). The stack bound is the wide
+// walk's and that of the reference's walk a ray may be handed to.
 template <bool ANY_HIT, class IO>
 int launch_trace(LmgpuScene* sc, const IO& io, int64_t max_rays, cudaStream_t stream)
 {
-    constexpr bool RENDER = render_rays<IO>::value;
-    const DeviceScene& s = RENDER ? sc->rdev : sc->dev;
-    const int cap = RENDER ? s.stack8_cap : std::max(s.stack8_cap, s.stack_cap);
+    static_assert(!render_rays<IO>::value, "renders launch their own traversals");
+    const DeviceScene& s = sc->dev;
+    const int cap = std::max(s.stack8_cap, s.stack_cap);
     if (cap <= 32) return launch_trace_stack<ANY_HIT, 32>(sc, s, io, max_rays, stream);
-    if (!RENDER && cap <= 64) return launch_trace_stack<ANY_HIT, RENDER ? 256 : 64>(sc, s, io, max_rays, stream);
-    if (!RENDER && cap <= 128) return launch_trace_stack<ANY_HIT, RENDER ? 256 : 128>(sc, s, io, max_rays, stream);
+    if (cap <= 64) return launch_trace_stack<ANY_HIT, 64>(sc, s, io, max_rays, stream);
+    if (cap <= 128) return launch_trace_stack<ANY_HIT, 128>(sc, s, io, max_rays, stream);
     if (cap <= 256) return launch_trace_stack<ANY_HIT, 256>(sc, s, io, max_rays, stream);
     return fail(LMGPU_ERR_UNSUPPORTED, "BVH deeper than the largest compiled traversal stack (256)");
 }

@@ -57,3 +57,31 @@ def test_any_split_renders_the_same_samples(cuda, tech, w, h, n, split):
     single, _ = _render(s, r, n, torch, fp64=False)
     np.testing.assert_allclose(single, whole, rtol=n * 6e-8, atol=1e-6)   # n additions of 2^-24 relative error each
     s.close()
+
+
+@pytest.mark.parametrize("tech,max_pv,rr,sampling", [("pt.mis", -1, 1, "stratified"), ("pt.direct", 14, 30, "uniform"),
+                                                     ("pt", -1, 4, "uniform"), ("pt.mis", 2, 1, "stratified"),
+                                                     ("pt.mis", 1, 1, "stratified"), ("pt.direct", 10, 5, "stratified")])
+def test_waves_of_any_size_and_the_batch_count_and_render_alike(cuda, tech, max_pv, rr, sampling):
+    import torch
+    s = _built(scenes.cornell_box(31, 17, variant="mixed"))
+    r = _renderer(tech, max_pv, rr, sampling)
+    n = 31 * 17 * 9 + 4
+    film, st = _render(s, r, n, torch)
+    for wave in (n, 1000, 257):
+        other, so = _render(s, r, n, torch, wave_paths=wave)
+        np.testing.assert_allclose(other, film, **SUMS)
+        assert (so.rays_traced, so.shadow_rays, so.paths, so.max_bounces_run) == \
+               (st.rays_traced, st.shadow_rays, st.paths, st.max_bounces_run)
+        assert so.waves == -(-n // wave)
+    if max_pv == 1:
+        assert st.rays_traced == 0 and not film.any()
+        return
+    b = SceneBatch([s])
+    for mode in ("waves", "overlap", "stream"):
+        b.configure(mode=mode, wave_paths=1024)
+        out = b.render([r], [n])[0].reshape(-1)
+        np.testing.assert_allclose(out, film * (31 * 17 / n), rtol=n * 6e-8, atol=1e-6)
+        assert b.last_stats["rays_traced"] == st.rays_traced and b.last_stats["shadow_rays"] == st.shadow_rays
+    b.close()
+    s.close()
