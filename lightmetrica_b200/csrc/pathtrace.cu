@@ -163,9 +163,12 @@ int trace_wave(LmgpuScene* sc, const IO& io, unsigned long long* work, int64_t m
             k_trace_naive<MODE == TRACE_ANY, IO><<<blocks, 128, 0, stream>>>(s, io);
         }
     } else {
+        auto few = k_trace_persistent<STACK, MODE | TRACE_SPREAD, IO>;
         auto k = k_trace_persistent<STACK, MODE, IO>;
-        const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(resident_blocks(k), (max_rays + 127) / 128));
-        k<<<blocks, 128, 0, stream>>>(s, io, sc->d_status, work, nullptr);
+        if (const int64_t blocks = spread_blocks(resident_blocks(few), max_rays))
+            few<<<blocks, 128, 0, stream>>>(s, io, sc->d_status, nullptr, nullptr);
+        else
+            k<<<resident_blocks(k), 128, 0, stream>>>(s, io, sc->d_status, work, nullptr);
     }
     LMGPU_CUDA_TRY(cudaGetLastError());
     return LMGPU_OK;

@@ -85,3 +85,25 @@ def test_waves_of_any_size_and_the_batch_count_and_render_alike(cuda, tech, max_
         assert b.last_stats["rays_traced"] == st.rays_traced and b.last_stats["shadow_rays"] == st.shadow_rays
     b.close()
     s.close()
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 127, 593, 4735, 4737, 9473, 151552, 151553])
+def test_few_rays_answer_as_among_many(cuda, n):
+    """Around one ray and 32 rays for each of 148 x 8 x 4 resident warps."""
+    import torch
+    pos, faces = random_soup(5003, seed=11, sigma=0.1)
+    s = _built(soup_primitives(pos, faces))
+    soa = {k: torch.from_numpy(v).to(cuda) for k, v in rays_soa(random_rays(400009, seed=12)).items()}
+    stream = torch.cuda.current_stream().cuda_stream
+
+    def ask(m):
+        out = {"tri_id": torch.zeros(m, dtype=torch.int32, device=cuda), **{k: torch.zeros(m, device=cuda) for k in "tuv"}}
+        occ = torch.zeros(m, dtype=torch.uint8, device=cuda)
+        rays = {k: v.data_ptr() for k, v in soa.items()}
+        s.intersect_device(rays, {k: v.data_ptr() for k, v in out.items()}, m, stream)
+        s.occluded_device(rays, occ.data_ptr(), m, stream)
+        s.status(stream)
+        return [out[k] for k in ("tri_id", "t", "u", "v")] + [occ]
+    for few, many in zip(ask(n), ask(400009)):
+        assert torch.equal(few, many[:n])
+    s.close()
