@@ -189,7 +189,7 @@ int lmgpu_intersect(LmgpuScene* scene, const LmgpuRaysSoA* rays, int64_t n,
 
 /* Same query from HOST buffers: rays AoS (8 floats per ray: o.xyz, d.xyz,
  * minT, maxT), outputs to host arrays (any may be NULL). Copies in, traces,
- * copies out, synchronises; 2^20-ray chunks on four streams overlap their
+ * copies out, synchronises; chunks of up to 2^20 rays on four streams overlap their
  * uploads, traversals and downloads. Page-locked buffers (cudaMallocHost,
  * cudaHostRegister) are copied directly; pageable ones, in batches of 2^16
  * rays or more, through the scene's pinned staging (192 MB, allocated on

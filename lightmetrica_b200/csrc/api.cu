@@ -739,10 +739,12 @@ int intersect_host_staged(LmgpuScene* scene, const float* rays_aos, int64_t n, v
                           bool stage_out)
 {
     HostPipeline& hp = scene->pipe;
-    const int64_t chunk = hp.chunk;
+    // Eight chunks or more, so that the host's copies, the transfers and the traversal
+    // overlap also in calls that would fit one of the pipeline's chunks.
+    const int64_t chunk = std::min(hp.chunk, std::max(STAGE_MIN_RAYS, (n / 8 + 1023) / 1024 * 1024));
     for (int k = 0; k < HostPipeline::SLOTS; k++) {
-        if (!hp.stage_rays[k]) LMGPU_CUDA_TRY(cudaMallocHost(&hp.stage_rays[k], (size_t)chunk * 8 * sizeof(float)));
-        if (!hp.stage_hits[k]) LMGPU_CUDA_TRY(cudaMallocHost(&hp.stage_hits[k], (size_t)chunk * 4 * sizeof(float)));
+        if (!hp.stage_rays[k]) LMGPU_CUDA_TRY(cudaMallocHost(&hp.stage_rays[k], (size_t)hp.chunk * 8 * sizeof(float)));
+        if (!hp.stage_hits[k]) LMGPU_CUDA_TRY(cudaMallocHost(&hp.stage_hits[k], (size_t)hp.chunk * 4 * sizeof(float)));
         if (!hp.done[k]) LMGPU_CUDA_TRY(cudaEventCreateWithFlags(&hp.done[k], cudaEventDisableTiming));
     }
     const int64_t nchunks = (n + chunk - 1) / chunk;
@@ -751,10 +753,17 @@ int intersect_host_staged(LmgpuScene* scene, const float* rays_aos, int64_t n, v
         const int k = static_cast<int>(c % HostPipeline::SLOTS);
         const int64_t b = c * chunk, m = std::min(chunk, n - b);
         LMGPU_CUDA_TRY(cudaEventSynchronize(hp.done[k]));
-        if (stage_out)
+        if (!stage_out) return LMGPU_OK;
+        CopyPool& pool = CopyPool::get();
+        const int parts = m * 16 < (int64_t(1) << 20) ? 1 : pool.size();
+        const int64_t part = (m / parts + 16) / 16 * 16;
+        pool.run(parts, [&](int i) {
+            const int64_t at = i * part, cnt = std::min(part, m - at);
+            if (cnt <= 0) return;
             for (int a = 0; a < 4; a++)
                 if (outs[a])
-                    parallel_copy(static_cast<char*>(outs[a]) + 4 * b, hp.stage_hits[k] + a * chunk, (size_t)m * 4);
+                    std::memcpy(static_cast<char*>(outs[a]) + 4 * (b + at), hp.stage_hits[k] + a * chunk + at, (size_t)cnt * 4);
+        });
         return LMGPU_OK;
     };
     int rc = LMGPU_OK;
