@@ -141,8 +141,8 @@ typedef struct {
     int32_t max_depth;
     int32_t layout;
     int64_t device_bytes;       /* bytes in HBM of the traversal data: the reference's tree (binary
-                                   and 8-wide), the render tree (8-wide), the triangle records and
-                                   leaf boxes */
+                                   and 8-wide), with a camera the render tree (the same), the triangle
+                                   records and leaf boxes */
     double build_seconds;       /* host BVH build time */
     float bounds_min[3];        /* Scene::GetAABBTriangles */
     float bounds_max[3];

@@ -92,7 +92,7 @@ __device__ __forceinline__ int32_t cast_ray(const DeviceScene& s, V3 o, V3 d, fl
     bool ok = true;
     // The renderers' walk and triangle test: the wavefront kernels' own.
     if (NAIVE) trace_naive<ANY>(s.tris_by_id, s.num_tris, r, h, nullptr);
-    else ok = trace8<ANY>(s.bvh8, s.tris8, s.check_boxes ? s.boxes8 : nullptr, r, h, stack, s.stack8_cap < STACK ? s.stack8_cap : STACK);
+    else ok = trace8<ANY>(s, r, h, stack, s.stack8_cap < STACK ? s.stack8_cap : STACK);
     if (!ok) { atomicOr(status, STATUS_STACK_OVERFLOW); h.tri = -1; }
     return h.tri;
 }

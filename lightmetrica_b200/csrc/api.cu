@@ -282,13 +282,16 @@ int create_impl(const LmgpuSceneDesc* desc, LmgpuScene** out)
     // The trees every traversal walks. The reference's: origins up to
     // WIDE_ORIGIN_LIMIT times the scene's largest coordinate (the boxes grow with the
     // bound; rays from farther away take the reference's own walk). The
-    // render tree: rays start in the scene's bounds or at the camera; far from the
-    // origin (coordinates beyond FAR_FROM_ORIGIN times the scene's extent) its candidate
-    // hits are also tested against their float leaf boxes.
+    // render tree: rays start in the scene's bounds or at the camera (without a camera
+    // nothing renders, and it is not collapsed); far from the origin (coordinates beyond
+    // FAR_FROM_ORIGIN times the scene's extent) every candidate hit is tested against its
+    // float leaf box, elsewhere those within NEAR_EDGE of a triangle's edge.
     constexpr double WIDE_ORIGIN_LIMIT = 8.0, FAR_FROM_ORIGIN = 8.0;
+    constexpr float NEAR_EDGE = 1.0f / 64.0f;
     Bvh8Tree wide, rwide;
     double scene_max = 0.0, extent = 0.0, wide_limit = 0.0;
     bool far = false;
+    std::vector<int32_t> tie_pos;
     if (desc->layout != LMGPU_LAYOUT_NAIVE && b.num_tris > 0) {
         for (int c = 0; c < 3; c++) {
             scene_max = std::max(scene_max, (double)std::max(std::fabs(b.bounds.mn[c]), std::fabs(b.bounds.mx[c])));
@@ -305,7 +308,7 @@ int create_impl(const LmgpuSceneDesc* desc, LmgpuScene** out)
         bool short_of_memory = false;
         std::thread side([&] {
             try {
-                collapse_bvh8(b, b.bvh2, b.tris, b.bvh2_root, b.root_box, WIDE_ORIGIN_LIMIT * scene_max, true, true,
+                collapse_bvh8(b, b.bvh2, b.tris, b.bvh2_root, b.root_box, WIDE_ORIGIN_LIMIT * scene_max, true,
                               desc->build_threads, wide);
             } catch (...) {
                 short_of_memory = true;
@@ -315,12 +318,19 @@ int create_impl(const LmgpuSceneDesc* desc, LmgpuScene** out)
         try {
             if (render_tree) {
                 build_render_tree(b, desc->build_threads);
-                collapse_bvh8(b, b.rbvh2, b.rtris, b.rbvh2_root, b.rroot_box, ray_max, false, far, desc->build_threads, rwide);
+                if (cam.valid) collapse_bvh8(b, b.rbvh2, b.rtris, b.rbvh2_root, b.rroot_box, ray_max, false, desc->build_threads, rwide);
+            }
+            if (cam.valid) {
+                const std::vector<TriRecord>& order = render_tree ? b.rtris : b.tris;
+                if (render_tree) set_splits(b.rbvh2);
+                tie_pos.resize(order.size());
+                for (size_t i = 0; i < order.size(); i++) tie_pos[order[i].tri_id] = (int32_t)i;
             }
         } catch (...) {
             main_short = true;
         }
         side.join();
+        if (!short_of_memory && !render_tree && cam.valid) set_splits(b.bvh2);   // (after the collapse that reads it)
         if (short_of_memory || main_short) return fail(LMGPU_ERR_OOM, "host allocation failed during the tree builds");
     }
 
@@ -463,7 +473,11 @@ int create_impl(const LmgpuSceneDesc* desc, LmgpuScene** out)
         r.bvh2 = nullptr;              // renders have no use for the reference's walk
         r.tris = nullptr;
     }
-    s->rdev.check_boxes = far ? 1 : 0;
+    s->rdev.box_margin = far ? 2.0f : NEAR_EDGE;
+    s->rdev.tie_nodes = d.bvh2;
+    if (render_tree && cam.valid) up(b.rbvh2, &s->rdev.tie_nodes);
+    up(tie_pos, &s->rdev.tie_pos);
+    s->rdev.tie_root = render_tree ? b.rbvh2_root : b.bvh2_root;
     if (rc != LMGPU_OK) { lmgpu_scene_destroy(s); return rc; }
 
     // Scratch: status word and the persistent kernels' work counter.
@@ -478,7 +492,7 @@ int create_impl(const LmgpuSceneDesc* desc, LmgpuScene** out)
 #if LMGPU_BOUNDS_CHECK
     if (desc->layout != LMGPU_LAYOUT_NAIVE) {
         rc = check_trees(s, s->dev, (int64_t)b.bvh2.size(), (int64_t)wide.nodes.size(), (int64_t)b.tris.size());
-        if (rc == LMGPU_OK && render_tree)
+        if (rc == LMGPU_OK && render_tree && cam.valid)
             rc = check_trees(s, s->rdev, 0, (int64_t)rwide.nodes.size(), (int64_t)rwide.tris.size());
         if (rc != LMGPU_OK) { lmgpu_scene_destroy(s); return rc; }
     }
@@ -494,6 +508,7 @@ int create_impl(const LmgpuSceneDesc* desc, LmgpuScene** out)
     // Everything uploaded for traversal: the reference's tree (binary and
     // 8-wide) and the render tree (8-wide), with their triangle records.
     int64_t bytes = (int64_t)b.tris.size() * sizeof(TriRecord) + (int64_t)b.bvh2.size() * sizeof(Bvh2Node);
+    bytes += (render_tree && cam.valid ? (int64_t)b.rbvh2.size() * sizeof(Bvh2Node) : 0) + (int64_t)tie_pos.size() * sizeof(int32_t);
     for (const Bvh8Tree* t : { &wide, &rwide })
         bytes += (int64_t)t->nodes.size() * sizeof(Bvh8Node) + (int64_t)t->tris.size() * sizeof(TriRecord) +
                  (int64_t)t->boxes.size() * sizeof(LeafBox);

@@ -233,7 +233,7 @@ int32_t flatten_bvh2(const std::vector<BuildNode>& nodes, int32_t ni, std::vecto
         o.by[0] = L.bound.mn[1]; o.by[1] = L.bound.mx[1]; o.by[2] = R.bound.mn[1]; o.by[3] = R.bound.mx[1];
         o.bz[0] = L.bound.mn[2]; o.bz[1] = L.bound.mx[2]; o.bz[2] = R.bound.mn[2]; o.bz[3] = R.bound.mx[2];
         o.axis = n.axis;
-        o.pad = 0;
+        o.split = 0;
     }
     const int32_t l = flatten_bvh2(nodes, n.left, out);
     const int32_t r = flatten_bvh2(nodes, n.right, out);
@@ -681,8 +681,18 @@ struct Collapse {
 
 }  // namespace
 
+void set_splits(std::vector<Bvh2Node>& nodes)
+{
+    std::vector<int32_t> first(nodes.size());         // pre-order: children follow their parent
+    for (size_t i = nodes.size(); i-- > 0;) {
+        auto begin = [&](int32_t ref) { return ref < 0 ? ~ref : first[(size_t)ref]; };
+        first[i] = begin(nodes[i].left);
+        nodes[i].split = begin(nodes[i].right);
+    }
+}
+
 void collapse_bvh8(const BuiltScene& s, const std::vector<Bvh2Node>& nodes, const std::vector<TriRecord>& tris,
-                   int32_t root, const float* root_box, double magnitude, bool exact, bool boxes, int threads,
+                   int32_t root, const float* root_box, double magnitude, bool exact, int threads,
                    Bvh8Tree& out)
 {
     out = Bvh8Tree{};
@@ -774,7 +784,6 @@ void collapse_bvh8(const BuiltScene& s, const std::vector<Bvh2Node>& nodes, cons
             part[t] = Bvh8Tree{};
         }
     }
-    if (!boxes) return;
     std::vector<LeafBox> by_id(tris.size());
     auto put = [&](int32_t ref, const float* x, const float* y, const float* z) {
         LeafBox b{ { x[0], y[0], z[0] }, { x[1], y[1], z[1] }, { 0.0f, 0.0f } };

@@ -71,8 +71,8 @@ struct PrimitiveInput {
     const float* transform;   // 16 floats column-major or nullptr
 };
 
-// An 8-wide compressed tree, its triangle records in leaf order and, when asked
-// for, the binary leaf's box of every record.
+// An 8-wide compressed tree, its triangle records in leaf order and the binary leaf's
+// box of every record.
 struct Bvh8Tree {
     std::vector<Bvh8Node> nodes;      // the root is node 0
     std::vector<TriRecord> tris;
@@ -86,10 +86,12 @@ struct Bvh8Tree {
 //   exact      the tree serves the reference-exact walk: every box is inflated by
 //              the distance outside its triangle at which TriAccel::Intersect
 //              can still report a hit for rays from within `magnitude`
-//   boxes      also write each record's binary leaf box
 void collapse_bvh8(const BuiltScene& s, const std::vector<Bvh2Node>& nodes, const std::vector<TriRecord>& tris,
-                   int32_t root, const float* root_box, double magnitude, bool exact, bool boxes, int threads,
+                   int32_t root, const float* root_box, double magnitude, bool exact, int threads,
                    Bvh8Tree& out);
+
+// Sets every node's `split`.
+void set_splits(std::vector<Bvh2Node>& nodes);
 
 // Builds everything; returns an empty string on success, else an error.
 std::string build_scene(const std::vector<PrimitiveInput>& prims, int threads, bool want_bvh,

@@ -7,10 +7,10 @@
 //   TriRecord[]  48 B each, the reference TriAccel constants
 //                (triaccel.h:31-47) in the wide tree's leaf order; leaves
 //                are contiguous runs ended by TRI_LAST_IN_LEAF.
-//   LeafBox[]    32 B each, the binary leaf's box of every triangle (the
-//                reference's tree; the render tree far from the origin).
+//   LeafBox[]    32 B each, the binary leaf's box of every triangle.
 // and, for the reference's own depth-first walk (rays the wide walk hands back,
 // work counts, full hit records):
+// (the render tree's binary nodes settle ties, see tie_takes)
 //   Bvh2Node[]   64 B each, DFS pre-order, both children's boxes stored in
 //                the parent; a child reference >= 0 is an internal node index, < 0
 //                a leaf whose first TriRecord is ~ref.
@@ -31,7 +31,7 @@ struct alignas(16) Bvh2Node {
     float bz[4];
     int32_t left, right;   // child references
     int32_t axis;          // split axis of this node (near-first order)
-    int32_t pad;
+    int32_t split;         // position of the right child's first triangle (set_splits)
 };
 static_assert(sizeof(Bvh2Node) == 64, "Bvh2Node is 64 B");
 

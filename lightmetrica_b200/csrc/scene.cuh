@@ -53,8 +53,11 @@ struct DeviceScene {
     int32_t stack8_cap;    // stack bound of the 8-wide walk
     const Bvh8Node* bvh8;         // root: node 0
     const TriRecord* tris8;       // its leaf order
-    const LeafBox* boxes8;        // binary leaf box per tris8 record (the reference's tree; renders with check_boxes)
-    int32_t check_boxes;          // renders: test boxes8 on every candidate hit (scene far from the origin)
+    const LeafBox* boxes8;        // binary leaf box per tris8 record
+    float box_margin;             // renders: hits nearer than this to a triangle's edge (barycentric) are tested against boxes8
+    const Bvh2Node* tie_nodes;    // renders: the binary tree (tie_takes)
+    const int32_t* tie_pos;       // its leaf position of each triangle id
+    int32_t tie_root;
     float wide_limit;             // the reference's tree: origins up to this magnitude take the 8-wide walk
     // The reference's own walk (the reference's tree only).
     int32_t root_ref;

@@ -15,6 +15,7 @@
 // 2.0 / 1.54 ms.
 #pragma once
 #include <type_traits>
+#include "scene.cuh"
 #include "trace.cuh"
 
 namespace lmgpu {
@@ -142,11 +143,28 @@ __device__ __forceinline__ const float4* walk8_leaf(const Bvh8Node* __restrict__
 
 // ------------------------------------------------------- candidate hits ----
 
-// The slab test of the record's binary leaf box, in the arithmetic of render
-// rays (multiply-adds): whether a walk through float boxes would have come to
-// this triangle. Renders far from the origin make it (DeviceScene::check_boxes):
-// there the triangle test's rounding reports hits outside the triangle, and the
-// 8-bit boxes let more of them through than float boxes do.
+// A render ray's hit is the one that a near-first walk of the binary tree through its
+// float boxes finds: the least t among the triangles whose leaf box the ray enters
+// before t (leaf_box_render), and among equal t the one visited last (tie_takes).
+// So the answer depends on neither the width of the nodes nor their rounding. Without
+// the box test, the triangle test's rounding reports hits just outside a triangle that
+// 8-bit boxes let through and float boxes do not (far from the origin, many). A hit well
+// inside its triangle is well inside the box, so that only hits near an edge are tested
+// (DeviceScene::box_margin). On every
+// hit the test takes the 1080p frame from 13.15 to 13.70 ms; near edges only it costs 2 %
+// (frame, six-scene batch and terrain alike).
+
+// Entry distance of a box, in the arithmetic of render rays (multiply-adds).
+__device__ __forceinline__ float box_entry(float lox, float hix, float loy, float hiy, float loz, float hiz, const TraversalRay& r)
+{
+    float x0, x1, y0, y1, z0, z1;
+    fma_pair(lox, hix, r.inv_min[0], r.inv_max[0], x0, x1);
+    fma_pair(loy, hiy, r.inv_min[1], r.inv_max[1], y0, y1);
+    fma_pair(loz, hiz, r.inv_min[2], r.inv_max[2], z0, z1);
+    return fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fminf(z0, z1));
+}
+
+// The slab test of the record's binary leaf box in the same arithmetic.
 __device__ __forceinline__ bool leaf_box_render(const LeafBox* __restrict__ boxes, int64_t at, const TraversalRay& r)
 {
     const float4 a = __ldg(reinterpret_cast<const float4*>(boxes + at));
@@ -158,6 +176,44 @@ __device__ __forceinline__ bool leaf_box_render(const LeafBox* __restrict__ boxe
     const float tn = fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fminf(z0, z1));
     const float tf = fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fmaxf(z0, z1));
     return tn <= tf && tf > r.tmin && tn < r.tmax;
+}
+
+// Whether triangle b, hit at the same t as triangle a, is the binary walk's answer: the one
+// visited later, unless its leaf is entered no sooner than t (a flat box may be; the walk
+// then culls it). Within a leaf the records are tested in order; where the two paths part,
+// the child entered later comes later, the right one if both are entered at once.
+__device__ __forceinline__ bool tie_takes(const Bvh2Node* __restrict__ nodes, const int32_t* __restrict__ pos, int32_t root,
+                                          int32_t a, int32_t b, float t, const TraversalRay& r)
+{
+    const int32_t pa = __ldg(pos + a), pb = __ldg(pos + b);
+    int32_t lo = min(pa, pb), hi = max(pa, pb);
+    bool parted = false, b_later = pb > pa;
+    float te = -FLT_MAX;                       // of the later one's leaf box
+    for (int32_t ref = root; ref >= 0;) {
+        const float4* n = reinterpret_cast<const float4*>(nodes + ref);
+        const float4 x = __ldg(n), y = __ldg(n + 1), z = __ldg(n + 2);
+        const int4 meta = __ldg(reinterpret_cast<const int4*>(n + 3));   // left, right, axis, split
+        const float tl = box_entry(x.x, x.y, y.x, y.y, z.x, z.y, r), tr = box_entry(x.z, x.w, y.z, y.w, z.z, z.w, r);
+        if (!parted && lo < meta.w && hi >= meta.w) {
+            if (tr < tl) { b_later = pb < pa; hi = lo; }   // right child first: the left one comes later
+            lo = hi;
+            parted = true;
+        }
+        const bool right = lo >= meta.w;
+        te = right ? tr : tl;
+        ref = right ? meta.y : meta.x;
+    }
+    return (!parted || te < t) == b_later;
+}
+
+// Whether a candidate (record `at`, triangle id, t <= r.tmax) replaces the hit h.
+template <bool ANY>
+__device__ __forceinline__ bool render_candidate(const DeviceScene& s, int64_t at, int32_t id, float t, float u, float v,
+                                                 const TraversalRay& r, const Hit& h, bool any)
+{
+    if (fminf(fminf(u, v), 1.0f - u - v) < s.box_margin && !leaf_box_render(s.boxes8, at, r)) return false;
+    if (ANY || any || t < r.tmax || h.tri < 0) return true;
+    return tie_takes(s.tie_nodes, s.tie_pos, s.tie_root, h.tri, id, t, r);
 }
 
 // Exact walk. The reference's answer for a ray is a fold over the triangles whose
@@ -219,12 +275,12 @@ __device__ __forceinline__ bool exact_wide_ok(const RayIn& in, float limit)
 // --------------------------------------------------------- one thread ----
 
 // Closest (or any) render hit by one thread; `stack` holds `cap` groups.
-// Between triangles hit at the same distance the higher id wins, whatever the
-// order of the tests. Returns false on stack overflow.
+// Returns false on stack overflow.
 template <bool ANY_HIT>
-__device__ __forceinline__ bool trace8(const Bvh8Node* __restrict__ nodes, const TriRecord* __restrict__ tris,
-                                       const LeafBox* __restrict__ boxes, TraversalRay& r, Hit& h, uint2* stack, int cap)
+__device__ __forceinline__ bool trace8(const DeviceScene& s, TraversalRay& r, Hit& h, uint2* stack, int cap)
 {
+    const Bvh8Node* __restrict__ nodes = s.bvh8;
+    const TriRecord* __restrict__ tris = s.tris8;
     const uint32_t oct = r.neg & 7u;
     Walk8 w;
     walk8_begin(w, oct);
@@ -251,14 +307,12 @@ __device__ __forceinline__ bool trace8(const Bvh8Node* __restrict__ nodes, const
         for (;;) {
             const float4 q0 = __ldg(p), q1 = __ldg(p + 1), q2 = __ldg(p + 2);
             float u, v, t;
+            const int32_t id = static_cast<int32_t>(__float_as_uint(q2.z));
             if (triaccel_intersect_fast(q0, q1, q2, r, r.tmax, u, v, t) &&
-                (!boxes || leaf_box_render(boxes, (p - reinterpret_cast<const float4*>(tris)) / 3, r))) {
-                const int32_t id = static_cast<int32_t>(__float_as_uint(q2.z));
-                if (t < r.tmax || id > h.tri) {
-                    r.tmax = t;
-                    h.tri = id; h.t = t; h.u = u; h.v = v;
-                    if (ANY_HIT) return true;
-                }
+                render_candidate<ANY_HIT>(s, (p - reinterpret_cast<const float4*>(tris)) / 3, id, t, u, v, r, h, ANY_HIT)) {
+                r.tmax = t;
+                h.tri = id; h.t = t; h.u = u; h.v = v;
+                if (ANY_HIT) return true;
             }
             if (__float_as_uint(q0.x) & TRI_LAST_IN_LEAF) {
                 if (w.leaves == 0) break;

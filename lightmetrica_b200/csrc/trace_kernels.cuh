@@ -103,8 +103,8 @@ __device__ __forceinline__ void reference_walk(const DeviceScene& s, int32_t* st
 // descent ends when every lane still in it holds leaves, and pauses once fewer
 // than LMGPU_TRACE_EXIT_BELOW lanes are in it. The order in which a ray's
 // triangles are tested thus depends on the warp's other rays, its result does
-// not: render rays break exact ties by triangle id, exact rays hand theirs to
-// the reference's walk. (Without postponing: 1.97 against 1.66 ms on the soup,
+// not: render rays break exact ties by the binary tree's order, exact rays hand
+// theirs to the reference's walk. (Without postponing: 1.97 against 1.66 ms on the soup,
 // 2.00 / 1.59 and 1.87 / 1.59 ms on the bounce and shadow rays.)
 // For a multi-scene I/O policy each lane switches to its new ray's scene at
 // refill; an empty scene is a miss. The COUNT instantiation (measurement
@@ -269,20 +269,12 @@ k_trace_persistent(const __grid_constant__ DeviceScene s, const __grid_constant_
                 const int32_t id = static_cast<int32_t>(__float_as_uint(q2.z));
                 float u, v, t;
                 if constexpr (RENDER) {
-                    if (triaccel_intersect_fast(q0, q1, q2, r, r.tmax, u, v, t)) {
-                        bool take = t < r.tmax || id > h.tri;
-                        bool check = s.check_boxes;
-                        if constexpr (TABLE) check = ray_scene(idx).check_boxes;
-                        if (check) {
-                            const LeafBox* boxes = s.boxes8;
-                            if constexpr (TABLE) boxes = ray_scene(idx).boxes8;
-                            take = take && leaf_box_render(boxes, (p - reinterpret_cast<const float4*>(tris)) / 3, r);
-                        }
-                        if (take) {
-                            r.tmax = t;
-                            h.tri = id; h.t = t; h.u = u; h.v = v;
-                            if (any) { done = true; break; }
-                        }
+                    if (triaccel_intersect_fast(q0, q1, q2, r, r.tmax, u, v, t) &&
+                        render_candidate<MODE == TRACE_ANY>(TABLE ? ray_scene(idx) : s, (p - reinterpret_cast<const float4*>(tris)) / 3, id,
+                                                            t, u, v, r, h, any)) {
+                        r.tmax = t;
+                        h.tri = id; h.t = t; h.u = u; h.v = v;
+                        if (any) { done = true; break; }
                     }
                 } else {
                     if (triaccel_intersect(q0, q1, q2, r, r.tmax, u, v, t)) {
