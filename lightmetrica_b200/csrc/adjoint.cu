@@ -761,7 +761,7 @@ int run_diff_waves(LmgpuScene* sc, const DiffConsts& c, float* image, const floa
         auto grid = [&](auto kernel, int64_t blocks) { return (unsigned)std::min<int64_t>(blocks, resident_blocks(kernel)); };
         ctx.rc.sample_base = c.sample_offset + base;
         k_wave_begin<<<1, 128, 0, stream>>>(st.counters);
-        k_pt_init<TECH, Ctx><<<(unsigned)full, 128, 0, stream>>>(ctx, st, n, 0, ring_rays(1), ring_shadow(0));
+        k_pt_init<TECH, Ctx><<<(unsigned)full, 128, 0, stream>>>(ctx, st, n, 0);
         for (int k = 1; k <= bounces; k++) {
             const int qin = (k - 1) & 1;
             const auto io = ray_queue<false>(st, qin, ring_rays(k), nullptr);

@@ -295,7 +295,7 @@ struct Wave {
     {
         const PathState& st = b->st[l];
         k_wave_begin<<<1, 128, 0, s>>>(st.counters);
-        k_pt_init<TECH, Ctx><<<(unsigned)((L.paths + 127) / 128), 128, 0, s>>>(ctx(b, l), st, 0, 0, ring_rays(1), ring_shadow(0));
+        k_pt_init<TECH, Ctx><<<(unsigned)((L.paths + 127) / 128), 128, 0, s>>>(ctx(b, l), st, 0, 0);
         if (TECH != LMGPU_RENDER_PT && !merged(b, 1)) shadow(b, L, l, 0, s);
         for (int k = 1; k < T; k++) bounce(b, L, l, k, s);
     }
@@ -346,7 +346,7 @@ struct Stream {
         const PathState& st = b->st[0];
         unsigned long long* work = b->d_work + 2 * q;
         k_stream_plan<<<1, 1, 0, s>>>(b->d_ctl, st.counters, q, b->d_stats, work);
-        k_pt_init<TECH, Ctx><<<(unsigned)((L.paths + 127) / 128), 128, 0, s>>>(make<Ctx>(b), st, 0, q, COUNTER_RAYS[q], COUNTER_SHADOW);
+        k_pt_init<TECH, Ctx><<<(unsigned)((L.paths + 127) / 128), 128, 0, s>>>(make<Ctx>(b), st, 0, q);
         launch_traversal<STACK, TRACE_CLOSEST>(b, L.trace_blocks, L.proto, ray_queue<true>(st, q, COUNTER_RAYS[q], b->d_table), work, s);
         k_pt_shade<TECH, Ctx><<<L.shade_blocks, 128, 0, s>>>(make<Ctx>(b), st, 0, q, nullptr);
         if (TECH != LMGPU_RENDER_PT)
@@ -711,10 +711,10 @@ int run_waves(LmgpuBatch* b, const Plan& pl, int64_t P, cudaStream_t s, int64_t&
         // Unbounded depth: finish the wave's remaining bounces directly.
         int k = pl.bounces + 1;
         for (;; k++) {
-            LMGPU_CUDA_TRY(cudaMemcpyAsync(b->h_counts, b->st[0].counters + ring_rays(0), RING * sizeof(uint32_t),
+            LMGPU_CUDA_TRY(cudaMemcpyAsync(b->h_counts, b->st[0].counters + RING_PAIRS, 2 * RING * sizeof(uint32_t),
                                            cudaMemcpyDeviceToHost, s));
             LMGPU_CUDA_TRY(cudaStreamSynchronize(s));
-            if (b->h_counts[k & (RING - 1)] == 0) break;
+            if (b->h_counts[ring_rays(k) - RING_PAIRS] == 0) break;
             W::bounce(b, L, 0, k, s);
             LMGPU_CUDA_TRY(cudaGetLastError());
         }
@@ -848,7 +848,7 @@ int lmgpu_batch_create(LmgpuScene* const* scenes, int32_t num_scenes, LmgpuBatch
     hm(reinterpret_cast<void**>(&b->h_table), n * sizeof(BatchEntry));
     hm(reinterpret_cast<void**>(&b->h_begins), (n + 1) * sizeof(int64_t));
     hm(reinterpret_cast<void**>(&b->h_stats), NSTATS * sizeof(unsigned long long));
-    hm(reinterpret_cast<void**>(&b->h_counts), 16);
+    hm(reinterpret_cast<void**>(&b->h_counts), 2 * RING * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemset(b->d_status, 0, sizeof(int32_t));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->cap_stream, cudaStreamNonBlocking);
     int least = 0, greatest = 0;

@@ -26,7 +26,7 @@ __device__ __align__(256) unsigned char g_noalloc_workspace[NOALLOC_WORKSPACE_BY
 constexpr int MAX_DEVICES = 64;
 std::mutex g_mu;
 void* g_workspace_ptr[MAX_DEVICES] = {};          // device address of the array, per device
-uint32_t g_host_counts[MAX_DEVICES][4] = {};       // queue-counter readback, per device
+uint32_t g_host_counts[MAX_DEVICES][8] = {};       // queue-counter readback, per device
 
 // Device address of the array on the current device. In host code the
 // array's name is a host-side stand-in, not a device address, so it is

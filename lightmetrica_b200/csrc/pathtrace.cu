@@ -179,7 +179,7 @@ int trace_wave(LmgpuScene* sc, const IO& io, unsigned long long* work, int64_t m
 // device, a question (copy, wait, next launch) about 12.
 constexpr int FIRST_CHECK = 8, CHECK_EVERY = 4;
 
-// `counts`: host memory of 4 words, or of the whole header (`with_stats`).
+// ws.host_counts: host memory of 2 * RING words, or of the whole header (`with_stats`).
 template <int TECH, int STACK, class F>
 int render_waves(LmgpuScene* sc, const LmgpuRenderParams& p, F* film, cudaStream_t stream, LmgpuRenderStats& stats,
                  Workspace& ws, bool with_stats)
@@ -224,16 +224,16 @@ int render_waves(LmgpuScene* sc, const LmgpuRenderParams& p, F* film, cudaStream
         stats.paths += cnt;
         if (c.max_pv != -1 && c.max_pv <= 1) continue;   // no path vertex beyond the camera
         LMGPU_CUDA_TRY(cudaMemsetAsync(st.counters, 0, COUNTER_WORDS * sizeof(uint32_t), stream));
-        k_pt_init<TECH, Ctx><<<(unsigned)((cnt + 127) / 128), 128, 0, stream>>>(ctx, st, cnt, 0, ring_rays(1), ring_shadow(0));
+        k_pt_init<TECH, Ctx><<<(unsigned)((cnt + 127) / 128), 128, 0, stream>>>(ctx, st, cnt, 0);
         LMGPU_CUDA_TRY(cudaGetLastError());
         const unsigned blocks = (unsigned)std::min<int64_t>((cnt + 127) / 128, shade_blocks);
         int k = 1;
         for (; c.max_pv == -1 || k < c.max_pv; k++) {
             if (k > FIRST_CHECK && (k - FIRST_CHECK - 1) % CHECK_EVERY == 0) {
-                LMGPU_CUDA_TRY(cudaMemcpyAsync(ws.host_counts, st.counters + ring_rays(0), RING * sizeof(uint32_t),
+                LMGPU_CUDA_TRY(cudaMemcpyAsync(ws.host_counts, st.counters + RING_PAIRS, 2 * RING * sizeof(uint32_t),
                                                cudaMemcpyDeviceToHost, stream));
                 LMGPU_CUDA_TRY(cudaStreamSynchronize(stream));
-                if (ws.host_counts[k & (RING - 1)] == 0) break;
+                if (ws.host_counts[ring_rays(k) - RING_PAIRS] == 0) break;
             }
             const int q = (k - 1) & 1;
             const auto rays = ray_queue<false>(st, q, ring_rays(k), nullptr);
@@ -403,7 +403,7 @@ int64_t workspace_paths_for_bytes(size_t bytes)
 }
 
 // Renders like lmgpu_render_device over a caller-owned wave workspace of
-// `ws_bytes` at `ws_mem` (device) and a host readback buffer of 4 counters:
+// `ws_bytes` at `ws_mem` (device) and a host readback buffer of 8 counters:
 // waves never exceed the workspace's capacity, and nothing is allocated.
 int render_device_preallocated(LmgpuScene* sc, const LmgpuRenderParams& p, void* film, cudaStream_t stream,
                                void* ws_mem, size_t ws_bytes, uint32_t* host_counts)
