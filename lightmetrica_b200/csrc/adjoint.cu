@@ -72,6 +72,7 @@ struct DiffConsts {
     uint64_t seed;
     int64_t sample_offset, num_samples, pixels;
     double inv_pixels;       // 1 / pixels
+    SampleOrder order;
     float scale;             // film rescale W*H/num_samples
     const float* albedo;     // 3 per triangle or null
     const float* emission;   // 3 per area light or null
@@ -371,7 +372,7 @@ __global__ void __launch_bounds__(128, 8) k_diff(const DeviceScene s, const Diff
     }
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < c.num_samples; j += stride) {
-        const uint64_t sample = (uint64_t)(c.sample_offset + j);
+        const uint64_t sample = (uint64_t)(c.sample_offset + ordered_sample(c.order, j));
         const uint64_t key = sample_key(c.seed, sample);
         if (BACKWARD) {
             rp.w[TAIL_SUM] = v3(0, 0, 0);
@@ -476,11 +477,14 @@ struct DiffScene : RenderContext {
     __device__ __forceinline__ const DeviceScene& scene(int) const { return s; }
     __device__ __forceinline__ const RenderConsts& consts(int) const { return rc; }
     __device__ __forceinline__ int64_t wave_count(int64_t n) const { return n; }
-    __device__ __forceinline__ int64_t sample_of(int, int64_t i) const { return rc.sample_base + i; }
+    __device__ __forceinline__ int64_t sample_of(int, int64_t i) const
+    {
+        return rc.sample_base + ordered_sample(rc.order, rc.path_base + i);
+    }
     __device__ __forceinline__ int begin_path(const PathState&, int64_t j, int64_t& i, int64_t& sample) const
     {
         i = j;
-        sample = rc.sample_base + j;
+        sample = sample_of(0, j);
         return 0;
     }
     __device__ __forceinline__ int path_depth(const PathState&, int64_t, int k) const { return k; }
@@ -740,6 +744,8 @@ int run_diff_waves(LmgpuScene* sc, const DiffConsts& c, float* image, const floa
     ctx.rc.seed = c.seed;
     ctx.rc.pixels = c.pixels;
     ctx.rc.inv_pixels = c.inv_pixels;
+    ctx.rc.sample_base = c.sample_offset;
+    ctx.rc.order = c.order;
     ctx.scale = c.scale;
     ctx.albedo = c.albedo;
     ctx.emission_of = c.emission;
@@ -759,7 +765,7 @@ int run_diff_waves(LmgpuScene* sc, const DiffConsts& c, float* image, const floa
         const int64_t full = (n + 127) / 128;
         const unsigned shade = (unsigned)std::min<int64_t>(full, 148 * 8);
         auto grid = [&](auto kernel, int64_t blocks) { return (unsigned)std::min<int64_t>(blocks, resident_blocks(kernel)); };
-        ctx.rc.sample_base = c.sample_offset + base;
+        ctx.rc.path_base = base;
         k_wave_begin<<<1, 128, 0, stream>>>(st.counters);
         k_pt_init<TECH, Ctx><<<(unsigned)full, 128, 0, stream>>>(ctx, st, n, 0);
         for (int k = 1; k <= bounces; k++) {
@@ -863,6 +869,7 @@ int launch_diff(LmgpuScene* sc, const LmgpuRenderParams* p, const LmgpuDiffParam
     c.num_samples = p->num_samples;
     c.pixels = (int64_t)sc->dev.cam.width * sc->dev.cam.height;
     c.inv_pixels = 1.0 / double(c.pixels);
+    c.order = sample_order(p->num_samples, sc->dev.cam.width, sc->dev.cam.height, p->sampling == LMGPU_SAMPLING_STRATIFIED);
     c.scale = float(double(c.pixels) / double(p->num_samples));
     c.albedo = dp ? dp->albedo : nullptr;
     c.emission = dp ? dp->emission : nullptr;

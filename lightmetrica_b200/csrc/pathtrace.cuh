@@ -83,9 +83,8 @@ __device__ __forceinline__ void stratified_raster(int64_t sample, int64_t pixels
 // plane, and uniform sampling (samples lie anywhere), keep the index order.
 // Measured against the index order: six-scene batch 26.6 -> 25.1 ms, terrain
 // 641 x 359 x 8 1.95 -> 1.91 ms, 1080p terrain frame 15.14 -> 15.10 ms. Plane by plane
-// within a block took 5 % longer on the batch and 2 % on the frame. (The differentiable
-// passes keep the index order: a warp on one pixel adds its gradients to one triangle,
-// 16.2 -> 16.3 ms.)
+// within a block took 5 % longer on the batch and 2 % on the frame. Differentiable
+// 512 x 512 x 32: 15.34 -> 15.03 ms.
 struct SampleOrder {
     int64_t ordered;       // samples in whole planes (0: index order)
     int64_t planes, pixels;

@@ -99,11 +99,11 @@ struct RenderConsts {
     int32_t max_pv;
     int32_t sampling;
     uint64_t seed;
-    int64_t sample_base;   // the scene's sample offset (differentiable passes: sample index of the wave's path 0)
+    int64_t sample_base;   // the scene's sample offset
     int64_t pixels;
     double inv_pixels;     // 1 / pixels
-    SampleOrder order;     // path numbers to sample indices (renders)
-    int64_t path_base;     // OneScene: path number of the wave's path 0
+    SampleOrder order;     // path numbers to sample indices
+    int64_t path_base;     // one scene: path number of the wave's path 0
 };
 
 template <class F>
