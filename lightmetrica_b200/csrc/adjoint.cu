@@ -351,13 +351,17 @@ __device__ __forceinline__ void bounce_loop(const DeviceScene& s, const DiffCons
     }
 }
 
-template <int TECH, bool NAIVE, int STACK, bool BACKWARD>
-// 8 resident blocks per SM (64 registers, some spills): on the refined
+template <int TECH, bool NAIVE, int STACK, bool BACKWARD, int BLOCKS>
+// BLOCKS resident blocks per SM. A budget that 4 a SM hold takes 4 (no spills): its time
+// is its longest path's, and each spilled value is a trip through local memory on it
+// (65 x 49 x 4, both passes with their calls: 312 -> 297 us).
+// Larger ones (under capture, or brute force) take 8
+// (64 registers, some spills): on the refined
 // Cornell box, forward / backward 22.2 / 33.1 ms against 24.9 / 36.2 ms at the
 // unconstrained 94-96 registers (5 blocks); 6, 10 and 12 blocks were slower
 // in total. The passes are latency-bound and gain more from resident warps
 // than they lose to spills.
-__global__ void __launch_bounds__(128, 8) k_diff(const DeviceScene s, const DiffConsts c, float* image, const float* dL,
+__global__ void __launch_bounds__(128, BLOCKS) k_diff(const DeviceScene s, const DiffConsts c, float* image, const float* dL,
                                               float* d_albedo, float* d_emission, int32_t* status)
 {
     uint2 stack[STACK];
@@ -817,8 +821,14 @@ int launch_diff_l(LmgpuScene* sc, const DiffConsts& c, bool backward, float* ima
                   float* de, cudaStream_t st)
 {
     const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((c.num_samples + 127) / 128, 148 * 16));
-    if (backward) k_diff<TECH, NAIVE, STACK, true><<<blocks, 128, 0, st>>>(sc->rdev, c, image, dL, da, de, sc->d_status);
-    else k_diff<TECH, NAIVE, STACK, false><<<blocks, 128, 0, st>>>(sc->rdev, c, image, dL, da, de, sc->d_status);
+    auto launch = [&](auto kernel) { kernel<<<blocks, 128, 0, st>>>(sc->rdev, c, image, dL, da, de, sc->d_status); };
+    if (blocks <= 148 * 4) {
+        if (backward) launch(k_diff<TECH, NAIVE, STACK, true, 4>);
+        else launch(k_diff<TECH, NAIVE, STACK, false, 4>);
+    } else {
+        if (backward) launch(k_diff<TECH, NAIVE, STACK, true, 8>);
+        else launch(k_diff<TECH, NAIVE, STACK, false, 8>);
+    }
     LMGPU_CUDA_TRY(cudaGetLastError());
     return LMGPU_OK;
 }
