@@ -41,7 +41,8 @@ constexpr uint32_t RAY_FINITE_INV = 8u;
 
 // Rays of the 8-wide walk (WIDE) keep inv_min = 1/d, clamped to +-1e18 so that
 // it stays finite, and inv_max = -o/d: a plane distance is then one
-// multiply-add, (lo - o)/d = fma(lo, 1/d, -o/d).
+// multiply-add, (lo - o)/d = fma(lo, 1/d, -o/d). inv_min's sign is `neg`'s: both
+// zeros give +1e18, since the walk picks near and far planes by `neg`.
 template <bool WIDE = false>
 __device__ __forceinline__ void setup_ray(TraversalRay& r, const RayIn& in)
 {
@@ -52,7 +53,7 @@ __device__ __forceinline__ void setup_ray(TraversalRay& r, const RayIn& in)
             r.o[c] = in.o[c];
             r.d[c] = in.d[c];
             float inv = __frcp_rn(in.d[c]);
-            if (!(fabsf(inv) <= 1e18f)) inv = copysignf(1e18f, in.d[c]);
+            if (!(fabsf(inv) <= 1e18f)) inv = in.d[c] < 0.0f ? -1e18f : 1e18f;
             r.inv_min[c] = inv;
             r.inv_max[c] = -(in.o[c] * inv);
             r.neg |= (in.d[c] < 0.0f ? 1u : 0u) << c;

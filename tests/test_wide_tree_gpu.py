@@ -101,3 +101,56 @@ def test_hits_and_visibility_equal_the_reference_walk(cuda, kind, n):
     s.status(stream)
     np.testing.assert_array_equal(occ.cpu().numpy().astype(bool), hit)
     s.close()
+
+
+def _equal_to_the_reference_walk(cuda, pos, faces, rays, impl="bvh"):
+    import torch
+    n = rays.shape[0]
+    s = create_scene(impl)
+    s.load(soup_primitives(pos, faces))
+    s.configure({})
+    s.build()
+    want = oracle.OracleScene(pos, faces, "bvh").intersect(rays)
+    got = s.intersect_host(rays)
+    np.testing.assert_array_equal(got["tri_id"], want["tri_id"])
+    hit = want["tri_id"] >= 0
+    for k in ("t", "u", "v"):
+        np.testing.assert_array_equal(got[k][hit], want[k][hit])
+    soa = {k: torch.from_numpy(v).to(cuda) for k, v in rays_soa(rays).items()}
+    occ = torch.zeros(n, dtype=torch.uint8, device=cuda)
+    stream = torch.cuda.current_stream().cuda_stream
+    s.occluded_device({k: v.data_ptr() for k, v in soa.items()}, occ.data_ptr(), n, stream)
+    s.status(stream)
+    np.testing.assert_array_equal(occ.cpu().numpy().astype(bool), hit)
+    s.close()
+    return hit
+
+
+@pytest.mark.parametrize("zeros", [1, 2])
+@pytest.mark.parametrize("kind", ["soup", "grid", "offset", "9"])
+def test_negated_zero_directions_hit_as_the_reference(cuda, kind, zeros):
+    """Direction components of either zero, alone and in pairs, from inside the boxes and from outside."""
+    pos, faces = _scene(kind)
+    n = 4001
+    rng = np.random.default_rng(31)
+    rays = _rays(pos, n, seed=30)
+    k = np.arange(n)
+    first = k % 3
+    d = rng.normal(size=(n, 3)).astype(np.float32)
+    for z in range(zeros):
+        d[k, (first + z) % 3] = np.copysign(np.float32(0), rng.choice([-1.0, 1.0], n).astype(np.float32))
+    rays[:, 3:6] = d / np.linalg.norm(d.astype(np.float64), axis=1, keepdims=True).astype(np.float32)
+    centre = pos.reshape(-1, 3)[faces].mean(1)[rng.integers(0, faces.shape[0], n)]
+    aim = k % 2 == 0                                 # towards a triangle from beside it: many hits
+    rays[aim, 0:3] = (centre - rays[:, 3:6] * rng.uniform(0.01, 0.5, (n, 1)).astype(np.float32))[aim]
+    zero = rays[:, 3:6] == 0
+    assert (np.signbit(rays[:, 3:6]) & zero).any() and (~np.signbit(rays[:, 3:6]) & zero).any()
+    hit = _equal_to_the_reference_walk(cuda, pos, faces, rays, "qbvh" if zeros == 2 else "bvh")
+    assert hit[np.signbit(rays[:, 3]) & zero[:, 0]].any()
+
+
+def test_a_negated_axis_hits(cuda):
+    pos = np.array([[-1, -1, -1], [1, -1, -1], [0, 1, -1]], np.float32)
+    rays = np.array([[0.01, 0.02, 0, -0.0, 0, -1, 0, FLT_MAX], [0.01, 0.02, 0, -0.0, -0.0, -1, 0, FLT_MAX],
+                     [0.01, 0.02, -2, -0.0, -0.0, 1, 0, FLT_MAX]], np.float32)
+    assert _equal_to_the_reference_walk(cuda, pos, np.array([[0, 1, 2]], np.uint32), rays).all()
