@@ -257,19 +257,27 @@ __device__ __forceinline__ void exact_candidate(const LeafBox* __restrict__ boxe
     r.tmax = window;
 }
 
-// Whether the inflated boxes cover this ray: a finite origin within the
-// magnitude they were built for, and every direction component zero or with a
-// finite inverse.
+// Whether the inflated boxes cover this ray, for scenes of largest coordinate M and
+// origins within limit = 8 M:
+//   * every non-zero direction component has an inverse below the clamp of setup_ray (1e18);
+//   * a zero axis, on which the walk's box ends at 1e18 times its distance, must not end
+//     the ray before its hit. Boxes that hold a hit reach at least 2^-21 * 8 M / 2 beyond
+//     the origin on such an axis (collapse_bvh8's margin of 4 ulps), that is 1.9e12 M,
+//     and a hit lies within 9.1 M of the origin on the direction's largest axis: any
+//     largest component above 5e-12 will do, and 2^-30 leaves a factor of 190;
+//   * inverses times grid steps (2^-83 and more) stay normal: at most 2^30.
+// NaN fails every comparison.
 __device__ __forceinline__ bool exact_wide_ok(const RayIn& in, float limit)
 {
     bool ok = true;
-    const float inf = __int_as_float(0x7f800000);
+    float longest = 0.0f;
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-        ok = ok && fabsf(in.o[c]) <= limit;
-        ok = ok && (in.d[c] == 0.0f || fabsf(__frcp_rn(in.d[c])) < inf) && fabsf(in.d[c]) < inf;
+        const float a = fabsf(in.d[c]);
+        ok = ok && fabsf(in.o[c]) <= limit && (a == 0.0f || a >= 0x1p-59f);
+        longest = fmaxf(longest, a);
     }
-    return ok;
+    return ok && longest >= 0x1p-30f && longest <= 0x1p30f;
 }
 
 // --------------------------------------------------------- one thread ----

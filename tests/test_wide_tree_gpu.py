@@ -154,3 +154,38 @@ def test_a_negated_axis_hits(cuda):
     rays = np.array([[0.01, 0.02, 0, -0.0, 0, -1, 0, FLT_MAX], [0.01, 0.02, 0, -0.0, -0.0, -1, 0, FLT_MAX],
                      [0.01, 0.02, -2, -0.0, -0.0, 1, 0, FLT_MAX]], np.float32)
     assert _equal_to_the_reference_walk(cuda, pos, np.array([[0, 1, 2]], np.uint32), rays).all()
+
+
+@pytest.mark.parametrize("scale", [1e-6, 1e-10, 1e-13, 1e-15, 1e-18, 1e-20, 1e-25, 1e-37, 1e9, 1e15, 1e25, 1e37])
+@pytest.mark.parametrize("kind", ["soup", "grid"])
+def test_directions_of_any_length_hit_as_the_reference(cuda, kind, scale):
+    """Unnormalised directions, with no, one and two zero components or ones far below the others; ray intervals that do
+    and do not begin or end on the way."""
+    pos, faces = _scene(kind)
+    n = 3001
+    rng = np.random.default_rng(41)
+    rays = _rays(pos, n, seed=40)
+    k = np.arange(n)
+    d = rng.normal(size=(n, 3)).astype(np.float32)
+    d[k % 5 == 1, 0] = 0.0
+    d[k % 5 == 2, 1:] = 0.0
+    d[k % 5 == 3, 2] *= np.float32(1e-9)
+    d[k % 5 == 4, 0] *= np.float32(1e-20)
+    d /= np.linalg.norm(d.astype(np.float64), axis=1, keepdims=True).astype(np.float32)
+    centre = pos[faces].mean(1)[rng.integers(0, faces.shape[0], n)]
+    aim = k % 2 == 0                                 # grazing the far side of the boxes, too: offsets of 1 down to 1e-5
+    away = (10.0 ** rng.uniform(-5, 0, (n, 1))).astype(np.float32)
+    rays[aim, 0:3] = (centre - d * away)[aim]
+    with np.errstate(under="ignore", over="ignore"):
+        rays[:, 3:6] = d * np.float32(scale)
+        rays[:, 6] = np.where(k % 3 == 0, np.float32(0.3 / scale if scale > 1e-38 else 0), 0)
+        rays[:, 7] = np.where(k % 4 == 0, np.minimum(2.0 / scale, FLT_MAX), FLT_MAX).astype(np.float32)
+    hit = _equal_to_the_reference_walk(cuda, pos, faces, rays)
+    assert hit.any() or scale < 1e-30
+
+
+def test_very_short_axis_directions_hit(cuda):
+    """The exit of a zero axis against an entry 1e15 and more away (in units of the direction's length)."""
+    pos = np.array([[-1, -1, -100], [1, -1, -100], [0, 1, -100]], np.float32)
+    rays = np.array([[0.49, -0.99, 0, 0, 0, -s, 0, FLT_MAX] for s in (1e-12, 1e-15, 1e-18, 1e-20, 1e-30)], np.float32)
+    assert _equal_to_the_reference_walk(cuda, pos, np.array([[0, 1, 2]], np.uint32), rays).all()
