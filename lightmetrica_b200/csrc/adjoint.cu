@@ -20,11 +20,11 @@
 //
 // Waves against one thread per sample (k_diff; measured on the refined Cornell box,
 // 512 x 512, 32 samples per pixel, up to 8 vertices, forward + backward):
-// one thread per sample over the binary tree 35.2 ms, over the 8-wide tree (more
-// registers, one ray's leaves hold up its warp) 61.5 ms, waves 16.0 ms.
-// One thread per sample stays for batches below WAVE_MIN_SAMPLES samples, whose
-// launches would cost more than the walk, and for streams being captured (a
-// wave's workspace is allocated in stream order).
+// one thread per sample over the binary render tree 9.8 + 17.9 ms, over the 8-wide tree
+// (more registers, and one ray's leaves hold up its warp) 18.4 + 36.6 ms, waves 14.2 ms in
+// all. So one thread walks the binary tree. It stays for batches below WAVE_MIN_SAMPLES
+// samples, whose launches would cost more than the walk, and for streams being captured
+// (a wave's workspace is allocated in stream order).
 //
 // The tail of a path of more vertices than a wave records (RECORDED_VERTS;
 // UNBOUNDED_VERTS where the depth has no bound) is run by one thread from the path's
@@ -80,7 +80,7 @@ struct DiffConsts {
 
 template <bool NAIVE, bool ANY, int STACK>
 __device__ __forceinline__ int32_t cast_ray(const DeviceScene& s, V3 o, V3 d, float tmin, float tmax, Hit& h,
-                                            uint2* stack, int32_t* status)
+                                            int2* stack, int32_t* status)
 {
     RayIn in;
     in.o[0] = o.x; in.o[1] = o.y; in.o[2] = o.z;
@@ -91,15 +91,15 @@ __device__ __forceinline__ int32_t cast_ray(const DeviceScene& s, V3 o, V3 d, fl
     h.tri = -1;
     if (s.num_tris == 0) return -1;
     bool ok = true;
-    // The renderers' walk and triangle test: the wavefront kernels' own.
+    // The render tree and arithmetic of the waves, over its binary nodes.
     if (NAIVE) trace_naive<ANY>(s.tris_by_id, s.num_tris, r, h, nullptr);
-    else ok = trace8<ANY>(s, r, h, stack, s.stack8_cap < STACK ? s.stack8_cap : STACK);
+    else ok = trace_bvh2_render<ANY>(s.bvh2, s.tris, s.root_ref, s.root_box, r, h, stack, s.stack_cap < STACK ? s.stack_cap : STACK);
     if (!ok) { atomicOr(status, STATUS_STACK_OVERFLOW); h.tri = -1; }
     return h.tri;
 }
 
 template <bool NAIVE, int STACK>
-__device__ __forceinline__ bool visible(const DeviceScene& s, V3 a, V3 b, uint2* stack, int32_t* status)
+__device__ __forceinline__ bool visible(const DeviceScene& s, V3 a, V3 b, int2* stack, int32_t* status)
 {
     const V3 d = b - a;
     const float len = sqrtf(length2(d));
@@ -246,7 +246,7 @@ __device__ __noinline__ void save_point(PathPoint* dst, const PathPoint& src) { 
 // instantiations compute the same path from the same state.
 template <int TECH, bool NAIVE, int STACK, bool BACKWARD, bool TAIL>
 __device__ __forceinline__ void bounce_loop(const DeviceScene& s, const DiffConsts& c, uint64_t key, int path_pixel,
-                                            PathPoint& pp, PathPoint* ck, bool* deep, Replay& rp, uint2* stack,
+                                            PathPoint& pp, PathPoint* ck, bool* deep, Replay& rp, int2* stack,
                                             float* image, const float* dL, float* d_albedo, EmissionSum& es,
                                             float* s_de, float* d_emission, int32_t* status)
 {
@@ -354,17 +354,14 @@ __device__ __forceinline__ void bounce_loop(const DeviceScene& s, const DiffCons
 template <int TECH, bool NAIVE, int STACK, bool BACKWARD, int BLOCKS>
 // BLOCKS resident blocks per SM. A budget that 4 a SM hold takes 4 (no spills): its time
 // is its longest path's, and each spilled value is a trip through local memory on it
-// (65 x 49 x 4, both passes with their calls: 312 -> 297 us).
-// Larger ones (under capture, or brute force) take 8
-// (64 registers, some spills): on the refined
-// Cornell box, forward / backward 22.2 / 33.1 ms against 24.9 / 36.2 ms at the
-// unconstrained 94-96 registers (5 blocks); 6, 10 and 12 blocks were slower
-// in total. The passes are latency-bound and gain more from resident warps
-// than they lose to spills.
+// (65 x 49 x 4, both passes with their calls: 315 -> 295 us).
+// Larger ones take 8 (64 registers, some spills): on the refined Cornell box, 512 x 512 x
+// 32, forward / backward 9.8 / 17.9 ms against 12.3 / 23.0 ms with 4. The passes are
+// latency-bound and gain more from resident warps than they lose to spills.
 __global__ void __launch_bounds__(128, BLOCKS) k_diff(const DeviceScene s, const DiffConsts c, float* image, const float* dL,
                                               float* d_albedo, float* d_emission, int32_t* status)
 {
-    uint2 stack[STACK];
+    int2 stack[STACK];
     Replay rp;
     __shared__ float s_de[3 * SHARED_LIGHTS];
     EmissionSum es;
@@ -601,11 +598,12 @@ __global__ void k_diff_emission(const double* part, int copies, int n, float* d_
 // queued ray. Their vertices count from RECORDED_VERTS on, so that every
 // contribution is "deeper than the record" (see the head of this file); the one
 // found by the first hit belongs to the wave's last vertex.
-template <int TECH, int STACK, bool BACKWARD>
+constexpr int TAIL_STACK = 256;
+template <int TECH, bool BACKWARD>
 __global__ void __launch_bounds__(128) k_diff_tail(const DiffScene<BACKWARD> ctx, const DiffConsts c, const PathState st, int q, int k0,
                                                    float* d_albedo, float* d_emission, int32_t* status)
 {
-    uint2 stack[STACK];
+    int2 stack[TAIL_STACK];
     Replay rp;
     __shared__ float s_de[3 * SHARED_LIGHTS];
     EmissionSum es;
@@ -634,12 +632,12 @@ __global__ void __launch_bounds__(128) k_diff_tail(const DiffScene<BACKWARD> ctx
         pp.nv = BACKWARD ? RECORDED_VERTS : k0 - 1;
         bool deep = false;
         if (BACKWARD) rp.w[RECORDED_VERTS - 1] = rp.w[TAIL_SUM] = rp.w[RUN_SUM] = v3(0, 0, 0);
-        bounce_loop<TECH, false, STACK, BACKWARD, false>(ctx.s, c, key, pixel, pp, &ck, &deep, rp, stack, ctx.image, ctx.dL, d_albedo,
+        bounce_loop<TECH, false, TAIL_STACK, BACKWARD, false>(ctx.s, c, key, pixel, pp, &ck, &deep, rp, stack, ctx.image, ctx.dL, d_albedo,
                                                          es, s_de, d_emission, status);
         if (BACKWARD) {
             st.L[i] = f4(rp.w[TAIL_SUM] + rp.w[RECORDED_VERTS - 1], 0.0f);
             if (deep)
-                bounce_loop<TECH, false, STACK, BACKWARD, true>(ctx.s, c, key, pixel, ck, nullptr, nullptr, rp, stack, ctx.image, ctx.dL,
+                bounce_loop<TECH, false, TAIL_STACK, BACKWARD, true>(ctx.s, c, key, pixel, ck, nullptr, nullptr, rp, stack, ctx.image, ctx.dL,
                                                                 d_albedo, es, s_de, d_emission, status);
         }
     }
@@ -789,7 +787,7 @@ int run_diff_waves(LmgpuScene* sc, const DiffConsts& c, float* image, const floa
             any<<<grid(any, full), 128, 0, stream>>>(s, shadow_queue(st, ring_shadow(bounces), ctx), sc->d_status,
                                                      work(ring_shadow_work(bounces)), nullptr);
         }
-        if (tail) k_diff_tail<TECH, STACK, BACKWARD><<<shade, 128, 0, stream>>>(ctx, c, st, bounces & 1, bounces + 1, da, de, sc->d_status);
+        if (tail) k_diff_tail<TECH, BACKWARD><<<shade, 128, 0, stream>>>(ctx, c, st, bounces & 1, bounces + 1, da, de, sc->d_status);
         if constexpr (BACKWARD) k_diff_flush<<<(unsigned)full, 128, 0, stream>>>(ctx, c, st, n, da);
         else k_diff_splat<<<(unsigned)full, 128, 0, stream>>>(ctx, st, n);
         e = cudaGetLastError();
@@ -845,17 +843,18 @@ template <int TECH>
 int launch_diff_t(LmgpuScene* sc, const DiffConsts& c, bool backward, float* image, const float* dL, float* da,
                   float* de, cudaStream_t st)
 {
-    const int cap = sc->rdev.stack8_cap;
-    if (cap <= 128 && diff_as_waves(sc, c, st)) {
-        if (cap <= 32)
+    const int cap = sc->rdev.stack_cap, cap8 = sc->rdev.stack8_cap;
+    if (cap8 <= 256 && cap <= TAIL_STACK && diff_as_waves(sc, c, st)) {
+        if (cap8 <= 32)
             return backward ? run_diff_waves<TECH, 32, true>(sc, c, image, dL, da, de, st)
                             : run_diff_waves<TECH, 32, false>(sc, c, image, dL, da, de, st);
         return backward ? run_diff_waves<TECH, 256, true>(sc, c, image, dL, da, de, st)
                         : run_diff_waves<TECH, 256, false>(sc, c, image, dL, da, de, st);
     }
-    if (cap <= 16) return launch_diff_s<TECH, 16>(sc, c, backward, image, dL, da, de, st);
-    if (cap <= 128) return launch_diff_s<TECH, 128>(sc, c, backward, image, dL, da, de, st);
-    return fail(LMGPU_ERR_UNSUPPORTED, "BVH too deep for the differentiable path (stack 128)");
+    if (cap <= 32) return launch_diff_s<TECH, 32>(sc, c, backward, image, dL, da, de, st);
+    if (cap <= 64) return launch_diff_s<TECH, 64>(sc, c, backward, image, dL, da, de, st);
+    if (cap <= 256) return launch_diff_s<TECH, 256>(sc, c, backward, image, dL, da, de, st);
+    return fail(LMGPU_ERR_UNSUPPORTED, "BVH too deep for the differentiable path (stack 256)");
 }
 
 int launch_diff(LmgpuScene* sc, const LmgpuRenderParams* p, const LmgpuDiffParams* dp, bool backward, float* image,

@@ -470,14 +470,19 @@ int create_impl(const LmgpuSceneDesc* desc, LmgpuScene** out)
         up(rwide.boxes, &r.boxes8);
         r.stack8_cap = rwide.depth;
         if (desc->max_stack_entries > 0 && desc->max_stack_entries < r.stack8_cap) r.stack8_cap = desc->max_stack_entries;
-        r.bvh2 = nullptr;              // renders have no use for the reference's walk
+        r.bvh2 = nullptr;
         r.tris = nullptr;
+        if (cam.valid) {
+            up(b.rbvh2, &r.bvh2);
+            up(b.rtris, &r.tris);
+        }
+        r.root_ref = b.rbvh2_root;
+        std::memcpy(r.root_box, b.rroot_box, sizeof(r.root_box));
+        r.stack_cap = 2 * b.rmax_depth + 4;
+        if (desc->max_stack_entries > 0 && desc->max_stack_entries < r.stack_cap) r.stack_cap = desc->max_stack_entries;
     }
     s->rdev.box_margin = far ? 2.0f : NEAR_EDGE;
-    s->rdev.tie_nodes = d.bvh2;
-    if (render_tree && cam.valid) up(b.rbvh2, &s->rdev.tie_nodes);
     up(tie_pos, &s->rdev.tie_pos);
-    s->rdev.tie_root = render_tree ? b.rbvh2_root : b.bvh2_root;
     if (rc != LMGPU_OK) { lmgpu_scene_destroy(s); return rc; }
 
     // Scratch: status word and the persistent kernels' work counter.
@@ -493,7 +498,7 @@ int create_impl(const LmgpuSceneDesc* desc, LmgpuScene** out)
     if (desc->layout != LMGPU_LAYOUT_NAIVE) {
         rc = check_trees(s, s->dev, (int64_t)b.bvh2.size(), (int64_t)wide.nodes.size(), (int64_t)b.tris.size());
         if (rc == LMGPU_OK && render_tree && cam.valid)
-            rc = check_trees(s, s->rdev, 0, (int64_t)rwide.nodes.size(), (int64_t)rwide.tris.size());
+            rc = check_trees(s, s->rdev, (int64_t)b.rbvh2.size(), (int64_t)rwide.nodes.size(), (int64_t)rwide.tris.size());
         if (rc != LMGPU_OK) { lmgpu_scene_destroy(s); return rc; }
     }
 #endif
@@ -505,10 +510,12 @@ int create_impl(const LmgpuSceneDesc* desc, LmgpuScene** out)
     info.max_depth = b.max_depth;
     info.layout = desc->layout;
     info.build_seconds = b.build_seconds;
-    // Everything uploaded for traversal: the reference's tree (binary and
-    // 8-wide) and the render tree (8-wide), with their triangle records.
+    // Everything uploaded for traversal: the reference's tree and (with a camera) the
+    // render tree, binary and 8-wide, with their triangle records.
     int64_t bytes = (int64_t)b.tris.size() * sizeof(TriRecord) + (int64_t)b.bvh2.size() * sizeof(Bvh2Node);
-    bytes += (render_tree && cam.valid ? (int64_t)b.rbvh2.size() * sizeof(Bvh2Node) : 0) + (int64_t)tie_pos.size() * sizeof(int32_t);
+    if (render_tree && cam.valid)
+        bytes += (int64_t)b.rbvh2.size() * sizeof(Bvh2Node) + (int64_t)b.rtris.size() * sizeof(TriRecord);
+    bytes += (int64_t)tie_pos.size() * sizeof(int32_t);
     for (const Bvh8Tree* t : { &wide, &rwide })
         bytes += (int64_t)t->nodes.size() * sizeof(Bvh8Node) + (int64_t)t->tris.size() * sizeof(TriRecord) +
                  (int64_t)t->boxes.size() * sizeof(LeafBox);

@@ -9,12 +9,12 @@
 //                are contiguous runs ended by TRI_LAST_IN_LEAF.
 //   LeafBox[]    32 B each, the binary leaf's box of every triangle.
 // and, for the reference's own depth-first walk (rays the wide walk hands back,
-// work counts, full hit records):
-// (the render tree's binary nodes settle ties, see tie_takes)
+// work counts, full hit records) and, of the render tree, for render rays walked by
+// one thread and for ties (tie_takes):
 //   Bvh2Node[]   64 B each, DFS pre-order, both children's boxes stored in
 //                the parent; a child reference >= 0 is an internal node index, < 0
 //                a leaf whose first TriRecord is ~ref.
-//   TriRecord[]  the same records in the reference's leaf order
+//   TriRecord[]  the same records in the binary tree's leaf order
 //                (bvhTriIndices of scene.bvh.cpp:193).
 #pragma once
 #include <stdint.h>

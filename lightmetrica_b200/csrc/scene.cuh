@@ -55,16 +55,15 @@ struct DeviceScene {
     const TriRecord* tris8;       // its leaf order
     const LeafBox* boxes8;        // binary leaf box per tris8 record
     float box_margin;             // renders: hits nearer than this to a triangle's edge (barycentric) are tested against boxes8
-    const Bvh2Node* tie_nodes;    // renders: the binary tree (tie_takes)
-    const int32_t* tie_pos;       // its leaf position of each triangle id
-    int32_t tie_root;
+    const int32_t* tie_pos;       // renders: leaf position of each triangle id in `tris`
     float wide_limit;             // the reference's tree: origins up to this magnitude take the 8-wide walk
-    // The reference's own walk (the reference's tree only).
+    // The binary tree: the reference's own walk; in the render view the render tree, for
+    // the one-thread walk and for ties (tie_takes).
     int32_t root_ref;
     int32_t stack_cap;
     float root_box[6];            // lo.xyz, hi.xyz
     const Bvh2Node* bvh2;
-    const TriRecord* tris;        // the reference's leaf order
+    const TriRecord* tris;        // in the binary tree's leaf order
     const TriRecord* tris_by_id;  // TriAccel order (naive layout)
     int64_t num_tris;
 

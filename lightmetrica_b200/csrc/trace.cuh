@@ -1,6 +1,7 @@
-// Rays, triangle tests and the reference's own binary walk (sm_100a). The
-// batched traversals walk the 8-wide tree (trace8.cuh); this walk answers the
-// rays that walk hands back, the work counts and the full hit records.
+// Rays, triangle tests and one-thread walks of the binary trees (sm_100a). The
+// batched traversals walk the 8-wide tree (trace8.cuh). The reference's own walk
+// (trace_bvh2) answers the rays that one hands back, the work counts and the full hit
+// records; render rays of one thread walk the binary render tree (trace_bvh2_render).
 //
 // Exactness contract: the closest hit (triangle id, t, u, v) is bit-identical
 // to the reference BVHScene::Intersect
@@ -39,14 +40,14 @@ struct TraversalRay {
 
 constexpr uint32_t RAY_FINITE_INV = 8u;
 
-// Rays of the 8-wide walk (WIDE) keep inv_min = 1/d, clamped to +-1e18 so that
+// Render rays and rays of the 8-wide walk (FMA) keep inv_min = 1/d, clamped to +-1e18 so that
 // it stays finite, and inv_max = -o/d: a plane distance is then one
 // multiply-add, (lo - o)/d = fma(lo, 1/d, -o/d). inv_min's sign is `neg`'s: both
 // zeros give +1e18, since the walk picks near and far planes by `neg`.
-template <bool WIDE = false>
+template <bool FMA = false>
 __device__ __forceinline__ void setup_ray(TraversalRay& r, const RayIn& in)
 {
-    if (WIDE) {
+    if (FMA) {
         r.neg = RAY_FINITE_INV;
 #pragma unroll
         for (int c = 0; c < 3; c++) {
@@ -153,6 +154,33 @@ __device__ __forceinline__ bool slab_finite(const TraversalRay& r,
     return tn <= tf && tf > r.tmin;
 }
 
+// x * s + b and y * s + b, each rounded once (packed, sm_100).
+__device__ __forceinline__ void fma_pair(float x, float y, float s, float b, float& a, float& c)
+{
+    asm("{\n\t.reg .b64 p, q, r;\n\t"
+        "mov.b64 p, {%2, %3};\n\t"
+        "mov.b64 q, {%4, %4};\n\t"
+        "mov.b64 r, {%5, %5};\n\t"
+        "fma.rn.f32x2 p, p, q, r;\n\t"
+        "mov.b64 {%0, %1}, p;\n\t}"
+        : "=f"(a), "=f"(c) : "f"(x), "f"(y), "f"(s), "f"(b));
+}
+
+// The slab test of render rays (setup_ray<true>): multiply-adds, near and far planes by
+// min and max. The box is hit iff this holds and t_enter < maxT.
+__device__ __forceinline__ bool slab_render(const TraversalRay& r, float lox, float hix, float loy, float hiy,
+                                            float loz, float hiz, float& t_enter)
+{
+    float x0, x1, y0, y1, z0, z1;
+    fma_pair(lox, hix, r.inv_min[0], r.inv_max[0], x0, x1);
+    fma_pair(loy, hiy, r.inv_min[1], r.inv_max[1], y0, y1);
+    fma_pair(loz, hiz, r.inv_min[2], r.inv_max[2], z0, z1);
+    const float tn = fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fminf(z0, z1));
+    const float tf = fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fmaxf(z0, z1));
+    t_enter = tn;
+    return tn <= tf && tf > r.tmin;
+}
+
 // Both child boxes of a binary node.
 __device__ __forceinline__ void slab_pair(const TraversalRay& r, float4 bx, float4 by, float4 bz,
                                           bool& pl, float& tl, bool& pr, float& tr)
@@ -238,7 +266,8 @@ struct TraceStats {
 
 // Leaf loop: every record of the leaf is tested against the running maxT;
 // a hit sets maxT = t so later records need t <= new maxT (scene.bvh.cpp:416-427).
-template <bool ANY_HIT>
+// RENDER: the triangle test of render rays.
+template <bool ANY_HIT, bool RENDER = false>
 __device__ __forceinline__ bool trace_leaf(const TriRecord* __restrict__ tris, int32_t first,
                                            TraversalRay& r, Hit& h, TraceStats* st)
 {
@@ -247,7 +276,8 @@ __device__ __forceinline__ bool trace_leaf(const TriRecord* __restrict__ tris, i
         const float4 q0 = __ldg(p), q1 = __ldg(p + 1), q2 = __ldg(p + 2);
         if (st) st->tris++;
         float u, v, t;
-        if (triaccel_intersect(q0, q1, q2, r, r.tmax, u, v, t)) {
+        if (RENDER ? triaccel_intersect_fast(q0, q1, q2, r, r.tmax, u, v, t)
+                   : triaccel_intersect(q0, q1, q2, r, r.tmax, u, v, t)) {
             r.tmax = t;
             h.tri = static_cast<int32_t>(__float_as_uint(q2.z));
             h.t = t; h.u = u; h.v = v;
@@ -331,6 +361,50 @@ __device__ __forceinline__ bool trace_bvh2(const Bvh2Node* __restrict__ nodes,
         if (ts.ref == REF_DONE) return true;
         if (trace_leaf<ANY_HIT>(tris, ~ts.ref, r, h, st) && ANY_HIT) return true;
         pop_next(ts, stack, r, st);
+    }
+}
+
+// Closest hit (or any hit) of a render ray (setup_ray<true>) by one thread through a
+// binary tree, the child entered first before the other. A visibility ray's maxT does
+// not change, so that its deferred children (node references alone) need no test when they
+// come up. `stack` holds `stack_cap` entries; returns false if that is exceeded.
+template <bool ANY_HIT>
+__device__ __forceinline__ bool trace_bvh2_render(const Bvh2Node* __restrict__ nodes, const TriRecord* __restrict__ tris,
+                                                  int32_t root_ref, const float* root_box, TraversalRay& r, Hit& h,
+                                                  int2* stack, int stack_cap)
+{
+    int32_t* refs = reinterpret_cast<int32_t*>(stack);
+    h.tri = -1;
+    TravState ts;
+    ts.sp = 0;
+    float te;
+    ts.ref = (slab_render(r, root_box[0], root_box[3], root_box[1], root_box[4], root_box[2], root_box[5], te) && te < r.tmax)
+                 ? root_ref : REF_DONE;
+    auto pop = [&] {
+        if (!ANY_HIT) pop_next(ts, stack, r, nullptr);
+        else ts.ref = ts.sp > 0 ? refs[--ts.sp] : REF_DONE;
+    };
+    for (;;) {
+        while (ts.ref >= 0 && ts.ref != REF_DONE) {
+            const float4* np = reinterpret_cast<const float4*>(nodes + ts.ref);
+            const float4 bx = __ldg(np), by = __ldg(np + 1), bz = __ldg(np + 2);
+            const int4 meta = __ldg(reinterpret_cast<const int4*>(np + 3));
+            float tl, tr;
+            const bool pl = slab_render(r, bx.x, bx.y, by.x, by.y, bz.x, bz.y, tl) && tl < r.tmax;
+            const bool pr = slab_render(r, bx.z, bx.w, by.z, by.w, bz.z, bz.w, tr) && tr < r.tmax;
+            const bool right_first = pr && (!pl || tr < tl);
+            if (pl && pr) {
+                if (ts.sp >= stack_cap) return false;
+                const int32_t far_ref = right_first ? meta.x : meta.y;
+                if (ANY_HIT) refs[ts.sp++] = far_ref;
+                else stack[ts.sp++] = make_int2(far_ref, __float_as_int(right_first ? tl : tr));
+            }
+            if (pl || pr) ts.ref = right_first ? meta.y : meta.x;
+            else pop();
+        }
+        if (ts.ref == REF_DONE) return true;
+        if (trace_leaf<ANY_HIT, true>(tris, ~ts.ref, r, h, nullptr) && ANY_HIT) return true;
+        pop();
     }
 }
 

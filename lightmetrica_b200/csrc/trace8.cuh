@@ -1,5 +1,5 @@
 // Traversal of the 8-wide compressed tree (Bvh8Node): the box test of a
-// node's eight children, the exact walk's certificate, and a one-thread walk.
+// node's eight children, the renders' candidate rule and the exact walk's certificate.
 //
 // A visit is about 250 instructions a warp, half of them on the ALU pipe (48 byte
 // permutes turn plane bytes into floats, 32 three-input min/max): with 22 of 32
@@ -29,18 +29,6 @@ __device__ __forceinline__ Words8 load32(const void* p)
         : "=r"(v.w[0]), "=r"(v.w[1]), "=r"(v.w[2]), "=r"(v.w[3]), "=r"(v.w[4]), "=r"(v.w[5]), "=r"(v.w[6]), "=r"(v.w[7])
         : "l"(p));
     return v;
-}
-
-// x * s + b and y * s + b, each rounded once (packed, sm_100).
-__device__ __forceinline__ void fma_pair(float x, float y, float s, float b, float& a, float& c)
-{
-    asm("{\n\t.reg .b64 p, q, r;\n\t"
-        "mov.b64 p, {%2, %3};\n\t"
-        "mov.b64 q, {%4, %4};\n\t"
-        "mov.b64 r, {%5, %5};\n\t"
-        "fma.rn.f32x2 p, p, q, r;\n\t"
-        "mov.b64 {%0, %1}, p;\n\t}"
-        : "=f"(a), "=f"(c) : "f"(x), "f"(y), "f"(s), "f"(b));
 }
 
 // Byte B of `word` as the float 2^15 + byte: one byte permute puts it into the
@@ -169,13 +157,8 @@ __device__ __forceinline__ bool leaf_box_render(const LeafBox* __restrict__ boxe
 {
     const float4 a = __ldg(reinterpret_cast<const float4*>(boxes + at));
     const float4 b = __ldg(reinterpret_cast<const float4*>(boxes + at) + 1);
-    float x0, x1, y0, y1, z0, z1;
-    fma_pair(a.x, a.w, r.inv_min[0], r.inv_max[0], x0, x1);
-    fma_pair(a.y, b.x, r.inv_min[1], r.inv_max[1], y0, y1);
-    fma_pair(a.z, b.y, r.inv_min[2], r.inv_max[2], z0, z1);
-    const float tn = fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fminf(z0, z1));
-    const float tf = fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fmaxf(z0, z1));
-    return tn <= tf && tf > r.tmin && tn < r.tmax;
+    float te;
+    return slab_render(r, a.x, a.w, a.y, b.x, a.z, b.y, te) && te < r.tmax;
 }
 
 // Whether triangle b, hit at the same t as triangle a, is the binary walk's answer: the one
@@ -213,7 +196,7 @@ __device__ __forceinline__ bool render_candidate(const DeviceScene& s, int64_t a
 {
     if (fminf(fminf(u, v), 1.0f - u - v) < s.box_margin && !leaf_box_render(s.boxes8, at, r)) return false;
     if (ANY || any || t < r.tmax || h.tri < 0) return true;
-    return tie_takes(s.tie_nodes, s.tie_pos, s.tie_root, h.tri, id, t, r);
+    return tie_takes(s.bvh2, s.tie_pos, s.root_ref, h.tri, id, t, r);
 }
 
 // Exact walk. The reference's answer for a ray is a fold over the triangles whose
@@ -278,58 +261,6 @@ __device__ __forceinline__ bool exact_wide_ok(const RayIn& in, float limit)
         longest = fmaxf(longest, a);
     }
     return ok && longest >= 0x1p-30f && longest <= 0x1p30f;
-}
-
-// --------------------------------------------------------- one thread ----
-
-// Closest (or any) render hit by one thread; `stack` holds `cap` groups.
-// Returns false on stack overflow.
-template <bool ANY_HIT>
-__device__ __forceinline__ bool trace8(const DeviceScene& s, TraversalRay& r, Hit& h, uint2* stack, int cap)
-{
-    const Bvh8Node* __restrict__ nodes = s.bvh8;
-    const TriRecord* __restrict__ tris = s.tris8;
-    const uint32_t oct = r.neg & 7u;
-    Walk8 w;
-    walk8_begin(w, oct);
-    h.tri = -1;
-    for (;;) {
-        // Descend to the next leaves: the lanes of a warp meet again before they
-        // test triangles.
-        while (w.leaves == 0) {
-            if ((w.mask & 0xffu) == 0) {
-                if (w.sp == 0) break;
-                const uint2 e = stack[--w.sp];
-                w.base = e.x;
-                w.mask = e.y;
-            }
-            const uint32_t node = walk8_next(w, oct);
-            if (w.mask & 0xffu) {
-                if (w.sp >= cap) return false;
-                stack[w.sp++] = make_uint2(w.base, w.mask);
-            }
-            walk8_visit(w, nodes, node, r, oct);
-        }
-        if (w.leaves == 0) return true;
-        const float4* p = walk8_leaf(nodes, tris, w.leaf_node, w.leaves);
-        for (;;) {
-            const float4 q0 = __ldg(p), q1 = __ldg(p + 1), q2 = __ldg(p + 2);
-            float u, v, t;
-            const int32_t id = static_cast<int32_t>(__float_as_uint(q2.z));
-            if (triaccel_intersect_fast(q0, q1, q2, r, r.tmax, u, v, t) &&
-                render_candidate<ANY_HIT>(s, (p - reinterpret_cast<const float4*>(tris)) / 3, id, t, u, v, r, h, ANY_HIT)) {
-                r.tmax = t;
-                h.tri = id; h.t = t; h.u = u; h.v = v;
-                if (ANY_HIT) return true;
-            }
-            if (__float_as_uint(q0.x) & TRI_LAST_IN_LEAF) {
-                if (w.leaves == 0) break;
-                p = walk8_leaf(nodes, tris, w.leaf_node, w.leaves);
-            } else {
-                p += 3;
-            }
-        }
-    }
 }
 
 }  // namespace lmgpu

@@ -72,3 +72,41 @@ def test_waves_equal_the_sum_of_one_thread_passes(cuda, technique, box, max_pv, 
             assert np.linalg.norm(got - want) <= 4 * np.sqrt(n) * 6e-8 * np.linalg.norm(want) + 1e-12
             assert np.linalg.norm(want) > 0 or max_pv == 2   # (one bounce: light seen directly, no albedo on any prefix)
     scene.close()
+
+
+@pytest.mark.parametrize("technique,max_pv,n", [("pt.mis", 9, 160 * 160 * 41), ("pt", 4, 1 << 21), ("pt.direct", 6, 777)])
+def test_a_captured_pass_equals_the_direct_one(cuda, technique, max_pv, n):
+    """Under capture every budget runs one thread per sample, over the binary render tree."""
+    import torch
+    prims = scenes.cornell_refined(2, 160, 160)
+    scene = create_scene("bvh")
+    scene.load(prims)
+    scene.configure({})
+    scene.build()
+    r = create_renderer(technique)
+    r.configure({"rr_depth": 3, "max_path_vertices": max_pv, "sampler": {"rng_seed": 6}})
+    albedo = torch.from_numpy(triangle_albedo(prims) * np.float32(0.8)).cuda()
+    emission = torch.from_numpy(light_emission(prims)).cuda()
+    dL = 1.0 + 0.5 * torch.rand((160, 160, 3), generator=torch.Generator(device="cuda").manual_seed(2), device="cuda")
+    diff, params = N.DiffParams(albedo.data_ptr(), emission.data_ptr()), r.params(n)
+    direct = _pass(scene, params, diff, torch, albedo, emission, dL, False) + \
+        _pass(scene, params, diff, torch, albedo, emission, dL, True)
+    img, da, de = torch.zeros(dL.numel(), device="cuda"), torch.zeros_like(albedo), torch.zeros_like(emission)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        s = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        N.check(N.lib().lmgpu_adjoint_forward(scene.handle, ctypes.byref(params), ctypes.byref(diff), img.data_ptr(), s, None))
+        N.check(N.lib().lmgpu_adjoint_backward(scene.handle, ctypes.byref(params), ctypes.byref(diff), dL.data_ptr(), da.data_ptr(),
+                                               de.data_ptr(), s, None))
+    graph.replay()
+    torch.cuda.synchronize()
+    scene.status(torch.cuda.current_stream().cuda_stream)
+    for got, want in zip((img, da, de), direct):
+        got = got.double().cpu().numpy()
+        # Sums of up to n single-precision terms in two orders; a ray within rounding of an edge or a tie may take another
+        # path in the other tree: a few of the samples, of the order of 1e-5 of them.
+        assert np.linalg.norm(got - want) <= (4 * np.sqrt(n) * 6e-8 + 1e-4) * np.linalg.norm(want)
+        assert np.linalg.norm(want) > 0
+    del graph
+    scene.close()
