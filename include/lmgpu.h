@@ -305,9 +305,9 @@ typedef struct {
 
 /* Forward pass: renders `params` with `diff` into a DEVICE image (W*H*3,
  * accumulated with atomics, already rescaled by W*H/num_samples; the caller
- * zeroes it). Same estimator as lmgpu_render. Both passes run budgets of 2^16
- * samples or more as waves of up to 2^23 paths over a workspace that is
- * allocated in stream order from a pool of the device (at most
+ * zeroes it). Same estimator as lmgpu_render. Both passes run large budgets (from 2^20
+ * or 2^21 samples on, see waves_pay in adjoint.cu) as waves of up to 2^23 paths over a
+ * workspace that is allocated in stream order from a pool of the device (at most
  * 220 + 16 * (max_path_vertices - 1) bytes per path; kept for the next call until
  * lmgpu_render_release); smaller budgets, and streams being captured, run
  * one thread per sample without it. */

@@ -22,9 +22,8 @@
 // 512 x 512, 32 samples per pixel, up to 8 vertices, forward + backward):
 // one thread per sample over the binary render tree 9.8 + 17.9 ms, over the 8-wide tree
 // (more registers, and one ray's leaves hold up its warp) 18.4 + 36.6 ms, waves 14.2 ms in
-// all. So one thread walks the binary tree. It stays for batches below WAVE_MIN_SAMPLES
-// samples, whose launches would cost more than the walk, and for streams being captured
-// (a wave's workspace is allocated in stream order).
+// all. So one thread walks the binary tree. It stays for the budgets of diff_as_waves, and
+// for streams being captured (a wave's workspace is allocated in stream order).
 //
 // The tail of a path of more vertices than a wave records (RECORDED_VERTS;
 // UNBOUNDED_VERTS where the depth has no bound) is run by one thread from the path's
@@ -201,15 +200,20 @@ __device__ __forceinline__ void contribute(const DiffConsts& c, const DeviceScen
     }
 }
 
-// Adds weight S / R to the albedo gradient of triangle t (diffuse only).
+// The albedo gradient S / R of a vertex of weight S on triangle t (diffuse only, else 0).
+__device__ __forceinline__ V3 albedo_grad(const DiffConsts& c, const DeviceScene& s, int t, V3 S)
+{
+    if (is_zero(S)) return S;
+    const Material m = diff_material(s, c, t);
+    if (m.type != LMGPU_BSDF_DIFFUSE) return v3(0, 0, 0);
+    return v3(m.R.x != 0.0f ? S.x / m.R.x : 0.0f, m.R.y != 0.0f ? S.y / m.R.y : 0.0f, m.R.z != 0.0f ? S.z / m.R.z : 0.0f);
+}
 __device__ __forceinline__ void add_albedo_grad(const DiffConsts& c, const DeviceScene& s, int t, V3 S, float* d_albedo)
 {
-    if (is_zero(S)) return;
-    const Material m = diff_material(s, c, t);
-    if (m.type != LMGPU_BSDF_DIFFUSE) return;
-    if (m.R.x != 0.0f) atomicAdd(d_albedo + 3 * (int64_t)t, S.x / m.R.x);
-    if (m.R.y != 0.0f) atomicAdd(d_albedo + 3 * (int64_t)t + 1, S.y / m.R.y);
-    if (m.R.z != 0.0f) atomicAdd(d_albedo + 3 * (int64_t)t + 2, S.z / m.R.z);
+    const V3 g = albedo_grad(c, s, t, S);
+    if (g.x != 0.0f) atomicAdd(d_albedo + 3 * (int64_t)t, g.x);
+    if (g.y != 0.0f) atomicAdd(d_albedo + 3 * (int64_t)t + 1, g.y);
+    if (g.z != 0.0f) atomicAdd(d_albedo + 3 * (int64_t)t + 2, g.z);
 }
 
 // End of a replayed path: the albedo gradient weight of recorded vertex i is
@@ -449,9 +453,8 @@ __global__ void __launch_bounds__(128, BLOCKS) k_diff(const DeviceScene s, const
 
 // ------------------------------------------------------------- waves ----
 
-// Samples from which a pass runs as waves.
-constexpr int64_t WAVE_MIN_SAMPLES = int64_t(1) << 16;
 constexpr int64_t WAVE_PATHS = int64_t(1) << 23;   // paths in flight (a workspace of 350 bytes a path at 8 vertices)
+constexpr int64_t MIN_WAVE_PATHS = int64_t(1) << 16;   // where device memory is short
 constexpr int UNBOUNDED_VERTS = 20;                // vertices a wave follows a path of unbounded depth
 constexpr int EMISSION_COPIES = 512;
 
@@ -571,18 +574,29 @@ __global__ void __launch_bounds__(128) k_diff_splat(const DiffScene<false> ctx, 
 // Adjoint, end of a wave: the albedo gradient weight of a vertex is the sum of
 // the weights of every contribution whose prefix contains it: the suffix sum of
 // the recorded weights plus the tail's (left in st.L by k_diff_tail, else 0).
-// Bound by its atomics: three per vertex with a non-zero weight.
+// Bound by its atomics, three per vertex with a non-zero weight, and neighbouring paths
+// mostly begin on the same triangle: the first vertices' gradients are summed over the
+// warp's runs of one triangle before they are added. 2^20 paths of a 64 x 64 image of 144
+// triangles: 1559 -> 750 us for the kernel.
 __global__ void __launch_bounds__(128) k_diff_flush(const DiffScene<true> ctx, const DiffConsts c, const PathState st, int64_t n,
                                                     float* d_albedo)
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    V3 S = f3(st.L[i]);
-    for (int v = ctx.vertices[i] - 1; v >= 0; v--) {
+    const int m = i < n ? ctx.vertices[i] : 0;
+    V3 S = i < n ? f3(st.L[i]) : v3(0, 0, 0);
+    for (int v = m - 1; v > 0; v--) {
         const float4 q = ctx.record[v * ctx.stride + i];
         S = S + f3(q);
         add_albedo_grad(c, ctx.s, __float_as_int(q.w), S, d_albedo);
     }
+    int tri = -1;
+    V3 g = v3(0, 0, 0);
+    if (m > 0) {
+        const float4 q = ctx.record[i];
+        tri = __float_as_int(q.w);
+        g = albedo_grad(c, ctx.s, tri, S + f3(q));
+    }
+    film_add_runs(d_albedo, tri, g);
 }
 
 __global__ void k_diff_emission(const double* part, int copies, int n, float* d_emission)
@@ -711,7 +725,7 @@ int run_diff_waves(LmgpuScene* sc, const DiffConsts& c, float* image, const floa
         if (e == cudaSuccess) break;
         cudaGetLastError();
         if (e != cudaErrorMemoryAllocation) return cuda_fail(e, "cudaMallocFromPoolAsync");
-        if (P <= WAVE_MIN_SAMPLES) return fail(LMGPU_ERR_OOM, "differentiable render workspace allocation failed");
+        if (P <= MIN_WAVE_PATHS) return fail(LMGPU_ERR_OOM, "differentiable render workspace allocation failed");
         P = (P + 1) / 2;
     }
     PathState st{};
@@ -802,10 +816,30 @@ int run_diff_waves(LmgpuScene* sc, const DiffConsts& c, float* image, const floa
     return LMGPU_OK;
 }
 
-// Whether a pass runs as waves (see the head of this file).
+// Whether a budget runs as waves. Waves pay for their launches (0.2 ms a pass) and for
+// path state in memory; one thread per sample for divergence, which grows with the
+// tree. Forward + backward of refined Cornell boxes, one thread -> waves, ms on the device
+// (pt: 6 vertices; pt.direct: 6; pt.mis: 9):
+//   samples                              2^18         2^19         2^20         2^21         2^23
+//   pt      576 triangles, 512 x 512     0.37 -> 0.67 0.58 -> 0.84 1.06 -> 1.20 2.05 -> 1.91 8.20 -> 6.10
+//   pt      36,864, 512 x 512            0.53 -> 1.02 0.85 -> 1.24 1.55 -> 1.74 2.94 -> 2.71 11.9 -> 8.38
+//   direct  144, 160 x 160                            1.24 -> 1.33 2.49 -> 2.38 4.86 -> 4.51 20.3 -> 17.4
+//   direct  576, 160 x 160                            1.01 -> 1.25 2.01 -> 2.16 4.23 -> 3.96 19.1 -> 15.1
+//   mis     36,864, 512 x 512            1.11 -> 1.78 1.72 -> 2.20 3.62 -> 3.00 7.06 -> 4.58 29.0 -> 14.0
+//   direct  144, 64 x 64                 0.84 -> 1.09 1.43 -> 1.71 2.70 -> 3.01 5.18 -> 5.77 21.1 -> 23.4
+//   mis     2,304, 64 x 64               0.86 -> 1.34 1.50 -> 1.89 3.06 -> 3.02 6.14 -> 5.35 25.7 -> 20.8
+// Light samples seen from the camera add up in the pixels that see the light, all in one
+// launch: on images of few pixels that holds waves up, unless the tree is large.
+bool waves_pay(const DiffConsts& c, int64_t triangles)
+{
+    const bool nee = c.technique != LMGPU_RENDER_PT;
+    if (nee && c.pixels < (1 << 13) && triangles < 1024) return false;
+    return c.num_samples >= int64_t(1) << (nee && c.pixels >= (1 << 14) ? 20 : 21);
+}
+
 bool diff_as_waves(const LmgpuScene* sc, const DiffConsts& c, cudaStream_t stream)
 {
-    if (sc->dev.layout == LMGPU_LAYOUT_NAIVE || c.num_samples < WAVE_MIN_SAMPLES || sc->rdev.num_tris == 0) return false;
+    if (sc->dev.layout == LMGPU_LAYOUT_NAIVE || sc->rdev.num_tris == 0 || !waves_pay(c, sc->rdev.num_tris)) return false;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess) {
         cudaGetLastError();

@@ -12,17 +12,22 @@ from lightmetrica_b200.diff import light_emission, triangle_albedo
 
 pytestmark = pytest.mark.gpu
 
-WAVE_MIN = 1 << 16      # samples from which a pass runs as waves
-PART = 1 << 15
+SIDE = 160              # an image whose larger budgets run as waves:
+WAVE_MIN = 1 << 20      # from this many samples on (pt: twice as many)
+PART = 1 << 17
 
 
 def _closed_box():
     """Mirrors and diffuse faces all around: no path leaves."""
-    prims = scenes.cornell_box(32, 32, variant="mixed")
+    prims = scenes.cornell_box(SIDE, SIDE, variant="mixed")
     prims.environment_light = None
     prims.add(scenes.Primitive(mesh=scenes._mesh([scenes._quad((0, 0, 1.0), (1, 0, 1.0), (1, 1, 1.0), (0, 1, 1.0), (0, 0, -1))]),
                                bsdf=scenes.PerfectMirrorBSDF((0.9, 0.9, 0.9))))
     prims.camera.eye = (0.5, 0.5, 0.9)
+    # Small triangles: of the 2^20 x 45 vertices each then gets about 10^4 gradient terms. (With 10^6 on each of 50, a
+    # single-precision sum in progress loses the terms below its half ulp, a share of 10^6 x 6e-8 of them.)
+    for p in prims.primitives:
+        p.mesh = scenes.subdivide(p.mesh, 3)
     return prims
 
 
@@ -43,13 +48,13 @@ def _pass(scene, params, diff, torch, albedo, emission, dL, backward):
 
 
 @pytest.mark.parametrize("technique,box,max_pv,rr,n", [
-    ("pt.mis", "mixed", 9, 3, WAVE_MIN), ("pt.direct", "classic", 2, 1, WAVE_MIN + 1), ("pt", "mixed", 9, -1, WAVE_MIN + 77),
+    ("pt.mis", "mixed", 9, 3, WAVE_MIN), ("pt.direct", "classic", 2, 1, WAVE_MIN + 1), ("pt", "mixed", 9, -1, 2 * WAVE_MIN + 77),
     ("pt.mis", "closed", 45, -1, WAVE_MIN),          # beyond the vertices a wave records: tails
-    ("pt", "closed", -1, 8, WAVE_MIN),               # unbounded depth: tails
+    ("pt", "closed", -1, 8, 2 * WAVE_MIN),           # unbounded depth: tails
     ("pt.direct", "closed", 33, -1, WAVE_MIN + 5)])  # exactly the recorded vertices
 def test_waves_equal_the_sum_of_one_thread_passes(cuda, technique, box, max_pv, rr, n):
     import torch
-    prims = _closed_box() if box == "closed" else scenes.cornell_box(32, 32, variant=box)
+    prims = _closed_box() if box == "closed" else scenes.cornell_box(SIDE, SIDE, variant=box)
     scene = create_scene("bvh")
     scene.load(prims)
     scene.configure({})
@@ -58,7 +63,7 @@ def test_waves_equal_the_sum_of_one_thread_passes(cuda, technique, box, max_pv, 
     r.configure({"rr_depth": rr, "max_path_vertices": max_pv, "sampler": {"rng_seed": 5}})
     albedo = torch.from_numpy(triangle_albedo(prims) * np.float32(0.9)).cuda()
     emission = torch.from_numpy(light_emission(prims)).cuda()
-    dL = 1.0 + 0.5 * torch.rand((32, 32, 3), generator=torch.Generator(device="cuda").manual_seed(1), device="cuda")
+    dL = 1.0 + 0.5 * torch.rand((SIDE, SIDE, 3), generator=torch.Generator(device="cuda").manual_seed(1), device="cuda")
     diff = N.DiffParams(albedo.data_ptr(), emission.data_ptr())
     for backward in (False, True):
         whole = _pass(scene, r.params(n), diff, torch, albedo, emission, dL, backward)
