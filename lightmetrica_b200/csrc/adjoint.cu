@@ -848,10 +848,23 @@ bool diff_as_waves(const LmgpuScene* sc, const DiffConsts& c, cudaStream_t strea
     return cap == cudaStreamCaptureStatusNone;
 }
 
+// Whether one thread per sample takes samples in the renders' order (SampleOrder). Its
+// warps then walk alike, and add to the same pixels and triangles one after the other. Index ->
+// renders' order, forward + backward, us:
+//   65 x 49 x 4, pt.direct, 144 triangles                     177 -> 186
+//   2^15 / 2^18 / 2^20, pt, 2,304 triangles, 256 x 128        323 -> 351 / 565 -> 463 / 1608 -> 1144
+//   2^18 / 2^20 / 2^23, pt.mis, 576 triangles, 64 x 64        853 -> 785 / 3125 -> 2756 / 26600 -> 23550
+//   2^18 / 2^20 / 2^23, pt.direct, 36 triangles, 64 x 64      1049 -> 1144 / 3358 -> 3870 / 26360 -> 27900
+bool ordered_pays(const DiffConsts& c, int64_t triangles)
+{
+    return c.num_samples >= (int64_t(1) << 18) && (c.technique == LMGPU_RENDER_PT || triangles >= 512);
+}
+
 template <int TECH, bool NAIVE, int STACK>
-int launch_diff_l(LmgpuScene* sc, const DiffConsts& c, bool backward, float* image, const float* dL, float* da,
+int launch_diff_l(LmgpuScene* sc, DiffConsts c, bool backward, float* image, const float* dL, float* da,
                   float* de, cudaStream_t st)
 {
+    if (!ordered_pays(c, sc->rdev.num_tris)) c.order.ordered = 0;
     const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((c.num_samples + 127) / 128, 148 * 16));
     auto launch = [&](auto kernel) { kernel<<<blocks, 128, 0, st>>>(sc->rdev, c, image, dL, da, de, sc->d_status); };
     if (blocks <= 148 * 4) {
