@@ -308,9 +308,10 @@ typedef struct {
  * zeroes it). Same estimator as lmgpu_render. Both passes run large budgets (from 2^20
  * or 2^21 samples on, see waves_pay in adjoint.cu) as waves of up to 2^23 paths over a
  * workspace that is allocated in stream order from a pool of the device (at most
- * 220 + 16 * (max_path_vertices - 1) bytes per path; kept for the next call until
- * lmgpu_render_release); smaller budgets, and streams being captured, run
- * one thread per sample without it. */
+ * 220 + 16 * (max_path_vertices - 1) bytes per path and 4 GiB in all; the pool keeps
+ * up to 4 GiB for the next call until lmgpu_render_release, or until another allocation
+ * of this library finds the device full). Smaller budgets, streams being captured, and
+ * passes whose workspace cannot be had run one thread per sample without it. */
 int lmgpu_adjoint_forward(LmgpuScene* scene, const LmgpuRenderParams* params,
                           const LmgpuDiffParams* diff, float* image_device,
                           void* stream, LmgpuRenderStats* stats);

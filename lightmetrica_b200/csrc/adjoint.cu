@@ -22,8 +22,9 @@
 // 512 x 512, 32 samples per pixel, up to 8 vertices, forward + backward):
 // one thread per sample over the binary render tree 9.8 + 17.9 ms, over the 8-wide tree
 // (more registers, and one ray's leaves hold up its warp) 18.4 + 36.6 ms, waves 14.2 ms in
-// all. So one thread walks the binary tree. It stays for the budgets of diff_as_waves, and
-// for streams being captured (a wave's workspace is allocated in stream order).
+// all. So one thread walks the binary tree. It stays for the budgets that waves_pay leaves,
+// for streams being captured (a wave's workspace is allocated in stream order), and where
+// that workspace cannot be had.
 //
 // The tail of a path of more vertices than a wave records (RECORDED_VERTS;
 // UNBOUNDED_VERTS where the depth has no bound) is run by one thread from the path's
@@ -454,7 +455,8 @@ __global__ void __launch_bounds__(128, BLOCKS) k_diff(const DeviceScene s, const
 // ------------------------------------------------------------- waves ----
 
 constexpr int64_t WAVE_PATHS = int64_t(1) << 23;   // paths in flight (a workspace of 350 bytes a path at 8 vertices)
-constexpr int64_t MIN_WAVE_PATHS = int64_t(1) << 16;   // where device memory is short
+constexpr int64_t MIN_WAVE_PATHS = int64_t(1) << 20;   // where memory is short; shorter still: one thread per sample
+constexpr uint64_t POOL_KEEP = uint64_t(1) << 32;     // bytes a device's pool keeps; a workspace takes no more
 constexpr int UNBOUNDED_VERTS = 20;                // vertices a wave follows a path of unbounded depth
 constexpr int EMISSION_COPIES = 512;
 // Doubles from one light's partial sum to the next: a 128-byte line each. Packed sums of
@@ -672,7 +674,8 @@ __global__ void __launch_bounds__(128) k_diff_tail(const DiffScene<BACKWARD> ctx
 
 // Stream-ordered memory of the waves' workspaces, one pool per device: calls
 // on several streams or threads each get their own, and what they return stays
-// in the pool for the next call until lmgpu_render_release.
+// in the pool for the next call, up to POOL_KEEP, until lmgpu_render_release or until another
+// allocation of this library finds the device full (device_malloc).
 struct DiffPool {
     std::mutex mu;
     cudaMemPool_t pool = nullptr;
@@ -698,13 +701,16 @@ cudaError_t diff_pool_of(int device, cudaMemPool_t* out)
         props.location.id = device;
         cudaError_t e = cudaMemPoolCreate(&p.pool, &props);
         if (e != cudaSuccess) { p.pool = nullptr; return e; }
-        uint64_t keep = UINT64_MAX;
+        uint64_t keep = POOL_KEEP;
         e = cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &keep);
         if (e != cudaSuccess) { cudaMemPoolDestroy(p.pool); p.pool = nullptr; return e; }
     }
     *out = p.pool;
     return cudaSuccess;
 }
+
+// (not a status of the library) nothing was launched: the workspace could not be had
+constexpr int WAVES_NO_MEMORY = 1 << 30;
 
 template <int TECH, int STACK, bool BACKWARD>
 int run_diff_waves(LmgpuScene* sc, const DiffConsts& c, float* image, const float* dL, float* da, float* de, cudaStream_t stream)
@@ -722,16 +728,17 @@ int run_diff_waves(LmgpuScene* sc, const DiffConsts& c, float* image, const floa
     const size_t emission_bytes = BACKWARD ? (size_t)copies * lights * EMISSION_LINE * sizeof(double) : 0;
     const size_t head = (256 + emission_bytes + 255) / 256 * 256;
     const size_t per_path = 16 * 13 + 8 + (BACKWARD ? 4 + 16 * (size_t)bounces : 0);
+    if (head > POOL_KEEP / 2) return WAVES_NO_MEMORY;
     cudaMemPool_t pool = nullptr;
     LMGPU_CUDA_TRY(diff_pool_of(sc->device, &pool));
-    int64_t P = std::min(c.num_samples, WAVE_PATHS);
+    int64_t P = std::min({ c.num_samples, WAVE_PATHS, (int64_t)((POOL_KEEP - head - 256) / per_path) });
     char* mem = nullptr;
     for (;;) {
         const cudaError_t e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&mem), head + (size_t)P * per_path + 256, pool, stream);
         if (e == cudaSuccess) break;
         cudaGetLastError();
         if (e != cudaErrorMemoryAllocation) return cuda_fail(e, "cudaMallocFromPoolAsync");
-        if (P <= MIN_WAVE_PATHS) return fail(LMGPU_ERR_OOM, "differentiable render workspace allocation failed");
+        if (P <= MIN_WAVE_PATHS) return WAVES_NO_MEMORY;
         P = (P + 1) / 2;
     }
     PathState st{};
@@ -898,11 +905,14 @@ int launch_diff_t(LmgpuScene* sc, const DiffConsts& c, bool backward, float* ima
 {
     const int cap = sc->rdev.stack_cap, cap8 = sc->rdev.stack8_cap;
     if (cap8 <= 256 && cap <= TAIL_STACK && diff_as_waves(sc, c, st)) {
+        int rc;
         if (cap8 <= 32)
-            return backward ? run_diff_waves<TECH, 32, true>(sc, c, image, dL, da, de, st)
-                            : run_diff_waves<TECH, 32, false>(sc, c, image, dL, da, de, st);
-        return backward ? run_diff_waves<TECH, 256, true>(sc, c, image, dL, da, de, st)
-                        : run_diff_waves<TECH, 256, false>(sc, c, image, dL, da, de, st);
+            rc = backward ? run_diff_waves<TECH, 32, true>(sc, c, image, dL, da, de, st)
+                          : run_diff_waves<TECH, 32, false>(sc, c, image, dL, da, de, st);
+        else
+            rc = backward ? run_diff_waves<TECH, 256, true>(sc, c, image, dL, da, de, st)
+                          : run_diff_waves<TECH, 256, false>(sc, c, image, dL, da, de, st);
+        if (rc != WAVES_NO_MEMORY) return rc;
     }
     if (cap <= 32) return launch_diff_s<TECH, 32>(sc, c, backward, image, dL, da, de, st);
     if (cap <= 64) return launch_diff_s<TECH, 64>(sc, c, backward, image, dL, da, de, st);

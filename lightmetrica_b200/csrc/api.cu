@@ -38,6 +38,16 @@ int cuda_fail(cudaError_t e, const char* what)
     return LMGPU_ERR_CUDA;
 }
 
+cudaError_t device_malloc_bytes(void** out, size_t bytes)
+{
+    cudaError_t e = cudaMalloc(out, bytes);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || release_diff_pool(dev) != LMGPU_OK) return e;
+    return cudaMalloc(out, bytes);
+}
+
 int64_t check_limit_from_env(const char* name)
 {
     const char* v = std::getenv(name);
@@ -90,7 +100,7 @@ int upload(LmgpuScene* s, const std::vector<T>& v, const T** out)
     *out = nullptr;
     if (v.empty()) return LMGPU_OK;
     void* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, v.size() * sizeof(T));
+    cudaError_t e = device_malloc(&p, v.size() * sizeof(T));
     if (e != cudaSuccess) return e == cudaErrorMemoryAllocation ? fail(LMGPU_ERR_OOM, "device allocation failed") : cuda_fail(e, "cudaMalloc");
     s->allocations.push_back(p);
     LMGPU_CUDA_TRY(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
@@ -488,7 +498,7 @@ int create_impl(const LmgpuSceneDesc* desc, LmgpuScene** out)
     // Scratch: status word and the persistent kernels' work counter.
     void* st = nullptr;
     const size_t scratch = 256 + LmgpuScene::WORK_SLOTS * sizeof(unsigned long long);
-    cudaError_t e = cudaMalloc(&st, scratch);
+    cudaError_t e = device_malloc(&st, scratch);
     if (e != cudaSuccess) { lmgpu_scene_destroy(s); return cuda_fail(e, "cudaMalloc(status)"); }
     s->allocations.push_back(st);
     s->d_status = static_cast<int32_t*>(st);
@@ -741,7 +751,7 @@ int ensure_host_pipeline(LmgpuScene* sc)
     for (int k = 0; k < HostPipeline::SLOTS; k++) {
         LMGPU_CUDA_TRY(cudaStreamCreateWithFlags(&hp.stream[k], cudaStreamNonBlocking));
         void* p = nullptr;
-        LMGPU_CUDA_TRY(cudaMalloc(&p, (size_t)hp.chunk * 12 * sizeof(float)));
+        LMGPU_CUDA_TRY(device_malloc(&p, (size_t)hp.chunk * 12 * sizeof(float)));
         sc->allocations.push_back(p);
         hp.rays[k] = static_cast<float*>(p);
         hp.hits[k] = hp.rays[k] + 8 * hp.chunk;

@@ -388,7 +388,7 @@ int ensure_batch_workspace(LmgpuBatch* b, int64_t paths, int pools)
     if (b->ws_mem) { cudaFree(b->ws_mem); b->ws_mem = nullptr; b->ws_capacity = 0; b->ws_pools = 0; }
     const size_t P = (size_t)paths;
     const size_t pool_bytes = (256 + P * BYTES_PER_PATH + 255) / 256 * 256;
-    cudaError_t e = cudaMalloc(&b->ws_mem, pool_bytes * pools);
+    cudaError_t e = device_malloc(&b->ws_mem, pool_bytes * pools);
     if (e != cudaSuccess) {
         b->ws_mem = nullptr;
         return e == cudaErrorMemoryAllocation ? fail(LMGPU_ERR_OOM, "batch workspace allocation failed")
@@ -835,7 +835,7 @@ int lmgpu_batch_create(LmgpuScene* const* scenes, int32_t num_scenes, LmgpuBatch
     cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, dev);
     const size_t n = (size_t)num_scenes;
     cudaError_t e = cudaSuccess;
-    auto dm = [&](void** p, size_t bytes) { if (e == cudaSuccess) e = cudaMalloc(p, bytes); };
+    auto dm = [&](void** p, size_t bytes) { if (e == cudaSuccess) e = device_malloc(p, bytes); };
     auto hm = [&](void** p, size_t bytes) { if (e == cudaSuccess) e = cudaMallocHost(p, bytes); };
     dm(reinterpret_cast<void**>(&b->d_table), n * sizeof(BatchEntry));
     dm(reinterpret_cast<void**>(&b->d_begins), (n + 1) * sizeof(int64_t));
@@ -939,7 +939,7 @@ int lmgpu_batch_render(LmgpuBatch* b, const LmgpuRenderParams* params, float* co
         cudaFree(b->hf_film);
         b->hf_film = nullptr;
         b->hf_film_bytes = 0;
-        LMGPU_CUDA_TRY(cudaMalloc(&b->hf_film, film_bytes));
+        LMGPU_CUDA_TRY(device_malloc(&b->hf_film, film_bytes));
         b->hf_film_bytes = film_bytes;
     }
     if (b->hf_out_bytes < out_bytes) {
@@ -948,7 +948,7 @@ int lmgpu_batch_render(LmgpuBatch* b, const LmgpuRenderParams* params, float* co
         b->hf_out = nullptr;
         b->hf_pinned = nullptr;
         b->hf_out_bytes = 0;
-        cudaError_t e = cudaMalloc(&b->hf_out, out_bytes);
+        cudaError_t e = device_malloc(&b->hf_out, out_bytes);
         if (e == cudaSuccess) e = cudaMallocHost(&b->hf_pinned, out_bytes);
         if (e != cudaSuccess) {
             cudaFree(b->hf_out);
@@ -991,7 +991,7 @@ int lmgpu_batch_profile(LmgpuBatch* b, const LmgpuRenderParams* params, void* co
     TraceProfileRun run;
     run.count = count_tests != 0;
     if (run.count) {
-        LMGPU_CUDA_TRY(cudaMalloc(&run.d_counts, 4 * sizeof(unsigned long long)));
+        LMGPU_CUDA_TRY(device_malloc(&run.d_counts, 4 * sizeof(unsigned long long)));
         cudaError_t e = cudaMemsetAsync(run.d_counts, 0, 4 * sizeof(unsigned long long), s);
         if (e != cudaSuccess) { cudaFree(run.d_counts); return cuda_fail(e, "profile counters"); }
     }
@@ -1058,7 +1058,7 @@ int lmgpu_batch_autotune(LmgpuBatch* b, const LmgpuRenderParams* params, double 
     if (rc != LMGPU_OK) return rc;
     void* film = nullptr;
     const size_t esize = pl.fp64 ? sizeof(double) : sizeof(float);
-    LMGPU_CUDA_TRY(cudaMalloc(&film, std::max<int64_t>(px, 1) * 3 * esize));
+    LMGPU_CUDA_TRY(device_malloc(&film, std::max<int64_t>(px, 1) * 3 * esize));
     std::vector<void*> films(n, film);
 
     const LmgpuBatchConfig start = b->cfg;

@@ -140,7 +140,7 @@ struct Scratch {
     ~Scratch() { cudaFree(mem); }
     int reserve(size_t bytes)
     {
-        cudaError_t e = cudaMalloc(&mem, bytes);
+        cudaError_t e = device_malloc(&mem, bytes);
         if (e != cudaSuccess) {
             mem = nullptr;
             return e == cudaErrorMemoryAllocation ? fail(LMGPU_ERR_OOM, "device allocation failed") : cuda_fail(e, "cudaMalloc");

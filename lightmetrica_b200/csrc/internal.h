@@ -72,6 +72,14 @@ int render_device_preallocated(LmgpuScene* sc, const LmgpuRenderParams& p, void*
 // Gives the differentiable passes' pooled workspace memory back (adjoint.cu).
 int release_diff_pool(int device);
 
+// cudaMalloc that asks again, once, after the idle memory of that pool has been given back.
+cudaError_t device_malloc_bytes(void** out, size_t bytes);
+template <class T>
+cudaError_t device_malloc(T** out, size_t bytes)
+{
+    return device_malloc_bytes(reinterpret_cast<void**>(out), bytes);
+}
+
 // Reads and clears the device status word; maps it to an LMGPU status.
 int consume_status(LmgpuScene* s, cudaStream_t stream);
 // The LMGPU status (and message) of a non-zero device status word.

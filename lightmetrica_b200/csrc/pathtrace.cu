@@ -141,7 +141,7 @@ int ensure_workspace(Workspace& ws, int64_t paths)
     if (ws.capacity >= paths && ws.mem) return LMGPU_OK;
     if (ws.mem) { cudaFree(ws.mem); ws.mem = nullptr; ws.capacity = 0; }
     const size_t P = (size_t)paths;
-    cudaError_t e = cudaMalloc(&ws.mem, WS_HEADER_BYTES + P * WS_BYTES_PER_PATH);
+    cudaError_t e = device_malloc(&ws.mem, WS_HEADER_BYTES + P * WS_BYTES_PER_PATH);
     if (e != cudaSuccess) return e == cudaErrorMemoryAllocation ? fail(LMGPU_ERR_OOM, "render workspace allocation failed")
                                                                  : cuda_fail(e, "cudaMalloc(workspace)");
     carve_state(ws.st, static_cast<char*>(ws.mem), P);
@@ -361,7 +361,7 @@ int ensure_host_film(HostFilmBuffers& hb, size_t film_bytes, size_t out_bytes)
         cudaFree(hb.film);
         hb.film = nullptr;
         hb.film_bytes = 0;
-        cudaError_t e = cudaMalloc(&hb.film, film_bytes);
+        cudaError_t e = device_malloc(&hb.film, film_bytes);
         if (e != cudaSuccess) { hb.film = nullptr; return cuda_fail(e, "cudaMalloc(film)"); }
         hb.film_bytes = film_bytes;
     }
@@ -371,7 +371,7 @@ int ensure_host_film(HostFilmBuffers& hb, size_t film_bytes, size_t out_bytes)
         hb.out = nullptr;
         hb.pinned = nullptr;
         hb.out_bytes = 0;
-        cudaError_t e = cudaMalloc(&hb.out, out_bytes);
+        cudaError_t e = device_malloc(&hb.out, out_bytes);
         if (e == cudaSuccess) e = cudaMallocHost(&hb.pinned, out_bytes);
         if (e != cudaSuccess) {
             cudaFree(hb.out);
@@ -452,7 +452,7 @@ int lmgpu_intersect_full_host(LmgpuScene* scene, const float* rays_aos, int64_t 
     const size_t N = static_cast<size_t>(n);
     char* buf = nullptr;
     const size_t bytes = N * (8 + 1 + 1 + 17 + 1) * sizeof(float);
-    LMGPU_CUDA_TRY(cudaMalloc(&buf, bytes));
+    LMGPU_CUDA_TRY(device_malloc(&buf, bytes));
     float* dr = reinterpret_cast<float*>(buf);
     int32_t* did = reinterpret_cast<int32_t*>(dr + 8 * N);
     float* dt = dr + 9 * N;

@@ -115,3 +115,64 @@ def test_a_captured_pass_equals_the_direct_one(cuda, technique, max_pv, n):
         assert np.linalg.norm(want) > 0
     del graph
     scene.close()
+
+
+def _idle(torch):
+    """Gives back what this library and torch keep idle; the device's free bytes."""
+    torch.cuda.synchronize()
+    N.check(N.lib().lmgpu_render_release())
+    torch.cuda.empty_cache()
+    return torch.cuda.mem_get_info()[0]
+
+
+def test_the_waves_workspace_is_bounded_and_gives_way(cuda):
+    """What idle passes keep stays below 4 GiB; on a nearly full device a pass runs without it, and a render gets it."""
+    import torch
+    prims = scenes.cornell_refined(2, SIDE, SIDE)
+    scene = create_scene("bvh")
+    scene.load(prims)
+    scene.configure({})
+    scene.build()
+    albedo, emission = torch.from_numpy(triangle_albedo(prims)).cuda(), torch.from_numpy(light_emission(prims)).cuda()
+    dL = torch.ones((SIDE, SIDE, 3), device="cuda")
+    diff = N.DiffParams(albedo.data_ptr(), emission.data_ptr())
+    r = create_renderer("pt.mis")
+
+    def gradients(n, max_pv):
+        r.configure({"rr_depth": 3, "max_path_vertices": max_pv, "sampler": {"rng_seed": 7}})
+        return _pass(scene, r.params(n), diff, torch, albedo, emission, dL, True)
+
+    def render(n):
+        r.configure({"rr_depth": 3, "max_path_vertices": 9, "sampler": {"rng_seed": 7}})
+        film, st = torch.zeros(SIDE * SIDE * 3, device="cuda"), N.RenderStats()
+        rc = N.lib().lmgpu_render_device(scene.handle, ctypes.byref(r.params(n, wave_paths=n)), ctypes.c_void_p(film.data_ptr()),
+                                         ctypes.c_void_p(torch.cuda.current_stream().cuda_stream), ctypes.byref(st))
+        torch.cuda.synchronize()
+        return rc
+
+    gradients(1 << 18, 9)                            # (kernels loaded, their local memory reserved)
+    render(1 << 18)
+    free = _idle(torch)
+    gradients(1 << 23, 33)                           # 732 bytes a path
+    torch.cuda.synchronize()
+    kept = free - torch.cuda.mem_get_info()[0]
+    assert (1 << 30) < kept <= (1 << 32) + (1 << 28)
+
+    n = 1 << 21                                      # waves of 2^20 paths would take 365 MB
+    want = gradients(n, 9)
+    free = _idle(torch)
+    room = 300 << 20
+    full = torch.empty(free - room, dtype=torch.uint8, device="cuda")
+    got = gradients(n, 9)
+    for a, b in zip(got, want):                      # (bounds as in the captured passes above)
+        assert np.linalg.norm(a - b) <= (4 * np.sqrt(n) * 6e-8 + 1e-4) * np.linalg.norm(b)
+    del full
+    _idle(torch)
+
+    gradients(n, 9)                                  # its workspace (730 MB) is idle now
+    torch.cuda.empty_cache()
+    full = torch.empty(torch.cuda.mem_get_info()[0] - room, dtype=torch.uint8, device="cuda")
+    assert render(n) == N.OK                         # 453 MB
+    del full
+    _idle(torch)
+    scene.close()
