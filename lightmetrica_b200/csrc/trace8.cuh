@@ -132,10 +132,15 @@ __device__ __forceinline__ const float4* walk8_leaf(const Bvh8Node* __restrict__
 // ------------------------------------------------------- candidate hits ----
 
 // A render ray's hit is the one that a near-first walk of the binary tree through its
-// float boxes finds: the least t among the triangles whose leaf box the ray enters
-// before t (leaf_box_render), and among equal t the one visited last (tie_takes).
-// So the answer depends on neither the width of the nodes nor their rounding. Without
-// the box test, the triangle test's rounding reports hits just outside a triangle that
+// float boxes finds, within rounding: triangles are tested in the order in which the ray's
+// walk finds their leaves; a hit near an edge counts if the ray enters the leaf's box before
+// the closest hit so far (leaf_box_render), and of equal t the one that the binary walk
+// visits last (tie_takes).
+// The order is the ray's own: nodes are visited depth first, and a postponed leaf is tested
+// before those found after it. The warp's other rays change when a leaf is tested, and so
+// which nodes are visited although a hit not yet known lies before them; the triangles in
+// those are entered after that hit and do not count, so the answer stays the same.
+// Without the box test, the triangle test's rounding reports hits just outside a triangle that
 // 8-bit boxes let through and float boxes do not (far from the origin, many). A hit well
 // inside its triangle is well inside the box, so that only hits near an edge are tested
 // (DeviceScene::box_margin). On every

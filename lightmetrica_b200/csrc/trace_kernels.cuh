@@ -101,10 +101,9 @@ __device__ __forceinline__ void reference_walk(const DeviceScene& s, int32_t* st
 // leaves of one visited node". A lane that finds leaves while it holds none
 // postpones them and goes on descending with the rest of the warp; the
 // descent ends when every lane still in it holds leaves, and pauses once fewer
-// than LMGPU_TRACE_EXIT_BELOW lanes are in it. The order in which a ray's
-// triangles are tested thus depends on the warp's other rays, its result does
-// not: render rays break exact ties by the binary tree's order, exact rays hand
-// theirs to the reference's walk. (Without postponing: 1.97 against 1.66 ms on the soup,
+// than LMGPU_TRACE_EXIT_BELOW lanes are in it. When a ray's triangles are
+// tested thus depends on the warp's other rays; in which order does not, nor does its
+// result (see the candidate rules in trace8.cuh). (Without postponing: 1.97 against 1.66 ms on the soup,
 // 2.00 / 1.59 and 1.87 / 1.59 ms on the bounce and shadow rays.)
 // For a multi-scene I/O policy each lane switches to its new ray's scene at
 // refill; an empty scene is a miss. The COUNT instantiation (measurement

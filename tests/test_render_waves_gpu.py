@@ -107,3 +107,38 @@ def test_few_rays_answer_as_among_many(cuda, n):
     for few, many in zip(ask(n), ask(400009)):
         assert torch.equal(few, many[:n])
     s.close()
+
+
+def _layered_grids(width, height):
+    """Four emitting grids some units of rounding apart, far from the origin: a leaf box may be entered after its own
+    triangle's t, and before or after the t of a triangle of another layer."""
+    prims = scenes.Primitives()
+    at, ulp = np.float32(300.0), np.float32(2.0 ** -15)
+    for layer, (n, radiance) in enumerate([(20, 1.0), (24, 2.0), (31, 4.0), (37, 8.0)]):
+        lin = np.linspace(-1, 1, n + 1).astype(np.float32)
+        x, y = np.meshgrid(lin, lin, indexing="ij")
+        pos = np.stack([x, y, np.zeros_like(x)], -1).reshape(-1, 3).astype(np.float32) + at
+        pos[:, 2] += np.float32(layer) * ulp
+        i, j = np.meshgrid(np.arange(n), np.arange(n), indexing="ij")
+        a = (i * (n + 1) + j).reshape(-1)
+        faces = np.concatenate([np.stack([a, a + n + 1, a + n + 2], 1), np.stack([a, a + n + 2, a + 1], 1)]).astype(np.uint32)
+        normals = np.tile(np.array([0, 0, 1], np.float32), (pos.shape[0], 1))
+        prims.add(scenes.Primitive(mesh=scenes.TriangleMesh(pos, faces, normals), bsdf=scenes.DiffuseBSDF((0, 0, 0)),
+                                   light=scenes.AreaLight((radiance,) * 3)))
+    film = scenes.HDRBitmapFilm(width, height)
+    prims.camera = scenes.PerspectiveCamera(film=film, eye=(340.3, 280.8, 1100.0), center=(300, 300, 300), up=(0, 1, 0), fovy=0.14)
+    return prims
+
+
+def test_a_rays_hit_does_not_depend_on_the_rays_beside_it(cuda):
+    """Waves of one size against another: other rays share a ray's warp, so its triangles are tested in another order.
+    Radiances are powers of two, whose sums are exact."""
+    import torch
+    s = _built(_layered_grids(96, 64))
+    r = _renderer("pt", 2, -1)
+    n = 96 * 64 * 8
+    film, _ = _render(s, r, n, torch)
+    assert len(np.unique(film)) > 4
+    for wave in (61, 997, 4736, 20000):
+        np.testing.assert_array_equal(_render(s, r, n, torch, wave_paths=wave)[0], film)
+    s.close()
