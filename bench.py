@@ -26,10 +26,9 @@ on the same scene and configuration, a bounded sample of the frame per step,
 counting the rays its scene traces.
 
 At N=1 the same line carries `sections`: the ray-intersection kernel (2^24
-rays x 1,048,576-triangle soup, scene types bvh and qbvh, bit-exact against
-the reference), the plain one-scene renderer on the headline frame, the
-adjoint path replay's backward/forward time, and the 64-scene batch against
-the plain renderers.
+rays x 1,048,576-triangle soup, bit-exact against the reference), the plain
+one-scene renderer on the headline frame, the adjoint pair's
+backward/forward time, and the 64-scene batch against the plain renderers.
 """
 from __future__ import annotations
 
@@ -50,7 +49,6 @@ sys.path.insert(0, ROOT)
 
 NUM_TRIS = 1 << 20
 NUM_RAYS = 1 << 24
-NODE_BYTES = 32      # compact binary node (6 f32 + 2 u32), per slab test
 WIDE_BOX_BYTES = 12  # an eighth of what a visit of an 8-wide node reads (96 B), per box test
 TRI_BYTES = 48       # TriAccel record, per triangle test
 RAY_IO_BYTES = 32 + 16
@@ -162,25 +160,23 @@ class ClockSampler:
                 "reasons": sorted(reasons), "samples": len(sm)}
 
 
-def profile_value(name, key):
-    """A `key: value` line of a committed ncu summary (profiles/<name>.md),
-    or None."""
-    p = os.path.join(ROOT, "profiles", name + ".md")
-    if os.path.exists(p):
-        with open(p) as f:
+# The committed ncu summary of the traversal kernels, and the node they walk: a
+# summary of another walk has no say in the figures below.
+TRACE_PROFILE, TRACE_NODE = "trace_wide", "Bvh8Node"
+
+
+def profile_value(key):
+    """A `key: value` line of the traversal's ncu summary (DRAM bytes per ray on a
+    smaller capture), or None where it is missing or names another walk's node."""
+    path = os.path.join(ROOT, "profiles", TRACE_PROFILE + ".md")
+    values = {}
+    if os.path.exists(path):
+        with open(path) as f:
             for line in f:
-                if line.startswith(key + ":"):
-                    return float(line.split(":", 1)[1])
-    return None
-
-
-def load_traffic(num_rays):
-    """DRAM bytes (read + write) of one full-size traversal launch of the
-    intersection API, from the committed ncu summary of the kernel: its line
-    `dram_bytes_per_ray: X` (measured on a smaller capture, scaled by the
-    rays of this launch), or None."""
-    v = profile_value("trace_closest_bvh2_intersect", "dram_bytes_per_ray")
-    return None if v is None else int(v * num_rays)
+                k, sep, v = line.partition(":")
+                if sep and k.strip() == k:
+                    values[k] = v.strip()
+    return float(values[key]) if values.get("node") == TRACE_NODE and key in values else None
 
 
 def frame_config(world, triangles):
@@ -323,9 +319,10 @@ def _batch_launches(cfg, stats, bounces):
 def frame_roofline(prof_count, prof_time):
     """Roofline of the dominant kernel of the frame, the closest-hit
     traversal of the path queues (and, beside it, the shadow traversal):
-    algorithmic bytes per ray (32 B ray + 16 B hit + 96 B per 8-wide node
-    visit, 12 B per box test, + 48 B per TriAccel test, the tests counted on the same samples by the counting kernel) over the
-    launches' summed device time."""
+    bytes the walk reads per ray from whatever level of memory (32 B ray + 16 B hit + 96 B
+    per 8-wide node visit, 12 B per box test, + 48 B per TriAccel test, the tests counted on
+    the same samples by the counting kernel) over the launches' summed device time.
+    `dram`: what the device memory moved of that (ncu, bytes per ray)."""
     peak, peak_kind = measured_peaks()
     out = {}
     for kind in ("closest", "shadow"):
@@ -342,15 +339,20 @@ def frame_roofline(prof_count, prof_time):
                      "tri_tests_per_ray": round(tb, 4), "rays": rays, "launches": t["launches"],
                      "avg_launch_ms": round(t["trace_ms"] / max(1, t["launches"]), 4),
                      "share_of_frame": round(t["trace_ms"] / prof_time["render_ms"], 4)}
+        dram = profile_value(f"frame_{kind}_dram_bytes_per_ray")
+        if dram is not None:
+            gbs = dram * rays / (t["trace_ms"] / 1e3) / 1e9
+            out[kind]["dram"] = {"bytes_per_ray": dram, "achieved": round(gbs, 1), "frac": round(gbs / peak, 4)}
     main = out["closest"]
-    traffic_per_ray = profile_value("pathtrace_terrain_1080p_batched", "closest_dram_bytes_per_ray")
+    traffic_per_ray = profile_value("frame_closest_dram_bytes_per_ray")
     return {"bound": "latency", "denominator": "hbm", "kernel": "k_trace_persistent (closest hit, path queues)",
             "achieved": main["achieved"], "peak": peak, "unit": "GB/s", "frac": main["frac"],
             "traffic": None if traffic_per_ray is None else int(traffic_per_ray * main["rays"] / main["launches"]),
             "peak_source": peak_kind,
-            "why_not_hbm": "the tree and triangles (~220 MB) mostly hit in L2; each ray's walk is a chain of "
-                           "dependent node visits of ~250 instructions, so the kernel is bound by the ALU pipe, "
-                           "divergence and fetch latency, not DRAM bandwidth",
+            "why_not_hbm": "achieved counts bytes read from any level of memory: the tree and triangles (~220 MB) "
+                           "mostly hit in L1 and L2 (DRAM's share is under kernels.*.dram). Each ray's walk is a chain "
+                           "of dependent node visits of ~250 instructions, so the kernel is bound by issue, the ALU "
+                           "pipe and L1, not by DRAM bandwidth",
             "kernels": out}
 
 
@@ -538,13 +540,14 @@ def _terrain_parity(r, layout="bvh"):
 
 # ------------------------------------------------------------- sections ----
 
-def intersect_section(args, dev, layout, cpu_baseline, want_ref_hits):
+def intersect_section(args, dev, cpu_baseline):
     """The ray-intersection kernel alone: 2^24 rays (origins U[-2,2]^3,
     directions uniform on the sphere) against 1,048,576 random triangles
-    (centres U[-1,1]^3, edges N(0, 0.01^2)), closest hit, scene type "bvh" or
-    "qbvh" (the same walk and hits). Bytes per ray: the reference walk's slab and
-    TriAccel tests. One launch per step over the batch (512 MB of rays, larger
-    than L2)."""
+    (centres U[-1,1]^3, edges N(0, 0.01^2)), closest hit. One launch per step over
+    the batch (512 MB of rays, larger than L2). The roofline's bytes are those that
+    the device memory moves per ray (ncu; without a summary, the ray and the hit);
+    `reference_work` is what the reference's own walk would do for these rays. The scene
+    type "qbvh" has the same walk: its hits are compared, untimed."""
     import torch
     from lightmetrica_b200 import native
     from lightmetrica_b200.scene import Scene, soup_primitives
@@ -553,10 +556,14 @@ def intersect_section(args, dev, layout, cpu_baseline, want_ref_hits):
     pos, faces = random_soup(NUM_TRIS, seed=1)
     num_rays = 1 << args.rays_log2
     rays = random_rays(num_rays, seed=2)
-    scene = Scene(layout)
-    scene.load(soup_primitives(pos, faces))
-    scene.configure({})
-    scene.build()
+    def built(layout):
+        s = Scene(layout)
+        s.load(soup_primitives(pos, faces))
+        s.configure({})
+        s.build()
+        return s
+
+    scene = built("bvh")
     info = scene.info()
     n = num_rays
     soa = {k: torch.from_numpy(v).to(dev) for k, v in rays_soa(rays).items()}
@@ -575,7 +582,8 @@ def intersect_section(args, dev, layout, cpu_baseline, want_ref_hits):
                                            ctypes.c_void_p(counters.data_ptr()), sptr))
     scene.status(stream.cuda_stream)
     node_tests, tri_tests = int(counters[0]), int(counters[1])
-    bytes_per_ray = RAY_IO_BYTES + NODE_BYTES * node_tests / n + TRI_BYTES * tri_tests / n
+    dram = profile_value("soup_dram_bytes_per_ray")
+    bytes_per_ray = RAY_IO_BYTES if dram is None else dram
     hit_frac = float((hits["tri_id"] >= 0).float().mean())
 
     steps, warm = max(3, args.steps), max(3, args.warmup)
@@ -594,23 +602,31 @@ def intersect_section(args, dev, layout, cpu_baseline, want_ref_hits):
     peak, peak_kind = measured_peaks()
     achieved = bytes_per_ray * n / (avg_ms / 1e3) / 1e9
     out = {"workload": f"ray-intersection: 2^{n.bit_length() - 1} rays x 1,048,576-triangle soup, closest hit",
-           "layout": f"{layout}: 8-wide compressed collapse of the reference tree, 128 B nodes (bit-exact)",
+           "layout": "8-wide compressed collapse of the reference tree, 128 B nodes (bit-exact)",
            "Mrays_per_s": round(n / (avg_ms / 1e3) / 1e6, 1),
            "kernel_ms": {"avg": round(avg_ms, 4), "min": round(min(launch_ms), 4), "max": round(max(launch_ms), 4)},
            "steps": steps, "hit_fraction": round(hit_frac, 4),
            "roofline": {"bound": "latency", "denominator": "hbm", "achieved": round(achieved, 1), "peak": peak,
-                        "unit": "GB/s", "frac": round(achieved / peak, 4), "traffic": load_traffic(n),
-                        "peak_source": peak_kind, "bytes_per_ray": round(bytes_per_ray, 2),
-                        "node_tests_per_ray": round(node_tests / n, 3), "tri_tests_per_ray": round(tri_tests / n, 4)},
+                        "unit": "GB/s", "frac": round(achieved / peak, 4),
+                        "traffic": None if dram is None else int(dram * n),
+                        "peak_source": peak_kind, "bytes_per_ray": round(bytes_per_ray, 2)},
+           "reference_work": {"node_tests_per_ray": round(node_tests / n, 3), "tri_tests_per_ray": round(tri_tests / n, 4)},
            "bvh_nodes": info["num_nodes"], "bvh_depth": info["max_depth"],
            "build_seconds": round(info["build_seconds"], 3)}
-    if not args.no_e2e and layout == "bvh":
+    if not args.no_e2e:
         out["e2e"] = run_e2e(args, scene, rays, hits, dev)
     ids = hits["tri_id"].cpu().numpy()
     tv = hits["t"].cpu().numpy()
     scene.close()
+    other = built("qbvh")
+    native.check(L.lmgpu_intersect(other.handle, ctypes.byref(R), n, ctypes.byref(Hh), sptr))
+    other.status(stream.cuda_stream)
+    hit = ids >= 0
+    out["qbvh_bit_exact"] = bool(np.array_equal(hits["tri_id"].cpu().numpy(), ids) and
+                                 np.array_equal(hits["t"].cpu().numpy()[hit], tv[hit]))
+    other.close()
     if cpu_baseline:
-        rate, kind, cores, done, secs, rh = cpu_reference_rate(pos, faces, rays, want_hits=want_ref_hits)
+        rate, kind, cores, done, secs, rh = cpu_reference_rate(pos, faces, rays, want_hits=True)
         out["cpu_baseline"] = {"value": round(rate, 4), "unit": "Mrays/s", "cores": cores, "kind": kind,
                                "sample": f"first {done} rays of the batch ({secs:.1f} s), reference BVHScene built once"}
         if rh is not None:
@@ -618,7 +634,7 @@ def intersect_section(args, dev, layout, cpu_baseline, want_ref_hits):
             out["vs_reference"] = {"rays_compared": int(done),
                                    "ids_bit_exact": bool(np.array_equal(ids[:done], rh[0])),
                                    "t_bit_equal": bool(np.array_equal(tv[:done][hit], rh[1][hit]))}
-    return out, ids, tv
+    return out
 
 
 def run_e2e(args, scene, rays, hits, dev):
@@ -763,14 +779,15 @@ def batch_section(args, dev):
     mirror), pt.mis with Russian roulette after depth 4. Three ways to render
     the same samples: the batch (one stream of waves over all scenes, each
     wave a replayed CUDA graph, configuration from the autotuner), the plain
-    one-scene-at-a-time wavefront renderer, and the plain one-scene megakernel
-    (one thread per path, one launch per scene). The batch and the plain
+    one-scene-at-a-time wavefront renderer, and the plain one-scene megakernel (one
+    thread per path, one launch per scene: the differentiable forward pass, which
+    runs so under stream capture; the graph of all scenes is replayed). The batch and the plain
     renderers trace the same paths, so their relMSE against any reference is
     equal; the films are compared to show it."""
     import torch
     from lightmetrica_b200 import create_renderer, create_scene, native, scenes
     from lightmetrica_b200.batch import SceneBatch
-    from lightmetrica_b200.diff import DifferentiableRender, light_emission, triangle_albedo
+    from lightmetrica_b200.diff import light_emission, triangle_albedo
     L = native.lib()
     t0 = time.perf_counter()
     items = [scenes.batch_scene(i) for i in range(64)]
@@ -841,12 +858,18 @@ def batch_section(args, dev):
     batched = [f.clone() for f in films]
 
     # Plain megakernel, one launch per scene (scene's own albedo and emission).
-    drs = [DifferentiableRender(sc, r, n) for sc, r, n in zip(built, rs, ns)]
     params = [(torch.from_numpy(triangle_albedo(d["prims"])).to(dev), torch.from_numpy(light_emission(d["prims"])).to(dev))
               for d in items]
+    mega = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(mega):
+        for sc, r, n, f, (a, e) in zip(built, rs, ns, films, params):
+            native.check(L.lmgpu_adjoint_forward(
+                sc.handle, ctypes.byref(r.params(n)), ctypes.byref(native.DiffParams(a.data_ptr(), e.data_ptr())),
+                f.data_ptr(), ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream), None))
 
     def mega_pass():
-        return [dr.forward(a, e) for dr, (a, e) in zip(drs, params)]
+        mega.replay()
     mega_pass()
 
     # Timed: the three renderers in turn, `rounds` times, best time of each
@@ -862,6 +885,7 @@ def batch_section(args, dev):
         mega_ms = min(mega_ms, ms)
         ms, _ = timed(lambda: batch.render_device(rs, ns, films, stats=False))
         batch_ms = min(batch_ms, ms)
+    del mega
     rel = []
     for a, b in zip(batched, plain):
         a64, b64 = a.double(), b.double()
@@ -892,11 +916,7 @@ def run_sections(args, dev, rank, world):
     out = {}
     if "intersect" in names:
         cpu = rank == 0 and not args.no_cpu_baseline
-        out["intersect"], ids, tv = intersect_section(args, dev, "bvh", cpu, want_ref_hits=cpu)
-        q, qids, qt = intersect_section(args, dev, "qbvh", False, False)
-        hit = ids >= 0
-        q["bit_exact_vs_bvh"] = bool(np.array_equal(qids, ids) and np.array_equal(qt[hit], tv[hit]))
-        out["intersect_qbvh"] = q
+        out["intersect"] = intersect_section(args, dev, cpu)
     if "render" in names:
         out["render_1080p_plain"] = render_section(args, dev)
     if "adjoint" in names:
