@@ -10,7 +10,7 @@
 //   LeafBox[]    32 B each, the binary leaf's box of every triangle.
 // and, for the reference's own depth-first walk (rays the wide walk hands back,
 // work counts, full hit records) and, of the render tree, for render rays walked by
-// one thread and for ties (tie_takes):
+// one thread and for the order of hits (order_takes):
 //   Bvh2Node[]   64 B each, DFS pre-order, both children's boxes stored in
 //                the parent; a child reference >= 0 is an internal node index, < 0
 //                a leaf whose first TriRecord is ~ref.

@@ -58,7 +58,7 @@ struct DeviceScene {
     const int32_t* tie_pos;       // renders: leaf position of each triangle id in `tris`
     float wide_limit;             // the reference's tree: origins up to this magnitude take the 8-wide walk
     // The binary tree: the reference's own walk; in the render view the render tree, for
-    // the one-thread walk and for ties (tie_takes).
+    // the one-thread walk and for the order of hits (order_takes).
     int32_t root_ref;
     int32_t stack_cap;
     float root_box[6];            // lo.xyz, hi.xyz

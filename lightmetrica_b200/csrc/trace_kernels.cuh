@@ -124,9 +124,12 @@ k_trace_persistent(const __grid_constant__ DeviceScene s, const __grid_constant_
     __shared__ int64_t back_sh[RENDER ? 1 : 4][RENDER ? 1 : BACK_LIST];   // rays handed back (exact)
     int back = 0;                              // entries in the warp's list
     bool hand_back = false;                    // this lane's ray joins it
-    int64_t n_closest = 0;
-    if constexpr (MODE == TRACE_MIXED) n_closest = io.closest.count();
-    const int64_t n = io.count();
+    // Queues of render rays hold fewer than 2^31 (both of a mixed launch: 2^29); one register
+    // fewer, where it keeps the closest-hit walk free of spills.
+    using Index = std::conditional_t<RENDER && !TABLE, int32_t, int64_t>;
+    Index n_closest = 0;
+    if constexpr (MODE == TRACE_MIXED) n_closest = (Index)io.closest.count();
+    const Index n = (Index)io.count();
     const unsigned lane = threadIdx.x & 31u;
     const int cap = s.stack8_cap < STACK ? s.stack8_cap : STACK;
     const Bvh8Node* nodes = s.bvh8;
@@ -141,21 +144,21 @@ k_trace_persistent(const __grid_constant__ DeviceScene s, const __grid_constant_
     w.leaves = 0;
     w.sp = 0;
     uint32_t pend_node = 0, pend = 0;          // postponed leaves
-    int64_t idx = -1;
+    Index idx = -1;
     bool live = false;
     bool exhausted = n <= 0;
     bool any = MODE == TRACE_ANY;              // this lane's ray stops at its first hit
-    auto load = [&](int64_t j) -> RayIn {
+    auto load = [&](Index j) -> RayIn {
         if constexpr (MODE == TRACE_MIXED) return any ? io.shadow.load(j - n_closest) : io.closest.load(j);
         else return io.load(j);
     };
-    auto store = [&](int64_t j) {
+    auto store = [&](Index j) {
         if constexpr (MODE == TRACE_MIXED) {
             if (any) io.shadow.store(j - n_closest, h, r);
             else io.closest.store(j, h, r);
         } else io.store(j, h, r);
     };
-    auto ray_scene = [&](int64_t j) -> const DeviceScene& {
+    auto ray_scene = [&](Index j) -> const DeviceScene& {
         if constexpr (MODE == TRACE_MIXED) return any ? io.shadow.ray_scene(j - n_closest) : io.closest.ray_scene(j);
         else if constexpr (TABLE) return io.ray_scene(j);
         else return s;
@@ -172,7 +175,7 @@ k_trace_persistent(const __grid_constant__ DeviceScene s, const __grid_constant_
             if (need == FULL && (exhausted ? back > 0 : back > BACK_LIST - 32)) {
                 __syncwarp();
                 for (int i = (int)lane; i < back; i += 32) {
-                    idx = back_sh[threadIdx.x >> 5][i];
+                    idx = (Index)back_sh[threadIdx.x >> 5][i];
                     reference_walk<MODE == TRACE_ANY, STACK>(s, status, load(idx), r, h);
                     store(idx);
                 }
@@ -196,8 +199,8 @@ k_trace_persistent(const __grid_constant__ DeviceScene s, const __grid_constant_
                 if (base + __popc(need) >= (unsigned long long)n) exhausted = true;
             }
             if (take) {
-                idx = (int64_t)base + __popc(need & ((1u << lane) - 1u));
-                if (idx < n) {
+                idx = (Index)base + __popc(need & ((1u << lane) - 1u));
+                if (base < (unsigned long long)n && idx < n) {
                     if constexpr (MODE == TRACE_MIXED) any = idx >= n_closest;
                     const RayIn in = load(idx);
                     setup_ray<true>(r, in);
@@ -268,10 +271,11 @@ k_trace_persistent(const __grid_constant__ DeviceScene s, const __grid_constant_
                 const int32_t id = static_cast<int32_t>(__float_as_uint(q2.z));
                 float u, v, t;
                 if constexpr (RENDER) {
+                    float window;
                     if (triaccel_intersect_fast(q0, q1, q2, r, r.tmax, u, v, t) &&
                         render_candidate<MODE == TRACE_ANY>(TABLE ? ray_scene(idx) : s, (p - reinterpret_cast<const float4*>(tris)) / 3, id,
-                                                            t, u, v, r, h, any)) {
-                        r.tmax = t;
+                                                            t, u, v, r, h.tri, any, window)) {
+                        r.tmax = window;
                         h.tri = id; h.t = t; h.u = u; h.v = v;
                         if (any) { done = true; break; }
                     }

@@ -79,11 +79,11 @@ def test_waves_equal_the_sum_of_one_thread_passes(cuda, technique, box, max_pv, 
     scene.close()
 
 
-@pytest.mark.parametrize("technique,max_pv,n", [("pt.mis", 9, 160 * 160 * 41), ("pt", 4, 1 << 21), ("pt.direct", 6, 777)])
-def test_a_captured_pass_equals_the_direct_one(cuda, technique, max_pv, n):
+@pytest.mark.parametrize("technique,max_pv,n,levels", [("pt.mis", 9, 160 * 160 * 41, 5), ("pt", 4, 1 << 21, 2), ("pt.direct", 6, 777, 2)])
+def test_a_captured_pass_equals_the_direct_one(cuda, technique, max_pv, n, levels):
     """Under capture every budget runs one thread per sample, over the binary render tree."""
     import torch
-    prims = scenes.cornell_refined(2, 160, 160)
+    prims = scenes.cornell_refined(levels, 160, 160)
     scene = create_scene("bvh")
     scene.load(prims)
     scene.configure({})
@@ -109,9 +109,9 @@ def test_a_captured_pass_equals_the_direct_one(cuda, technique, max_pv, n):
     scene.status(torch.cuda.current_stream().cuda_stream)
     for got, want in zip((img, da, de), direct):
         got = got.double().cpu().numpy()
-        # Sums of up to n single-precision terms in two orders; a ray within rounding of an edge or a tie may take another
-        # path in the other tree: a few of the samples, of the order of 1e-5 of them.
-        assert np.linalg.norm(got - want) <= (4 * np.sqrt(n) * 6e-8 + 1e-4) * np.linalg.norm(want)
+        # Sums of single-precision terms in two orders: n of them on a few hundred triangles, about 2^8 on each of 36,864.
+        # (Both walks answer rays within rounding of a shared edge alike: by the wide walk's own order, 1.4e-4 apart.)
+        assert np.linalg.norm(got - want) <= (4 * np.sqrt(n if levels == 2 else 256) * 6e-8 + 2e-5) * np.linalg.norm(want)
         assert np.linalg.norm(want) > 0
     del graph
     scene.close()
