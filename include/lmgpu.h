@@ -126,8 +126,9 @@ typedef struct {
     int32_t layout;             /* LMGPU_LAYOUT_* */
     int32_t build_threads;      /* host threads for the BVH build, 0 = all */
     int32_t max_stack_entries;  /* traversal stack bound per ray, 0 = automatic (enough for every
-                                   walk: the wide tree's depth, and 2 * tree depth + 4 in the
-                                   reference's own walk); a smaller bound makes the walks that
+                                   walk: the wide tree's depth, 2 * tree depth + 4 in the
+                                   reference's own walk, the render tree's depth + 2 in
+                                   one-thread differentiable passes); a smaller bound makes the walks that
                                    need more fail with LMGPU_ERR_STACK_OVERFLOW (the status word
                                    the kernels raise). The multi-scene batch always uses the
                                    largest compiled bound. */

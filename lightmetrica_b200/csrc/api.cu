@@ -488,7 +488,7 @@ int create_impl(const LmgpuSceneDesc* desc, LmgpuScene** out)
         }
         r.root_ref = b.rbvh2_root;
         std::memcpy(r.root_box, b.rroot_box, sizeof(r.root_box));
-        r.stack_cap = 2 * b.rmax_depth + 4;
+        r.stack_cap = b.rmax_depth + 2;    // (a near-first walk defers at most one child a level)
         if (desc->max_stack_entries > 0 && desc->max_stack_entries < r.stack_cap) r.stack_cap = desc->max_stack_entries;
     }
     s->rdev.box_margin = far ? 2.0f : NEAR_EDGE;
