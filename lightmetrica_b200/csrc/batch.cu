@@ -1,10 +1,9 @@
 // Multi-scene batch: many independent scenes rendered as one stream of
 // waves, each wave captured once into a CUDA graph and replayed.
 //
-// The one-scene driver (pathtrace.cu) reads every queue count back to the
-// host to size its next launch, so a small scene spends most of its time in
-// launch gaps and host round trips, and the GPU renders one scene at a time.
-// Here the waves run over the concatenated sample sequence of all scenes
+// The one-scene driver (pathtrace.cu) renders one scene at a time: the bounces
+// of a small scene are launches of a few microseconds, each with its own tail of
+// long rays, and every call ends with the host. Here the waves run over the concatenated sample sequence of all scenes
 // (SceneTable context: per-path scene index, per-ray scene in traversal),
 // launches have fixed grids that read their counts on the device, and one
 // wave (init, K bounces of trace / shade / shadow, splat, wave advance) is a

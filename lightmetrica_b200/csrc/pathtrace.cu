@@ -3,7 +3,7 @@
 //
 // Path state lives in HBM as structure-of-arrays (float4 records, 16-byte
 // coalesced accesses); surviving paths and shadow rays are appended to
-// compacted queues with one warp-aggregated atomic per warp (ballot/popc).
+// compacted queues with one atomic per block and kind (block_append).
 // Queue lengths stay on the device; the driver asks for them only to end deep waves.
 #include <cuda_runtime.h>
 #include <algorithm>

@@ -84,7 +84,7 @@ struct PathState {
     int32_t* depth;    // per path index k of its next bounce (StreamTable)
     int32_t* free_slots;   // free path slots (StreamTable)
     int32_t* retire;   // paths finished this iteration (StreamTable; counters[3])
-    // Bounds-checked build: the queues' capacities (queue_append) and the
+    // Bounds-checked build: the queues' capacities (block_append) and the
     // status word that records an append beyond one.
     uint32_t cap[4];
     int32_t* status;
@@ -639,9 +639,10 @@ __host__ __device__ inline ShadowIO<Ctx> shadow_queue(const PathState& st, int w
 // then for pt.direct / pt.mis next-event estimation at it, Russian roulette
 // and BSDF sampling; pt samples the BSDF first and applies Russian roulette
 // with numPathVertices = k (pathtrace.cpp:223-260).
-// 8 resident blocks per SM (64 registers, a few spilled bytes): on the
-// 1080p terrain frame 6, 7 and 10 blocks took 159.6, 159.7 and 164.0 ms
-// against 156.7 ms; the 64-scene batch was within 0.5 % for all four.
+// 8 resident blocks per SM (64 registers, a few spilled bytes). 6, 7 and 10 blocks (72, 71 and
+// 48 registers) against it: 1080p frame x 8 14.17, 14.17, 14.03 against 13.72 ms; six-scene
+// batch 22.57, 22.61, 22.36 against 22.02 ms; 512 x 512 x 32 gradients 15.00, 14.99, 14.07
+// against 13.68 ms.
 #ifndef LMGPU_PT_SHADE_MIN_BLOCKS
 #define LMGPU_PT_SHADE_MIN_BLOCKS 8
 #endif

@@ -124,8 +124,9 @@ k_trace_persistent(const __grid_constant__ DeviceScene s, const __grid_constant_
     __shared__ int64_t back_sh[RENDER ? 1 : 4][RENDER ? 1 : BACK_LIST];   // rays handed back (exact)
     int back = 0;                              // entries in the warp's list
     bool hand_back = false;                    // this lane's ray joins it
-    // Queues of render rays hold fewer than 2^31 (both of a mixed launch: 2^29); one register
-    // fewer, where it keeps the closest-hit walk free of spills.
+    // 32 bits where they save the closest-hit walk its spills: the queues of one-scene waves, also
+    // the two of a mixed launch, hold fewer than 2^31 rays (a path's state takes 216 bytes and adds
+    // at most two, so that more would need 230 GB).
     using Index = std::conditional_t<RENDER && !TABLE, int32_t, int64_t>;
     Index n_closest = 0;
     if constexpr (MODE == TRACE_MIXED) n_closest = (Index)io.closest.count();
