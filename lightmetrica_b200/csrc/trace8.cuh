@@ -168,12 +168,13 @@ __device__ __forceinline__ bool leaf_box_render(const LeafBox* __restrict__ boxe
     return slab_render(r, a.x, a.w, a.y, b.x, a.z, b.y, te);
 }
 
-// Of two hits whose windows end at the same distance `end`, whether triangle b's is the binary
-// walk's answer rather than a's: the one visited later, if its leaf is entered before that, else the
-// one visited first. Within a leaf the records are tested in order; where the two paths part,
-// the child entered later comes later, the right one if both are entered at once.
+// Of two hits whose windows end at the same distance `end`, whether triangle b's (at tb) is the
+// binary walk's answer rather than a's (at ta): the one visited later, if its leaf is entered
+// before that, else the one visited first; in one leaf the nearer, of equal t the later record.
+// Where the two paths part, the child entered later comes later, the right one if both are
+// entered at once.
 __device__ __forceinline__ bool order_takes(const Bvh2Node* __restrict__ nodes, const int32_t* __restrict__ pos, int32_t root,
-                                            int32_t a, int32_t b, float end, const TraversalRay& r)
+                                            int32_t a, int32_t b, float ta, float tb, float end, const TraversalRay& r)
 {
     const int32_t pa = __ldg(pos + a), pb = __ldg(pos + b);
     int32_t lo = min(pa, pb), hi = max(pa, pb);
@@ -193,14 +194,15 @@ __device__ __forceinline__ bool order_takes(const Bvh2Node* __restrict__ nodes, 
         te = right ? tr : tl;
         ref = right ? meta.y : meta.x;
     }
-    return (!parted || te < end) == b_later;
+    if (!parted) return tb < ta || (tb == ta && b_later);
+    return (te < end) == b_later;
 }
 
-// Whether a candidate (record `at`, triangle id, t <= r.tmax) replaces the hit `best` (-1: none),
+// Whether a candidate (record `at`, triangle id, t <= r.tmax) replaces the hit h (h.tri -1: none),
 // whose window ends at r.tmax; `window`: the end of the candidate's own.
 template <bool ANY>
 __device__ __forceinline__ bool render_candidate(const DeviceScene& s, int64_t at, int32_t id, float t, float u, float v,
-                                                 const TraversalRay& r, int32_t best, bool any, float& window)
+                                                 const TraversalRay& r, const Hit& h, bool any, float& window)
 {
     window = t;
     if (fminf(fminf(u, v), 1.0f - u - v) < s.box_margin) {
@@ -209,8 +211,8 @@ __device__ __forceinline__ bool render_candidate(const DeviceScene& s, int64_t a
         if (ANY || any) return te < r.tmax;
         window = fmaxf(t, te);
     }
-    if (ANY || any || window < r.tmax || best < 0) return true;
-    return window == r.tmax && order_takes(s.bvh2, s.tie_pos, s.root_ref, best, id, window, r);
+    if (ANY || any || window < r.tmax || h.tri < 0) return true;
+    return window == r.tmax && order_takes(s.bvh2, s.tie_pos, s.root_ref, h.tri, id, h.t, t, window, r);
 }
 
 // Exact walk. The reference's answer for a ray is a fold over the triangles whose

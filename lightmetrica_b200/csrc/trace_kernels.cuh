@@ -275,7 +275,7 @@ k_trace_persistent(const __grid_constant__ DeviceScene s, const __grid_constant_
                     float window;
                     if (triaccel_intersect_fast(q0, q1, q2, r, r.tmax, u, v, t) &&
                         render_candidate<MODE == TRACE_ANY>(TABLE ? ray_scene(idx) : s, (p - reinterpret_cast<const float4*>(tris)) / 3, id,
-                                                            t, u, v, r, h.tri, any, window)) {
+                                                            t, u, v, r, h, any, window)) {
                         r.tmax = window;
                         h.tri = id; h.t = t; h.u = u; h.v = v;
                         if (any) { done = true; break; }
